@@ -133,7 +133,7 @@ attn_latent_decode_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         }
     } else if (warp == 8 || warp == 9) {
         // ------------------------------------------------ scores
-        if (lane == 0) {
+        if (tc::elect_one()) {
             constexpr uint32_t idesc = tc::idesc_bf16_f32(kTcRows, kTcTok);
             const uint32_t q_addr = tc::smem_u32(sQ), s_addr = tc::smem_u32(sS);
             bool ok = tc::mbar_wait_abortable(&q_full, 0, a.budget, &s_abort);
@@ -165,7 +165,7 @@ attn_latent_decode_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         }
     } else if (warp == 10) {
         // ------------------------------------------------ outputs
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const uint32_t idesc_all = tc::idesc_bf16_f32_bmn(kTcRows, 64 * nv);
             constexpr uint32_t idesc_one = tc::idesc_bf16_f32_bmn(kTcRows, 64);
             const uint32_t p_addr = tc::smem_u32(sP), s_addr = tc::smem_u32(sS);

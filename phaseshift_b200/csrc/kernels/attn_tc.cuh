@@ -297,7 +297,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         // ------------------------------------------------ score issuers: warp 10 issues S(t) for even t, warp 11 for odd t.
         // A tcgen05.mma costs its issuing thread about 80 cycles whatever its size, and a 128 x 64 x 16 product is only 32
         // cycles of tensor work, so one thread cannot keep the pipe fed; two threads take turns.
-        if (lane == 0) {
+        if (tc::elect_one()) {
             constexpr uint32_t idesc_s = tc::idesc_bf16_f32(kTcRows, kTcTok);
             const int b = warp - 10;
             const uint32_t q_addr = tc::smem_u32(sQ), k_addr0 = tc::smem_u32(sK);
@@ -327,7 +327,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         }
     } else if (warp == 12) {
         // ------------------------------------------------ output issuer: O += P(t) V(t)
-        if (lane == 0) {
+        if (tc::elect_one()) {
             constexpr uint32_t idesc_o = tc::idesc_bf16_f32_bmn(kTcRows, DV);
             const uint32_t v_addr0 = tc::smem_u32(SHARED ? sK : sV), p_addr = tc::smem_u32(sP);
             for (int t = 0; t < T; ++t) {

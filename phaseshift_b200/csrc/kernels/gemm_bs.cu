@@ -508,7 +508,9 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
-        if (lane == 0) {
+        pre = __shfl_sync(0xffffffffu, pre, 0);              // thread 0 filled the ring; the elected lane goes on
+        GI.u = __shfl_sync(0xffffffffu, GI.u, 0);
+        if (tc::elect_one()) {
             int issued = pre;
             // activation half of a (single-panel) stage of the streamed path
             auto issue_acts = [&](int slot, int t, int p) {
@@ -553,7 +555,7 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (tc::elect_one()) {
             int it = 0, pi = 0, seg = 0, t, p0, p1, s = 0;      // it: stages consumed, pi: panels consumed
             uint32_t full_phase = 0;
             BsSegIter S{u0, u1, P};
@@ -640,7 +642,7 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
     } else if (warp == 6) {
         // ------------------------------------------------ scale-factor copies (tcgen05.cp), ahead of the MMAs (streamed path)
-        if (kSplitSf && lane == 0) {
+        if (kSplitSf && tc::elect_one()) {
             int it = 0, t, p0, p1, s = 0;
             uint32_t full_phase = 0;
             BsSegIter S{u0, u1, P};

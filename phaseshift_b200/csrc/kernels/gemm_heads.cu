@@ -67,7 +67,7 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const uint32_t tmem = tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const int early = min(iters, kGhStages);
             const uint32_t bytes = kW + g.box_rows * kGhK * 2;
             for (int it = 0; it < early; ++it) {
@@ -87,7 +87,7 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const uint32_t idesc = tc::idesc_bf16_f32(kGhM, g.nb);
             for (int it = 0; it < iters; ++it) {
                 const int s = it % kGhStages;

@@ -72,7 +72,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     (void)x_tile_bytes;
 
     if (warp == 0) {
-        if (lane == 0 && k_iters > 0) {
+        if (k_iters > 0 && tc::elect_one()) {
             for (int it = 0; it < k_iters; ++it) {
                 const int s = it % STAGES;
                 const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
@@ -84,7 +84,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const uint32_t idesc = tc::idesc_bf16_f32(kSmBM, g.nb);
             bool ok = true;
             for (int it = 0; it < k_iters && ok; ++it) {

@@ -158,7 +158,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (tc::elect_one()) {
             for (int it = 0; it < k_iters; ++it) {
                 const int s = it % kGemmStages;
                 const uint32_t ph = (uint32_t)(it / kGemmStages) & 1u;
@@ -171,7 +171,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (tc::elect_one()) {
             constexpr uint32_t idesc = tc::idesc_bf16_f32(kBM, BN);
             bool ok = true;
             for (int it = 0; it < k_iters && ok; ++it) {
@@ -283,30 +283,30 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer: this CTA's half of both operands
-        const uint32_t full0 = tc::cluster_addr(&full_bar[0], 0);
-        const uint32_t bytes = 2 * kABytes + p.bn * kBK * 2;
-        int s = 0;
-        uint32_t ph = 1;                 // the first round finds every stage free
-        bool ok = true;
-        for (int t = pair; t < p.tiles && ok; t += pairs) {
-            int tm, tn;
-            place(t, tm, tn);
-            const int ra = tm * kPairBM + (int)rank * kBM, rw = tn * p.bn + (int)rank * (p.bn >> 1);
-            for (int k = 0; k < k_iters; ++k) {
-                ok = tc::mbar_wait_warp(&empty_bar[s], ph, g.budget, &s_abort);
-                if (!ok) break;
-                if (tc::elect_one()) {
+        if (tc::elect_one()) {
+            const uint32_t full0 = tc::cluster_addr(&full_bar[0], 0);
+            const uint32_t bytes = 2 * kABytes + p.bn * kBK * 2;
+            int s = 0;
+            uint32_t ph = 1;                 // the first round finds every stage free
+            bool ok = true;
+            for (int t = pair; t < p.tiles && ok; t += pairs) {
+                int tm, tn;
+                place(t, tm, tn);
+                const int ra = tm * kPairBM + (int)rank * kBM, rw = tn * p.bn + (int)rank * (p.bn >> 1);
+                for (int k = 0; k < k_iters; ++k) {
+                    ok = tc::mbar_wait_abortable(&empty_bar[s], ph, g.budget, &s_abort);
+                    if (!ok) break;
                     unsigned char* st = smem + s * kPairStageBytes;
                     if (rank == 0) tc::mbar_expect_tx(&full_bar[s], bytes);
                     tc::tma_load_2d_pair(st, &map_a, k * kBK, ra, full0 + 8 * s);
                     tc::tma_load_2d_pair(st + kABytes, &map_w, k * kBK, rw, full0 + 8 * s);
+                    if (++s == kPairStages) { s = 0; ph ^= 1u; }
                 }
-                if (++s == kPairStages) { s = 0; ph ^= 1u; }
             }
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer of the pair
-        if (rank == 0) {
+        if (rank == 0 && tc::elect_one()) {
             const uint32_t idesc = tc::idesc_bf16_f32(kPairBM, p.bn);
             const uint32_t lo0 = (tc::smem_u32(smem) >> 4) | tc::kDescSw128LoFlags;
             int s = 0, n = 0, done = 0;
@@ -314,27 +314,25 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             bool ok = true;
             for (int t = pair; t < p.tiles && ok; t += pairs, ++n) {
                 const int buf = n & 1;
-                if (n >= 2 && !tc::mbar_wait_warp(&acc_empty[buf], ((uint32_t)(n >> 1) & 1u) ^ 1u, g.budget, &s_abort)) break;
+                if (n >= 2 && !tc::mbar_wait_abortable(&acc_empty[buf], ((uint32_t)(n >> 1) & 1u) ^ 1u, g.budget, &s_abort)) break;
                 tc::fence_after_sync();
                 const uint32_t acc = tmem_acc + (uint32_t)buf * 256u;
                 for (int k = 0; k < k_iters; ++k) {
-                    ok = tc::mbar_wait_warp(&full_bar[s], ph, g.budget, &s_abort);
+                    ok = tc::mbar_wait_abortable(&full_bar[s], ph, g.budget, &s_abort);
                     if (!ok) break;
                     tc::fence_after_sync();
-                    if (tc::elect_one()) {
-                        const uint32_t a = lo0 + s * (kPairStageBytes >> 4), b = a + (kABytes >> 4);
+                    const uint32_t a = lo0 + s * (kPairStageBytes >> 4), b = a + (kABytes >> 4);
 #pragma unroll
-                        for (int kk = 0; kk < kBK / 16; ++kk)       // 16 bf16 = 32 bytes inside the 128-byte swizzle row
-                            tc::mma_bf16_ss_pair(acc, tc::desc_pack(a + 2 * kk, tc::kDescSw128Hi), tc::desc_pack(b + 2 * kk, tc::kDescSw128Hi), idesc,
-                                                 (k > 0 || kk > 0) ? 1u : 0u);
-                        tc::mma_commit_pair(&empty_bar[s]);
-                        if (k == k_iters - 1) tc::mma_commit_pair(&acc_full[buf]);
-                    }
+                    for (int kk = 0; kk < kBK / 16; ++kk)       // 16 bf16 = 32 bytes inside the 128-byte swizzle row
+                        tc::mma_bf16_ss_pair(acc, tc::desc_pack(a + 2 * kk, tc::kDescSw128Hi), tc::desc_pack(b + 2 * kk, tc::kDescSw128Hi), idesc,
+                                             (k > 0 || kk > 0) ? 1u : 0u);
+                    tc::mma_commit_pair(&empty_bar[s]);
+                    if (k == k_iters - 1) tc::mma_commit_pair(&acc_full[buf]);
                     ++done;
                     if (++s == kPairStages) { s = 0; ph ^= 1u; }
                 }
             }
-            if (lane == 0) s_consumed = done;
+            s_consumed = done;
         }
     } else {
         // ------------------------------------------------ epilogue: two warps per TMEM lane quadrant, alternating 32 columns
@@ -344,7 +342,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             const int buf = n & 1;
             int tm, tn;
             place(t, tm, tn);
-            if (!tc::mbar_wait_warp(&acc_full[buf], (uint32_t)(n >> 1) & 1u, g.budget, &s_abort)) break;
+            if (!__all_sync(0xffffffffu, tc::mbar_wait_abortable(&acc_full[buf], (uint32_t)(n >> 1) & 1u, g.budget, &s_abort))) break;
             tc::fence_after_sync();
             const int row = tm * kPairBM + (int)rank * kBM + quad * 32 + lane;
 #pragma unroll 1

@@ -68,7 +68,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const uint32_t tmem_acc = tmem_base_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             for (int it = 0; it < k_iters; ++it) {
                 const int s = it % STAGES;
                 const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
@@ -80,7 +80,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             const uint32_t idesc = tc::idesc_bf16_f32(kMgM, (tile.z + 15) / 16 * 16);
             bool ok = true;
             for (int it = 0; it < k_iters && ok; ++it) {
