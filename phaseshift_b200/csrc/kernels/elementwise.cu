@@ -81,6 +81,56 @@ __global__ void rmsnorm_kernel(const __nv_bfloat16* x, int ldx, const __nv_bfloa
     }
 }
 
+// The same for rows of whole 16-byte vectors without an addend (every norm in front of a GEMM): a thread keeps NV vectors of its row
+// in registers, so the row is read once, in 16-byte loads that are all in flight together.  2048 rows of 2560: 15.0 us by the kernel
+// above (scalar loads, the row through shared memory), 6.1 us by this one (3.4 TB/s); 8 rows: 6.5 and 2.0 us, which is latency.
+template <int NV>
+__global__ void __launch_bounds__(512) rmsnorm_vec_kernel(const __nv_bfloat16* x, int ldx, const __nv_bfloat16* w, float eps, int H, __nv_bfloat16* out,
+                                                          int ldo, int one_plus) {
+    __shared__ float red[32];
+    const int nv = H >> 3;
+    uint4 v[NV], wv[NV];
+    cudaTriggerProgrammaticLaunchCompletion();
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        wv[j] = i < nv ? __ldg(reinterpret_cast<const uint4*>(w) + i) : make_uint4(0, 0, 0, 0);
+    }
+    cudaGridDependencySynchronize();
+    const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)blockIdx.x * ldx);
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        v[j] = i < nv ? xr[i] : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const uint32_t u[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 f = bf16x2_bits_to_f32x2(u[e]);
+            ss += f.x * f.x + f.y * f.y;
+        }
+    }
+    ss = block_sum(ss, red);
+    const float inv = rsqrtf(ss / (float)H + eps), one = one_plus ? 1.f : 0.f;
+    uint4* o = reinterpret_cast<uint4*>(out + (size_t)blockIdx.x * ldo);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i >= nv) break;
+        const uint32_t u[4] = {v[j].x, v[j].y, v[j].z, v[j].w}, q[4] = {wv[j].x, wv[j].y, wv[j].z, wv[j].w};
+        uint32_t r[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 f = bf16x2_bits_to_f32x2(u[e]), g = bf16x2_bits_to_f32x2(q[e]);
+            r[e] = f32x2_to_bf16x2_bits(f.x * inv * (one + g.x), f.y * inv * (one + g.y));
+        }
+        o[i] = make_uint4(r[0], r[1], r[2], r[3]);
+    }
+}
+
 __global__ void add_kernel(const __nv_bfloat16* a, int lda, const __nv_bfloat16* b, int ldb, __nv_bfloat16* out,
                            int ldo, int H) {
     const int r = blockIdx.y;
@@ -133,6 +183,15 @@ PS_API int ps_embedding_mxfp8(const void* ids, const void* codes, const void* sc
 PS_API int ps_rmsnorm(const void* x, int ldx, const void* add, int ld_add, void* sum_out, int ld_sum, const void* w,
                       float eps, int rows, int H, void* out, int ldo, int one_plus, cudaStream_t stream) {
     if (rows <= 0 || H <= 0 || H > 32768) return (int)cudaErrorInvalidValue;
+    if (add == nullptr && H % 8 == 0 && H <= 16384 && ldx % 8 == 0 && ldo % 8 == 0 && ((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) % 16 == 0) {
+        using namespace ps;
+        const int nv = H / 8;
+        auto go = [&](auto kernel, int per) {
+            return launch_pdl(kernel, dim3(rows), dim3(((nv + per - 1) / per + 31) / 32 * 32), 0, stream, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w,
+                              eps, H, (__nv_bfloat16*)out, ldo, one_plus);
+        };
+        return nv <= 512 ? go(rmsnorm_vec_kernel<1>, 1) : nv <= 1024 ? go(rmsnorm_vec_kernel<2>, 2) : go(rmsnorm_vec_kernel<4>, 4);
+    }
     static bool attr_set = false;
     if (!attr_set) {
         cudaFuncSetAttribute(ps::rmsnorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);

@@ -9,6 +9,13 @@
 // them with `tcgen05.ld` (lane = weight row, column = batch row), so the partial stores are coalesced.
 // All mbarrier waits are bounded; a timeout sets PS_DEV_WAIT_TIMEOUT, frees the tensor memory and returns.
 //
+// A decoding step is a chain of about five such products per layer, 3 to 15 us of weights each, so what lies between them counts: all
+// kernels here are launched programmatically, the product asks for its first 128 KB of weights per SM before its rows exist, and the
+// reduction of a residual product norms the rows for the next one (gemm_smallm_norm_kernel).
+// May a product that starts early hold what its predecessors need?  It takes 64 columns of tensor memory and 97 KB; a predecessor
+// that wants more than what is left (512 columns or 200 KB: attention, CTA-pair and block-scaled GEMMs) either never triggers early
+// or fills the SM by its shared memory, so both are never resident together.
+//
 // The reference serves this regime with its RowBlock2/4/8 WMMA kernels (src/phaseshift/models/qwen35/
 // kernels/optimized/linear/psq4.hip:221-349); here it runs from a bf16 expansion that 180 GB of HBM can
 // afford to keep resident next to the block-quantised weights.
@@ -50,6 +57,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int k_iters = min(g.iters_per_split, total_iters - it0);
     const int x_bytes = g.x_box_rows * kSmBK * 2;
 
+    cudaTriggerProgrammaticLaunchCompletion();
     // rows of the X tile beyond the fetched box must read as zero
     for (int i = threadIdx.x; i < STAGES * kXStride / 16; i += kSmThreads) reinterpret_cast<uint4*>(sX)[i] = make_uint4(0, 0, 0, 0);
     tc::fence_proxy_async_smem();
@@ -73,12 +81,20 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
     if (warp == 0) {
         if (k_iters > 0 && tc::elect_one()) {
+            // the first weights are on their way before the kernel that writes the rows is done
+            const int early = min(k_iters, STAGES);
+            for (int it = 0; it < early; ++it) {
+                tc::mbar_expect_tx(&full_bar[it], kWBytes + x_bytes);
+                tc::tma_load_2d(sW + it * kWBytes, &map_w, (it0 + it) * kSmBK, tile_n * kSmBM, &full_bar[it]);
+            }
+            cudaGridDependencySynchronize();
             for (int it = 0; it < k_iters; ++it) {
                 const int s = it % STAGES;
-                const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-                if (it >= STAGES && !tc::mbar_wait(&empty_bar[s], ph ^ 1u, g.budget)) { atomicExch(&s_abort, 1); break; }
-                tc::mbar_expect_tx(&full_bar[s], kWBytes + x_bytes);
-                tc::tma_load_2d(sW + s * kWBytes, &map_w, (it0 + it) * kSmBK, tile_n * kSmBM, &full_bar[s]);
+                if (it >= STAGES) {
+                    if (!tc::mbar_wait(&empty_bar[s], ((uint32_t)(it / STAGES) & 1u) ^ 1u, g.budget)) { atomicExch(&s_abort, 1); break; }
+                    tc::mbar_expect_tx(&full_bar[s], kWBytes + x_bytes);
+                    tc::tma_load_2d(sW + s * kWBytes, &map_w, (it0 + it) * kSmBK, tile_n * kSmBM, &full_bar[s]);
+                }
                 tc::tma_load_2d(sX + s * kXStride, &map_x, (it0 + it) * kSmBK, 0, &full_bar[s]);
                 s_issued = it + 1;
             }
@@ -87,6 +103,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         if (tc::elect_one()) {
             const uint32_t idesc = tc::idesc_bf16_f32(kSmBM, g.nb);
             bool ok = true;
+            cudaGridDependencySynchronize();             // the waits below are for this kernel's copies, not for its predecessor
             for (int it = 0; it < k_iters && ok; ++it) {
                 const int s = it % STAGES;
                 const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
@@ -104,6 +121,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
     } else {
         // epilogue warps 2..5 -> TMEM lane quadrant (warp % 4); lane = weight row, column = batch row
+        cudaGridDependencySynchronize();                 // the previous product's sums have been read
         const int quad = warp & 3;
         const bool done = k_iters > 0 ? tc::mbar_wait(&acc_bar, 0, g.budget) : true;
         tc::fence_after_sync();
@@ -147,10 +165,112 @@ struct SmallMReduceArgs {
     int epilogue;            // 0 store, 1 residual, 2 / 3 / 5 SwiGLU / ReGLU / GeGLU on interleaved (gate, up) columns, 4 tanh-gelu
     const __nv_bfloat16* residual; int ld_res;
     void* out; int ldo; int out_f32;
+    const __nv_bfloat16* norm_w; float eps; __nv_bfloat16* normed; int ld_normed;      // gemm_smallm_norm_kernel
 };
 
-// One thread per output pair (two neighbouring columns); splits are added in ascending order.
+// Sum of the splits of four neighbouring columns (c a multiple of 4) of row m, in ascending order; four loads in flight.
+__device__ __forceinline__ float4 smallm_sum4(const SmallMReduceArgs& a, int m, int c) {
+    const float4* p = reinterpret_cast<const float4*>(a.partial + (size_t)m * a.N + c);
+    const size_t step = (size_t)a.M * a.N / 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    int s = 0;
+    for (; s + 4 <= a.splits; s += 4) {
+        const float4 q[4] = {p[s * step], p[(s + 1) * step], p[(s + 2) * step], p[(s + 3) * step]};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { v.x += q[i].x; v.y += q[i].y; v.z += q[i].z; v.w += q[i].w; }
+    }
+    for (; s < a.splits; ++s) { const float4 q = p[s * step]; v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w; }
+    return v;
+}
+__device__ __forceinline__ float smallm_gated(const SmallMReduceArgs& a, float g, float u) {
+    const float gt = bf16_to_f32(f32_to_bf16(g)), up = bf16_to_f32(f32_to_bf16(u));
+    return (a.epilogue == 3 ? fmaxf(gt, 0.f) : a.epilogue == 5 ? gelu_tanh_f(gt) : silu_f(gt)) * up;
+}
+
+// One thread per four output columns (N a multiple of 4, rows of `out` and the residual 16- / 8-byte aligned).
+__global__ void gemm_smallm_reduce4_kernel(const SmallMReduceArgs a) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    const int quads = a.N >> 2;
+    const int id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= a.M * quads) return;
+    const int m = id / quads, c = (id - m * quads) * 4;
+    float4 v = smallm_sum4(a, m, c);
+    if (a.epilogue == 2 || a.epilogue == 3 || a.epilogue == 5) {
+        *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(a.out) + (size_t)m * a.ldo + (c >> 1)) =
+            f32x2_to_bf16x2_bits(smallm_gated(a, v.x, v.y), smallm_gated(a, v.z, v.w));
+        return;
+    }
+    if (a.epilogue == 1) {
+        const uint2 rb = *reinterpret_cast<const uint2*>(a.residual + (size_t)m * a.ld_res + c);
+        const float2 r0 = bf16x2_bits_to_f32x2(rb.x), r1 = bf16x2_bits_to_f32x2(rb.y);
+        v.x = bf16_to_f32(f32_to_bf16(v.x)) + r0.x; v.y = bf16_to_f32(f32_to_bf16(v.y)) + r0.y;
+        v.z = bf16_to_f32(f32_to_bf16(v.z)) + r1.x; v.w = bf16_to_f32(f32_to_bf16(v.w)) + r1.y;
+    }
+    if (a.epilogue == 4) { v.x = gelu_tanh_f(v.x); v.y = gelu_tanh_f(v.y); v.z = gelu_tanh_f(v.z); v.w = gelu_tanh_f(v.w); }
+    if (a.out_f32) *reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + (size_t)m * a.ldo + c) = v;
+    else *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(a.out) + (size_t)m * a.ldo + c) =
+        make_uint2(f32x2_to_bf16x2_bits(v.x, v.y), f32x2_to_bf16x2_bits(v.z, v.w));
+}
+
+// Residual epilogue and the next projection's RMSNorm (scale 1 + w) in one launch: the four CTAs of a cluster share a row, exchange
+// their sums of squares through distributed shared memory and write the new residual and its normed row.  Replaces a reduction
+// and a norm launch (2.9 + 6.5 us for 8 rows of 2560); with the early weights above, a step of 8 rows through 8 layers of 2560 x 9216
+// went from 1190 to 931 us, one of 32 rows through 4 layers of 5120 x 17408 from 2010 to 1780.  What bounds it: latency.
+constexpr int kSmNormCtas = 4, kSmNormThreads = 256, kSmNormItems = 4;       // rows of up to 4 * 4 * 4 * 256 columns
+__global__ void __cluster_dims__(kSmNormCtas, 1, 1) __launch_bounds__(kSmNormThreads) gemm_smallm_norm_kernel(const SmallMReduceArgs a) {
+    __shared__ float red[32], s_part;
+    const int m = blockIdx.x / kSmNormCtas, per = (a.N / 4 + kSmNormCtas - 1) / kSmNormCtas;
+    const uint32_t rank = tc::cluster_ctarank();
+    const int first = (int)rank * per, last = min(first + per, a.N / 4);         // this CTA's groups of four columns
+    cudaTriggerProgrammaticLaunchCompletion();
+    uint2 w[kSmNormItems];
+#pragma unroll
+    for (int j = 0; j < kSmNormItems; ++j) {
+        const int i = first + threadIdx.x + j * kSmNormThreads;
+        w[j] = i < last ? __ldg(reinterpret_cast<const uint2*>(a.norm_w) + i) : make_uint2(0, 0);
+    }
+    cudaGridDependencySynchronize();
+    float4 x[kSmNormItems];
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < kSmNormItems; ++j) {
+        const int i = first + threadIdx.x + j * kSmNormThreads, c = 4 * i;
+        x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i >= last) continue;
+        const float4 v = smallm_sum4(a, m, c);
+        const uint2 rb = *reinterpret_cast<const uint2*>(a.residual + (size_t)m * a.ld_res + c);
+        const float2 r0 = bf16x2_bits_to_f32x2(rb.x), r1 = bf16x2_bits_to_f32x2(rb.y);
+        const uint2 o = make_uint2(f32x2_to_bf16x2_bits(bf16_to_f32(f32_to_bf16(v.x)) + r0.x, bf16_to_f32(f32_to_bf16(v.y)) + r0.y),
+                                   f32x2_to_bf16x2_bits(bf16_to_f32(f32_to_bf16(v.z)) + r1.x, bf16_to_f32(f32_to_bf16(v.w)) + r1.y));
+        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(a.out) + (size_t)m * a.ldo + c) = o;
+        const float2 x0 = bf16x2_bits_to_f32x2(o.x), x1 = bf16x2_bits_to_f32x2(o.y);
+        x[j] = make_float4(x0.x, x0.y, x1.x, x1.y);
+        ss += x0.x * x0.x + x0.y * x0.y + x1.x * x1.x + x1.y * x1.y;
+    }
+    ss = block_sum(ss, red);
+    if (threadIdx.x == 0) s_part = ss;
+    tc::cluster_sync();
+    ss = 0.f;
+#pragma unroll
+    for (int r = 0; r < kSmNormCtas; ++r) ss += tc::cluster_load_f32(&s_part, r);
+    const float inv = rsqrtf(ss / (float)a.N + a.eps);
+#pragma unroll
+    for (int j = 0; j < kSmNormItems; ++j) {
+        const int i = first + threadIdx.x + j * kSmNormThreads;
+        if (i >= last) continue;
+        const float2 w0 = bf16x2_bits_to_f32x2(w[j].x), w1 = bf16x2_bits_to_f32x2(w[j].y);
+        *reinterpret_cast<uint2*>(a.normed + (size_t)m * a.ld_normed + 4 * i) =
+            make_uint2(f32x2_to_bf16x2_bits(x[j].x * inv * (1.f + w0.x), x[j].y * inv * (1.f + w0.y)),
+                       f32x2_to_bf16x2_bits(x[j].z * inv * (1.f + w1.x), x[j].w * inv * (1.f + w1.y)));
+    }
+    tc::cluster_sync();              // nobody leaves while its sum may still be read
+}
+
+// Any even N and any alignment: one thread per output pair (two neighbouring columns); splits are added in ascending order.
 __global__ void gemm_smallm_reduce_kernel(const SmallMReduceArgs a) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     const int pairs = a.N >> 1;
     const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= (long long)a.M * pairs) return;
@@ -161,8 +281,7 @@ __global__ void gemm_smallm_reduce_kernel(const SmallMReduceArgs a) {
         v0 += p.x; v1 += p.y;
     }
     if (a.epilogue == 2 || a.epilogue == 3 || a.epilogue == 5) {
-        const float gt = bf16_to_f32(f32_to_bf16(v0)), up = bf16_to_f32(f32_to_bf16(v1));
-        reinterpret_cast<__nv_bfloat16*>(a.out)[(size_t)m * a.ldo + (c >> 1)] = f32_to_bf16((a.epilogue == 3 ? fmaxf(gt, 0.f) : a.epilogue == 5 ? gelu_tanh_f(gt) : silu_f(gt)) * up);
+        reinterpret_cast<__nv_bfloat16*>(a.out)[(size_t)m * a.ldo + (c >> 1)] = f32_to_bf16(smallm_gated(a, v0, v1));
         return;
     }
     if (a.epilogue == 1) {
@@ -218,14 +337,24 @@ PS_API int ps_gemm_smallm_splits(int N, int K) {
 }
 
 // out[M,N] = epilogue(A[M,K] . W[N,K]^T) for 1 <= M <= 64; A, W bf16 row-major (lda, ldw multiples of 8,
-// 16-byte aligned bases), N even, `partial` = ps_gemm_smallm_splits(N, K) * M * N floats of scratch.
-PS_API int ps_gemm_smallm(const void* a, int lda, const void* w, int ldw, int M, int N, int K, int epilogue, const void* residual,
-                          int ld_res, void* out, int ldo, int out_f32, void* partial, void* status, cudaStream_t stream) {
+// 16-byte aligned bases), N even, `partial` = ps_gemm_smallm_splits(N, K) * M * N floats of scratch (16-byte aligned).
+// With `norm_w` (residual epilogue, bf16 output): `normed` [M, N] bf16 receives out / rms(out) * (1 + norm_w) as well; N a multiple of
+// 4, at most ps_gemm_smallm_norm_cols(), and 8-byte aligned rows of out, residual, norm_w and normed.
+PS_API int ps_gemm_smallm_norm_cols() { return 16 * ps::kSmNormItems * ps::kSmNormThreads; }
+
+PS_API int ps_gemm_smallm_normed(const void* a, int lda, const void* w, int ldw, int M, int N, int K, int epilogue, const void* residual,
+                                 int ld_res, void* out, int ldo, int out_f32, const void* norm_w, float eps, void* normed, int ld_normed,
+                                 void* partial, void* status, cudaStream_t stream) {
     using namespace ps;
     if (M < 1 || M > 64 || N <= 0 || (N & 1) || K <= 0 || (K % 8) || (lda % 8) || (ldw % 8) || ((uintptr_t)a % 16) ||
         ((uintptr_t)w % 16) || partial == nullptr)
         return (int)cudaErrorInvalidValue;
-    if ((epilogue == 2 || epilogue == 3 || epilogue == 5) && out_f32) return (int)cudaErrorInvalidValue;
+    const bool gated = epilogue == 2 || epilogue == 3 || epilogue == 5;
+    if (gated && out_f32) return (int)cudaErrorInvalidValue;
+    auto rows8 = [](const void* p, int ld) { return (uintptr_t)p % 8 == 0 && ld % 4 == 0; };       // bf16 rows in 8-byte pieces
+    if (norm_w != nullptr && (epilogue != 1 || out_f32 || N % 4 || N > ps_gemm_smallm_norm_cols() || (uintptr_t)norm_w % 8 || !rows8(out, ldo) ||
+                              !rows8(residual, ld_res) || !rows8(normed, ld_normed)))
+        return (int)cudaErrorInvalidValue;
     SmallMArgs g;
     g.M = M; g.N = N; g.K = K;
     g.nb = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
@@ -248,13 +377,21 @@ PS_API int ps_gemm_smallm(const void* a, int lda, const void* w, int ldw, int M,
         attr_set = true;
     }
     dim3 grid((N + kSmBM - 1) / kSmBM, g.splits);
-    gemm_smallm_kernel<STAGES><<<grid, kSmThreads, smem, stream>>>(map_w, map_x, g);
-    err = PS_LAUNCH_CHECK();
+    err = launch_pdl(gemm_smallm_kernel<STAGES>, grid, dim3(kSmThreads), smem, stream, map_w, map_x, g);
     if (err) return err;
     SmallMReduceArgs r;
     r.partial = g.partial; r.splits = g.splits; r.M = M; r.N = N; r.epilogue = epilogue;
     r.residual = (const __nv_bfloat16*)residual; r.ld_res = ld_res; r.out = out; r.ldo = ldo; r.out_f32 = out_f32;
+    r.norm_w = (const __nv_bfloat16*)norm_w; r.eps = eps; r.normed = (__nv_bfloat16*)normed; r.ld_normed = ld_normed;
+    if (norm_w != nullptr) return launch_pdl(gemm_smallm_norm_kernel, dim3(M * kSmNormCtas), dim3(kSmNormThreads), 0, stream, r);
+    if (N % 4 == 0 && (uintptr_t)partial % 16 == 0 && (epilogue != 1 || rows8(residual, ld_res)) &&
+        (gated ? (uintptr_t)out % 4 == 0 && ldo % 2 == 0 : out_f32 ? (uintptr_t)out % 16 == 0 && ldo % 4 == 0 : rows8(out, ldo)))
+        return launch_pdl(gemm_smallm_reduce4_kernel, dim3((unsigned)((M * (N >> 2) + 255) / 256)), dim3(256), 0, stream, r);
     const long long n = (long long)M * (N >> 1);
-    gemm_smallm_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(r);
-    return PS_LAUNCH_CHECK();
+    return launch_pdl(gemm_smallm_reduce_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, r);
+}
+
+PS_API int ps_gemm_smallm(const void* a, int lda, const void* w, int ldw, int M, int N, int K, int epilogue, const void* residual,
+                          int ld_res, void* out, int ldo, int out_f32, void* partial, void* status, cudaStream_t stream) {
+    return ps_gemm_smallm_normed(a, lda, w, ldw, M, N, K, epilogue, residual, ld_res, out, ldo, out_f32, nullptr, 0.f, nullptr, 0, partial, status, stream);
 }

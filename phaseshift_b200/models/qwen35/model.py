@@ -12,6 +12,7 @@ from typing import Dict, List, Optional, Sequence
 
 import torch
 
+from ...ops.specs import NextNorm
 from ...runtime.batch import StepBatch
 from ...runtime.state import ModelState
 from ..common import StepOutput
@@ -53,7 +54,7 @@ class Qwen35Runner:
         L = self.w.layers[li]
         return L.mixer.in_proj if L.kind == 0 else L.mixer.qkv_proj
 
-    def _row_parallel(self, inp: torch.Tensor, W, residual: torch.Tensor, name: str, rows: int, nxt=None):
+    def _row_parallel(self, inp: torch.Tensor, W, residual: torch.Tensor, name: str, rows: int, nxt=None, norm_next=None):
         """Row-parallel projection + residual.  Single rank: residual fused in the projection epilogue.
         Tensor parallel, few rows: the projection kernel also performs the cross-rank sum (fused one-shot
         all-reduce over NVLink); otherwise the partial goes through the all-reduce kernel / library.
@@ -67,7 +68,7 @@ class Qwen35Runner:
             ssq = (ssq_out, -(-W.N // 128))
         kw = {"prefetch": nxt} if self.use_ssq else {}
         if tp is None or tp.size <= 1:
-            return ops.linear(inp, W, name=name, residual=residual, ssq_out=ssq_out, **kw), ssq
+            return ops.linear(inp, W, name=name, residual=residual, ssq_out=ssq_out, norm_next=norm_next, **kw), ssq
         comb = tp.combine_for(W.N) if (rows <= tp.max_fused_rows(W) and hasattr(ops, "buf")) else None
         if comb is not None:
             tp.stats["fused"] += 1
@@ -102,6 +103,7 @@ class Qwen35Runner:
                 x_ssq = (e_ssq, 1)
             else:
                 x = ops.embed(b, rows, w.embed, st.status)
+        x_normed = None                          # rows of x that the previous projection has normed for the next one
         taps = {}
         taps_cat = None
         if tap_layers and hasattr(ops, "buf"):
@@ -120,7 +122,10 @@ class Qwen35Runner:
                 if hasattr(ops, "buf"):
                     proj = ops.buf("gdn_proj", rows, n_main + m.ba_proj.N)
                     batched = rows >= 2 and m.in_proj.rowmajor_bf16 is not None and not ops.exact_rows
-                    if rows <= FUSED_BA_MAX_ROWS and not batched:
+                    if batched and m.in_ba is not None:
+                        xn = None
+                        ops.linear(x, m.in_ba, name="gdn_in", norm_w=L.input_norm, eps=eps, out=proj, x_normed=x_normed)
+                    elif rows <= FUSED_BA_MAX_ROWS and not batched:
                         # decode / verify: the GDN kernel projects beta/decay inputs itself from the
                         # normalised row that in_proj leaves behind -> one launch fewer per layer
                         xn = ops.buf("gdn_xn", rows, x.shape[1])
@@ -144,11 +149,12 @@ class Qwen35Runner:
                                     log=None if gdn_log is None else gdn_log[li], to_alt=gdn_to_alt)
                 self._tap(lp + "linear_attn.out_proj.weight", o, b.n_rows)
                 with ops.range("gdn.out_proj"):
-                    r, r_ssq = self._row_parallel(o, m.out_proj, x, "r", rows, L.gate_up)
+                    mid = NextNorm(L.post_norm, eps, "xn_mid")
+                    r, r_ssq = self._row_parallel(o, m.out_proj, x, "r", rows, L.gate_up, mid)
             else:
                 self._tap(lp + "self_attn.q_proj.weight", x, b.n_rows, L.input_norm)
                 with ops.range("attn.qkv_proj"):
-                    qkv = ops.linear(x, m.qkv_proj, name="attn_qkv", norm_w=L.input_norm, eps=eps,
+                    qkv = ops.linear(x, m.qkv_proj, name="attn_qkv", norm_w=L.input_norm, eps=eps, x_normed=x_normed,
                                      **({"ssq_in": x_ssq, "prefetch": m.o_proj} if self.use_ssq else {}))
                 with ops.range("attn.prep"):
                     q = ops.attn_prep(qkv, m, self.hq, self.hkv, b, st.kv[li], st)
@@ -156,16 +162,19 @@ class Qwen35Runner:
                     ctx = ops.paged_attention(q, qkv, self.hq, self.hkv, b, st.kv[li], st, b.max_visible_launch)
                 self._tap(lp + "self_attn.o_proj.weight", ctx, b.n_rows)
                 with ops.range("attn.o_proj"):
-                    r, r_ssq = self._row_parallel(ctx, m.o_proj, x, "r", rows, L.gate_up)
+                    mid = NextNorm(L.post_norm, eps, "xn_mid")
+                    r, r_ssq = self._row_parallel(ctx, m.o_proj, x, "r", rows, L.gate_up, mid)
             self._tap(lp + "mlp.gate_proj.weight", r, b.n_rows, L.post_norm)
             with ops.range("mlp.gate_up"):
-                act = ops.linear(r, L.gate_up, name="mlp_act", norm_w=L.post_norm, eps=eps, swiglu=True,
+                act = ops.linear(r, L.gate_up, name="mlp_act", norm_w=L.post_norm, eps=eps, swiglu=True, x_normed=mid.rows,
                                  **({"ssq_in": r_ssq, "prefetch": L.down} if self.use_ssq else {}))
             self._tap(lp + "mlp.down_proj.weight", act, b.n_rows)
             # ping-pong the residual stream so a layer never writes the buffer it still reads
             xname = "x_a" if (li & 1) == 0 else "x_b"
             with ops.range("mlp.down"):
-                x, x_ssq = self._row_parallel(act, L.down, r, xname, rows, self._first_proj(li + 1))
+                nn = NextNorm(w.layers[li + 1].input_norm if li + 1 < len(w.layers) else w.final_norm, eps, "xn_next")
+                x, x_ssq = self._row_parallel(act, L.down, r, xname, rows, self._first_proj(li + 1), nn)
+                x_normed = nn.rows
             if li in tap_layers:
                 if taps_cat is None:
                     taps[li] = x
@@ -175,9 +184,9 @@ class Qwen35Runner:
         tokens = logits = hidden = None
         if n_out > 0:
             if b.identity_out and self.use_ssq:
-                hidden, h_ssq = x[:n_out], x_ssq          # pure decode batch: no gather, and the row statistics carry over
+                hidden, h_ssq, h_normed = x[:n_out], x_ssq, None if x_normed is None else x_normed[:n_out]          # pure decode batch: no gather, and the row statistics carry over
             else:
-                hidden, h_ssq = ops.gather_rows(x, b.out_rows, n_out, "out_hidden", st.status), None
+                hidden, h_ssq, h_normed = ops.gather_rows(x, b.out_rows, n_out, "out_hidden", st.status), None, None
             self._tap(_P + "lm_head.weight", hidden, n_out, w.final_norm)
             if (greedy_only and sample and mask is None and self.tp is None and hasattr(ops, "can_fuse_argmax")
                     and ops.can_fuse_argmax(w.lm_head, n_out)):
@@ -185,7 +194,7 @@ class Qwen35Runner:
                     tokens = ops.linear_argmax(hidden, w.lm_head, norm_w=w.final_norm, eps=eps)
                 return StepOutput(tokens, None, hidden, taps, taps_cat)
             with ops.range("head.lm_head"):
-                logits = ops.linear(hidden, w.lm_head, name="logits", norm_w=w.final_norm, eps=eps, out_f32=True,
+                logits = ops.linear(hidden, w.lm_head, name="logits", norm_w=w.final_norm, eps=eps, out_f32=True, x_normed=h_normed,
                                     **({"ssq_in": h_ssq} if self.use_ssq else {}))
             if sample:
                 with ops.range("head.sample"):

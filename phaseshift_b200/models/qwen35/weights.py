@@ -202,6 +202,8 @@ class GdnW:
     dt_bias: torch.Tensor     # [Hv_local] f32
     norm_w: torch.Tensor      # [Dv] bf16
     out_proj: LinearW
+    # in_proj and ba_proj as one row-major matrix whose slices they are (bf16 weights on a CUDA device): several rows take one product
+    in_ba: Optional[LinearW] = None
 
 
 @dataclass
@@ -455,6 +457,15 @@ def build_engine_weights(cfg: Qwen35Config, get, preset: str = "bf16", device="c
                 lw.make_tiled(keep_canonical or role == "gdn_small" or (lw.fmt == "bf16" and layout != "stream"))
         return lw
 
+    def joined(a: LinearW, b: LinearW) -> Optional[LinearW]:
+        """One row-major matrix for two bf16 projections of the same input; theirs become slices of it."""
+        if not on_cuda or a.rowmajor_bf16 is None or b.rowmajor_bf16 is None:
+            return None
+        n, kp = a.N + b.N, a.k_padded
+        both = torch.cat([a.q.codes, b.q.codes], 0)
+        a.q.codes, b.q.codes = both[:a.N], both[a.N:]
+        return LinearW(QuantizedTensor("bf16", (n, a.K), kp, both))
+
     def dev(t: torch.Tensor, dtype=torch.bfloat16) -> torch.Tensor:
         return t.to(device=device, dtype=dtype).contiguous()
 
@@ -476,7 +487,7 @@ def build_engine_weights(cfg: Qwen35Config, get, preset: str = "bf16", device="c
             out_proj = lin([(a + "out_proj.weight", None, hr(vh, Dv))], "gdn_out", l)
             mixer = GdnW(in_proj, ba, dev(cw), dev(_rows(src.tensor(a + "A_log"), vh, 1), torch.float32),
                          dev(_rows(src.tensor(a + "dt_bias"), vh, 1), torch.float32), dev(src.tensor(a + "norm.weight")),
-                         out_proj)
+                         out_proj, joined(in_proj, ba))
         else:
             a = lp + "self_attn."
             qkv = lin([(a + "q_proj.weight", hr(geo.q_heads, 2 * D), None), (a + "k_proj.weight", hr(geo.kv_heads, D), None),

@@ -21,7 +21,7 @@ from ..models.qwen35.weights import AttnW, GdnW, LinearW
 from ..runtime.batch import ROW_BUCKETS, StepBatch
 from ..runtime.state import GdnLayerState, KVLayer, ModelState
 from . import _lib
-from .specs import AttnSpec, DeltaSpec, GatedNorm, GlaSpec, HeadsSpec, LatentSpec, MoeSpec, Pending, Routed, StreamWrite
+from .specs import AttnSpec, DeltaSpec, GatedNorm, GlaSpec, HeadsSpec, LatentSpec, MoeSpec, NextNorm, Pending, Routed, StreamWrite
 from ._lib import c_float, c_int, c_ll, ptr
 
 WFMT = {"bf16": 0, "nvfp4": 1, "mxfp8": 2}
@@ -144,8 +144,12 @@ class CudaOps(OpTrace):
                eps: float = 0.0, residual: Optional[torch.Tensor] = None, swiglu: bool = False, reglu: bool = False, gelu: bool = False,
                geglu: bool = False, out_f32: bool = False, out: Optional[torch.Tensor] = None,
                xn_out: Optional[torch.Tensor] = None, tp_combine=None, ssq_in=None,
-               ssq_out: Optional[torch.Tensor] = None, prefetch: Optional[LinearW] = None, tp_scatter=None) -> torch.Tensor:
-        """``tp_combine`` (a parallel.tp.TpCombineStruct): the projection is row-parallel and the kernel sums
+               ssq_out: Optional[torch.Tensor] = None, prefetch: Optional[LinearW] = None, tp_scatter=None,
+               norm_next: Optional[NextNorm] = None, x_normed: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """``norm_next``: the norm that the output rows pass on their way into the next projection; where this projection's kernels
+        can, they leave the normed rows in ``norm_next.rows``.  ``x_normed``: rows of `x` that such a kernel normed with `norm_w`
+        (None: the norm is still to be done).
+        ``tp_combine`` (a parallel.tp.TpCombineStruct): the projection is row-parallel and the kernel sums
         the ranks' partial results over NVLink before the residual epilogue.
         ``ssq_in`` = (tensor [rows, SSQ_LD] fp32, n): n partial sums of squares per row of ``x`` left by the kernel
         that produced it, consumed by the fused RMSNorm; ``ssq_out``: receives the partial sums of the rows this
@@ -187,7 +191,8 @@ class CudaOps(OpTrace):
                    and not self.exact_rows)
         self.sel_counts["gemm" if (sel == "gemm" or batched) else "stream"] += 1
         if sel == "gemm" or batched:
-            return self.linear_large(x, W, norm_w=norm_w, eps=eps, residual=residual, epi=epi, out_f32=out_f32, out=out)
+            return self.linear_large(x, W, norm_w=norm_w, eps=eps, residual=residual, epi=epi, out_f32=out_f32, out=out, norm_next=norm_next,
+                                     x_normed=x_normed)
         pro = PRO_RMSNORM if norm_w is not None else PRO_NONE
         if W.tiled is None:
             W.make_tiled()
@@ -256,17 +261,18 @@ class CudaOps(OpTrace):
         self.sel_counts["f32"] = self.sel_counts.get("f32", 0) + 1
         return out
 
-    def linear_large(self, x: torch.Tensor, W: LinearW, *, norm_w, eps, residual, epi: int, out_f32, out):
+    def linear_large(self, x: torch.Tensor, W: LinearW, *, norm_w, eps, residual, epi: int, out_f32, out, norm_next: Optional[NextNorm] = None,
+                     x_normed: Optional[torch.Tensor] = None):
         """Prefill-sized projection: (RMSNorm kernel) -> weight expansion to a bf16 scratch matrix -> tcgen05
         GEMM with the residual / SwiGLU / dtype epilogue fused."""
         M, K = x.shape
-        a = x if norm_w is None else self.rmsnorm(x, norm_w, eps, "gemm_norm_in")
-        if W.tiled is None:
-            W.make_tiled()
+        a = x if norm_w is None else x_normed if x_normed is not None else self.rmsnorm(x, norm_w, eps, "gemm_norm_in")
         kp = W.k_padded
         if W.rowmajor_bf16 is not None:
             wd = W.rowmajor_bf16
         else:
+            if W.tiled is None:
+                W.make_tiled()
             need = W.N * kp
             if self.wscratch is None or self.wscratch.numel() < need:
                 self.wscratch = torch.empty(need, dtype=torch.bfloat16, device=self.device)
@@ -284,9 +290,15 @@ class CudaOps(OpTrace):
             if part is None or part.numel() < need:
                 part = torch.empty(max(need, 1 << 22), dtype=torch.float32, device=self.device)
                 self.ws[("smallm_partial", 0)] = part
-            _lib.call("ps_gemm_smallm", ptr(a), c_int(a.stride(0)), ptr(wd), c_int(kp), c_int(M), c_int(W.N), c_int(kp), c_int(epi),
+            normed = None
+            if (norm_next is not None and epi == EPI_RESIDUAL and not out_f32 and W.N % 4 == 0 and W.N <= L.ps_gemm_smallm_norm_cols()
+                    and all(t.stride(0) % 4 == 0 and t.data_ptr() % 8 == 0 for t in (out, residual))):
+                normed = norm_next.rows = self.buf(norm_next.name, M, W.N)
+            _lib.call("ps_gemm_smallm_normed", ptr(a), c_int(a.stride(0)), ptr(wd), c_int(kp), c_int(M), c_int(W.N), c_int(kp), c_int(epi),
                       ptr(residual), c_int(residual.stride(0) if residual is not None else 0), ptr(out), c_int(out.stride(0)),
-                      c_int(1 if out_f32 else 0), ptr(part), ptr(self.status))
+                      c_int(1 if out_f32 else 0), ptr(norm_next.weight if normed is not None else None),
+                      c_float(norm_next.eps if normed is not None else 0.0), ptr(normed), c_int(normed.stride(0) if normed is not None else 0),
+                      ptr(part), ptr(self.status))
             self.launches += 2
             return out
         _lib.call("ps_gemm_bf16_tc", ptr(a), c_int(a.stride(0)), ptr(wd), c_int(kp), c_int(M), c_int(W.N), c_int(kp),

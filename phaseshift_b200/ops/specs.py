@@ -312,6 +312,16 @@ class GatedNorm:
 
 
 @dataclass
+class NextNorm:
+    """The RMSNorm (scale 1 + weight) between a residual projection and the one that follows it.  ``rows``: the normed rows, where the
+    residual projection left them (buffer `name` of the op set); None: the next projection norms its own input."""
+    weight: torch.Tensor
+    eps: float
+    name: str
+    rows: Optional[torch.Tensor] = None
+
+
+@dataclass
 class Pending:
     """What the next residual update still has to add: the normed sum of two branches (each [rows, width] with its norm
     weight), a plain projection output or a mixture's sum, times `coef`; and a `bias` vector (f32 [width])."""
