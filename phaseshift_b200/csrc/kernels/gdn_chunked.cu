@@ -17,19 +17,21 @@
 //      tensor-core products with T, and the decayed operands Qd = D q, Kd = (D_C/D_s) k, written to scratch.
 //   2. gdn_history : stores the raw inputs of each sequence's last rows in the conv ring (a separate
 //      launch so no CTA reads history that another CTA of the same step is overwriting).
-//   3. gdn_chunk_scan_tc : one CTA per (sequence, value head, 64-column slice of Dv) walks the chunks:
+//   3. gdn_chunk_scan_umma : one CTA per (sequence, value head, 64-column slice of Dv) walks the chunks:
 //      Delta = U - W S0 ;  O = Qd S0 + QKd Delta ;  S = D_C S0 + Kd^T Delta.  Three small tensor-core
-//      products per chunk, no serial solve on the critical path; the state stays in accumulator registers.
-//      (gdn_chunk_scan is the same walk with fp32 CUDA-core products, selected by PS_GDN_SCAN=fp32.)
+//      products per chunk on tcgen05, no serial solve on the critical path; the state stays in tensor memory.
+//      (gdn_chunk_scan_tc is the same walk on mma.sync for head sizes of 64, gdn_chunk_scan with fp32 CUDA-core
+//      products, selected by PS_GDN_SCAN=fp32.)
 //   4. gdn_post : RMSNorm over the head's Dv outputs (direct weight) * SiLU(z) -> bf16.
 //
 // All decay ratios have s <= t and g <= 0, so every exponential is <= 1.  The state and every accumulation
-// are fp32; the tensor-core products take TF32 operands (mma.sync m16n8k8, round-to-nearest copies).
+// are fp32; the tensor-core products take TF32 operands (round-to-nearest copies; mma.sync in the preparation, tcgen05 in the scan).
 // The reference's chunked kernel (src/phaseshift/models/qwen35/kernels/optimized/gdn/recurrence.hip:
 // 128-519) uses chunk 32, bf16 WMMA products (hi+lo split in "exact" mode) and a 32-step serial forward
 // substitution per column inside the sequential walk.  Decode and speculative verification keep using
 // the row-sequential kernel (gdn_recurrent.cu), whose per-row arithmetic is independent of the batch.
 #include "ps_common.cuh"
+#include "ps_tcgen05.cuh"
 
 namespace ps {
 
@@ -49,8 +51,23 @@ struct GdnPrepArgs {
     int min_rows;                                // sequences with at most this many rows are left to the row kernel
     float* scratch;                              // per (chunk, head): W, Qd, Kd [64,Dk]; U [64,Dv]; QKd [64,64]
     float* dc;                                   // per (chunk, head): D_C
-    int round_tf32;                              // 1: W, Qd, Kd, QKd are stored rounded to TF32 (the tensor-core scan copies them
+    int round_tf32;                              // 1: W, Qd, Kd, QKd are stored rounded to TF32 (the tensor-core scans copy them
                                                  // into shared memory asynchronously and cannot round on the way)
+    int images;                                  // 1: ... and as the tcgen05 scan's operand tiles (GdnImage)
+};
+
+// Scratch of one (chunk, head) for the tcgen05 scan: operand tiles as that kernel's shared memory holds them (rows of 128 bytes = 32
+// floats along K, 16-byte pieces swizzled by the row, panel by panel), so that one bulk copy fetches each.  Same size as the row-major form.
+template <int DK, int DV> struct GdnImage {
+    static constexpr int kWQ = 0, kKd = 2 * kChunk * DK, kU = kKd + kChunk * DK, kQK = kU + kChunk * DV;      // offsets in floats
+    __device__ static __forceinline__ int at(int rows, int r, int k) {           // element (r, k) of a tile of `rows` rows
+        return ((k >> 5) * rows + r) * 32 + ((((k & 31) >> 2) ^ (r & 7)) << 2) + (k & 3);
+    }
+    __device__ static __forceinline__ int w(int r, int k) { return kWQ + at(2 * kChunk, r, k); }               // W over Qd, K = DK
+    __device__ static __forceinline__ int qd(int r, int k) { return kWQ + at(2 * kChunk, kChunk + r, k); }
+    __device__ static __forceinline__ int kdt(int d, int r) { return kKd + at(DK, d, r); }                     // Kd^T, K = rows of the chunk
+    __device__ static __forceinline__ int ut(int r, int n) { return kU + n * kChunk + r; }                     // U^T
+    __device__ static __forceinline__ int qk(int r, int c) { return kQK + at(kChunk, r, c); }
 };
 
 __host__ __device__ inline size_t chunk_scratch_floats(int Dk, int Dv) { return (size_t)kChunk * (3 * Dk + Dv + kChunk); }
@@ -80,6 +97,9 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const float (&a)[4], flo
                    "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
 }
 
+// SiLU with the hardware's division (2 ulp of 32 bits); its results are rounded to TF32 before they are multiplied.
+__device__ __forceinline__ float gdn_silu(float x) { return __fdividef(x, 1.f + __expf(-x)); }
+
 // grid = (max chunks, Hv), block = 256 threads, two CTAs per SM (shared memory: Q and K tiles, the raw q|k input tile
 // that A, T and the block-row temporaries later overwrite; V is convolved straight from global memory into Q's tile
 // once Q is dead).
@@ -93,7 +113,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
     float* sV = sQ;
     float* sG = sK + kChunk * PK;          // [64]
     float* sBeta = sG + kChunk;            // [64]
-    float* sU = sBeta + kChunk;            // union: raw bf16 q|k tile [67][2 DK], later A [64][65], T [64][68], M [3][16][17]
+    float* sU = sBeta + kChunk;            // union: raw bf16 q|k tile [67][2 DK], later A [64][65], T [64][68], M [32][36]
     __nv_bfloat16* sRaw = reinterpret_cast<__nv_bfloat16*>(sU);
     float* sA = sU;
     float* sT = sA + kChunk * 65;          // 64 * 65 floats keep the T rows 16-byte aligned
@@ -112,9 +132,21 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
     float* scr = a.scratch + ((size_t)blockIdx.x * a.Hv + h) * chunk_scratch_floats(DK, DV);
     float* gW = scr; float* gQd = gW + kChunk * DK; float* gKd = gQd + kChunk * DK;
     float* gU = gKd + kChunk * DK; float* gQK = gU + kChunk * DV;
+    using Image = GdnImage<DK, DV>;
 
     // ---- stage the raw inputs of rows -3 .. 63 (this head's q | k channels) with wide loads
-    {
+    const bool inner = r0 >= 3 && C == kChunk;              // every row of the tile is one of this step's
+    if (inner && (a.ld_proj % 8) == 0) {
+        // all copies in flight at once
+        constexpr int PPR = CQK / 8;
+        const __nv_bfloat16* src0 = a.proj + (row0 - 3) * a.ld_proj;
+        for (int p = t; p < RAWR * PPR; p += 256) {
+            const int rr = p / PPR, c = (p % PPR) * 8;
+            const __nv_bfloat16* src = src0 + (size_t)rr * a.ld_proj + (c < DK ? q_off + c : k_off + (c - DK));
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(sRaw + rr * CQK + c)), "l"(src) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    } else {
         const bool vec = (a.ld_proj % 8) == 0;
         constexpr int PPR = CQK / 8;
         for (int p = t; p < RAWR * PPR; p += 256) {
@@ -159,6 +191,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
         sG[lane] = g0; sG[lane + 32] = g1 + tot0;
         sBeta[lane] = b0; sBeta[lane + 32] = b1;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     // ---- conv + SiLU of q and k: a thread owns a channel pair over a run of rows and slides its taps through registers
     {
@@ -178,17 +211,35 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
             float ya = wa01.x * x3.x; ya = fmaf(wa01.y, x2.x, ya); ya = fmaf(wa23.x, x1.x, ya); ya = fmaf(wa23.y, x0.x, ya);
             float yb = wb01.x * x3.y; yb = fmaf(wb01.y, x2.y, yb); yb = fmaf(wb23.x, x1.y, yb); yb = fmaf(wb23.y, x0.y, yb);
             x3 = x2; x2 = x1; x1 = x0;
-            *reinterpret_cast<float2*>(dst + r * PK) = make_float2(silu_f(ya), silu_f(yb));
+            *reinterpret_cast<float2*>(dst + r * PK) = make_float2(gdn_silu(ya), gdn_silu(yb));
         }
     }
     __syncthreads();
-    // ---- L2 norms: warp w owns rows 8w .. 8w+7
-    for (int r = warp * 8; r < warp * 8 + 8; ++r) {
-        float qq = 0.f, kk = 0.f;
-        for (int d = lane; d < DK; d += 32) { const float qv = sQ[r * PK + d], kv = sK[r * PK + d]; qq += qv * qv; kk += kv * kv; }
-        qq = warp_sum(qq); kk = warp_sum(kk);
-        const float qn = rsqrtf(qq + 1e-6f) * rsqrtf((float)DK), kn = rsqrtf(kk + 1e-6f);
-        for (int d = lane; d < DK; d += 32) { sQ[r * PK + d] *= qn; sK[r * PK + d] *= kn; }
+    // ---- L2 norms: warp w owns rows 8w .. 8w+7, four at a time so that their reductions overlap
+    {
+        constexpr int V = DK / 32;
+        for (int rb = warp * 8; rb < warp * 8 + 8; rb += 4) {
+            float q[4][V], k[4][V], n[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                n[i] = n[4 + i] = 0.f;
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    q[i][v] = sQ[(rb + i) * PK + lane + 32 * v]; k[i][v] = sK[(rb + i) * PK + lane + 32 * v];
+                    n[i] = fmaf(q[i][v], q[i][v], n[i]); n[4 + i] = fmaf(k[i][v], k[i][v], n[4 + i]);
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) n[i] += __shfl_xor_sync(0xffffffffu, n[i], o);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float qn = rsqrtf(n[i] + 1e-6f) * rsqrtf((float)DK), kn = rsqrtf(n[4 + i] + 1e-6f);
+#pragma unroll
+                for (int v = 0; v < V; ++v) { sQ[(rb + i) * PK + lane + 32 * v] = q[i][v] * qn; sK[(rb + i) * PK + lane + 32 * v] = k[i][v] * kn; }
+            }
+        }
     }
     __syncthreads();
     // ---- A (strictly lower) and QKd (lower incl. diagonal) on the tensor cores: warp -> rows 16 mt .., columns
@@ -221,7 +272,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
                 const int tt = 16 * mt + g + (e >> 1) * 8, ss = 32 * ch + 8 * nt + 2 * tq + (e & 1);
                 const float dec = ss <= tt ? __expf(sG[tt] - sG[ss]) : 0.f;
                 sA[tt * 65 + ss] = ss < tt ? sBeta[tt] * dec * kk[nt][e] : 0.f;
-                gQK[tt * kChunk + ss] = a.round_tf32 ? to_tf32(dec * qk[nt][e]) : dec * qk[nt][e];
+                (a.images ? scr[Image::qk(tt, ss)] : gQK[tt * kChunk + ss]) = a.round_tf32 ? to_tf32(dec * qk[nt][e]) : dec * qk[nt][e];
             }
     }
     __syncthreads();
@@ -229,7 +280,11 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
     constexpr int VPARTS = 512 / DV, VRUN = kChunk / VPARTS;             // DV / 2 channel pairs x VPARTS row runs = 256 threads
     const int vc = 2 * (t % (DV / 2)), vrb = (t / (DV / 2)) * VRUN;
     uint32_t vraw[VRUN + 3];
-    {
+    if (inner && (a.ld_proj & 1) == 0) {
+        const __nv_bfloat16* src = a.proj + (row0 + vrb - 3) * a.ld_proj + v_off + vc;
+#pragma unroll
+        for (int i = 0; i < VRUN + 3; ++i) vraw[i] = __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)i * a.ld_proj));
+    } else {
         const bool even = (a.ld_proj & 1) == 0;
 #pragma unroll
         for (int i = 0; i < VRUN + 3; ++i) {
@@ -264,7 +319,23 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
         for (int i = 0; i < 16; ++i) sT[(16 * b + i) * kTP + 16 * b + j] = x[i];
     } else {
         const float GC = sG[kChunk - 1];
-        for (int i = t - kChunk; i < kChunk * DK / 4; i += 256 - kChunk) {
+        if (a.images) {
+            for (int i = t - kChunk; i < kChunk * DK / 4; i += 256 - kChunk) {
+                const int r = (i * 4) / DK, d = (i * 4) % DK;
+                const float eq = __expf(sG[r]);
+                const float4 q = *reinterpret_cast<const float4*>(sQ + r * PK + d);
+                *reinterpret_cast<float4*>(scr + Image::qd(r, d)) = make_float4(to_tf32(eq * q.x), to_tf32(eq * q.y), to_tf32(eq * q.z), to_tf32(eq * q.w));
+            }
+            // Kd^T: a thread takes eight rows of the chunk of one channel, whole 32-byte sectors of the tile
+            for (int i = t - kChunk; i < kChunk * DK / 8; i += 256 - kChunk) {
+                const int d = i % DK, r = i / DK * 8;
+                float k[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) k[j] = to_tf32(__expf(GC - sG[r + j]) * sK[(r + j) * PK + d]);
+                *reinterpret_cast<float4*>(scr + Image::kdt(d, r)) = make_float4(k[0], k[1], k[2], k[3]);
+                *reinterpret_cast<float4*>(scr + Image::kdt(d, r + 4)) = make_float4(k[4], k[5], k[6], k[7]);
+            }
+        } else for (int i = t - kChunk; i < kChunk * DK / 4; i += 256 - kChunk) {
             const int r = (i * 4) / DK, d = (i * 4) % DK;
             const float eq = __expf(sG[r]), ek = __expf(GC - sG[r]);
             const float4 q = *reinterpret_cast<const float4*>(sQ + r * PK + d), k = *reinterpret_cast<const float4*>(sK + r * PK + d);
@@ -293,32 +364,53 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
             float ya = wa01.x * x3.x; ya = fmaf(wa01.y, x2.x, ya); ya = fmaf(wa23.x, x1.x, ya); ya = fmaf(wa23.y, x0.x, ya);
             float yb = wb01.x * x3.y; yb = fmaf(wb01.y, x2.y, yb); yb = fmaf(wb23.x, x1.y, yb); yb = fmaf(wb23.y, x0.y, yb);
             x3 = x2; x2 = x1; x1 = x0;
-            *reinterpret_cast<float2*>(dst + r * PV) = make_float2(silu_f(ya), silu_f(yb));
+            *reinterpret_cast<float2*>(dst + r * PV) = make_float2(gdn_silu(ya), gdn_silu(yb));
         }
     }
-    // ---- T, block rows 1 .. 3: T_ij = -T_ii (sum_{k = j .. i-1} A_ik T_kj) for all j < i at once
-    for (int bi = 1; bi < 4; ++bi) {
-        for (int e = t; e < bi * 256; e += 256) {
-            const int bj = e >> 8, r = (e >> 4) & 15, c = e & 15;
-            const float* Ar = sA + (16 * bi + r) * 65;
-            float acc0 = 0.f, acc1 = 0.f;
-            for (int k = 16 * bj; k < 16 * bi; k += 2) {
-                acc0 = fmaf(Ar[k], sT[k * kTP + 16 * bj + c], acc0);
-                acc1 = fmaf(Ar[k + 1], sT[(k + 1) * kTP + 16 * bj + c], acc1);
-            }
-            sM[(bj * 16 + r) * 17 + c] = acc0 + acc1;
-        }
-        __syncthreads();
-        for (int e = t; e < bi * 256; e += 256) {
-            const int bj = e >> 8, r = (e >> 4) & 15, c = e & 15;
-            const float* Tr = sT + (16 * bi + r) * kTP + 16 * bi;
-            float acc = 0.f;
+    // ---- T below the diagonal blocks: -T_22 (A_21 T_11) for the two pairs of 16-row blocks, then for the two 32-row halves
+    __syncthreads();
+    {
+        const int pr = t >> 7, r = (t >> 3) & 15, c = 2 * (t & 7);                 // pair, row and columns of its 16 x 16 block
+        const int lo = 32 * pr, hi = lo + 16;
+        float x0 = 0.f, x1 = 0.f;
 #pragma unroll
-            for (int k = 0; k < 16; ++k) acc = fmaf(Tr[k], sM[(bj * 16 + k) * 17 + c], acc);     // T_ii is zero above its diagonal
-            sT[(16 * bi + r) * kTP + 16 * bj + c] = -acc;
+        for (int k = 0; k < 16; ++k) {
+            const float av = sA[(hi + r) * 65 + lo + k];
+            const float2 tv = *reinterpret_cast<const float2*>(sT + (lo + k) * kTP + lo + c);
+            x0 = fmaf(av, tv.x, x0); x1 = fmaf(av, tv.y, x1);
         }
+        sM[(16 * pr + r) * 36 + c] = x0; sM[(16 * pr + r) * 36 + c + 1] = x1;
+        sT[(lo + r) * kTP + hi + c] = 0.f; sT[(lo + r) * kTP + hi + c + 1] = 0.f;      // the halves are used whole below
         __syncthreads();
+        x0 = x1 = 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const float tv = sT[(hi + r) * kTP + hi + k];
+            const float2 mv = *reinterpret_cast<const float2*>(sM + (16 * pr + k) * 36 + c);
+            x0 = fmaf(tv, mv.x, x0); x1 = fmaf(tv, mv.y, x1);
+        }
+        sT[(hi + r) * kTP + lo + c] = -x0; sT[(hi + r) * kTP + lo + c + 1] = -x1;
     }
+    __syncthreads();
+    {
+        const int r = t >> 3, c = 4 * (t & 7);
+        auto product = [&](const float* left, int lp, const float* right, int rp) {    // row r of left [32 x 32] times right's columns c ..
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+            for (int k = 0; k < 32; ++k) {
+                const float l = left[r * lp + k];
+                const float4 v = *reinterpret_cast<const float4*>(right + k * rp + c);
+                x.x = fmaf(l, v.x, x.x); x.y = fmaf(l, v.y, x.y); x.z = fmaf(l, v.z, x.z); x.w = fmaf(l, v.w, x.w);
+            }
+            return x;
+        };
+        const float4 m = product(sA + 32 * 65, 65, sT, kTP);
+        *reinterpret_cast<float4*>(sM + r * 36 + c) = m;
+        __syncthreads();
+        const float4 x = product(sT + 32 * kTP + 32, kTP, sM, 36);
+        *reinterpret_cast<float4*>(sT + (32 + r) * kTP + c) = make_float4(-x.x, -x.y, -x.z, -x.w);
+    }
+    __syncthreads();
     // ---- W = T diag(beta D) K (warps 0-3) and U = T diag(beta) V (warps 4-7) on the tensor cores: warp -> rows
     //      16 mt .., all columns of its matrix; T is lower triangular, so k-steps beyond the row tile are skipped
     {
@@ -347,6 +439,20 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
         if (isW && a.round_tf32) {
 #pragma unroll
             for (int nt = 0; nt < NTW; ++nt) { acc[nt][0] = to_tf32(acc[nt][0]); acc[nt][1] = to_tf32(acc[nt][1]); acc[nt][2] = to_tf32(acc[nt][2]); acc[nt][3] = to_tf32(acc[nt][3]); }
+        }
+        if (a.images) {
+#pragma unroll
+            for (int nt = 0; nt < NTW; ++nt) {
+                const int r = 16 * mt + g, c = 8 * nt + 2 * tq;
+                if (isW && nt < ntiles) {
+                    *reinterpret_cast<float2*>(scr + Image::w(r, c)) = make_float2(acc[nt][0], acc[nt][1]);
+                    *reinterpret_cast<float2*>(scr + Image::w(r + 8, c)) = make_float2(acc[nt][2], acc[nt][3]);
+                } else if (nt < ntiles) {
+                    scr[Image::ut(r, c)] = acc[nt][0]; scr[Image::ut(r, c + 1)] = acc[nt][1];
+                    scr[Image::ut(r + 8, c)] = acc[nt][2]; scr[Image::ut(r + 8, c + 1)] = acc[nt][3];
+                }
+            }
+            return;
         }
 #pragma unroll
         for (int nt = 0; nt < NTW; ++nt)
@@ -392,6 +498,7 @@ struct GdnScanArgs {
     float* state;                 // [slots, Hv, Dk, Dv] fp32, updated in place
     const GdnSeqDesc2* seqs;
     float* o;                     // [rows, Hv, Dv] fp32
+    uint32_t* status; long long budget;      // tcgen05 scan
 };
 
 __device__ __forceinline__ void fma8(float (&acc)[8], float w, const float4& s0, const float4& s1) {
@@ -701,6 +808,210 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_tc_kernel(const GdnScanArg
     }
 }
 
+// ---- the scan on tcgen05 (Dk = Dv = 128): the same products, with the state in tensor memory.  One CTA per (sequence, value head,
+// 64 columns of Dv); per chunk (TF32 operands from shared memory, fp32 accumulators):
+//     [P; R] = [W; Qd] S          128 x 64 x 128 into D1 (rows of P: lanes 0 .. 63)
+//     Delta = U - P               lanes 0 .. 63 to shared memory as Delta^T, rounded to TF32
+//     S     += Kd^T Delta         128 x 64 x 64 into D2, which the threads have scaled by D_C before
+//     [.; R] += [0; QKd] Delta    128 x 64 x 64 into D1 (the zero rows stay in shared memory)
+// then a TF32 copy of S goes to shared memory as the next chunk's operand and R to global memory.  The preparation kernel has laid the
+// operands out as shared-memory tiles (GdnImage), so one thread fetches a chunk with five bulk copies, each as soon as the products
+// that read the previous chunk's tile are done.
+// Warps 0-7: lane quadrant (warp & 3), columns 32 (warp >> 2) .. + 31; warp 8: copies; warp 9: products.
+// Rounding as in the mma.sync scan it replaces, which took 5.2 us per chunk (1500 of 9800 cycles to issue copies twice, 2700 and 2500
+// for the large products, bound by fragment loads from shared memory) and now takes 3.3 us.  2048 rows: 165 us before, 106 now with 32
+// heads, 169 and 115 with 48 (64 and 96 CTAs).  What bounds a chunk: fetching its 128 KB of tiles, of which none has a second buffer.
+template <int DK, int DV>
+__global__ void __launch_bounds__(320, 1) gdn_chunk_scan_umma_kernel(const GdnScanArgs a) {
+    static_assert(DK == 128 && kChunk == 64 && kSlice == 64, "the tiles' row counts");
+    using Image = GdnImage<DK, DV>;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    constexpr int kBytesWQ = 128 * DK * 4, kBytesKd = DK * kChunk * 4, kBytesA3 = 128 * kChunk * 4, kBytesS = kSlice * DK * 4, kBytesD = kSlice * kChunk * 4;
+    unsigned char* sWQ = smem;                   // [4 panels][128 rows][128 B]
+    unsigned char* sKd = sWQ + kBytesWQ;         // [2][128][128 B]
+    unsigned char* sA3 = sKd + kBytesKd;         // [2][64 zero rows, 64 of QKd][128 B]
+    unsigned char* sS = sA3 + kBytesA3;          // S^T: [4 panels][64 columns][128 B]
+    unsigned char* sD = sS + kBytesS;            // Delta^T: [2 panels][64 columns][128 B]
+    float* sU = reinterpret_cast<float*>(sD + kBytesD);      // U^T: [64 columns][64 rows]
+    __shared__ __align__(8) uint64_t wq_full, u_full, kq_full, s_ready, d_ready, m1_done, m2_done, m3_done;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int s_abort, s_wq, s_u, s_kq;     // fills of each tile issued
+
+    const int c0 = blockIdx.x * kSlice, h = blockIdx.y, Hv = a.Hv;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const GdnSeqDesc2 sd = a.seqs[blockIdx.z];
+    if (sd.n_rows <= a.min_rows || sd.slot < 0) return;
+    PS_CHECK(PS_SLOT_OK(sd.slot) && PS_ROWS_OK(sd.row_start, sd.n_rows));
+    int gc = 0;
+    for (int s = 0; s < (int)blockIdx.z; ++s) {
+        const GdnSeqDesc2 d = a.seqs[s];
+        if (d.n_rows > a.min_rows && d.slot >= 0) gc += (d.n_rows + kChunk - 1) / kChunk;
+    }
+    const int nc = (sd.n_rows + kChunk - 1) / kChunk;
+    const float* scr0 = a.scratch + ((size_t)gc * Hv + h) * chunk_scratch_floats(DK, DV);
+    const size_t scr_step = (size_t)Hv * chunk_scratch_floats(DK, DV);
+
+    if (threadIdx.x == 0) {
+        tc::mbar_init(&wq_full, 1); tc::mbar_init(&u_full, 1); tc::mbar_init(&kq_full, 1);
+        tc::mbar_init(&s_ready, 8); tc::mbar_init(&d_ready, 4);
+        tc::mbar_init(&m1_done, 1); tc::mbar_init(&m2_done, 1); tc::mbar_init(&m3_done, 1);
+        tc::fence_barrier_init();
+        s_abort = 0; s_wq = s_u = s_kq = 0;
+    }
+    if (warp == 9) {
+        tc::tmem_alloc(&tmem_slot, 128);
+        tc::tmem_relinquish();
+    }
+    for (int i = threadIdx.x; i < 2 * 64 * 8; i += 320)       // the zero rows of both panels
+        *reinterpret_cast<uint4*>(sA3 + (i >> 9) * (128 * 128) + (i & 511) * 16) = make_uint4(0, 0, 0, 0);
+    tc::fence_proxy_async_smem();
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t d1 = tmem_slot, d2 = d1 + 64;
+
+    if (warp == 8) {
+        // ------------------------------------------------ copies
+        if (tc::elect_one()) {
+            for (int c = 0; c < nc; ++c) {
+                const float* scr = scr0 + c * scr_step;
+                const uint32_t before = (uint32_t)(c - 1) & 1u;
+                if (c > 0 && !tc::mbar_wait_abortable(&m1_done, before, a.budget, &s_abort)) break;      // [W; Qd] has been read
+                tc::mbar_expect_tx(&wq_full, kBytesWQ);
+                tc::bulk_load(sWQ, scr + Image::kWQ, kBytesWQ, &wq_full);
+                s_wq = c + 1;
+                // U is free with the Delta that was made of it, Kd and QKd with the products of that Delta
+                if (c > 0 && !tc::mbar_wait_abortable(&d_ready, before, a.budget, &s_abort)) break;
+                tc::mbar_expect_tx(&u_full, kBytesD);
+                tc::bulk_load(sU, scr + Image::kU + c0 * kChunk, kBytesD, &u_full);
+                s_u = c + 1;
+                if (c > 0 && !tc::mbar_wait_abortable(&m3_done, before, a.budget, &s_abort)) break;
+                tc::mbar_expect_tx(&kq_full, kBytesKd + kChunk * kChunk * 4);
+                tc::bulk_load(sKd, scr + Image::kKd, kBytesKd, &kq_full);
+#pragma unroll
+                for (int p = 0; p < 2; ++p) tc::bulk_load(sA3 + p * (128 * 128) + 64 * 128, scr + Image::kQK + p * (kChunk * 32), kChunk * 128, &kq_full);
+                s_kq = c + 1;
+            }
+        }
+    } else if (warp == 9) {
+        // ------------------------------------------------ products
+        if (tc::elect_one()) {
+            constexpr uint32_t idesc = tc::idesc_tf32_f32(128, kSlice);
+            auto lo = [](const void* p) { return (tc::smem_u32(p) >> 4) | tc::kDescSw128LoFlags; };
+            const uint32_t wq = lo(sWQ), kd = lo(sKd), a3 = lo(sA3), st = lo(sS), dt = lo(sD);
+            // K-step j of 8: panel j / 4, 32 bytes inside its rows; panels of `ra` and `rb` rows
+            auto product = [&](uint32_t acc, uint32_t al, uint32_t bl, int steps, int ra, int rb, bool add) {
+#pragma unroll 4
+                for (int j = 0; j < steps; ++j)
+                    tc::mma_tf32_ss(acc, tc::desc_pack(al + (j >> 2) * (ra * 8) + (j & 3) * 2, tc::kDescSw128Hi),
+                                    tc::desc_pack(bl + (j >> 2) * (rb * 8) + (j & 3) * 2, tc::kDescSw128Hi), idesc, add || j > 0 ? 1u : 0u);
+            };
+            for (int c = 0; c < nc; ++c) {
+                const uint32_t ph = (uint32_t)c & 1u;
+                if (!tc::mbar_wait_abortable(&s_ready, ph, a.budget, &s_abort) || !tc::mbar_wait_abortable(&wq_full, ph, a.budget, &s_abort)) break;
+                tc::fence_after_sync();
+                product(d1, wq, st, DK / 8, 128, kSlice, false);
+                tc::mma_commit(&m1_done);
+                if (!tc::mbar_wait_abortable(&d_ready, ph, a.budget, &s_abort) || !tc::mbar_wait_abortable(&kq_full, ph, a.budget, &s_abort)) break;
+                tc::fence_after_sync();
+                product(d2, kd, dt, kChunk / 8, DK, kSlice, true);
+                tc::mma_commit(&m2_done);
+                product(d1, a3, dt, kChunk / 8, 128, kSlice, true);
+                tc::mma_commit(&m3_done);
+            }
+        }
+    } else {
+        // ------------------------------------------------ state, Delta and outputs
+        const int quad = warp & 3, n0 = (warp >> 2) * 32, row = quad * 32 + lane;         // row: TMEM lane
+        const uint32_t at = ((uint32_t)(quad * 32) << 16) + (uint32_t)n0;
+        float* Sg = a.state + (((size_t)sd.slot * Hv + h) * DK + row) * DV + c0 + n0;
+        const float* dcs = a.dc + (size_t)gc * Hv + h;
+        auto wait = [&](uint64_t* bar, uint32_t ph) {
+            const bool ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(bar, ph, a.budget, &s_abort));
+            if (ok) tc::fence_after_sync();
+            return ok;
+        };
+        // state row `row`, columns n0 .. + 31: TF32 copy as the operand S^T, and the accumulator scaled by the chunk's decay
+        auto put_state = [&](uint32_t (&v)[32], float decay) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                const int n = n0 + j;
+                *reinterpret_cast<float*>(sS + quad * (kSlice * 128) + n * 128 + (((lane >> 2) ^ (n & 7)) << 4) + (lane & 3) * 4) = to_tf32(__uint_as_float(v[j]));
+                v[j] = __float_as_uint(__uint_as_float(v[j]) * decay);
+            }
+            tc::tmem_st_32x32(d2 + at, v);
+            tc::tmem_st_wait();
+            tc::fence_proxy_async_smem();
+        };
+        auto arrive = [&](uint64_t* bar) {
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(bar);
+        };
+        uint32_t v[32];
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+            const uint4 q = *reinterpret_cast<const uint4*>(Sg + j);
+            v[j] = q.x; v[j + 1] = q.y; v[j + 2] = q.z; v[j + 3] = q.w;
+        }
+        put_state(v, dcs[0]);
+        arrive(&s_ready);
+        for (int c = 0; c < nc; ++c) {
+            const uint32_t ph = (uint32_t)c & 1u;
+            const float next = c + 1 < nc ? dcs[(size_t)(c + 1) * Hv] : 1.f;
+            if (quad < 2) {
+                if (!wait(&m1_done, ph) || !wait(&u_full, ph)) break;
+                tc::tmem_ld_32x32(d1 + at, v);
+                tc::tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    const int n = n0 + j;
+                    *reinterpret_cast<float*>(sD + quad * (kSlice * 128) + n * 128 + (((lane >> 2) ^ (n & 7)) << 4) + (lane & 3) * 4) =
+                        to_tf32(sU[n * kChunk + row] - __uint_as_float(v[j]));
+                }
+                tc::fence_proxy_async_smem();
+                arrive(&d_ready);
+            }
+            if (!wait(&m2_done, ph)) break;
+            tc::tmem_ld_32x32(d2 + at, v);
+            tc::tmem_ld_wait();
+            if (c + 1 < nc) put_state(v, next);
+            else {
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(Sg + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            }
+            if (quad >= 2) {
+                if (!wait(&m3_done, ph)) break;
+                tc::tmem_ld_32x32(d1 + at, v);
+                tc::tmem_ld_wait();
+            }
+            arrive(&s_ready);
+            const int r = c * kChunk + row - 64;
+            if (quad >= 2 && r < sd.n_rows) {
+                float* o = a.o + ((size_t)(sd.row_start + r) * Hv + h) * DV + c0 + n0;
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(o + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            }
+        }
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (s_abort != 0 && threadIdx.x == 0) {
+        set_status(a.status, PS_DEV_WAIT_TIMEOUT);
+        // copies still in flight get a bounded chance to land before the shared memory goes back to the next CTA
+        const long long b = a.budget < 4000000ll ? a.budget : 4000000ll;
+        if (s_wq > 0) tc::mbar_wait(&wq_full, (uint32_t)(s_wq - 1) & 1u, b);
+        if (s_u > 0) tc::mbar_wait(&u_full, (uint32_t)(s_u - 1) & 1u, b);
+        if (s_kq > 0) tc::mbar_wait(&kq_full, (uint32_t)(s_kq - 1) & 1u, b);
+    }
+    __syncthreads();
+    if (warp == 9) {
+        tc::fence_after_sync();
+        tc::tmem_dealloc(d1, 128);
+    }
+}
+
 // One warp per (row, head): RMSNorm over the head's Dv outputs * SiLU(z).  E = Dv / 32 contiguous values per lane.
 // grid = ceil(rows * Hv / 8), block = 256 threads
 template <int E>
@@ -748,38 +1059,46 @@ PS_API long long ps_gdn_chunked_scratch_floats(int rows, int n_seqs, int Hv, int
 namespace ps {
 template <int DK, int DV>
 static int launch_chunked(const GdnPrepArgs& p, const GdnScanArgs& s, int max_chunks, cudaStream_t stream) {
-    const size_t raw_b = (size_t)(kChunk + 3) * (2 * DK) * 2, at_b = sizeof(float) * (kChunk * 65 + kChunk * kTP + 3 * 16 * 17);
+    const size_t raw_b = (size_t)(kChunk + 3) * (2 * DK) * 2, at_b = sizeof(float) * (kChunk * 65 + kChunk * kTP + 32 * 36);
     const size_t smem_a = sizeof(float) * (2 * kChunk * (DK + 4) + 2 * kChunk) + (raw_b > at_b ? raw_b : at_b);
     const size_t smem_b = sizeof(float) * (3 * kChunk * (DK + 4) + DK * (kSlice + 4) + kChunk * (kSlice + 4) + kChunk * 65);
     const size_t smem_t = sizeof(float) * (2 * kChunk * (DK + 4) + kChunk * (DK + 8) + DK * (kSlice + 8) + kChunk * (kSlice + 8) +
                                            kChunk * (kChunk + 4));
+    // a chunk's tiles, S^T, Delta^T and U^T of the tcgen05 scan, and slack for their alignment
+    const size_t smem_u = sizeof(float) * (2 * kChunk * DK + DK * kChunk + 2 * kChunk * kChunk + kSlice * DK + 2 * kSlice * kChunk) + 1024;
     static bool set = false;
     static int use_tc = 1;
+    constexpr bool kUmma = DK == 128 && DV == 128;
     if (!set) {
         cudaFuncSetAttribute(gdn_chunk_prep_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a);
         cudaFuncSetAttribute(gdn_chunk_scan_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b);
-        cudaFuncSetAttribute(gdn_chunk_scan_tc_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t);
+        if constexpr (kUmma) cudaFuncSetAttribute(gdn_chunk_scan_umma_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_u);
+        else cudaFuncSetAttribute(gdn_chunk_scan_tc_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t);
         const char* e = getenv("PS_GDN_SCAN");            // "fp32": the CUDA-core scan (all-fp32 products)
         use_tc = (e == nullptr || e[0] != 'f') ? 1 : 0;
         set = true;
     }
     GdnPrepArgs pp = p;
     pp.round_tf32 = use_tc;
+    pp.images = use_tc && kUmma;
     gdn_chunk_prep_kernel<DK, DV><<<dim3(max_chunks, p.Hv), 256, smem_a, stream>>>(pp);
     int err = PS_LAUNCH_CHECK();
     if (err) return err;
-    if (use_tc) gdn_chunk_scan_tc_kernel<DK, DV><<<dim3(DV / kSlice, p.Hv, p.n_seqs), 256, smem_t, stream>>>(s);
-    else gdn_chunk_scan_kernel<DK, DV><<<dim3(DV / kSlice, p.Hv, p.n_seqs), 256, smem_b, stream>>>(s);
+    const dim3 grid(DV / kSlice, p.Hv, p.n_seqs);
+    if (!use_tc) gdn_chunk_scan_kernel<DK, DV><<<grid, 256, smem_b, stream>>>(s);
+    else if constexpr (kUmma) gdn_chunk_scan_umma_kernel<DK, DV><<<grid, 320, smem_u, stream>>>(s);
+    else gdn_chunk_scan_tc_kernel<DK, DV><<<grid, 256, smem_t, stream>>>(s);
     return PS_LAUNCH_CHECK();
 }
 }  // namespace ps
 
+// (All launches, 2048 rows: 343 us before the tcgen05 scan and the shorter preparation, 239 now with 32 heads; 421 and 309 with 48.)
 // Chunked GDN mixer for prefill-sized steps.  `scratch` holds ps_gdn_chunked_scratch_floats() floats,
 // `dc` one float per (chunk, head), `o` [rows, Hv, Dv] floats.
 PS_API int ps_gdn_chunked(const void* proj, int ld_proj, int rows, int Hk, int Hv, int Dk, int Dv, const void* conv_w,
                           const void* A_log, const void* dt_bias, const void* norm_w, float eps, void* conv_state, int ring,
                           void* state, const void* seqs, int n_seqs, const void* row_slot, const void* row_pos,
-                          int min_rows, void* scratch, void* dc, void* o, void* out, cudaStream_t stream) {
+                          int min_rows, void* scratch, void* dc, void* o, void* out, void* status, cudaStream_t stream) {
     using namespace ps;
     if (rows <= 0 || n_seqs <= 0 || Hk <= 0 || (Hv % Hk) || ring < 4) return (int)cudaErrorInvalidValue;
     GdnPrepArgs p;
@@ -787,9 +1106,10 @@ PS_API int ps_gdn_chunked(const void* proj, int ld_proj, int rows, int Hk, int H
     p.conv_w = (const __nv_bfloat16*)conv_w; p.A_log = (const float*)A_log; p.dt_bias = (const float*)dt_bias;
     p.conv_state = (__nv_bfloat16*)conv_state; p.ring = ring; p.row_slot = (const int*)row_slot; p.row_pos = (const int*)row_pos;
     p.seqs = (const GdnSeqDesc2*)seqs; p.n_seqs = n_seqs; p.min_rows = min_rows; p.scratch = (float*)scratch; p.dc = (float*)dc;
+    p.round_tf32 = p.images = 0;
     GdnScanArgs s;
     s.scratch = p.scratch; s.dc = p.dc; s.Hv = Hv; s.Dv = Dv; s.n_seqs = n_seqs; s.min_rows = min_rows; s.state = (float*)state; s.seqs = p.seqs;
-    s.o = (float*)o;
+    s.o = (float*)o; s.status = (uint32_t*)status; s.budget = g_ps_wait_budget_cycles;
     const int max_chunks = (rows + kChunk - 1) / kChunk + n_seqs;
     int err;
     if (Dk == 128 && Dv == 128) err = launch_chunked<128, 128>(p, s, max_chunks, stream);
