@@ -540,6 +540,16 @@ class CudaOps(OpTrace):
                       c_int(split_tokens), c_int(self.max_splits), *gate, ptr(out))
             self.launches += 2
             return out
+        if (self.attn_decode_tc and st.kv_fmt == 1
+                and _lib.lib().ps_attn_decode_fp8_ok(c_int(hq), c_int(hkv), c_int(D), c_int(st.sc.page_tokens), c_int(split_tokens))):
+            _lib.call("ps_attn_decode_fp8", ptr(q), ptr(kv.k), ptr(kv.v), ptr(kv.k_scale), ptr(kv.v_scale), ptr(st.block_table),
+                      c_int(st.max_blocks), c_int(st.sc.page_tokens), c_int(st.num_pages), ptr(b.row_slot), ptr(row_pos), c_int(rows),
+                      c_int(hq), c_int(hkv), c_int(D), sm, c_int(split_tokens), c_int(self.max_splits), c_int(max_visible), ptr(pacc),
+                      ptr(pml), ptr(st.status))
+            _lib.call("ps_paged_attention_merge", ptr(pacc), ptr(pml), ptr(row_pos), c_int(rows), c_int(hq), c_int(D),
+                      c_int(split_tokens), c_int(self.max_splits), *gate, ptr(out))
+            self.launches += 2
+            return out
         _lib.call("ps_paged_attention_ex", ptr(q), ptr(kv.k), ptr(kv.v), ptr(kv.k_scale), ptr(kv.v_scale),
                   ptr(st.block_table), c_int(st.max_blocks), c_int(st.sc.page_tokens), c_int(st.num_pages),
                   ptr(b.row_slot), ptr(row_pos), c_int(rows), c_int(hq), c_int(hkv), c_int(D),
