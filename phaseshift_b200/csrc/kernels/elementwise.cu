@@ -42,13 +42,29 @@ __global__ void embedding_mxfp8_kernel(const int* ids, const uint8_t* codes, con
     const bool ok = id >= 0 && id < vocab;
     if (!ok && threadIdx.x == 0) set_status(status, PS_DEV_BAD_INDEX);
     float ss = 0.f;
-    for (int i = threadIdx.x; i < H; i += blockDim.x) {
-        float v = 0.f;
-        if (ok) v = e4m3_to_f32(codes[(size_t)id * H + i]) * __uint_as_float((uint32_t)scales[(size_t)id * (H / 32) + i / 32] << 23);
-        const __nv_bfloat16 o = f32_to_bf16(v);
-        out[(size_t)r * ldo + i] = o;
-        const float of = bf16_to_f32(o);
-        ss += of * of;
+    // eight codes per load and thread (byte by byte a row of 5120 took 11.5 us, most of a step's start)
+    for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
+        uint2 c = make_uint2(0, 0);
+        float sc = 0.f;
+        if (ok) {
+            c = __ldg(reinterpret_cast<const uint2*>(codes + (size_t)id * H) + i);
+            sc = __uint_as_float((uint32_t)scales[(size_t)id * (H / 32) + i / 4] << 23);
+        }
+        uint32_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const uint32_t w = e < 2 ? c.x : c.y;
+            const float v0 = ok ? e4m3_to_f32((uint8_t)(w >> (16 * (e & 1)))) * sc : 0.f, v1 = ok ? e4m3_to_f32((uint8_t)(w >> (16 * (e & 1) + 8))) * sc : 0.f;
+            o[e] = f32x2_to_bf16x2_bits(v0, v1);
+            const float2 f = bf16x2_bits_to_f32x2(o[e]);
+            ss += f.x * f.x + f.y * f.y;
+        }
+        __nv_bfloat16* d = out + (size_t)r * ldo + 8 * i;
+        if (ldo % 8 == 0) *reinterpret_cast<uint4*>(d) = make_uint4(o[0], o[1], o[2], o[3]);
+        else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { const __nv_bfloat162 two = *reinterpret_cast<const __nv_bfloat162*>(&o[e]); d[2 * e] = two.x; d[2 * e + 1] = two.y; }
+        }
     }
     if (ssq != nullptr) {
         ss = block_sum(ss, red);
