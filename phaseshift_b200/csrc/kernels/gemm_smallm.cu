@@ -31,7 +31,8 @@ struct SmallMArgs {
     int x_box_rows;         // rows fetched per X tile (multiple of 8)
     int iters_per_split;    // k-iterations (of 64) per split
     int splits;
-    float* partial;         // [splits, M, N] fp32
+    float* partial;         // [splits, M, ld] fp32
+    int ld;
     uint32_t* status;
     long long budget;       // clock-cycle budget of every mbarrier wait
 };
@@ -127,7 +128,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         tc::fence_after_sync();
         const int n = tile_n * kSmBM + quad * 32 + lane;
         if (done && s_abort == 0) {
-            float* dst = g.partial + (size_t)split * g.M * g.N;
+            float* dst = g.partial + (size_t)split * g.M * g.ld;
             for (int c0 = 0; c0 < g.nb; c0 += 32) {
                 uint32_t r[32];
                 if (k_iters > 0) {
@@ -140,7 +141,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 if (n < g.N) {
 #pragma unroll
                     for (int j = 0; j < 32; ++j)
-                        if (c0 + j < g.M) dst[(size_t)(c0 + j) * g.N + n] = __uint_as_float(r[j]);
+                        if (c0 + j < g.M) dst[(size_t)(c0 + j) * g.ld + n] = __uint_as_float(r[j]);
                 }
             }
         }
@@ -327,8 +328,11 @@ static int sm_map_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t
 PS_API int ps_gemm_smallm_splits(int N, int K) {
     const int tiles = (N + ps::kSmBM - 1) / ps::kSmBM;
     const int iters = (K + ps::kSmBK - 1) / ps::kSmBK;
-    int splits = (296 + tiles - 1) / tiles;                 // two CTAs on each of 148 SMs
-    const int max_splits = iters / 8 > 0 ? iters / 8 : 1;   // at least 8 k-iterations (128 KB of weights) per CTA
+    // as many CTAs as fit at once, two on each of 148 SMs: a few more than that and the step waits for a second round of them (with
+    // the count rounded up instead, 18432 x 2560 ran as 432 CTAs and 2560 x 9216 as 300: steps of 8, 12 and 32 rows took 858, 983 and
+    // 1456 us, with this rule 797, 922 and 1384)
+    int splits = 296 / tiles;
+    const int max_splits = iters / 4 > 0 ? iters / 4 : 1;   // at least 4 k-iterations (64 KB of weights) per CTA
     if (splits > max_splits) splits = max_splits;
     if (splits < 1) splits = 1;
     if (splits > 16) splits = 16;
@@ -362,7 +366,9 @@ PS_API int ps_gemm_smallm_normed(const void* a, int lda, const void* w, int ldw,
     g.splits = ps_gemm_smallm_splits(N, K);
     const int iters = (K + kSmBK - 1) / kSmBK;
     g.iters_per_split = (iters + g.splits - 1) / g.splits;
-    g.partial = (float*)partial; g.status = (uint32_t*)status; g.budget = g_ps_wait_budget_cycles;
+    // one split and nothing to do with its sums: they are the output
+    const bool direct = g.splits == 1 && epilogue == 0 && out_f32;
+    g.partial = direct ? (float*)out : (float*)partial; g.ld = direct ? ldo : N; g.status = (uint32_t*)status; g.budget = g_ps_wait_budget_cycles;
     CUtensorMap map_w, map_x;
     int err = sm_map_2d(&map_w, w, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, kSmBM);
     if (err) return err;
@@ -378,7 +384,7 @@ PS_API int ps_gemm_smallm_normed(const void* a, int lda, const void* w, int ldw,
     }
     dim3 grid((N + kSmBM - 1) / kSmBM, g.splits);
     err = launch_pdl(gemm_smallm_kernel<STAGES>, grid, dim3(kSmThreads), smem, stream, map_w, map_x, g);
-    if (err) return err;
+    if (err || direct) return err;
     SmallMReduceArgs r;
     r.partial = g.partial; r.splits = g.splits; r.M = M; r.N = N; r.epilogue = epilogue;
     r.residual = (const __nv_bfloat16*)residual; r.ld_res = ld_res; r.out = out; r.ldo = ldo; r.out_f32 = out_f32;
