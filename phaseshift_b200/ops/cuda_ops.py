@@ -285,11 +285,11 @@ class CudaOps(OpTrace):
             L = _lib.lib()
             L.ps_gemm_smallm_splits.restype = ctypes.c_int
             splits = L.ps_gemm_smallm_splits(c_int(W.N), c_int(kp))
-            need = splits * M * W.N
-            part = self.ws.get(("smallm_partial", 0))
-            if part is None or part.numel() < need:
-                part = torch.empty(max(need, 1 << 22), dtype=torch.float32, device=self.device)
-                self.ws[("smallm_partial", 0)] = part
+            # one buffer per power of two: a larger step must not free what a captured step of fewer rows writes to
+            cap = 1 << max(22, (splits * M * W.N - 1).bit_length())
+            part = self.ws.get(("smallm_partial", cap))
+            if part is None:
+                part = self.ws[("smallm_partial", cap)] = torch.empty(cap, dtype=torch.float32, device=self.device)
             normed = None
             if (norm_next is not None and epi == EPI_RESIDUAL and not out_f32 and W.N % 4 == 0 and W.N <= L.ps_gemm_smallm_norm_cols()
                     and all(t.stride(0) % 4 == 0 and t.data_ptr() % 8 == 0 for t in (out, residual))):
