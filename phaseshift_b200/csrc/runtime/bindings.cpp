@@ -22,8 +22,11 @@ static py::dict plan_to_dict(const StepPlan& p) {
     return d;
 }
 
+void bind_step_batch(py::module_& m);          // step_batch.cpp
+
 PYBIND11_MODULE(ps_runtime, m) {
     m.doc() = "phaseshift_b200 host runtime (C++)";
+    bind_step_batch(m);
     py::register_exception<Error>(m, "RuntimeCoreError");
 
     m.def("checked_add", &checked_add); m.def("checked_mul", &checked_mul); m.def("align_up", &align_up);

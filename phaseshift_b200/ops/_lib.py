@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes
 import os
 from pathlib import Path
+from typing import Dict
 
 import torch
 
@@ -67,7 +68,8 @@ def ptr(t) -> ctypes.c_void_p:
 
 
 def stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # (the raw handle without the Stream object that torch.cuda.current_stream() builds)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def check(err: int, what: str) -> None:
@@ -75,13 +77,31 @@ def check(err: int, what: str) -> None:
         raise KernelLibraryError(f"{what} failed with cudaError {err}")
 
 
+_LAUNCHERS: Dict[str, object] = {}
+
+
 def call(name: str, *args) -> None:
     """Call launcher ``name`` with pre-converted ctypes args and the current stream appended."""
-    fn = getattr(lib(), name)
-    fn.restype = ctypes.c_int
+    fn = _LAUNCHERS.get(name)
+    if fn is None:
+        fn = getattr(lib(), name)
+        fn.restype = ctypes.c_int
+        _LAUNCHERS[name] = fn
     check(fn(*args, stream()), name)
 
 
-c_int = ctypes.c_int
+# A step outside of a graph passes about two thousand sizes and flags to the launchers, nearly always the same ones.
+_INTS: Dict[int, ctypes.c_int] = {}
+
+
+def c_int(v: int) -> ctypes.c_int:
+    o = _INTS.get(v)
+    if o is None:
+        if len(_INTS) >= 1 << 16:
+            _INTS.clear()
+        o = _INTS[v] = ctypes.c_int(v)
+    return o
+
+
 c_float = ctypes.c_float
 c_ll = ctypes.c_longlong

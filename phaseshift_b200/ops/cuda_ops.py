@@ -86,6 +86,8 @@ class CudaOps(OpTrace):
         self.force_tc = os.environ.get("PS_FORCE_TC", "0") == "1"   # single-row steps on the tensor-core kernel too
         self.bs_prefetch = os.environ.get("PS_BS_PREFETCH", "1") != "0"
         self._bs_plan_cache: Dict[tuple, bool] = {}
+        self._norm_cols = int(_lib.lib().ps_gemm_smallm_norm_cols())
+        self._smallm_splits: Dict[Tuple[int, int], int] = {}                 # by (N, padded K)
         self.tickets = torch.zeros(ROW_BUCKETS[-1], dtype=torch.int32, device=device)      # one per sequence, zero between launches
         self.sel_counts: Dict[str, int] = {"tc_resident": 0, "tc_streamed": 0, "stream": 0, "gemm": 0}   # projection calls per kernel
         self.fallbacks: Dict[str, int] = {}
@@ -283,16 +285,17 @@ class CudaOps(OpTrace):
         if W.rowmajor_bf16 is not None and M <= 64 and W.N % 2 == 0:
             # batched decode: swap-AB split-K weight-streaming GEMM (gemm_smallm.cu)
             L = _lib.lib()
-            L.ps_gemm_smallm_splits.restype = ctypes.c_int
-            splits = L.ps_gemm_smallm_splits(c_int(W.N), c_int(kp))
+            splits = self._smallm_splits.get((W.N, kp))
+            if splits is None:
+                splits = self._smallm_splits[W.N, kp] = int(L.ps_gemm_smallm_splits(c_int(W.N), c_int(kp)))
             # one buffer per power of two: a larger step must not free what a captured step of fewer rows writes to
             cap = 1 << max(22, (splits * M * W.N - 1).bit_length())
             part = self.ws.get(("smallm_partial", cap))
             if part is None:
                 part = self.ws[("smallm_partial", cap)] = torch.empty(cap, dtype=torch.float32, device=self.device)
             normed = None
-            if (norm_next is not None and epi == EPI_RESIDUAL and not out_f32 and W.N % 4 == 0 and W.N <= L.ps_gemm_smallm_norm_cols()
-                    and all(t.stride(0) % 4 == 0 and t.data_ptr() % 8 == 0 for t in (out, residual))):
+            if (norm_next is not None and epi == EPI_RESIDUAL and not out_f32 and W.N % 4 == 0 and W.N <= self._norm_cols
+                    and not (out.stride(0) | residual.stride(0)) & 3 and not (out.data_ptr() | residual.data_ptr()) & 7):
                 normed = norm_next.rows = self.buf(norm_next.name, M, W.N)
             _lib.call("ps_gemm_smallm_normed", ptr(a), c_int(a.stride(0)), ptr(wd), c_int(kp), c_int(M), c_int(W.N), c_int(kp), c_int(epi),
                       ptr(residual), c_int(residual.stride(0) if residual is not None else 0), ptr(out), c_int(out.stride(0)),

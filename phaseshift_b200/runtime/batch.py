@@ -14,6 +14,8 @@ from typing import List, Optional, Sequence
 import numpy as np
 import torch
 
+from ..core.native import runtime
+
 ROW_BUCKETS = (1, 2, 4, 8, 16, 32, 64, 128, 256, 512, 1024, 2048)
 
 
@@ -51,10 +53,12 @@ class StepBatch:
         self.max_rows, self.max_seqs, self.device = max_rows, max_seqs, device
         use_pin = (device.type == "cuda") if pinned is None else pinned
         n_int = 3 * max_rows + 4 * max_seqs + 2 * max_rows    # ids, slot, pos | seq descs | output rows | pos of short sequences' rows
-        self.h_int = torch.zeros(n_int, dtype=torch.int32, pin_memory=use_pin)
-        self.h_samp = torch.zeros(max_rows * SAMPLING_ROW_DTYPE.itemsize, dtype=torch.uint8, pin_memory=use_pin)
-        self.d_int = torch.zeros(n_int, dtype=torch.int32, device=device)
-        self.d_samp = torch.zeros_like(self.h_samp, device=device)
+        # one buffer for the integers and the sampling rows behind them, so that a step's description is one copy
+        ints, samp = -(-n_int * 4 // 16) * 16, max_rows * SAMPLING_ROW_DTYPE.itemsize
+        self.h_all = torch.zeros(ints + samp, dtype=torch.uint8, pin_memory=use_pin)
+        self.d_all = torch.zeros(ints + samp, dtype=torch.uint8, device=device)
+        self.h_int, self.h_samp = self.h_all[:n_int * 4].view(torch.int32), self.h_all[ints:]
+        self.d_int, self.d_samp = self.d_all[:n_int * 4].view(torch.int32), self.d_all[ints:]
         self.n_rows = self.n_seqs = self.n_out = 0
         self.max_visible = 1
         # graph_static: the step is replayed from a captured CUDA graph, so launch geometry must not
@@ -72,44 +76,15 @@ class StepBatch:
         # (the per-row attention kernel leaves those rows' outputs alone: the tiled kernel of the same step wrote them) and
         # -1 for padding rows
         self.row_pos_short = self.d_int[o:o + max_rows]
-        self._np = self.h_int.numpy()
         self._np_samp = self.h_samp.numpy().view(SAMPLING_ROW_DTYPE)
+        self._fill = runtime().fill_step
         self.seqs: List[SeqRows] = []
 
     def fill(self, seqs: Sequence[SeqRows]) -> None:
-        mr, ms = self.max_rows, self.max_seqs
-        a = self._np
-        a[:] = 0
-        a[mr:3 * mr] = -1          # padding rows of a bucket: slot -1 / position -1, skipped by the kernels
-        short0 = 3 * mr + 4 * ms + mr
-        a[short0:short0 + mr] = -1
-        r = 0
-        n_out = 0
-        max_vis = 1
-        if len(seqs) > ms:
-            raise ValueError("too many sequences for this batch")
-        for i, s in enumerate(seqs):
-            n = len(s.token_ids)
-            if r + n > mr:
-                raise ValueError("too many rows for this batch")
-            a[r:r + n] = np.asarray(s.token_ids, dtype=np.int32)
-            a[mr + r:mr + r + n] = s.slot
-            a[2 * mr + r:2 * mr + r + n] = np.arange(s.pos_start, s.pos_start + n, dtype=np.int32)
-            a[short0 + r:short0 + r + n] = a[2 * mr + r:2 * mr + r + n] if n <= self.SHORT_SEQ_ROWS else -2
-            a[3 * mr + 4 * i:3 * mr + 4 * i + 4] = (r, n, s.slot, s.pos_start)
-            for j, orow in enumerate(s.output_rows):
-                a[3 * mr + 4 * ms + n_out] = r + orow
-                sp = self._np_samp[n_out]
-                sp["mode"] = 1 if s.temperature <= 0.0 else 2
-                sp["temperature"], sp["top_p"], sp["top_k"] = s.temperature, s.top_p, s.top_k
-                sp["seed"], sp["sample_index"] = s.seed, s.sample_index + j
-                n_out += 1
-            max_vis = max(max_vis, s.pos_start + n)
-            r += n
-        self.n_rows, self.n_seqs, self.n_out, self.max_visible = r, len(seqs), n_out, max_vis
-        # output row i is step row i for every i (a pure decode batch): the output gather is the identity
-        self.identity_out = n_out == r and bool(np.array_equal(a[3 * mr + 4 * ms:3 * mr + 4 * ms + n_out],
-                                                               np.arange(n_out, dtype=np.int32)))
+        self.n_rows, self.n_out, self.max_visible, self.identity_out = self._fill(
+            self.h_int.data_ptr(), self.h_samp.data_ptr(), self.max_rows, self.max_seqs, self.SHORT_SEQ_ROWS, seqs)
+        # (identity_out: output row i is step row i for every i -- a pure decode batch -- so the output gather is the identity)
+        self.n_seqs = len(seqs)
         self.seqs = list(seqs)
 
     @property
@@ -117,8 +92,7 @@ class StepBatch:
         return self.max_context if self.graph_static else self.max_visible
 
     def upload(self) -> None:
-        self.d_int.copy_(self.h_int, non_blocking=True)
-        self.d_samp.copy_(self.h_samp, non_blocking=True)
+        self.d_all.copy_(self.h_all, non_blocking=True)
 
     def h2d_bytes(self) -> int:
-        return self.h_int.numel() * 4 + self.h_samp.numel()
+        return self.h_all.numel()

@@ -109,6 +109,12 @@ class Engine:
             from ..core.arena import ArenaSet
             self.arenas = ArenaSet(int(arena_gib * (1 << 30)), self.device.index or 0)
         self.state = ModelState(self.cfg, state_cfg, self.device, self.ops.act_dtype, geo, arenas=self.arenas)
+        if self.device.type == "cuda":
+            # both status words side by side, so that a step reads them back in one copy
+            self.status_pair = torch.zeros(2, dtype=torch.int32, device=self.device)
+            self.state.status = self.status_pair[0:1]
+            if hasattr(self.ops, "status"):
+                self.ops.status = self.status_pair[1:2]
         self._arm_checked_limits()
         self.runner = self.family.runner(weights, self.state, self.ops, tp)
         self.tp = tp
@@ -512,9 +518,7 @@ class Engine:
         if self.device.type == "cuda":
             if out.tokens is not None and n_out:
                 self.h_tokens[:n_out].copy_(out.tokens[:n_out], non_blocking=True)
-            self.h_status[0:1].copy_(self.state.status, non_blocking=True)
-            if ops_status is not None:
-                self.h_status[1:2].copy_(ops_status, non_blocking=True)
+            self.h_status.copy_(self.status_pair, non_blocking=True)
             if read_back is not None:
                 self.h_extra[:read_back.numel()].copy_(read_back, non_blocking=True)
             torch.cuda.current_stream().synchronize()
