@@ -49,8 +49,8 @@ __global__ void __launch_bounds__(256) gdn_rows_kernel(const GdnArgs a) {
     constexpr int R = DK / RG;          // rows per thread
     constexpr int CH = 2 * DK + DV;     // conv channels owned by this head
     __shared__ float s_q[DK], s_k[DK], s_v[DV], s_red[32], s_red4[192];
-    __shared__ float s_part[RG][DV], s_partq[RG][DV];
-    __shared__ float s_vec[DV];
+    __shared__ __align__(16) float s_part[RG][DV], s_partq[RG][DV];      // float4 accesses
+    __shared__ __align__(16) float s_vec[DV];
 
     const int h = blockIdx.x;
     const GdnSeqDesc sd = a.seqs[blockIdx.y];
