@@ -7,12 +7,15 @@
 // partial sums [split, M, N] and a second tiny kernel adds the splits in a fixed order (deterministic) and
 // applies the residual / SwiGLU / dtype epilogue.  Accumulators live in tensor memory; epilogue warps read
 // them with `tcgen05.ld` (lane = weight row, column = batch row), so the partial stores are coalesced.
+// The tensor core drops what falls below an accumulator's last bit, so the error grows with the number of products added to one
+// accumulator: each CTA keeps two, one for either half of its run of K, and adds them in 32 bits.  With one accumulator a run of 80
+// k-iterations (34816 x 5120) was 5.6e-6 off 64 bits, one of 20 (18432 x 2560) 1.3e-6; with two 2.7e-6 and 6.0e-7 (times the same).
 // All mbarrier waits are bounded; a timeout sets PS_DEV_WAIT_TIMEOUT, frees the tensor memory and returns.
 //
 // A decoding step is a chain of about five such products per layer, 3 to 15 us of weights each, so what lies between them counts: all
 // kernels here are launched programmatically, the product asks for its first 128 KB of weights per SM before its rows exist, and the
 // reduction of a residual product norms the rows for the next one (gemm_smallm_norm_kernel).
-// May a product that starts early hold what its predecessors need?  It takes 64 columns of tensor memory and 97 KB; a predecessor
+// May a product that starts early hold what its predecessors need?  It takes up to 128 columns of tensor memory and 97 KB; a predecessor
 // that wants more than what is left (512 columns or 200 KB: attention, CTA-pair and block-scaled GEMMs) either never triggers early
 // or fills the SM by its shared memory, so both are never resident together.
 //
@@ -57,6 +60,8 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int it0 = split * g.iters_per_split;
     const int k_iters = min(g.iters_per_split, total_iters - it0);
     const int x_bytes = g.x_box_rows * kSmBK * 2;
+    const int first_run = (k_iters + 1) / 2;                    // k-iterations of the first accumulator; the rest go to the second
+    const uint32_t acc_cols = g.nb <= 32 ? 32 : 64;
 
     cudaTriggerProgrammaticLaunchCompletion();
     // rows of the X tile beyond the fetched box must read as zero
@@ -71,7 +76,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         tc::tma_prefetch_desc(&map_x);
     }
     if (warp == 1) {
-        tc::tmem_alloc(&tmem_base_slot, 64);        // up to 64 fp32 columns x 128 lanes
+        tc::tmem_alloc(&tmem_base_slot, 2 * acc_cols);        // two accumulators of up to 64 fp32 columns x 128 lanes
         tc::tmem_relinquish();
     }
     tc::fence_before_sync();
@@ -112,10 +117,12 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 s_consumed = it + 1;
                 tc::fence_after_sync();
                 const uint32_t w_addr = tc::smem_u32(sW + s * kWBytes), x_addr = tc::smem_u32(sX + s * kXStride);
+                const uint32_t acc = it < first_run ? tmem_acc : tmem_acc + acc_cols;
+                const bool begun = it > 0 && it != first_run;
 #pragma unroll
                 for (int kk = 0; kk < kSmBK / 16; ++kk)
-                    tc::mma_bf16_ss(tmem_acc, tc::smem_desc_sw128(w_addr + kk * 32), tc::smem_desc_sw128(x_addr + kk * 32), idesc,
-                                    (it > 0 || kk > 0) ? 1u : 0u);
+                    tc::mma_bf16_ss(acc, tc::smem_desc_sw128(w_addr + kk * 32), tc::smem_desc_sw128(x_addr + kk * 32), idesc,
+                                    (begun || kk > 0) ? 1u : 0u);
                 tc::mma_commit(&empty_bar[s]);
             }
             tc::mma_commit(&acc_bar);
@@ -131,8 +138,16 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             float* dst = g.partial + (size_t)split * g.M * g.ld;
             for (int c0 = 0; c0 < g.nb; c0 += 32) {
                 uint32_t r[32];
-                if (k_iters > 0) {
-                    tc::tmem_ld_32x32(tmem_acc + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, r);
+                const uint32_t at = tmem_acc + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
+                if (k_iters > 1) {
+                    uint32_t q[32];
+                    tc::tmem_ld_32x32(at, r);
+                    tc::tmem_ld_32x32(at + acc_cols, q);
+                    tc::tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(q[j]));
+                } else if (k_iters > 0) {
+                    tc::tmem_ld_32x32(at, r);
                     tc::tmem_ld_wait();
                 } else {
 #pragma unroll
@@ -157,7 +172,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     __syncthreads();
     if (warp == 1) {
         tc::fence_after_sync();
-        tc::tmem_dealloc(tmem_acc, 64);
+        tc::tmem_dealloc(tmem_acc, 2 * acc_cols);
     }
 }
 

@@ -73,3 +73,21 @@ def test_rmsnorm_rows(rows, H, pad):
         want = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + EPS) * (one_plus + w.double())
         assert float((out[:rows, :H].double() - want).norm() / want.norm()) < 2.0 ** -8 + 1e-5
         assert bool((out[rows] == 7).all()) and bool((out[:, H:] == 7).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(32, 34816, 5120), (8, 18432, 2560), (2, 37888, 2560), (64, 20480, 5184), (5, 4096, 128), (3, 131, 64)])
+def test_smallm_sums_lose_no_more_than_half_a_run(M, N, K):
+    """Error against 64 bits of products whose CTAs have long runs of K, and of ones with a single step or none to spare."""
+    from phaseshift_b200.ops import _lib
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    N += N & 1
+    a = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * 0.02).bfloat16()
+    out = torch.empty(M, N, device="cuda")
+    _run(a, w, out)
+    ref = torch.cat([a.double() @ p.double().T for p in w.split(8192)], 1)
+    # an addition to the accumulator drops half a last place on average, 2^-25 to 2^-24 of its value; over a run the sum grows as the
+    # square root of its length, so n additions cost about n 2^-25 of the result.  A run is half of what a CTA adds up, at 4 per 64 of
+    # K; below that the 32-bit sum of a few runs and the stored result are left (2^-24 each).
+    steps = -(-(-(-K // 64)) // _lib.lib().ps_gemm_smallm_splits(ci(N), ci(K)))
+    assert float((out.double() - ref).norm() / ref.norm()) < 4 * -(-steps // 2) * 2.0 ** -25 + 4 * 2.0 ** -24
