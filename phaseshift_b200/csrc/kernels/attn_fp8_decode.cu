@@ -2,31 +2,36 @@
 //
 // Every row reads its whole cache, so the kernel is a stream over K and V that has to keep up with HBM.  The CUDA-core kernel
 // (paged_attention.cu) widens the codes into shared memory and multiplies on the FMA pipe: issue-bound at 0.11 of the measured copy
-// bandwidth (32 rows of 0.4 - 8 K tokens, 24 heads on 4 KV heads of 256: 418 us for 270 MB, here 108 us, 2.5 TB/s; the last splits of
+// bandwidth (32 rows of 0.4 - 8 K tokens, 24 heads on 4 KV heads of 256: 418 us, here 117 us for 287 MB, 2.5 TB/s; the last splits of
 // the longest rows bound it).  Here each warp works for
 // itself on every fourth run of 16 tokens, straight from global memory to tensor-core fragments (mma.sync m16n8k16, f16 operands, in
 // which an E4M3 code is exact; one conversion per two codes, nothing goes through shared memory):
 //   * S = Q K^T: the query heads of the KV head are rows 0-7 of A.  The order of the head's dimensions along K of the product is free
 //     (the same on both sides), so that a lane's fragments are 16 consecutive codes of one token: one load, and 8 bytes of Q.
-//     Q is bf16: scaled by a power of two per head it is exact in f16 down to 2^-28 of the head's largest entry.
-//   * softmax in 32 bits, online per warp.  The value row's scale 2^e f joins the weight: w = 2^(s + e - m) f, m the largest s + e.
-//   * O += P V: w is split into two f16 terms (22 bits; the largest w is 2^12 to 2^13, so that what lies 2^-36 below it still counts), the high
+//     Q is bf16: scaled by a power of two per head it is exact in f16 down to 2^-30 of the head's largest entry.
+//   * softmax in 32 bits, online per warp.  The value row's scale 2^e f joins the weight: w = exp(s) 2^e f over the largest such product.
+//   * O += P V: w is split into two f16 terms (23 bits; the largest w is 2^12 to 2^14, so that what lies 2^-36 below it still counts), the high
 //     one in rows 0-7 of A and the low one in the unused rows 8-15 of the same product.  A lane's fragments of V are 16 consecutive
 //     codes of four tokens; a byte permutation pairs them.
+// The tensor core drops what falls below the last bit of an accumulator.  So a score is the 32-bit sum of a product per 64 dimensions, and a
+// value's accumulator goes to sums in shared memory after 16 runs.  The partial sums are as exact as those of the CUDA-core kernel, which
+// rounds every addition (against 64 bits: 2.5e-8 and 4.1e-8 with splits of 64 tokens, 1.5e-7 and 6.3e-7 with 4096; with scores kept as binary
+// logarithms and single accumulators 1.0e-7 and 7.6e-7, in 113 us).  Two terms of w show only where single tokens with scales thousands of times the others'
+// make up the result (1.3e-7 and 1.1e-7); a third product for what they drop takes 131 us.
 // The warps' results meet in shared memory; the partials are those of the merge pass of paged_attention.cu.
 // A row's arithmetic depends only on its position and the split length, not on the batch.
 #include "ps_common.cuh"
 
 namespace ps {
 
-constexpr int kF8Threads = 128, kF8Warps = kF8Threads / 32, kF8Tok = 16;
+constexpr int kF8Threads = 128, kF8Warps = kF8Threads / 32, kF8Tok = 16, kF8Chain = 16;
 
 struct AttnFp8Args {
     const __nv_bfloat16* q;                      // [rows, Hq, D]
     const uint8_t* k_pool; const uint8_t* v_pool; const float* k_scale; const float* v_scale;
     const int* block_table; int max_blocks, page_tokens, num_pages;
     const int* row_slot; const int* row_pos;
-    int Hq, Hkv; float scale_log2;
+    int Hq, Hkv; float scale;
     int split_tokens, max_splits;
     float* part_acc; float* part_ml;
     uint32_t* status;
@@ -53,10 +58,10 @@ template <int D>
 __global__ void __launch_bounds__(kF8Threads, 2) attn_fp8_decode_kernel(const AttnFp8Args a) {
     constexpr int KC = D / 64, VC = D / 128;         // 16-byte pieces of a lane per K token, per V token
     constexpr int QP = D + 8;                        // pitch of a head's queries (f16)
-    constexpr float kTop = 12.f;
+    constexpr float kLog2e = 1.4426950408889634f, kTop = 8192.f;      // 2^13: the largest f16 weight is between 2^12 and 2^14
     __shared__ __align__(16) __half s_q[8 * QP];
     __shared__ float s_qs[8];                        // score factor of a head: softmax scale / power of two of its queries
-    __shared__ __align__(16) float s_acc[kF8Warps][8][D];
+    __shared__ float s_acc[kF8Warps][8 * D];         // [2 x accumulator][lane]
     __shared__ float s_m[kF8Warps][8], s_l[kF8Warps][8];
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
@@ -81,7 +86,7 @@ __global__ void __launch_bounds__(kF8Threads, 2) attn_fp8_decode_kernel(const At
         const float up = __uint_as_float((uint32_t)(e + 127) << 23);
 #pragma unroll
         for (int i = 0; i < D / 32; ++i) s_q[h * QP + lane + 32 * i] = __float2half_rn(x[i] * up);
-        if (lane == 0) s_qs[h] = a.scale_log2 / up;
+        if (lane == 0) s_qs[h] = a.scale / up;
     }
     __syncthreads();
     const float qs = s_qs[g];
@@ -89,7 +94,8 @@ __global__ void __launch_bounds__(kF8Threads, 2) attn_fp8_decode_kernel(const At
     float o[VC * 16][4];
 #pragma unroll
     for (int i = 0; i < VC * 16; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
-    float m_s = -1.0e30f, m_w = -1.0e30f, l = 0.f;   // head g: references of the sum and of the weights, and the sum (this lane's tokens)
+    // head g: largest score and the sum of e^(s - m_s) (this lane's tokens); the weights' reference e^r_s 2^r_e, a score and a whole number
+    float m_s = -1.0e30f, l = 0.f, r_s = -1.0e30f, r_e = 0.f;
     bool bad = false;
     const size_t tok_bytes = D;
     // 16 tokens' place in the pools; false: not mapped
@@ -116,6 +122,23 @@ __global__ void __launch_bounds__(kF8Threads, 2) attn_fp8_decode_kernel(const At
             ksc[2 * n] = k2.x; ksc[2 * n + 1] = k2.y; vsc[2 * n] = v2.x; vsc[2 * n + 1] = v2.y;
         }
     };
+    // Adds the accumulators (both terms of the weights) to the lane's sums in shared memory, times `f` and `e`, and clears them.  The
+    // tensor core drops what falls below an accumulator's last bit, so no more than kF8Chain products are added to one.
+    float kept = 0.f;                                // factor of the sums in shared memory to the present reference
+    float* mine = s_acc[warp] + lane;
+    auto flush = [&](float f, float e) {
+#pragma unroll
+        for (int i = 0; i < VC * 16; ++i) {
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                float* p = mine + 32 * (2 * i + x);
+                *p = ((kept > 0.f ? *p * kept : 0.f) + (o[i][x] + o[i][x + 2])) * f * e;
+            }
+            o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+        }
+        kept = 1.f;
+    };
+    int runs = 0;
     int tok = begin + kF8Tok * warp;
     load_k(tok);
     for (; tok < end; tok += kF8Tok * kF8Warps) {
@@ -129,9 +152,10 @@ __global__ void __launch_bounds__(kF8Threads, 2) attn_fp8_decode_kernel(const At
 #pragma unroll
                 for (int i = 0; i < VC; ++i)
                     vr[n][i] = __ldg(reinterpret_cast<const uint4*>(a.v_pool + (at + 2 * t + (n & 1) + 8 * (n >> 1)) * tok_bytes + 128 * i + 16 * g));
-            float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int j = 0; j < KC; ++j)
+            for (int j = 0; j < KC; ++j) {
+                float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const uint2 qa = *reinterpret_cast<const uint2*>(s_q + g * QP + 64 * j + 16 * t + 4 * i);
@@ -142,8 +166,11 @@ __global__ void __launch_bounds__(kF8Threads, 2) attn_fp8_decode_kernel(const At
                     }
                 }
 #pragma unroll
+                for (int n = 0; n < 4; ++n) sum[n] += c[n >> 1][n & 1];
+            }
+#pragma unroll
             for (int n = 0; n < 4; ++n) {
-                s[n] = c[n >> 1][n & 1] * (qs * ksc[n]);
+                s[n] = sum[n] * (qs * ksc[n]);
                 const int e = max(-126, min(126, (int)((__float_as_uint(vsc[n]) >> 23) & 255u) - 127));
                 lv[n] = (float)e;
                 fv[n] = vsc[n] * __uint_as_float((uint32_t)(127 - e) << 23);
@@ -161,26 +188,42 @@ __global__ void __launch_bounds__(kF8Threads, 2) attn_fp8_decode_kernel(const At
                     for (int i = 0; i < VC; ++i) vr[n][i] = make_uint4(0, 0, 0, 0);
                 }
         }
-        float ms = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
-        float mw = fmaxf(fmaxf(s[0] + lv[0], s[1] + lv[1]), fmaxf(s[2] + lv[2], s[3] + lv[3]));
+        // exponents of the weights: differences of scores and of whole numbers first, so that what is rounded is small where a weight is
+        // near the largest
+        float x[4];
 #pragma unroll
-        for (int x = 1; x <= 2; x <<= 1) {
-            ms = fmaxf(ms, __shfl_xor_sync(0xffffffffu, ms, x));
-            mw = fmaxf(mw, __shfl_xor_sync(0xffffffffu, mw, x));
+        for (int n = 0; n < 4; ++n) x[n] = fmaf(s[n] - r_s, kLog2e, lv[n] - r_e);
+        float ms = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3])), top = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
+#pragma unroll
+        for (int d = 1; d <= 2; d <<= 1) {
+            ms = fmaxf(ms, __shfl_xor_sync(0xffffffffu, ms, d));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, d));
         }
-        ms = fmaxf(m_s, ms); mw = fmaxf(m_w, mw);
-        l *= f8_ex2(m_s - ms);
-        if (__any_sync(0xffffffffu, mw != m_w)) {
-            const float alpha = f8_ex2(m_w - mw);
+        ms = fmaxf(m_s, ms);
+        l *= f8_ex2((m_s - ms) * kLog2e);
+        m_s = ms;
+        const bool up = top > 0.f;
+        if (__any_sync(0xffffffffu, up)) {           // a weight above the reference
+            top = fmaxf(fmaxf(fmaf(s[0] - ms, kLog2e, lv[0]), fmaf(s[1] - ms, kLog2e, lv[1])), fmaxf(fmaf(s[2] - ms, kLog2e, lv[2]), fmaf(s[3] - ms, kLog2e, lv[3])));
+#pragma unroll
+            for (int d = 1; d <= 2; d <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, d));
+            float alpha = 1.f;
+            if (up) {
+                const float e = ceilf(top);
+                alpha = f8_ex2(fmaf(r_s - ms, kLog2e, r_e - e));
+                r_s = ms; r_e = e;
+                kept *= alpha;
+#pragma unroll
+                for (int n = 0; n < 4; ++n) x[n] = fmaf(s[n] - r_s, kLog2e, lv[n] - r_e);
+            }
 #pragma unroll
             for (int i = 0; i < VC * 16; ++i) { o[i][0] *= alpha; o[i][1] *= alpha; o[i][2] *= alpha; o[i][3] *= alpha; }
         }
-        m_s = ms; m_w = mw;
         __half hi[4], lo[4];
 #pragma unroll
         for (int n = 0; n < 4; ++n) {
-            l += f8_ex2(s[n] - m_s);
-            const float w = f8_ex2(s[n] + lv[n] - m_w + kTop) * fv[n];
+            l += f8_ex2((s[n] - m_s) * kLog2e);
+            const float w = f8_ex2(x[n]) * (fv[n] * kTop);
             hi[n] = __float2half_rn(w);
             lo[n] = __float2half_rn(w - __half2float(hi[n]));
         }
@@ -199,41 +242,34 @@ __global__ void __launch_bounds__(kF8Threads, 2) attn_fp8_decode_kernel(const At
                     mma_f16(o[16 * i + 4 * w + 2 * p + 1], a0, a1, a2, a3, e4m3x2_to_f16x2(x >> 16), e4m3x2_to_f16x2(y >> 16));
                 }
         }
+        if (++runs == kF8Chain) { flush(1.f, 1.f); runs = 0; }
     }
     if (bad) set_status(a.status, PS_DEV_BAD_INDEX);
-    // ---- this warp's sums: both terms of the weights together, on the reference of the sum
+    // ---- this warp's sums, on the reference of the scores
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
-    const float f = l > 0.f ? f8_ex2(m_w - kTop - m_s) : 0.f;
-#pragma unroll
-    for (int i = 0; i < VC; ++i)
-#pragma unroll
-        for (int b = 0; b < 16; ++b) {
-            // product columns 2t, 2t + 1 are dimensions 128 i + 32 t + b and + 16 + b
-            s_acc[warp][g][128 * i + 32 * t + b] = (o[16 * i + b][0] + o[16 * i + b][2]) * f;
-            s_acc[warp][g][128 * i + 32 * t + 16 + b] = (o[16 * i + b][1] + o[16 * i + b][3]) * f;
-        }
+    const float f = l > 0.f ? f8_ex2((r_s - m_s) * kLog2e) / kTop : 0.f, fe = r_e < -126.f ? 0.f : __uint_as_float((uint32_t)((int)r_e + 127) << 23);
+    flush(f, fe);
     if (t == 0) { s_m[warp][g] = m_s; s_l[warp][g] = l; }
     __syncthreads();
-    // ---- the four warps' sums, in warp order
-    for (int i = threadIdx.x; i < G * (D / 4); i += kF8Threads) {
-        const int h = i / (D / 4), d = i % (D / 4) * 4;
-        float m = s_m[0][h];
+    // ---- the four warps' sums, in warp order: a lane's head and four neighbouring dimensions at a time
+    if (g >= G) return;
+    float c[kF8Warps], m = s_m[0][g], sum = 0.f;
 #pragma unroll
-        for (int w = 1; w < kF8Warps; ++w) m = fmaxf(m, s_m[w][h]);
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        float sum = 0.f;
+    for (int w = 1; w < kF8Warps; ++w) m = fmaxf(m, s_m[w][g]);
 #pragma unroll
-        for (int w = 0; w < kF8Warps; ++w) {
-            const float c = f8_ex2(s_m[w][h] - m);
-            const float4 y = *reinterpret_cast<const float4*>(&s_acc[w][h][d]);
-            x.x = fmaf(c, y.x, x.x); x.y = fmaf(c, y.y, x.y); x.z = fmaf(c, y.z, x.z); x.w = fmaf(c, y.w, x.w);
-            sum = fmaf(c, s_l[w][h], sum);
-        }
-        const size_t idx = ((size_t)row * a.Hq + kvh * G + h) * a.max_splits + split;
-        *reinterpret_cast<float4*>(a.part_acc + idx * D + d) = x;
-        if (d == 0) { a.part_ml[2 * idx] = sum > 0.f ? m * 0.6931471805599453f : -3.0e38f; a.part_ml[2 * idx + 1] = sum; }
+    for (int w = 0; w < kF8Warps; ++w) { c[w] = f8_ex2((s_m[w][g] - m) * kLog2e); sum = fmaf(c[w], s_l[w][g], sum); }
+    const size_t idx = ((size_t)row * a.Hq + kvh * G + g) * a.max_splits + split;
+    for (int q = warp; q < VC * 8; q += kF8Warps) {
+        const int i = 4 * (q >> 1), x = q & 1;       // product columns 2t + x of accumulators i .. i + 3
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int w = 0; w < kF8Warps; ++w)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = fmaf(c[w], s_acc[w][32 * (2 * (i + j) + x) + lane], v[j]);
+        *reinterpret_cast<float4*>(a.part_acc + idx * D + 128 * (i >> 4) + 32 * t + 16 * x + (i & 15)) = make_float4(v[0], v[1], v[2], v[3]);
     }
+    if (warp == 0 && t == 0) { a.part_ml[2 * idx] = sum > 0.f ? m : -3.0e38f; a.part_ml[2 * idx + 1] = sum; }
 }
 
 }  // namespace ps
@@ -255,7 +291,7 @@ PS_API int ps_attn_decode_fp8(const void* q, const void* k_pool, const void* v_p
     a.q = (const __nv_bfloat16*)q; a.k_pool = (const uint8_t*)k_pool; a.v_pool = (const uint8_t*)v_pool; a.k_scale = (const float*)k_scale;
     a.v_scale = (const float*)v_scale; a.block_table = (const int*)block_table; a.max_blocks = max_blocks; a.page_tokens = page_tokens;
     a.num_pages = num_pages; a.row_slot = (const int*)row_slot; a.row_pos = (const int*)row_pos; a.Hq = Hq; a.Hkv = Hkv;
-    a.scale_log2 = sm_scale * 1.4426950408889634f; a.split_tokens = split_tokens; a.max_splits = max_splits; a.part_acc = (float*)part_acc;
+    a.scale = sm_scale; a.split_tokens = split_tokens; a.max_splits = max_splits; a.part_acc = (float*)part_acc;
     a.part_ml = (float*)part_ml; a.status = (uint32_t*)status;
     int n_splits = (max_visible + split_tokens - 1) / split_tokens;
     if (n_splits < 1) n_splits = 1;

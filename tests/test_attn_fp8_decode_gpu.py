@@ -78,3 +78,55 @@ def test_fp8_rows_beyond_the_position_do_not_count():
         pool[5, :, 11:] = 0x7f
         scale[5, :, 11:] = float("nan")
     assert torch.equal(first, ops.attention(q, AttnSpec(12, 2, 256, 1 / 16), b, kv, st, 75)) and bool(torch.isfinite(first.float()).all())
+
+
+@pytest.mark.parametrize("hq,hkv,D,positions,split,scale_q,spread", [
+    (24, 4, 256, [500, 1000, 4000], 64, 1.0, 0.0), (16, 4, 256, list(range(64, 4096, 500)), 256, 1.0, 0.0), (16, 2, 128, [100, 3000], 512, 1.0, 0.0),
+    (24, 4, 256, [500, 8000], 2048, 6.0, 0.0), (12, 2, 256, list(range(5, 1000, 40)), 64, 1.0, 3.0), (24, 4, 256, [8000], 4096, 0.05, 0.0)])
+def test_fp8_partials_are_as_exact_as_those_of_the_other_kernel(hq, hkv, D, positions, split, scale_q, spread, monkeypatch):
+    """The partial sums in 32 bits, merged in 64: short and long splits, peaked and flat weights, row scales far apart."""
+    from phaseshift_b200.models.qwen35.config import tiny_config
+    from phaseshift_b200.ops.cuda_ops import CudaOps
+    from phaseshift_b200.ops.specs import AttnSpec
+    from phaseshift_b200.runtime.batch import SeqRows, StepBatch
+    from phaseshift_b200.runtime.state import ModelState, StateConfig
+    monkeypatch.setenv("PS_ATTN_SPLIT_TOKENS", str(split))
+    dev, n, longest = torch.device("cuda:0"), len(positions), max(positions) + 1
+    cfg = tiny_config(num_attention_heads=hq, num_key_value_heads=hkv, head_dim=D)
+    st = ModelState(cfg, StateConfig(max_slots=n, max_seq_len=longest, page_tokens=16, kv_dtype="fp8_e4m3"), dev)
+    kv = next(x for x in st.kv if x is not None)
+    g = torch.Generator(device="cuda").manual_seed(split)
+    pages = torch.split(torch.arange(1, 1 + sum(p // 16 + 1 for p in positions), device=dev), [p // 16 + 1 for p in positions])
+    for s, at in enumerate(pages):
+        st.block_table[s, :len(at)] = at.to(torch.int32)
+    for pool, scale in ((kv.k, kv.k_scale), (kv.v, kv.v_scale)):
+        x = torch.randn(pool.shape, device="cuda", generator=g) + (0.3 if scale is kv.v_scale else 0.0)
+        top = x.abs().amax(-1) / 448
+        pool.view(torch.float8_e4m3fn).copy_((x / top[..., None]).to(torch.float8_e4m3fn))
+        scale.copy_(top * torch.exp2(torch.randn(top.shape, device="cuda", generator=g) * (spread if scale is kv.v_scale else 0.0)))
+    q = (torch.randn(n, hq * D, device="cuda", generator=g) * scale_q).bfloat16()
+    b = StepBatch(n, n, dev)
+    b.fill([SeqRows(s, p, [0], (0,)) for s, p in enumerate(positions)])
+    b.upload()
+    want = torch.empty(n, hq, D, dtype=torch.float64, device="cuda")
+    for s, p in enumerate(positions):
+        k, v = ((pool.view(torch.float8_e4m3fn)[pages[s]].double() * scale[pages[s]].double()[..., None]).transpose(1, 2).reshape(-1, hkv, D)[:p + 1]
+                for pool, scale in ((kv.k, kv.k_scale), (kv.v, kv.v_scale)))
+        for h in range(hq):
+            want[s, h] = torch.softmax(q[s].double().reshape(hq, D)[h] @ k[:, h * hkv // hq].T * D ** -0.5, 0) @ v[:, h * hkv // hq]
+    err = []
+    for on in (True, False):
+        ops = CudaOps(cfg, dev, max_seq_len=longest)
+        ops.attn_decode_tc, ops.exact_rows = on, True             # (the split length as it is set)
+        ops.attention(q, AttnSpec(hq, hkv, D, D ** -0.5), b, kv, st, longest)
+        torch.cuda.synchronize()
+        assert int(st.status[0]) == 0 and ops.split_tokens == split
+        part = {key: t.double().reshape(n, hq, ops.max_splits, -1) for (name, _), t in ops.ws.items() for key in ("attn_part_acc", "attn_part_ml") if name.startswith(key)}
+        got = torch.empty_like(want)
+        for s, p in enumerate(positions):
+            ml, acc = (part[key][s, :, :p // split + 1] for key in ("attn_part_ml", "attn_part_acc"))
+            w = torch.exp(ml[..., 0] - ml[..., 0].amax(1, keepdim=True))
+            got[s] = (w[..., None] * acc).sum(1) / (w * ml[..., 1]).sum(1)[:, None]
+        err.append(float((got - want).norm() / want.norm()))
+    # the same inputs and splits on both sides: 32-bit sums in another order, no less exact (0.2 to 0.95 of the other's error)
+    assert err[0] <= err[1]
