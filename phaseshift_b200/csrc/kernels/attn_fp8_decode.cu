@@ -8,7 +8,8 @@
 // which an E4M3 code is exact; one conversion per two codes, nothing goes through shared memory):
 //   * S = Q K^T: the query heads of the KV head are rows 0-7 of A.  The order of the head's dimensions along K of the product is free
 //     (the same on both sides), so that a lane's fragments are 16 consecutive codes of one token: one load, and 8 bytes of Q.
-//     Q is bf16: scaled by a power of two per head it is exact in f16 down to 2^-30 of the head's largest entry.
+//     Q is bf16: scaled by a power of two per head it is exact in f16 down to 2^-30 of the head's largest entry; what f16 drops of smaller
+//     ones is multiplied in rows 8-15 of the same product.
 //   * softmax in 32 bits, online per warp.  The value row's scale 2^e f joins the weight: w = exp(s) 2^e f over the largest such product.
 //   * O += P V: w is split into two f16 terms (23 bits; the largest w is 2^12 to 2^14, so that what lies 2^-36 below it still counts), the high
 //     one in rows 0-7 of A and the low one in the unused rows 8-15 of the same product.  A lane's fragments of V are 16 consecutive
@@ -59,7 +60,7 @@ __global__ void __launch_bounds__(kF8Threads, 2) attn_fp8_decode_kernel(const At
     constexpr int KC = D / 64, VC = D / 128;         // 16-byte pieces of a lane per K token, per V token
     constexpr int QP = D + 8;                        // pitch of a head's queries (f16)
     constexpr float kLog2e = 1.4426950408889634f, kTop = 8192.f;      // 2^13: the largest f16 weight is between 2^12 and 2^14
-    __shared__ __align__(16) __half s_q[8 * QP];
+    __shared__ __align__(16) __half s_q[16 * QP];    // the heads' queries, and behind them 2^24 times what f16 drops of them
     __shared__ float s_qs[8];                        // score factor of a head: softmax scale / power of two of its queries
     __shared__ float s_acc[kF8Warps][8 * D];         // [2 x accumulator][lane]
     __shared__ float s_m[kF8Warps][8], s_l[kF8Warps][8];
@@ -85,7 +86,12 @@ __global__ void __launch_bounds__(kF8Threads, 2) attn_fp8_decode_kernel(const At
         if (top > 0.f && top < 3.0e38f) e = max(-126, min(126, 13 - ((int)(__float_as_uint(top) >> 23) - 127)));
         const float up = __uint_as_float((uint32_t)(e + 127) << 23);
 #pragma unroll
-        for (int i = 0; i < D / 32; ++i) s_q[h * QP + lane + 32 * i] = __float2half_rn(x[i] * up);
+        for (int i = 0; i < D / 32; ++i) {
+            const __half q = __float2half_rn(x[i] * up);
+            const float r = x[i] * up - __half2float(q);
+            s_q[h * QP + lane + 32 * i] = q;
+            s_q[(8 + h) * QP + lane + 32 * i] = __float2half_rn(r * 16777216.f);
+        }
         if (lane == 0) s_qs[h] = a.scale / up;
     }
     __syncthreads();
@@ -158,15 +164,17 @@ __global__ void __launch_bounds__(kF8Threads, 2) attn_fp8_decode_kernel(const At
                 float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const uint2 qa = *reinterpret_cast<const uint2*>(s_q + g * QP + 64 * j + 16 * t + 4 * i);
+                    const __half* q = s_q + g * QP + 64 * j + 16 * t + 4 * i;
+                    const uint2 qa = *reinterpret_cast<const uint2*>(q);
+                    const uint2 qb = *reinterpret_cast<const uint2*>(q + 8 * QP);
 #pragma unroll
                     for (int n = 0; n < 2; ++n) {
                         const uint32_t w = i == 0 ? kr[n][j].x : i == 1 ? kr[n][j].y : i == 2 ? kr[n][j].z : kr[n][j].w;
-                        mma_f16(c[n], qa.x, 0u, qa.y, 0u, e4m3x2_to_f16x2(w), e4m3x2_to_f16x2(w >> 16));
+                        mma_f16(c[n], qa.x, qb.x, qa.y, qb.y, e4m3x2_to_f16x2(w), e4m3x2_to_f16x2(w >> 16));
                     }
                 }
 #pragma unroll
-                for (int n = 0; n < 4; ++n) sum[n] += c[n >> 1][n & 1];
+                for (int n = 0; n < 4; ++n) sum[n] += fmaf(1.f / 16777216.f, c[n >> 1][2 + (n & 1)], c[n >> 1][n & 1]);
             }
 #pragma unroll
             for (int n = 0; n < 4; ++n) {

@@ -130,3 +130,45 @@ def test_fp8_partials_are_as_exact_as_those_of_the_other_kernel(hq, hkv, D, posi
         err.append(float((got - want).norm() / want.norm()))
     # the same inputs and splits on both sides: 32-bit sums in another order, no less exact (0.2 to 0.95 of the other's error)
     assert err[0] <= err[1]
+
+
+def test_fp8_rows_with_query_entries_of_very_different_sizes():
+    """Small query entries that decide the scores because the keys are zero where the large ones are: 2^-24 to 2^-45 of the largest."""
+    from phaseshift_b200.models.qwen35.config import tiny_config
+    from phaseshift_b200.ops.cuda_ops import CudaOps
+    from phaseshift_b200.ops.specs import AttnSpec
+    from phaseshift_b200.runtime.batch import SeqRows, StepBatch
+    from phaseshift_b200.runtime.state import ModelState, StateConfig
+    dev, hq, hkv, D, last = torch.device("cuda:0"), 8, 2, 256, 200
+    cfg = tiny_config(num_attention_heads=hq, num_key_value_heads=hkv, head_dim=D)
+    st = ModelState(cfg, StateConfig(max_slots=1, max_seq_len=last + 1, page_tokens=16, kv_dtype="fp8_e4m3"), dev)
+    kv = next(x for x in st.kv if x is not None)
+    pages = torch.arange(1, 2 + last // 16, device=dev)
+    st.block_table[0, :len(pages)] = pages.to(torch.int32)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    for pool in (kv.k, kv.v):
+        x = torch.randn(pool.shape, device="cuda", generator=g) * 50
+        if pool is kv.k:
+            x[..., ::64] = 0
+        pool.view(torch.float8_e4m3fn).copy_(x.to(torch.float8_e4m3fn))
+    size = torch.exp2(-torch.tensor([24., 28, 30, 32, 34, 37, 40, 45], device="cuda"))[:, None]
+    q = torch.randn(hq, D, device="cuda", generator=g) * size * 2.0 ** 20
+    q[:, ::64] = 2.0 ** 20
+    # scores of about one for every head of a KV head: its heads' sizes differ, so the keys' scale suits the middle one
+    kv.k_scale.fill_(1.0)
+    kv.k_scale[:, 0], kv.k_scale[:, 1] = 2.0 ** 6, 2.0 ** 14
+    kv.v_scale.fill_(0.01)
+    q = q.reshape(1, -1).bfloat16()
+    b = StepBatch(1, 1, dev)
+    b.fill([SeqRows(0, last, [0], (0,))])
+    b.upload()
+    k, v = ((pool.view(torch.float8_e4m3fn)[pages].double() * scale[pages].double()[..., None]).transpose(1, 2).reshape(-1, hkv, D)[:last + 1]
+            for pool, scale in ((kv.k, kv.k_scale), (kv.v, kv.v_scale)))
+    ops = CudaOps(cfg, dev, max_seq_len=last + 1)
+    got = ops.attention(q, AttnSpec(hq, hkv, D, D ** -0.5), b, kv, st, last + 1).double().reshape(hq, D)
+    assert int(st.status[0]) == 0
+    for h in range(hq):
+        s = q.double().reshape(hq, D)[h] @ k[:, h * hkv // hq].T * D ** -0.5
+        want = torch.softmax(s, 0) @ v[:, h * hkv // hq]
+        # the output's rounding to bf16, and scores in 32 bits (2^-24 each for the products, their sums and the scale's factor: 2^-20 of one)
+        assert float((got[h] - want).norm() / want.norm()) < 2.0 ** -8 + 2.0 ** -20 * float(s.abs().max()), h
