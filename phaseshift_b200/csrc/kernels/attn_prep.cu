@@ -36,7 +36,7 @@ struct AttnPrepArgs {
 constexpr int kPrepWarps = 8, kPrepMaxD = 512;
 __global__ void __launch_bounds__(kPrepWarps * 32) attn_prep_kernel(const AttnPrepArgs a) {
     extern __shared__ __align__(16) double s_turn[];               // [rotary_dim / 2][2]: cosine, sine
-    __shared__ float s_vals[kPrepWarps][kPrepMaxD];
+    __shared__ __align__(16) float s_vals[kPrepWarps][kPrepMaxD];       // float2 accesses
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
     const int row = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, D = a.D, half = a.rotary_dim / 2;

@@ -18,7 +18,7 @@ struct GemmF32Args {
 };
 
 __global__ void __launch_bounds__(256) gemm_f32_kernel(GemmF32Args g) {
-    __shared__ float sa[kFK][kFT + 4], sw[kFK][kFT + 4];
+    __shared__ __align__(16) float sa[kFK][kFT + 4], sw[kFK][kFT + 4];
     const int m0 = blockIdx.y * kFT, n0 = blockIdx.x * kFT, t = threadIdx.x, tx = t & 15, ty = t >> 4;
     g.a += blockIdx.z * g.stride_a; g.w += blockIdx.z * g.stride_w; g.out += blockIdx.z * g.stride_o;
     if (g.gate != nullptr) g.gate += blockIdx.z * g.stride_g;

@@ -187,7 +187,7 @@ struct MoeGemmF32Args {
 
 // grid = (column tiles, tiles of the list at most)
 __global__ void __launch_bounds__(256) moe_gemm_f32_kernel(const MoeGemmF32Args g) {
-    __shared__ float sa[kMfK][kMfT + 4], sw[kMfK][kMfT + 4];
+    __shared__ __align__(16) float sa[kMfK][kMfT + 4], sw[kMfK][kMfT + 4];
     if ((int)blockIdx.y >= g.tiles[0]) return;
     const int4 tile = reinterpret_cast<const int4*>(g.tiles)[1 + blockIdx.y];
     const int n0 = blockIdx.x * kMfT, t = threadIdx.x, tx = t & 15, ty = t >> 4;
