@@ -28,7 +28,14 @@ struct AttnPrepArgs {
     const int* block_table; int max_blocks; int page_tokens; int num_pages; int kv_fp8;
     uint32_t* status;
     int pairs;                         // rows of qkv take 4-byte loads
+    int wide;                          // the queries and the pools take 4-byte stores
 };
+
+// Two neighbouring values rounded to bf16 at element `at`, which is even.
+__device__ __forceinline__ void prep_store2(__nv_bfloat16* dst, int at, float x, float y, int wide) {
+    if (wide) *reinterpret_cast<uint32_t*>(dst + at) = f32x2_to_bf16x2_bits(x, y);
+    else { dst[at] = f32_to_bf16(x); dst[at + 1] = f32_to_bf16(y); }
+}
 
 // grid = (CTAs per row, rows), block = 8 warps; a warp takes whole heads of the row, one after the other.  The row's rotation angles --
 // 64-bit sines and cosines, the same for every head -- are computed once per CTA: computed per head, as before, they were most of the
@@ -97,15 +104,15 @@ __global__ void __launch_bounds__(kPrepWarps * 32) attn_prep_kernel(const AttnPr
             }
         __syncwarp();
         if (kind == 0) {
-            uint32_t* dst = reinterpret_cast<uint32_t*>(a.q_out + ((size_t)row * a.Hq + head) * D);
-            for (int d = lane; d < D / 2; d += 32) dst[d] = f32x2_to_bf16x2_bits(vals[2 * d], vals[2 * d + 1]);
+            __nv_bfloat16* dst = a.q_out + ((size_t)row * a.Hq + head) * D;
+            for (int d = 2 * lane; d < D; d += 64) prep_store2(dst, d, vals[d], vals[d + 1], a.wide);
             continue;
         }
         const size_t tok = ((size_t)page * a.Hkv + head) * a.page_tokens + off;
         void* pool = kind == 1 ? a.k_pool : a.v_pool;
         if (!a.kv_fp8) {
-            uint32_t* dst = reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(pool) + tok * D);
-            for (int d = lane; d < D / 2; d += 32) dst[d] = f32x2_to_bf16x2_bits(vals[2 * d], vals[2 * d + 1]);
+            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(pool) + tok * D;
+            for (int d = 2 * lane; d < D; d += 64) prep_store2(dst, d, vals[d], vals[d + 1], a.wide);
             continue;
         }
         // coded rows: K after bf16 rounding of the turned value, V as given; the row's scale from its maximum
@@ -131,7 +138,11 @@ __global__ void __launch_bounds__(kPrepWarps * 32) attn_prep_kernel(const AttnPr
                 uint32_t w = 0;
 #pragma unroll
                 for (int e = 0; e < 4; ++e) w |= (uint32_t)f32_to_e4m3(vals[d + e] * inv) << (8 * e);
-                *reinterpret_cast<uint32_t*>(dst + d) = w;
+                if (a.wide) *reinterpret_cast<uint32_t*>(dst + d) = w;
+                else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) dst[d + e] = (uint8_t)(w >> (8 * e));
+                }
             }
             if (lane == 0) *scale = sc;
         }
@@ -155,6 +166,7 @@ PS_API int ps_attn_prep(const void* qkv, int ld_qkv, int rows, int Hq, int Hkv, 
     a.v_scale = (float*)v_scale; a.block_table = (const int*)block_table; a.max_blocks = max_blocks;
     a.page_tokens = page_tokens; a.num_pages = num_pages; a.kv_fp8 = kv_fp8; a.status = (uint32_t*)status;
     a.pairs = ld_qkv % 2 == 0 && (uintptr_t)qkv % 4 == 0;
+    a.wide = ((uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool) % 4 == 0;
     // many rows: one CTA per row; few: the heads over several, so that the row does not wait for its warps' second round
     const int ctas = rows >= 64 ? 1 : (Hq + 2 * Hkv + kPrepWarps - 1) / kPrepWarps;
     return launch_pdl(attn_prep_kernel, dim3(ctas, rows), dim3(kPrepWarps * 32), (size_t)rotary_dim * sizeof(double), stream, a);

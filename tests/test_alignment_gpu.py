@@ -1,0 +1,46 @@
+"""Rows that begin at any element: kernels with wide loads and stores take them by narrower ones and leave the same bytes."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+ci, cf = ctypes.c_int, ctypes.c_float
+
+
+def _vp(t):
+    return ctypes.c_void_p(t.data_ptr() if t is not None else None)
+
+
+def _shifted(t, by):
+    """A copy of `t` that begins `by` elements into its allocation."""
+    raw = torch.zeros(t.numel() + by, dtype=t.dtype, device=t.device)
+    raw[by:].copy_(t.reshape(-1))
+    return raw[by:].view(t.shape)
+
+
+@pytest.mark.parametrize("fmt", [0, 1])
+@pytest.mark.parametrize("rows", [3, 70])
+def test_rotation_and_append_to_rows_at_odd_addresses(fmt, rows):
+    from phaseshift_b200.ops import _lib
+    hq, hkv, D, rot, page, pages = 6, 2, 128, 64, 16, 8
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    qkv = torch.randn(rows, (2 * hq + 2 * hkv) * D, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(2, D, device="cuda", generator=g) * 0.1).bfloat16()
+    freq = 1e4 ** (-torch.arange(rot // 2, dtype=torch.float64, device="cuda") / (rot // 2))
+    slot = torch.zeros(rows, dtype=torch.int32, device="cuda")
+    pos = torch.arange(rows, dtype=torch.int32, device="cuda")
+    table = torch.arange(1, pages, dtype=torch.int32, device="cuda").view(1, -1)
+    got = []
+    for by in (0, 1):
+        q = _shifted(torch.zeros(rows, hq * D, dtype=torch.bfloat16, device="cuda"), by)
+        pool = torch.zeros(pages, hkv, page, D, dtype=torch.uint8 if fmt else torch.bfloat16, device="cuda")
+        k, v = _shifted(pool, by), _shifted(pool, by)
+        scale = torch.zeros(2, pages, hkv, page, device="cuda")
+        status = torch.zeros(1, dtype=torch.int32, device="cuda")
+        _lib.call("ps_attn_prep", _vp(_shifted(qkv, by)), ci(qkv.shape[1]), ci(rows), ci(hq), ci(hkv), ci(D), ci(rot), _vp(w[0]), _vp(w[1]), cf(1e-6), _vp(freq),
+                  _vp(slot), _vp(pos), _vp(q), _vp(k), _vp(v), _vp(scale[0]), _vp(scale[1]), _vp(table), ci(pages - 1), ci(page), ci(pages), ci(fmt), _vp(status))
+        torch.cuda.synchronize()
+        assert int(status[0]) == 0
+        got.append([q.clone(), k.clone(), v.clone(), scale])
+    assert all(torch.equal(a, b) for a, b in zip(*got)) and bool(got[0][1].float().abs().sum() > 0)
