@@ -34,8 +34,9 @@ __global__ void embedding_kernel(const int* ids, const __nv_bfloat16* table, int
 }
 
 // MXFP8 table (E4M3 codes + UE8M0 scale per 32): dequantising gather.
+// `wide_in`, `wide_out`: codes take 8-byte loads, rows of `out` 16-byte stores.
 __global__ void embedding_mxfp8_kernel(const int* ids, const uint8_t* codes, const uint8_t* scales, int vocab,
-                                       int H, __nv_bfloat16* out, int ldo, uint32_t* status, float* ssq, int ssq_ld) {
+                                       int H, __nv_bfloat16* out, int ldo, uint32_t* status, float* ssq, int ssq_ld, int wide_in, int wide_out) {
     __shared__ float red[32];
     const int r = blockIdx.x;
     const int id = ids[r];
@@ -47,7 +48,12 @@ __global__ void embedding_mxfp8_kernel(const int* ids, const uint8_t* codes, con
         uint2 c = make_uint2(0, 0);
         float sc = 0.f;
         if (ok) {
-            c = __ldg(reinterpret_cast<const uint2*>(codes + (size_t)id * H) + i);
+            const uint8_t* src = codes + (size_t)id * H + 8 * i;
+            if (wide_in) c = __ldg(reinterpret_cast<const uint2*>(src));
+            else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { c.x |= (uint32_t)src[e] << (8 * e); c.y |= (uint32_t)src[4 + e] << (8 * e); }
+            }
             sc = __uint_as_float((uint32_t)scales[(size_t)id * (H / 32) + i / 4] << 23);
         }
         uint32_t o[4];
@@ -60,7 +66,7 @@ __global__ void embedding_mxfp8_kernel(const int* ids, const uint8_t* codes, con
             ss += f.x * f.x + f.y * f.y;
         }
         __nv_bfloat16* d = out + (size_t)r * ldo + 8 * i;
-        if (ldo % 8 == 0) *reinterpret_cast<uint4*>(d) = make_uint4(o[0], o[1], o[2], o[3]);
+        if (wide_out) *reinterpret_cast<uint4*>(d) = make_uint4(o[0], o[1], o[2], o[3]);
         else {
 #pragma unroll
             for (int e = 0; e < 4; ++e) { const __nv_bfloat162 two = *reinterpret_cast<const __nv_bfloat162*>(&o[e]); d[2 * e] = two.x; d[2 * e + 1] = two.y; }
@@ -192,7 +198,8 @@ PS_API int ps_embedding_mxfp8(const void* ids, const void* codes, const void* sc
     if (rows <= 0 || (H % 32)) return (int)cudaErrorInvalidValue;
     ps::embedding_mxfp8_kernel<<<rows, 256, 0, stream>>>((const int*)ids, (const uint8_t*)codes,
                                                          (const uint8_t*)scales, vocab, H, (__nv_bfloat16*)out, ldo,
-                                                         (uint32_t*)status, (float*)ssq, ssq_ld);
+                                                         (uint32_t*)status, (float*)ssq, ssq_ld, (uintptr_t)codes % 8 == 0,
+                                                         ldo % 8 == 0 && (uintptr_t)out % 16 == 0);
     return PS_LAUNCH_CHECK();
 }
 

@@ -44,3 +44,25 @@ def test_rotation_and_append_to_rows_at_odd_addresses(fmt, rows):
         assert int(status[0]) == 0
         got.append([q.clone(), k.clone(), v.clone(), scale])
     assert all(torch.equal(a, b) for a, b in zip(*got)) and bool(got[0][1].float().abs().sum() > 0)
+
+
+@pytest.mark.parametrize("H,rows", [(32, 1), (2560, 5)])
+def test_quantised_embedding_rows_at_odd_addresses(H, rows):
+    from phaseshift_b200.ops import _lib
+    vocab = 40
+    g = torch.Generator(device="cuda").manual_seed(H)
+    codes = torch.randint(0, 256, (vocab, H), device="cuda", generator=g, dtype=torch.uint8)
+    codes[(codes & 0x7F) == 0x7F] = 0                       # (the two NaN codes)
+    scales = torch.randint(100, 140, (vocab, H // 32), device="cuda", generator=g, dtype=torch.uint8)
+    ids = torch.randint(0, vocab, (rows,), device="cuda", generator=g, dtype=torch.int32)
+    want = (codes.view(torch.float8_e4m3fn).float().view(vocab, -1, 32) * torch.exp2(scales.float() - 127)[..., None]).view(vocab, H).bfloat16()[ids.long()]
+    for c_by, o_by, pad in ((0, 0, 0), (1, 0, 0), (4, 1, 0), (0, 4, 8), (3, 0, 1)):
+        c = _shifted(codes, c_by)
+        out = _shifted(torch.full((rows, H + pad), 7.0, dtype=torch.bfloat16, device="cuda"), o_by)
+        ssq = torch.zeros(rows, device="cuda")
+        status = torch.zeros(1, dtype=torch.int32, device="cuda")
+        _lib.call("ps_embedding_mxfp8", _vp(ids), _vp(c), _vp(scales), ci(rows), ci(vocab), ci(H), _vp(out), ci(H + pad), _vp(status), _vp(ssq), ci(1))
+        torch.cuda.synchronize()
+        assert int(status[0]) == 0 and torch.equal(out[:, :H], want) and bool((out[:, H:] == 7).all())
+        # a 32-bit sum of H squares: H 2^-24 of it at most
+        assert torch.allclose(ssq.double(), want.double().pow(2).sum(1), rtol=H * 2.0 ** -24, atol=0)
