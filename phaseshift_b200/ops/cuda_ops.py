@@ -295,7 +295,8 @@ class CudaOps(OpTrace):
                 part = self.ws[("smallm_partial", cap)] = torch.empty(cap, dtype=torch.float32, device=self.device)
             normed = None
             if (norm_next is not None and epi == EPI_RESIDUAL and not out_f32 and W.N % 4 == 0 and W.N <= self._norm_cols
-                    and not (out.stride(0) | residual.stride(0)) & 3 and not (out.data_ptr() | residual.data_ptr()) & 7):
+                    and not (out.stride(0) | residual.stride(0)) & 3
+                    and not (out.data_ptr() | residual.data_ptr() | norm_next.weight.data_ptr()) & 7):
                 normed = norm_next.rows = self.buf(norm_next.name, M, W.N)
             _lib.call("ps_gemm_smallm_normed", ptr(a), c_int(a.stride(0)), ptr(wd), c_int(kp), c_int(M), c_int(W.N), c_int(kp), c_int(epi),
                       ptr(residual), c_int(residual.stride(0) if residual is not None else 0), ptr(out), c_int(out.stride(0)),

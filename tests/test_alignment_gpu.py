@@ -66,3 +66,27 @@ def test_quantised_embedding_rows_at_odd_addresses(H, rows):
         assert int(status[0]) == 0 and torch.equal(out[:, :H], want) and bool((out[:, H:] == 7).all())
         # a 32-bit sum of H squares: H 2^-24 of it at most
         assert torch.allclose(ssq.double(), want.double().pow(2).sum(1), rtol=H * 2.0 ** -24, atol=0)
+
+
+@pytest.mark.parametrize("by", [0, 1])
+def test_residual_projection_before_a_norm_whose_weights_lie_anywhere(by):
+    """The norm joins the projection's reduction where it can; other weights leave it to the next projection, which gives the same rows."""
+    from phaseshift_b200.models.qwen35.config import tiny_config
+    from phaseshift_b200.models.qwen35.weights import LinearW
+    from phaseshift_b200.ops.cuda_ops import CudaOps
+    from phaseshift_b200.ops.specs import NextNorm
+    from phaseshift_b200.quant.formats import quantize
+    dev = torch.device("cuda:0")
+    ops = CudaOps(tiny_config(), dev)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    W, V = (LinearW(quantize(torch.randn(256, 256, device="cuda", generator=g) / 16, "bf16")) for _ in range(2))
+    x, res = (torch.randn(4, 256, device="cuda", generator=g).bfloat16() for _ in range(2))
+    nxt = NextNorm(_shifted((torch.randn(256, device="cuda", generator=g) * 0.1).bfloat16(), by), 1e-6, "xn")
+    r = ops.linear(x, W, name="r", residual=res, norm_next=nxt)
+    assert (nxt.rows is None) == bool(by)
+    y = ops.linear(r, V, name="y", norm_w=nxt.weight, eps=1e-6, x_normed=nxt.rows, out_f32=True)
+    rd = (x.double() @ W.q.codes.double().T).bfloat16().double() + res.double()
+    assert float((r.double() - rd).norm() / rd.norm()) < 2.0 ** -7          # the product and the sum, each rounded to bf16 (2^-8)
+    rd = r.double()
+    want = (rd * torch.rsqrt(rd.pow(2).mean(-1, keepdim=True) + 1e-6) * (1 + nxt.weight.double())) @ V.q.codes.double().T
+    assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -8      # the normed rows, rounded to bf16
