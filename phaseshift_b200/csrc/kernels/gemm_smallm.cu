@@ -355,8 +355,12 @@ PS_API int ps_gemm_smallm_splits(int N, int K) {
     return (iters + per - 1) / per;                         // drop empty trailing splits
 }
 
+// One run of K and nothing to do with its sums: they are the output, and no scratch is needed.
+PS_API int ps_gemm_smallm_direct(int splits, int epilogue, int out_f32) { return splits == 1 && epilogue == 0 && out_f32; }
+
 // out[M,N] = epilogue(A[M,K] . W[N,K]^T) for 1 <= M <= 64; A, W bf16 row-major (lda, ldw multiples of 8,
-// 16-byte aligned bases), N even, `partial` = ps_gemm_smallm_splits(N, K) * M * N floats of scratch (16-byte aligned).
+// 16-byte aligned bases), N even, `partial` = ps_gemm_smallm_splits(N, K) * M * N floats of scratch (16-byte aligned; unused where
+// ps_gemm_smallm_direct).
 // With `norm_w` (residual epilogue, bf16 output): `normed` [M, N] bf16 receives out / rms(out) * (1 + norm_w) as well; N a multiple of
 // 4, at most ps_gemm_smallm_norm_cols(), and 8-byte aligned rows of out, residual, norm_w and normed.
 PS_API int ps_gemm_smallm_norm_cols() { return 16 * ps::kSmNormItems * ps::kSmNormThreads; }
@@ -366,7 +370,7 @@ PS_API int ps_gemm_smallm_normed(const void* a, int lda, const void* w, int ldw,
                                  void* partial, void* status, cudaStream_t stream) {
     using namespace ps;
     if (M < 1 || M > 64 || N <= 0 || (N & 1) || K <= 0 || (K % 8) || (lda % 8) || (ldw % 8) || ((uintptr_t)a % 16) ||
-        ((uintptr_t)w % 16) || partial == nullptr)
+        ((uintptr_t)w % 16))
         return (int)cudaErrorInvalidValue;
     const bool gated = epilogue == 2 || epilogue == 3 || epilogue == 5;
     if (gated && out_f32) return (int)cudaErrorInvalidValue;
@@ -381,8 +385,8 @@ PS_API int ps_gemm_smallm_normed(const void* a, int lda, const void* w, int ldw,
     g.splits = ps_gemm_smallm_splits(N, K);
     const int iters = (K + kSmBK - 1) / kSmBK;
     g.iters_per_split = (iters + g.splits - 1) / g.splits;
-    // one split and nothing to do with its sums: they are the output
-    const bool direct = g.splits == 1 && epilogue == 0 && out_f32;
+    const bool direct = ps_gemm_smallm_direct(g.splits, epilogue, out_f32);
+    if (!direct && partial == nullptr) return (int)cudaErrorInvalidValue;
     g.partial = direct ? (float*)out : (float*)partial; g.ld = direct ? ldo : N; g.status = (uint32_t*)status; g.budget = g_ps_wait_budget_cycles;
     CUtensorMap map_w, map_x;
     int err = sm_map_2d(&map_w, w, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, kSmBM);

@@ -288,11 +288,13 @@ class CudaOps(OpTrace):
             splits = self._smallm_splits.get((W.N, kp))
             if splits is None:
                 splits = self._smallm_splits[W.N, kp] = int(L.ps_gemm_smallm_splits(c_int(W.N), c_int(kp)))
-            # one buffer per power of two: a larger step must not free what a captured step of fewer rows writes to
-            cap = 1 << max(22, (splits * M * W.N - 1).bit_length())
-            part = self.ws.get(("smallm_partial", cap))
-            if part is None:
-                part = self.ws[("smallm_partial", cap)] = torch.empty(cap, dtype=torch.float32, device=self.device)
+            direct, part = bool(L.ps_gemm_smallm_direct(c_int(splits), c_int(epi), c_int(1 if out_f32 else 0))), None
+            if not direct:
+                # one buffer per power of two: a larger step must not free what a captured step of fewer rows writes to
+                cap = 1 << max(22, (splits * M * W.N - 1).bit_length())
+                part = self.ws.get(("smallm_partial", cap))
+                if part is None:
+                    part = self.ws[("smallm_partial", cap)] = torch.empty(cap, dtype=torch.float32, device=self.device)
             normed = None
             if (norm_next is not None and epi == EPI_RESIDUAL and not out_f32 and W.N % 4 == 0 and W.N <= self._norm_cols
                     and not (out.stride(0) | residual.stride(0)) & 3
@@ -303,7 +305,7 @@ class CudaOps(OpTrace):
                       c_int(1 if out_f32 else 0), ptr(norm_next.weight if normed is not None else None),
                       c_float(norm_next.eps if normed is not None else 0.0), ptr(normed), c_int(normed.stride(0) if normed is not None else 0),
                       ptr(part), ptr(self.status))
-            self.launches += 2
+            self.launches += 1 if direct else 2
             return out
         _lib.call("ps_gemm_bf16_tc", ptr(a), c_int(a.stride(0)), ptr(wd), c_int(kp), c_int(M), c_int(W.N), c_int(kp),
                   c_int(epi), ptr(residual), c_int(residual.stride(0) if residual is not None else 0), ptr(out),
