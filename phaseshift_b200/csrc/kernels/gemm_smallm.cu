@@ -415,8 +415,3 @@ PS_API int ps_gemm_smallm_normed(const void* a, int lda, const void* w, int ldw,
     const long long n = (long long)M * (N >> 1);
     return launch_pdl(gemm_smallm_reduce_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, r);
 }
-
-PS_API int ps_gemm_smallm(const void* a, int lda, const void* w, int ldw, int M, int N, int K, int epilogue, const void* residual,
-                          int ld_res, void* out, int ldo, int out_f32, void* partial, void* status, cudaStream_t stream) {
-    return ps_gemm_smallm_normed(a, lda, w, ldw, M, N, K, epilogue, residual, ld_res, out, ldo, out_f32, nullptr, 0.f, nullptr, 0, partial, status, stream);
-}
