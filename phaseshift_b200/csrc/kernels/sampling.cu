@@ -17,6 +17,7 @@ struct SampleArgs {
     const uint32_t* mask; int mask_words;   // optional [rows, mask_words]; bit set = token allowed
     const uint8_t* mask_active;             // optional [rows]
     int* out;                               // [rows]; -1 on failure / empty constraint
+    int ctas;                               // CTAs of a row
     uint32_t* status;
 };
 
@@ -89,13 +90,13 @@ struct RowCluster {
     __device__ __forceinline__ void leave() const { if (size > 1) tc::cluster_sync(); }
 };
 
-// grid = (cluster size, rows).  One CTA per row read a 152 K vocabulary in 25 us (one row), latency-bound on one SM; eight take 9.8.
+// grid = rows x a.ctas, one cluster per row.  One CTA per row read a 152 K vocabulary in 25 us (one row), latency-bound on one SM; eight take 9.8.
 __global__ void __launch_bounds__(kSampThreads) sample_kernel(const SampleArgs a) {
     __shared__ Best sh_best[32];
     __shared__ double sh_d[32];
     __shared__ double sh_slots[2][2];
-    RowCluster cl{gridDim.x, blockIdx.x, 0, sh_slots};
-    const int row = blockIdx.y;
+    RowCluster cl{(uint32_t)a.ctas, blockIdx.x % (uint32_t)a.ctas, 0, sh_slots};
+    const int row = blockIdx.x / (uint32_t)a.ctas;
     const uint32_t first = cl.rank * kSampThreads + threadIdx.x, stride = cl.size * kSampThreads;
     const SamplingRow p = a.params[row];
     const bool lead = cl.rank == 0 && threadIdx.x == 0;
@@ -213,9 +214,10 @@ PS_API int ps_sample(const void* logits, int ld, int vocab, int rows, const void
     a.mask_active = (const uint8_t*)mask_active; a.out = (int*)out; a.status = (uint32_t*)status;
     // CTAs per row: two per SM in all, and at least four thousand tokens each
     int size = 8;
-    while (size > 1 && (rows * size > 296 || vocab < 4096 * size)) size >>= 1;
+    while (size > 1 && ((long long)rows * size > 296 || vocab < 4096 * size)) size >>= 1;
+    a.ctas = size;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(size, rows); cfg.blockDim = dim3(kSampThreads); cfg.stream = stream;
+    cfg.gridDim = dim3((unsigned)rows * size); cfg.blockDim = dim3(kSampThreads); cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = size; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
