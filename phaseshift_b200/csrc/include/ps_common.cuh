@@ -160,6 +160,13 @@ __device__ __forceinline__ void set_status(uint32_t* status, uint32_t code) {
     if (status != nullptr) atomicCAS(status, 0u, code);
 }
 
+// SMs of the current device.
+inline int sm_count() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
+    return n;
+}
+
 // Launch with programmatic dependent launch allowed: the kernel may be scheduled while its stream
 // predecessor is still draining; it must call cudaGridDependencySynchronize() before touching anything
 // the predecessor wrote.  PS_PDL=0 in the environment turns the attribute off.

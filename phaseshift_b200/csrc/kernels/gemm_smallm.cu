@@ -343,10 +343,10 @@ static int sm_map_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t
 PS_API int ps_gemm_smallm_splits(int N, int K) {
     const int tiles = (N + ps::kSmBM - 1) / ps::kSmBM;
     const int iters = (K + ps::kSmBK - 1) / ps::kSmBK;
-    // as many CTAs as fit at once, two on each of 148 SMs: a few more than that and the step waits for a second round of them (with
+    // as many CTAs as fit at once, two on each SM (296 here): a few more than that and the step waits for a second round of them (with
     // the count rounded up instead, 18432 x 2560 ran as 432 CTAs and 2560 x 9216 as 300: steps of 8, 12 and 32 rows took 858, 983 and
     // 1456 us, with this rule 797, 922 and 1384)
-    int splits = 296 / tiles;
+    int splits = 2 * ps::sm_count() / tiles;
     const int max_splits = iters / 4 > 0 ? iters / 4 : 1;   // at least 4 k-iterations (64 KB of weights) per CTA
     if (splits > max_splits) splits = max_splits;
     if (splits < 1) splits = 1;

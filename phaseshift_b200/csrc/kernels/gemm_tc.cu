@@ -442,9 +442,7 @@ static int pair_tile_cols(int tiles_m, int N, int pairs) {
 }
 
 static int launch_pair(const void* a, int lda, const void* w, int ldw, const GemmArgs& g, cudaStream_t stream) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     PairArgs p;
     p.g = g;
     p.tiles_m = (g.M + kPairBM - 1) / kPairBM;

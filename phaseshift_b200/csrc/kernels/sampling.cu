@@ -214,7 +214,8 @@ PS_API int ps_sample(const void* logits, int ld, int vocab, int rows, const void
     a.mask_active = (const uint8_t*)mask_active; a.out = (int*)out; a.status = (uint32_t*)status;
     // CTAs per row: two per SM in all, and at least four thousand tokens each
     int size = 8;
-    while (size > 1 && ((long long)rows * size > 296 || vocab < 4096 * size)) size >>= 1;
+    const int room = 2 * sm_count();
+    while (size > 1 && ((long long)rows * size > room || vocab < 4096 * size)) size >>= 1;
     a.ctas = size;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)rows * size); cfg.blockDim = dim3(kSampThreads); cfg.stream = stream;

@@ -91,3 +91,12 @@ def test_smallm_sums_lose_no_more_than_half_a_run(M, N, K):
     # K; below that the 32-bit sum of a few runs and the stored result are left (2^-24 each).
     steps = -(-(-(-K // 64)) // _lib.lib().ps_gemm_smallm_splits(ci(N), ci(K)))
     assert float((out.double() - ref).norm() / ref.norm()) < 4 * -(-steps // 2) * 2.0 ** -25 + 4 * 2.0 ** -24
+
+
+def test_runs_of_k_fit_the_device_at_once():
+    from phaseshift_b200.ops import _lib
+    room = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    for N in (8, 130, 2560, 5120, 12352, 18432, 34816, 151936):
+        for K in (64, 520, 2560, 5120, 17408):
+            splits = _lib.lib().ps_gemm_smallm_splits(ci(N), ci(K))
+            assert splits == 1 or (splits <= 16 and splits * -(-N // 128) <= room)
