@@ -24,31 +24,51 @@ struct Name {
     }
 };
 
-long long to_int(PyObject* o) {
-    if (PyLong_Check(o)) {
-        const long long v = PyLong_AsLongLong(o);
-        if (v == -1 && PyErr_Occurred()) throw py::error_already_set();
-        return v;
+// A Python integer for `o`, as an assignment to an element of an integer array takes it: integers of any type, floats and texts (cut and
+// read by int()), but no arrays.  `wraps`: numpy's and torch's own integers keep their low bits, where Python's have to fit.
+py::object as_integer(PyObject* o, bool& wraps) {
+    wraps = !PyLong_Check(o);
+    PyObject* i = PyNumber_Index(o);
+    if (i == nullptr && (PyFloat_Check(o) || PyUnicode_Check(o) || !PySequence_Check(o)) && PyErr_ExceptionMatches(PyExc_TypeError)) {
+        PyErr_Clear();
+        wraps = false;
+        i = PyNumber_Long(o);
+        if (i == nullptr && PyUnicode_Check(o) && PyErr_ExceptionMatches(PyExc_ValueError)) {
+            PyErr_Clear();
+            throw py::type_error("a number is needed");
+        }
     }
-    PyObject* i = PyNumber_Index(o);                     // numpy and torch integers
     if (i == nullptr) throw py::error_already_set();
-    const long long v = PyLong_AsLongLong(i);
-    Py_DECREF(i);
-    if (v == -1 && PyErr_Occurred()) throw py::error_already_set();
-    return v;
+    return py::reinterpret_steal<py::object>(i);
 }
-int32_t to_i32(PyObject* o, const char* what) {
-    const long long v = to_int(o);
+int32_t fit_i32(PyObject* i, const char* what) {
+    const long long v = PyLong_AsLongLong(i);
+    if (v == -1 && PyErr_Occurred()) throw py::error_already_set();
     if (v < INT32_MIN || v > INT32_MAX) throw std::overflow_error(std::string(what) + " does not fit 32 bits");
     return (int32_t)v;
 }
+int32_t to_i32(PyObject* o, const char* what) {
+    if (PyLong_CheckExact(o)) return fit_i32(o, what);
+    bool wraps;
+    const py::object i = as_integer(o, wraps);
+    return wraps ? (int32_t)(uint32_t)PyLong_AsUnsignedLongLongMask(i.ptr()) : fit_i32(i.ptr(), what);
+}
 uint64_t to_u64(PyObject* o) {
-    PyObject* i = PyNumber_Index(o);
-    if (i == nullptr) throw py::error_already_set();
-    const unsigned long long v = PyLong_AsUnsignedLongLong(i);
-    Py_DECREF(i);
+    bool wraps;
+    const py::object i = as_integer(o, wraps);
+    if (wraps) return PyLong_AsUnsignedLongLongMask(i.ptr());
+    const unsigned long long v = PyLong_AsUnsignedLongLong(i.ptr());
     if (v == (unsigned long long)-1 && PyErr_Occurred()) throw py::error_already_set();
     return v;
+}
+uint32_t to_u32(PyObject* o, const char* what) {
+    bool wraps;
+    const py::object i = as_integer(o, wraps);
+    if (wraps) return (uint32_t)PyLong_AsUnsignedLongLongMask(i.ptr());
+    const long long v = PyLong_AsLongLong(i.ptr());
+    if (v == -1 && PyErr_Occurred()) throw py::error_already_set();
+    if (v < 0 || v > UINT32_MAX) throw std::overflow_error(std::string(what) + " does not fit 32 bits");
+    return (uint32_t)v;
 }
 double to_double(PyObject* o) {
     const double v = PyFloat_AsDouble(o);
@@ -67,6 +87,15 @@ struct Items {
     Py_ssize_t size() const { return PySequence_Fast_GET_SIZE(fast); }
     PyObject* operator[](Py_ssize_t i) const { return PySequence_Fast_GET_ITEM(fast, i); }
 };
+
+// A sequence's token ids are one row of numbers: a list, a tuple, a range, an array or a tensor of one dimension.
+void check_row(const py::object& o) {
+    if (PyList_CheckExact(o.ptr()) || PyTuple_CheckExact(o.ptr())) return;
+    if (PyBytes_Check(o.ptr()) || PyUnicode_Check(o.ptr())) throw py::value_error("token_ids are numbers");
+    if (PyAnySet_Check(o.ptr()) || PyDict_Check(o.ptr())) throw py::type_error("token_ids is a sequence");
+    if (PyObject_Size(o.ptr()) < 0) throw py::error_already_set();
+    if (py::hasattr(o, "ndim") && py::cast<long long>(o.attr("ndim")) != 1) throw py::value_error("token_ids has one dimension");
+}
 
 // ints: [ids | row_slot | row_pos] of `max_rows`, [max_seqs][4] descriptors, output rows and short-sequence positions of `max_rows`;
 // samp: sampling rows.  Returns (rows, output rows, largest visible length, output row i is step row i for every i).
@@ -88,11 +117,13 @@ py::tuple fill_step(uintptr_t ints, uintptr_t samp, int max_rows, int max_seqs, 
     bool identity = true;
     for (int i = 0; i < n; ++i) {
         PyObject* s = list[i];
-        const Items tok(n_ids.of(s));
+        const py::object given = n_ids.of(s);
+        check_row(given);
+        const Items tok(given);
         const int k = (int)tok.size();
         if (k > max_rows - r) throw py::value_error("too many rows for this batch");
         const int32_t sl = to_i32(n_slot.of(s).ptr(), "slot"), p0 = to_i32(n_pos.of(s).ptr(), "pos_start");
-        if (p0 > INT32_MAX - k) throw std::overflow_error("pos_start does not fit 32 bits");
+        if ((long long)p0 + k - 1 > INT32_MAX) throw std::overflow_error("pos_start does not fit 32 bits");
         for (int j = 0; j < k; ++j) {
             ids[r + j] = to_i32(tok[j], "token id");
             slot[r + j] = sl;
@@ -109,11 +140,10 @@ py::tuple fill_step(uintptr_t ints, uintptr_t samp, int max_rows, int max_seqs, 
             row.mode = t <= 0.0 ? ps::kSamplingGreedy : ps::kSamplingStochastic;
             row.temperature = (float)t;
             row.top_p = (float)to_double(n_top_p.of(s).ptr());
-            const long long top_k = to_int(n_top_k.of(s).ptr());
-            if (top_k < 0 || top_k > UINT32_MAX) throw std::overflow_error("top_k does not fit 32 bits");
-            row.top_k = (uint32_t)top_k;
+            row.top_k = to_u32(n_top_k.of(s).ptr(), "top_k");
             row.seed = to_u64(n_seed.of(s).ptr());
             row.sample_index = to_u64(n_index.of(s).ptr());
+            if (row.sample_index + (uint64_t)(rows.size() - 1) < row.sample_index) throw std::overflow_error("sample_index does not fit 64 bits");
             for (Py_ssize_t j = 0; j < rows.size(); ++j, ++n_out) {
                 outs[n_out] = r + to_i32(rows[j], "output row");
                 identity = identity && outs[n_out] == n_out;

@@ -61,3 +61,25 @@ def test_fill_matches_a_loop_over_the_requests():
 def test_fill_refuses(seqs, error):
     with pytest.raises(error):
         StepBatch(8, 2, torch.device("cpu")).fill(seqs)
+
+
+def test_fill_takes_numbers_as_an_integer_array_takes_them():
+    """Floats and texts are cut and read, numpy's integers keep their low bits, and a row may end at the last position of 32 bits."""
+    b = StepBatch(8, 4, torch.device("cpu"))
+    b.fill([SeqRows(1.0, 3.0, [1.0, 2.7, "7"], [1.0], temperature=np.float32(0.5), top_k=20.0, seed=5.0, sample_index=4.0),
+            SeqRows(np.int64(2), np.int64(9), np.array([4, 2 ** 32 + 5], dtype=np.int64), torch.tensor([1]), top_k=np.int64(-1), seed=np.int64(-2)),
+            SeqRows(0, 2 ** 31 - 1, torch.tensor([6]), (x for x in [0])), SeqRows(0, 0, np.array([3.0], dtype=np.float32))])
+    a = b.h_int.numpy()
+    assert a[:7].tolist() == [1, 2, 7, 4, 5, 6, 3] and a[8:15].tolist() == [1, 1, 1, 2, 2, 0, 0]
+    assert a[16:23].tolist() == [3, 4, 5, 9, 10, 2 ** 31 - 1, 0] and b.n_out == 3
+    s = b._np_samp
+    assert [int(x) for x in s["top_k"][:2]] == [20, 2 ** 32 - 1] and [int(x) for x in s["seed"][:2]] == [5, 2 ** 64 - 2] and int(s["sample_index"][0]) == 4
+
+
+@pytest.mark.parametrize("seqs,error", [([SeqRows(0, 0, [1, 2], (0, 1), sample_index=2 ** 64 - 1)], OverflowError), ([SeqRows(0, 2 ** 31 - 1, [1, 2])], OverflowError),
+                                        ([SeqRows(0, 0, (x for x in [1, 2]), (0,))], TypeError), ([SeqRows(0, 0, {1, 2}, (0,))], TypeError),
+                                        ([SeqRows(0, 0, {1: 2}, (0,))], TypeError), ([SeqRows(0, 0, b"ab", (0,))], ValueError),
+                                        ([SeqRows(0, 0, torch.ones(2, 1, dtype=torch.int64), (0,))], ValueError), ([SeqRows(0, 0, [np.ones(1)], (0,))], TypeError)])
+def test_fill_refuses_what_is_no_row_of_numbers(seqs, error):
+    with pytest.raises(error):
+        StepBatch(8, 4, torch.device("cpu")).fill(seqs)
