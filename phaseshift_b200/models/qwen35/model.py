@@ -122,7 +122,7 @@ class Qwen35Runner:
                 if hasattr(ops, "buf"):
                     proj = ops.buf("gdn_proj", rows, n_main + m.ba_proj.N)
                     batched = rows >= 2 and m.in_proj.rowmajor_bf16 is not None and not ops.exact_rows
-                    if batched and m.in_ba is not None:
+                    if batched and m.in_ba is not None and ops.use_tc_gemm:
                         xn = None
                         ops.linear(x, m.in_ba, name="gdn_in", norm_w=L.input_norm, eps=eps, out=proj, x_normed=x_normed)
                     elif rows <= FUSED_BA_MAX_ROWS and not batched:
