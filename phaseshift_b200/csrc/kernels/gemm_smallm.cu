@@ -355,12 +355,9 @@ PS_API int ps_gemm_smallm_splits(int N, int K) {
     return (iters + per - 1) / per;                         // drop empty trailing splits
 }
 
-// One run of K and nothing to do with its sums: they are the output, and no scratch is needed.
-PS_API int ps_gemm_smallm_direct(int splits, int epilogue, int out_f32) { return splits == 1 && epilogue == 0 && out_f32; }
-
 // out[M,N] = epilogue(A[M,K] . W[N,K]^T) for 1 <= M <= 64; A, W bf16 row-major (lda, ldw multiples of 8,
-// 16-byte aligned bases), N even, `partial` = ps_gemm_smallm_splits(N, K) * M * N floats of scratch (16-byte aligned; unused where
-// ps_gemm_smallm_direct).
+// 16-byte aligned bases), N even, `partial` = ps_gemm_smallm_splits(N, K) * M * N floats of scratch (16-byte aligned; none for one
+// run of K stored in 32 bits, whose sums are the output).
 // With `norm_w` (residual epilogue, bf16 output): `normed` [M, N] bf16 receives out / rms(out) * (1 + norm_w) as well; N a multiple of
 // 4, at most ps_gemm_smallm_norm_cols(), and 8-byte aligned rows of out, residual, norm_w and normed.
 PS_API int ps_gemm_smallm_norm_cols() { return 16 * ps::kSmNormItems * ps::kSmNormThreads; }
@@ -385,7 +382,7 @@ PS_API int ps_gemm_smallm_normed(const void* a, int lda, const void* w, int ldw,
     g.splits = ps_gemm_smallm_splits(N, K);
     const int iters = (K + kSmBK - 1) / kSmBK;
     g.iters_per_split = (iters + g.splits - 1) / g.splits;
-    const bool direct = ps_gemm_smallm_direct(g.splits, epilogue, out_f32);
+    const bool direct = g.splits == 1 && epilogue == 0 && out_f32;
     if (!direct && partial == nullptr) return (int)cudaErrorInvalidValue;
     g.partial = direct ? (float*)out : (float*)partial; g.ld = direct ? ldo : N; g.status = (uint32_t*)status; g.budget = g_ps_wait_budget_cycles;
     CUtensorMap map_w, map_x;

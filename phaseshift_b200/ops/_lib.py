@@ -97,12 +97,13 @@ _INTS: Dict[int, ctypes.c_int] = {}
 def c_int(v: int) -> ctypes.c_int:
     if type(v) is not int:               # (4.0 and True would find 4 and 1)
         return ctypes.c_int(v)
-    o = _INTS.get(v)
-    if o is None:
+    try:
+        return _INTS[v]
+    except KeyError:
         if len(_INTS) >= 1 << 16:
             _INTS.clear()
         o = _INTS[v] = ctypes.c_int(v)
-    return o
+        return o
 
 
 c_float = ctypes.c_float

@@ -288,7 +288,7 @@ class CudaOps(OpTrace):
             splits = self._smallm_splits.get((W.N, kp))
             if splits is None:
                 splits = self._smallm_splits[W.N, kp] = int(L.ps_gemm_smallm_splits(c_int(W.N), c_int(kp)))
-            direct, part = bool(L.ps_gemm_smallm_direct(c_int(splits), c_int(epi), c_int(1 if out_f32 else 0))), None
+            direct, part = splits == 1 and epi == EPI_STORE and out_f32, None         # (the kernel's sums are the output)
             if not direct:
                 # one buffer per power of two: a larger step must not free what a captured step of fewer rows writes to
                 cap = 1 << max(22, (splits * M * W.N - 1).bit_length())
