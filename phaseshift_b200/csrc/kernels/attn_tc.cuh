@@ -284,8 +284,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         }
     } else if (warp == 10 || warp == 11) {
         // ------------------------------------------------ score issuers: warp 10 issues S(t) for even t, warp 11 for odd t.
-        // A tcgen05.mma costs its issuing thread about 80 cycles whatever its size, and a 128 x 64 x 16 product is only 32
-        // cycles of tensor work, so one thread cannot keep the pipe fed; two threads take turns.
+        // Two issuers because a tcgen05.mma under `lane == 0` cost its thread about 80 cycles whatever its size, where a 128 x 64 x 16
+        // product is 32 cycles of tensor work; under elect.sync an instruction costs a few, and one issuer has not been tried since.
         if (tc::elect_one()) {
             constexpr uint32_t idesc_s = tc::idesc_bf16_f32(kTcRows, kTcTok);
             const int b = warp - 10;

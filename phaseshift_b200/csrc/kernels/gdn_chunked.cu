@@ -13,8 +13,8 @@
 //   1. gdn_chunk_prep : one CTA per (chunk, value head): causal depthwise conv (kernel 4) + SiLU with the
 //      taps sliding through registers, L2 normalisation (q also scaled by Dk^-0.5), beta = sigmoid(b),
 //      g = -exp(A_log) softplus(a + dt_bias); then A and QKd from K K^T and Q K^T on the tensor cores, T by
-//      forward substitution on the identity (one thread per column, out of registers), W and U as
-//      tensor-core products with T, and the decayed operands Qd = D q, Kd = (D_C/D_s) k, written to scratch.
+//      forward substitution in the four 16 x 16 diagonal blocks (one thread per column, out of registers) and
+//      -T_22 A_21 T_11 below them, for blocks of 16 and then of 32 rows, W and U as tensor-core products with T, and the decayed operands Qd = D q, Kd = (D_C/D_s) k, written to scratch.
 //   2. gdn_history : stores the raw inputs of each sequence's last rows in the conv ring (a separate
 //      launch so no CTA reads history that another CTA of the same step is overwriting).
 //   3. gdn_chunk_scan_umma : one CTA per (sequence, value head, 64-column slice of Dv) walks the chunks:
@@ -822,7 +822,9 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_tc_kernel(const GdnScanArg
 // Warps 0-7: lane quadrant (warp & 3), columns 32 (warp >> 2) .. + 31; warp 8: copies; warp 9: products.
 // Rounding as in the mma.sync scan it replaces, which took 5.2 us per chunk (1500 of 9800 cycles to issue copies twice, 2700 and 2500
 // for the large products, bound by fragment loads from shared memory) and now takes 3.3 us.  2048 rows: 165 us before, 106 now with 32
-// heads, 169 and 115 with 48 (64 and 96 CTAs).  What bounds a chunk: fetching its 128 KB of tiles, of which none has a second buffer.
+// heads, 169 and 115 with 48 (64 and 96 CTAs).  What bounds it: too few CTAs, and in each the chain of a chunk -- product, accumulator to
+// registers, operand to shared memory, barrier, next product -- at 6500 cycles with the tensor pipe 17 % and DRAM 29 % busy.  Fetching the
+// 128 KB of tiles is not the bound: with second buffers for them the scan took 105 us instead of 106.
 template <int DK, int DV>
 __global__ void __launch_bounds__(320, 1) gdn_chunk_scan_umma_kernel(const GdnScanArgs a) {
     static_assert(DK == 128 && kChunk == 64 && kSlice == 64, "the tiles' row counts");

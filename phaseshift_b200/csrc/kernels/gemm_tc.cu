@@ -104,9 +104,10 @@ __device__ __forceinline__ void gemm_store_32(const GemmArgs& g, int row, int co
     }
 }
 
-// BN x kGemmStages x CTAs per SM: <128, 3, 2> up to K = 1024, <128, 4, 1> for N < 256 (everything larger goes to CTA pairs, below);
-// <32, 5, 2> for M <= 128 (batched decode on resident bf16 weights), where the problem is a weight stream: narrow N tiles give every SM a slice even
-// when N is 5120, and two co-resident CTAs per SM keep ~40 KB of weights in flight without wave quantisation.
+// BN x kGemmStages x CTAs per SM, in this order: <32, 5, 2> for M <= 128 and N >= 512 (on resident bf16 weights: more rows than the few-row
+// GEMM takes), where the problem is a weight stream: narrow N tiles give every SM a slice even when N is 5120, and two co-resident CTAs per SM
+// keep ~40 KB of weights in flight without wave quantisation; <128, 3, 2> up to K = 1024; CTA pairs (below) for M > 128 and N >= 256;
+// <128, 4, 1> for what is left: N < 256, and M <= 128 with N < 512.
 template <int BN, int kGemmStages, int kMinBlocks>
 __global__ void __launch_bounds__(kGemmThreads, kMinBlocks)
 gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,

@@ -519,11 +519,12 @@ class CudaOps(OpTrace):
             split_tokens = max(split_tokens, -(-(-(-max_visible // want)) // 32) * 32)
         pacc = self.buf("attn_part_acc" + geom, rows, hq * self.max_splits * D, torch.float32)
         pml = self.buf("attn_part_ml" + geom, rows, hq * self.max_splits * 2, torch.float32)
-        # Decode / verify rows on the tensor cores: bf16 pages, head dim 256, every sequence handled here has at most 16 rows
+        # Decode / verify rows on the tensor cores: bf16 pages, head dims of whole 64s, every sequence handled here has at most 16 rows
         # (the query heads that share a KV head are packed into one MMA tile).  A row's result does not depend on the other
         # rows of its tile (every tile row has its own scores, reference maximum and accumulator lane), so Exact mode -- whose
-        # verified rows must reproduce single-row decoding bit for bit -- uses it as well.  FP8 pages and other shapes keep the
-        # per-row kernel.  PS_ATTN_DECODE=legacy switches it off.
+        # verified rows must reproduce single-row decoding bit for bit -- uses it as well.  FP8 pages of head dims 128 and 256
+        # have their own kernel below (ps_attn_decode_fp8); other shapes keep the per-row kernel.  PS_ATTN_DECODE=legacy
+        # switches both off.
         if (self.attn_decode_tc and D % 64 == 0 and st.kv_fmt == 0 and st.sc.page_tokens in (16, 32, 64) and hq // hkv <= 8
                 and not (kv.k is kv.v and (spec.bias is not None or spec.temp_coef != 0.0))
                 and (b.graph_static or row_pos is b.row_pos_short or all(len(sq.token_ids) <= 16 for sq in b.seqs))):
