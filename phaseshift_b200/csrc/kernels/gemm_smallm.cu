@@ -8,8 +8,9 @@
 // applies the residual / SwiGLU / dtype epilogue.  Accumulators live in tensor memory; epilogue warps read
 // them with `tcgen05.ld` (lane = weight row, column = batch row), so the partial stores are coalesced.
 // The tensor core drops what falls below an accumulator's last bit, so the error grows with the number of products added to one
-// accumulator: each CTA keeps two, one for either half of its run of K, and adds them in 32 bits.  With one accumulator a run of 80
-// k-iterations (34816 x 5120) was 5.6e-6 off 64 bits, one of 20 (18432 x 2560) 1.3e-6; with two 2.7e-6 and 6.0e-7 (times the same).
+// accumulator: a CTA with more than kSmRun k-iterations keeps two, one for either half of its run of K, and adds them in 32 bits (shorter
+// runs do with one: with two, 8 rows took 0.15 us longer per product).  With one accumulator a run of 80
+// k-iterations (34816 x 5120) was 5.6e-6 off 64 bits, one of 20 (18432 x 2560) 1.3e-6; with two 2.7e-6 and 6.0e-7.
 // All mbarrier waits are bounded; a timeout sets PS_DEV_WAIT_TIMEOUT, frees the tensor memory and returns.
 //
 // A decoding step is a chain of about five such products per layer, 3 to 15 us of weights each, so what lies between them counts: all
@@ -26,7 +27,7 @@
 
 namespace ps {
 
-constexpr int kSmBM = 128, kSmBK = 64, kSmThreads = 192;
+constexpr int kSmBM = 128, kSmBK = 64, kSmThreads = 192, kSmRun = 8;
 
 struct SmallMArgs {
     int M, N, K;
@@ -60,7 +61,8 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int it0 = split * g.iters_per_split;
     const int k_iters = min(g.iters_per_split, total_iters - it0);
     const int x_bytes = g.x_box_rows * kSmBK * 2;
-    const int first_run = (k_iters + 1) / 2;                    // k-iterations of the first accumulator; the rest go to the second
+    // k-iterations of the first accumulator; the rest go to the second, which runs of up to kSmRun do without
+    const int first_run = k_iters > kSmRun ? (k_iters + 1) / 2 : k_iters;
     const uint32_t acc_cols = g.nb <= 32 ? 32 : 64;
 
     cudaTriggerProgrammaticLaunchCompletion();
@@ -139,7 +141,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             for (int c0 = 0; c0 < g.nb; c0 += 32) {
                 uint32_t r[32];
                 const uint32_t at = tmem_acc + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
-                if (k_iters > 1) {
+                if (k_iters > first_run) {
                     uint32_t q[32];
                     tc::tmem_ld_32x32(at, r);
                     tc::tmem_ld_32x32(at + acc_cols, q);
