@@ -15,6 +15,8 @@ from .weights import GebuzenWeights, ParallelLayerW
 
 
 class GebuzenRunner:
+    any_rows = True          # a step computes the rows it has, not its bucket's (runtime/engine.py: _eager_rows)
+
     def __init__(self, weights: GebuzenWeights, state, ops, tp=None):
         if tp is not None and tp.size > 1:
             raise ValueError("Gebuzen models run on one rank")

@@ -24,6 +24,8 @@ FUSED_BA_MAX_ROWS = 8
 
 
 class Qwen35Runner:
+    any_rows = True          # a step computes the rows it has, not its bucket's (runtime/engine.py: _eager_rows)
+
     def __init__(self, weights: EngineWeights, state: ModelState, ops, tp=None):
         self.w, self.state, self.ops, self.tp = weights, state, ops, tp
         self.cfg: Qwen35Config = weights.cfg

@@ -89,18 +89,24 @@ class CudaOps(OpTrace):
         self._norm_cols = int(_lib.lib().ps_gemm_smallm_norm_cols())
         self._smallm_splits: Dict[Tuple[int, int], int] = {}                 # by (N, padded K)
         self.tickets = torch.zeros(ROW_BUCKETS[-1], dtype=torch.int32, device=device)      # one per sequence, zero between launches
+        # rows of the eager step that runs, and the row bucket whose buffers it takes the first rows of (equal: a buffer for every size)
+        self.step_rows = self.step_bucket = 0
         self.sel_counts: Dict[str, int] = {"tc_resident": 0, "tc_streamed": 0, "stream": 0, "gemm": 0}   # projection calls per kernel
         self.fallbacks: Dict[str, int] = {}
 
     # ------------------------------------------------------------------ workspace
     CANARY = 0xA5
     CANARY_BYTES = 256
+    STEP_OUTPUTS = frozenset(("logits", "sampled", "out_hidden"))        # outlive their step: a buffer for every number of rows
 
     def buf(self, name: str, rows: int, cols: int, dtype=torch.bfloat16) -> torch.Tensor:
         key = (name, rows)
         t = self.ws.get(key)
         if t is None or t.shape[1] != cols or t.dtype != dtype:
-            if self.checked:
+            if rows == self.step_rows != self.step_bucket and name not in self.STEP_OUTPUTS:
+                # a step of fewer rows than its bucket: the first rows of the bucket's buffer, so that steps of many sizes keep one set
+                t = self.buf(name, self.step_bucket, cols, dtype)[:rows]
+            elif self.checked:
                 # checked build: every workspace sits between two guard regions that `check_canaries` inspects
                 n = rows * cols * torch.empty(0, dtype=dtype).element_size()
                 raw = torch.full((n + 2 * self.CANARY_BYTES,), self.CANARY, dtype=torch.uint8, device=self.device)

@@ -507,12 +507,15 @@ class Engine:
             out = self._run_graph(bucket, b, n_out, variant, greedy)
         else:
             self.ops.exact_rows = exact
+            run = self._eager_rows(n_rows, bucket)
+            self.ops.step_rows, self.ops.step_bucket = run, bucket
             try:
-                out = self.runner.forward(b, bucket if self.backend == "cuda" else n_rows, n_out, tap_layers=tap_layers,
+                out = self.runner.forward(b, run, n_out, tap_layers=tap_layers,
                                           gdn_log=gdn_log, gdn_to_alt=gdn_to_alt, mask=mask, mask_active=mask_active,
                                           sample=sample, **({"greedy_only": True} if greedy else {}))
             finally:
                 self.ops.exact_rows = False
+                self.ops.step_rows = self.ops.step_bucket = 0
         toks: List[int] = []
         ops_status = getattr(self.ops, "status", None)
         if self.device.type == "cuda":
@@ -552,6 +555,19 @@ class Engine:
             if hasattr(self.ops, "reset_after_error"):
                 self.ops.reset_after_error()
         return toks, out, status
+
+    EAGER_ROW_STEP = 16
+
+    def _eager_rows(self, n_rows: int, bucket: int) -> int:
+        """Rows that a step outside of a graph computes: only those it has, in whole 16s (the rows of a matrix instruction and a
+        bound on the number of shapes; up to 16 rows the buckets are as fine), where the family's kernels take any number of
+        rows.  Computing the bucket's rows instead, a prompt of 1500 tokens ran every product and norm over 2048.  Several ranks keep
+        the bucket: their exchange buffers are laid out by it."""
+        if self.backend != "cuda":
+            return n_rows
+        if n_rows <= 16 or not getattr(self.runner, "any_rows", False) or (self.tp is not None and self.tp.size > 1):
+            return bucket
+        return min(bucket, -(-n_rows // self.EAGER_ROW_STEP) * self.EAGER_ROW_STEP)
 
     def profile_step(self, rows: Sequence[SeqRows], seq_objs: Sequence[Sequence_], **kw) -> Dict[str, dict]:
         """Run one step eagerly with per-op-family device timing (ops/trace.py).  Returns name -> {calls, ms}; the
