@@ -228,11 +228,96 @@ __device__ __forceinline__ void load_act_block(const __nv_bfloat16* xr, const __
 __host__ __device__ __forceinline__ int sf_atom_off(int r, int j) { return (r & 31) * 16 + ((r >> 5) & 3) * 4 + j; }
 
 // Threads per CTA: warp 0 producer, warp 1 MMA issuer, warps 2..5 epilogue, warp 6 scale-copy issuer; the resident variant
-// adds five more warps that only help in the activation prologue (one (slot, block) pair per thread instead of two in a row).
+// adds five more warps that only help in the activation prologue (one (slot, block) pair per thread instead of two in a row), the
+// streamed variant four more epilogue warps.
 // Warp 6 issues the scale-factor copies (tcgen05.cp) one stage ahead of the MMA warp: the two instruction streams of a
 // stage (copies: ~55 cycles each, MMAs: ~86 each at N = 16) run in parallel instead of back to back in one thread.
-template <bool RES> constexpr int bs_threads() { return RES ? 384 : kBsThreads + 32; }
+template <bool RES> constexpr int bs_threads() { return RES ? 384 : kBsThreads + 32 + 128; }
 template <bool RES> constexpr int bs_group() { return RES ? 2 : 1; }      // K-panels per pipeline stage
+
+// Staging of the streamed epilogue: each half of the tile's batch rows in blocks of 32, all but the last at once (32-bit words: a feature of
+// two neighbouring rows), then the last ones.
+constexpr int bs_staging_bytes(int nb) { return 2 * (nb / 64 - 1) * 16 * 128 * 4; }
+// Position of feature f inside a staged row pair: 16-byte pieces permuted so that both the lanes that write neighbouring features and those
+// that read every fourth piece meet different banks.
+__device__ __forceinline__ int bs_staged(int f) { const int c = f >> 2; return ((c ^ ((c >> 2) & 7)) << 2) | (f & 3); }
+
+// Eight neighbouring bf16 outputs of batch row m from column n0 on, with the residual added, to their row or to the rank that owns it.
+__device__ __forceinline__ void bs_store_piece(const BsArgs& g, int m, int n0, int n_lim, uint32_t (&w)[4]) {
+    if (m >= g.M || n0 >= n_lim) return;
+    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(g.out) + (size_t)m * g.ldo + n0;
+    if (g.rs.size > 1) {
+        // tensor parallel: the piece goes to the rank that owns row m (peer store)
+        const int owner = m / g.rs.rpr;
+        dst = g.rs.recv[owner] + ((size_t)g.rs.rank * g.rs.rpr + (m - owner * g.rs.rpr)) * g.rs.ld + n0;
+    }
+    const bool full = n0 + 8 <= n_lim;
+    if (g.epilogue == EPI_RESIDUAL) {
+        const __nv_bfloat16* rp = g.residual + (size_t)m * g.ld_res + n0;
+        if (full && (reinterpret_cast<uintptr_t>(rp) & 15) == 0) {
+            const uint4 rv = *reinterpret_cast<const uint4*>(rp);
+            const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 a2 = bf16x2_bits_to_f32x2(w[e]), r2 = bf16x2_bits_to_f32x2(rw[e]);
+                w[e] = f32x2_to_bf16x2_bits(a2.x + r2.x, a2.y + r2.y);
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 a2 = bf16x2_bits_to_f32x2(w[e]);
+                const float r0 = n0 + 2 * e < n_lim ? bf16_to_f32(rp[2 * e]) : 0.f;
+                const float r1 = n0 + 2 * e + 1 < n_lim ? bf16_to_f32(rp[2 * e + 1]) : 0.f;
+                w[e] = f32x2_to_bf16x2_bits(a2.x + r0, a2.y + r1);
+            }
+        }
+    }
+    if (full && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+        *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (n0 + e < n_lim) dst[e] = __ushort_as_bfloat16((unsigned short)(w[e >> 1] >> (16 * (e & 1))));
+    }
+}
+__device__ __forceinline__ float bs_swiglu(float g, float u) { return __fdividef(g, 1.f + __expf(-g)) * u; }
+
+// Staged row pairs to the output: pair q of `blocks` blocks per half holds rows `row0` + half (NB / 2) + 2 (q % (16 blocks)) and the next.
+template <int NB>
+__device__ __forceinline__ void bs_write_rows(const BsArgs& g, const uint32_t* sE, int blocks, int row0, int tn, int et) {
+    const int pairs = 32 * blocks;
+    auto row_of = [&](int q) { const int h = q >= 16 * blocks ? 1 : 0; return row0 + h * (NB / 2) + 2 * (q - h * 16 * blocks); };
+    if (g.epilogue == EPI_SWIGLU) {
+        for (int i = et; i < pairs * 8; i += 256) {
+            const int q = i >> 3, pc = i & 7, m = row_of(q);
+            uint32_t a[4], b[4];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const uint4 x = *reinterpret_cast<const uint4*>(sE + q * 128 + bs_staged(16 * pc + 4 * p));       // (gate, up) twice, two rows each
+                const float2 g0 = bf16x2_bits_to_f32x2(x.x), u0 = bf16x2_bits_to_f32x2(x.y), g1 = bf16x2_bits_to_f32x2(x.z), u1 = bf16x2_bits_to_f32x2(x.w);
+                a[p] = f32x2_to_bf16x2_bits(bs_swiglu(g0.x, u0.x), bs_swiglu(g1.x, u1.x));
+                b[p] = f32x2_to_bf16x2_bits(bs_swiglu(g0.y, u0.y), bs_swiglu(g1.y, u1.y));
+            }
+            const int n0 = tn * (kBsTileN / 2) + 8 * pc;
+            bs_store_piece(g, m, n0, g.N >> 1, a);
+            bs_store_piece(g, m + 1, n0, g.N >> 1, b);
+        }
+        return;
+    }
+    for (int i = et; i < pairs * 16; i += 256) {
+        const int q = i >> 4, pc = i & 15, m = row_of(q);
+        uint32_t a[4], b[4];
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const uint4 x = *reinterpret_cast<const uint4*>(sE + q * 128 + bs_staged(8 * pc + 4 * p));
+            a[2 * p] = __byte_perm(x.x, x.y, 0x5410); a[2 * p + 1] = __byte_perm(x.z, x.w, 0x5410);
+            b[2 * p] = __byte_perm(x.x, x.y, 0x7632); b[2 * p + 1] = __byte_perm(x.z, x.w, 0x7632);
+        }
+        const int n0 = tn * kBsTileN + 8 * pc;
+        bs_store_piece(g, m, n0, g.N, a);
+        bs_store_piece(g, m + 1, n0, g.N, b);
+    }
+}
 
 template <int FMT, int NB, bool RES>
 __global__ void __launch_bounds__(bs_threads<RES>(), 1)
@@ -273,14 +358,17 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* sBres = smem + (size_t)g.stages * kStage;                          // resident activation codes
-    __nv_bfloat16* sEpi = reinterpret_cast<__nv_bfloat16*>(sBres);                    // streamed path: 128 x 128 bf16 output staging
+    // streamed path, bf16 outputs of one rank's own sums: eight epilogue warps, outputs staged in shared memory
+    const bool staged = !RES && !g.out_f32 && g.tp.size <= 1;
     uint32_t* sSfRes = reinterpret_cast<uint32_t*>(sBres + (size_t)g.res_slots * kBTile);   // [slot][APP][32 rows] scale words
     __shared__ __align__(8) uint64_t full_bar[kBsMaxStages], empty_bar[kBsMaxStages], acc_full[2], acc_empty[2], drain_bar;
     __shared__ __align__(8) uint64_t sf_ready[4], sf_free[4];      // scale-factor columns of a stage parity: copied / consumed
     __shared__ uint32_t tmem_base_slot;
     __shared__ volatile int s_abort;
     __shared__ int s_issued, s_consumed;
-    __shared__ float s_inv_rms[32], s_red[32 * kWarps], s_ssq[4 * 32];
+    __shared__ float s_inv_rms[32], s_red[RES ? 32 * kWarps : 1], s_ssq[4 * 32];
+    __shared__ __align__(16) float s_rs[2][RES ? 4 : NB];        // streamed path: factors of a tile's batch rows, by the segment's parity
+    __shared__ int s_last;
 
     cudaTriggerProgrammaticLaunchCompletion();
     const bool prof = g.prof != nullptr && blockIdx.x == 0;
@@ -314,7 +402,7 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         if (!RES) tc::tma_prefetch_desc(&map_x);
     } else if (threadIdx.x == 64) {
         for (int s = 0; s < stages; ++s) tc::mbar_init(&empty_bar[s], 1);
-        for (int b = 0; b < 2; ++b) { tc::mbar_init(&acc_full[b], 1); tc::mbar_init(&acc_empty[b], 4); }
+        for (int b = 0; b < 2; ++b) { tc::mbar_init(&acc_full[b], 1); tc::mbar_init(&acc_empty[b], staged ? 8 : 4); }
         tc::mbar_init(&drain_bar, 1);
         for (int b = 0; b < 4; ++b) { tc::mbar_init(&sf_ready[b], 1); tc::mbar_init(&sf_free[b], 1); }
         tc::fence_barrier_init();
@@ -675,6 +763,131 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 }
             }
         }
+    } else if (staged) {
+        // ------------------------------------------------ epilogue of the streamed path: two warps per TMEM lane quadrant (warp % 4), one
+        // for either half of the batch rows.  The accumulator (one: the scale factors take the rest of the tensor memory) is only held
+        // until its values are in registers, as bf16 pairs of rows; everything else -- staging, activation, stores -- runs under the next
+        // tile's products.  With four warps that held it until the outputs were stored, a tile of 256 rows took 22600 cycles here beside
+        // 15000 of products (34816 x 5120, 2048 rows).
+        // Control flow depends only on values that are uniform over the 256 threads, so every barrier is reached by all of them
+        // even after a wait has run out (`ok` only gates memory work).
+        const int quad = warp & 3, half = warp > 6 ? 1 : 0, et = half * 128 + (int)threadIdx.x - (half ? 224 : 64);
+        const int row_l = quad * 32 + lane;                 // feature inside the tile == TMEM lane
+        constexpr int FIRST = NB > 64 ? NB / 64 - 1 : 1;
+        uint32_t* sE = reinterpret_cast<uint32_t*>(sBres) + bs_staged(row_l);
+        auto all_sync = []() { asm volatile("bar.sync 2, 256;" ::: "memory"); };
+        int seg = 0, t, p0, p1;
+        BsSegIter S{u0, u1, P};
+        bool ok = true;
+        long long prof_ewait = 0, prof_ework = 0;
+        while (S.next(t, p0, p1)) {
+            const int buf = ACC_BUFS == 2 ? (seg & 1) : 0;
+            const int tn = t / g.tiles_m, tm = t - tn * g.tiles_m, row0 = tm * NB;
+            float* rs = s_rs[seg & 1];
+            if (et < NB) rs[et] = g.row_scale != nullptr && row0 + et < g.M ? g.out_scale * g.row_scale[row0 + et] : g.out_scale;
+            const long long te0 = prof ? clock64() : 0;
+            ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&acc_full[buf], (uint32_t)((seg / ACC_BUFS) & 1), g.budget, &s_abort)) && ok;
+            const long long te1 = prof ? clock64() : 0;
+            prof_ewait += te1 - te0;
+            tc::fence_after_sync();
+            all_sync();                                     // the factors are there, and what was staged before has been read
+            const uint32_t acc = tmem_base + (uint32_t)(buf * ACC_STRIDE) + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * (NB / 2));
+            const bool complete = p0 == 0 && p1 == P;
+            auto release = [&]() {
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&acc_empty[buf]);
+            };
+            // Tiles cut over several CTAs: every contributor stores its raw fp32 partial and bumps the tile's counter; the one that arrives
+            // last (all partials are then complete) adds them in CTA order -- the same sum whoever does it.  Nobody waits for anybody.
+            int c_first = blockIdx.x, c_last = blockIdx.x;
+            bool finisher = true;
+            if (!complete) {
+                c_first = unit_owner(g.total_units, gridDim.x, t * P);
+                c_last = unit_owner(g.total_units, gridDim.x, (t + 1) * P - 1);
+                // a CTA holds at most two cut segments: the tail of one tile (slot 0) and the head of another (slot 1)
+                float* wp = g.ws + (size_t)(2 * blockIdx.x + (p0 == 0 ? 1 : 0)) * (NB * 128) + (size_t)(half * (NB / 2)) * 128 + row_l;
+                if (ok) {
+#pragma unroll 1
+                    for (int c0 = 0; c0 < NB / 2; c0 += 32) {
+                        if (row0 + half * (NB / 2) + c0 >= g.M) break;      // columns of dead rows are never read back
+                        uint32_t r[32];
+                        tc::tmem_ld_32x32(acc + c0, r);
+                        tc::tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) wp[(size_t)(c0 + j) * 128] = __uint_as_float(r[j]);
+                    }
+                }
+                release();
+                __threadfence();
+                all_sync();
+                if (et == 0) {
+                    const uint32_t prev = atomicAdd(g.flags + t, 1u);
+                    const bool last = prev + 1u == (uint32_t)(c_last - c_first + 1);
+                    if (last) g.flags[t] = 0u;                       // ready for the next launch
+                    __threadfence();
+                    s_last = last ? 1 : 0;
+                }
+                all_sync();
+                finisher = s_last != 0;                              // (written again only after the next segment's barriers)
+            }
+            if (finisher) {
+                // 32 batch rows of this half as pairs of bf16
+                auto block = [&](int b, uint32_t (&y)[16]) {
+                    const int c0 = half * (NB / 2) + 32 * b;
+                    float v[32];
+                    if (!ok || row0 + c0 >= g.M) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = 0.f;
+                    } else if (complete) {
+                        uint32_t r[32];
+                        tc::tmem_ld_32x32(acc + 32 * b, r);
+                        tc::tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+                    } else {
+                        // the contributors' partials, this CTA's included, in CTA order
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = 0.f;
+#pragma unroll 1
+                        for (int cc = c_first; cc <= c_last; ++cc) {
+                            const float* pp = g.ws + (size_t)(2 * cc + (cc == c_first ? 1 : 0)) * (NB * 128) + (size_t)c0 * 128 + row_l;
+                            float pv[32];
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) pv[j] = __ldcg(pp + (size_t)j * 128);
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) v[j] += pv[j];
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < 32; j += 4) {
+                        const float4 f = *reinterpret_cast<const float4*>(rs + c0 + j);
+                        y[j / 2] = f32x2_to_bf16x2_bits(v[j] * f.x, v[j + 1] * f.y);
+                        y[j / 2 + 1] = f32x2_to_bf16x2_bits(v[j + 2] * f.z, v[j + 3] * f.w);
+                    }
+                };
+                uint32_t y[16];
+#pragma unroll 1
+                for (int b = 0; b < FIRST; ++b) {
+                    block(b, y);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) sE[((half * FIRST + b) * 16 + j) * 128] = y[j];
+                }
+                block(FIRST, y);
+                if (complete) release();
+                const uint32_t* staged_rows = reinterpret_cast<const uint32_t*>(sBres);
+                all_sync();
+                if (ok) bs_write_rows<NB>(g, staged_rows, FIRST, row0, tn, et);
+                all_sync();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) sE[(half * 16 + j) * 128] = y[j];
+                all_sync();
+                if (ok) bs_write_rows<NB>(g, staged_rows, 1, row0 + 32 * FIRST, tn, et);
+            }
+            ++seg;
+            if (prof) prof_ework += clock64() - te1;
+        }
+        if (prof && et == 0) { g.prof[9] = clock64(); g.prof[11] = prof_ewait; g.prof[12] = prof_ework; g.prof[13] = seg; }
     } else if (warp < 6) {
         // ------------------------------------------------ epilogue: warps 2..5 own TMEM lane quadrant (warp % 4)
         // Control flow below depends only on values that are uniform over the 128 epilogue threads, so every
@@ -703,14 +916,6 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             const long long te1 = prof ? clock64() : 0;
             prof_ewait += te1 - te0;
             ok = __all_sync(0xffffffffu, ok);           // warp-uniform: the shuffles below need every lane
-            if constexpr (!RES) {
-                // the streamed epilogue has named barriers inside its row-block loop: agree on `ok` across the four warps
-                if (!ok) s_abort = 1;
-                epi_bar_sync();
-                if (etid == 0) s_ssq[1] = s_abort == 0 ? 1.f : 0.f;
-                epi_bar_sync();
-                ok = s_ssq[1] != 0.f;
-            }
             tc::fence_after_sync();
             const uint32_t acc = tmem_base + (uint32_t)(buf * ACC_STRIDE) + lane_addr;
             const int tn = t / g.tiles_m, tm = t - tn * g.tiles_m;
@@ -755,11 +960,7 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             }
             if (finisher) {
                 const bool tp_on = g.tp.size > 1;
-                const bool staged = !RES && !g.out_f32 && !tp_on;       // bf16 output of many rows: staged through shared memory
-                bool released = false;
-                // the staged epilogue never forms the per-row sums, so it must not publish any (what is in s_ssq then is whatever
-                // the finisher test left there)
-                const bool want_ssq = g.ssq_out != nullptr && g.epilogue != EPI_SWIGLU && !staged;
+                const bool want_ssq = g.ssq_out != nullptr && g.epilogue != EPI_SWIGLU;
                 uint32_t tp_val = 0; size_t tp_par = 0;
                 if (tp_on) {
                     tp_val = g.tp.counter[t] + 1u;
@@ -782,7 +983,7 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         }
                         // all contributors' partials (this CTA's included), a few at a time so their loads overlap;
                         // added in CTA order
-                        constexpr int FB = CH == 16 ? 4 : 2;
+                        constexpr int FB = CH == 16 ? 4 : RES ? 2 : 1;
                         for (int cb = c_first; !complete && cb <= c_last; cb += FB) {
                             float pv[FB][CH];
 #pragma unroll
@@ -805,24 +1006,6 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         float rs_lane = g.out_scale;
                         if constexpr (RES) rs_lane *= s_inv_rms[(c0 + lane) & 31];
                         else if (g.row_scale != nullptr && m_base + lane < g.M) rs_lane *= g.row_scale[m_base + lane];
-                        if (staged) {
-                            // lean bodies, one per epilogue kind (no per-element mode branches): values go to the staging
-                            // block as rows of 128 (64 after SwiGLU) bf16; rows past M are staged too and never written out
-                            __nv_bfloat16* srow = sEpi + (c0 & 127) * (g.epilogue == EPI_SWIGLU ? 64 : 128);
-                            if (g.epilogue == EPI_SWIGLU) {
-#pragma unroll
-                                for (int j = 0; j < CH; ++j) {
-                                    const float yb = bf16_to_f32(f32_to_bf16(v[j] * __shfl_sync(0xffffffffu, rs_lane, j & 31)));
-                                    const float other = __shfl_xor_sync(0xffffffffu, yb, 1);
-                                    const float o = __fdividef(yb, 1.f + __expf(-yb)) * other;
-                                    if (!(lane & 1)) srow[j * 64 + (row_l >> 1)] = f32_to_bf16(o);
-                                }
-                            } else {
-#pragma unroll
-                                for (int j = 0; j < CH; ++j)
-                                    srow[j * 128 + row_l] = f32_to_bf16(v[j] * __shfl_sync(0xffffffffu, rs_lane, j & 31));
-                            }
-                        } else {
                         float resv[CH];
                         const bool use_res = g.epilogue == EPI_RESIDUAL && !tp_on;
 #pragma unroll
@@ -865,70 +1048,9 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                                 }
                             }
                         }
-                        }
-                        if (staged && (((c0 + CH) & 127) == 0 || c0 + CH >= NB || tm * NB + c0 + CH >= g.M)) {
-                            // a block of up to 128 batch rows is staged: release the accumulator if it was the last one,
-                            // then write the rows out (and add the residual) in 16-byte pieces, full row segments per warp
-                            const int rb0 = tm * NB + ((c0 + CH - 1) & ~127);
-                            const bool last_block = c0 + CH >= NB || tm * NB + c0 + CH >= g.M;
-                            if (last_block && complete) {
-                                tc::fence_before_sync();
-                                __syncwarp();
-                                if (lane == 0) tc::mbar_arrive(&acc_empty[buf]);
-                                released = true;
-                            }
-                            epi_bar_sync();
-                            const int cols = g.epilogue == EPI_SWIGLU ? 64 : 128, cpr = cols >> 3;
-                            const int n_base = g.epilogue == EPI_SWIGLU ? (tn * kBsTileN) >> 1 : tn * kBsTileN;
-                            const int n_lim = g.epilogue == EPI_SWIGLU ? g.N >> 1 : g.N;
-                            const int rcnt = min(128, g.M - rb0);
-                            __nv_bfloat16* outp = reinterpret_cast<__nv_bfloat16*>(g.out);
-                            for (int i = etid; i < rcnt * cpr; i += 128) {
-                                const int rr = i / cpr, ch = i - rr * cpr;
-                                const int m = rb0 + rr, n0 = n_base + ch * 8;
-                                if (n0 >= n_lim) continue;
-                                const uint4 sv = *reinterpret_cast<const uint4*>(sEpi + rr * cols + ch * 8);
-                                uint32_t w[4] = {sv.x, sv.y, sv.z, sv.w};
-                                __nv_bfloat16* dst = outp + (size_t)m * g.ldo + n0;
-                                if (g.rs.size > 1) {
-                                    // tensor parallel: the piece goes to the rank that owns row m (peer store)
-                                    const int owner = m / g.rs.rpr;
-                                    dst = g.rs.recv[owner] + ((size_t)g.rs.rank * g.rs.rpr + (m - owner * g.rs.rpr)) * g.rs.ld + n0;
-                                }
-                                const bool full = n0 + 8 <= n_lim;
-                                if (g.epilogue == EPI_RESIDUAL) {
-                                    const __nv_bfloat16* rp = g.residual + (size_t)m * g.ld_res + n0;
-                                    if (full && (reinterpret_cast<uintptr_t>(rp) & 15) == 0) {
-                                        const uint4 rv = *reinterpret_cast<const uint4*>(rp);
-                                        const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
-#pragma unroll
-                                        for (int e = 0; e < 4; ++e) {
-                                            const float2 a2 = bf16x2_bits_to_f32x2(w[e]), r2 = bf16x2_bits_to_f32x2(rw[e]);
-                                            w[e] = f32x2_to_bf16x2_bits(a2.x + r2.x, a2.y + r2.y);
-                                        }
-                                    } else {
-#pragma unroll
-                                        for (int e = 0; e < 4; ++e) {
-                                            const float2 a2 = bf16x2_bits_to_f32x2(w[e]);
-                                            const float r0 = n0 + 2 * e < n_lim ? bf16_to_f32(rp[2 * e]) : 0.f;
-                                            const float r1 = n0 + 2 * e + 1 < n_lim ? bf16_to_f32(rp[2 * e + 1]) : 0.f;
-                                            w[e] = f32x2_to_bf16x2_bits(a2.x + r0, a2.y + r1);
-                                        }
-                                    }
-                                }
-                                if (full && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-                                    *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
-                                } else {
-#pragma unroll
-                                    for (int e = 0; e < 8; ++e)
-                                        if (n0 + e < n_lim) dst[e] = reinterpret_cast<const __nv_bfloat16*>(w)[e];
-                                }
-                            }
-                            epi_bar_sync();             // the staging block is free again
-                        }
                     }
                 }
-                if (complete && !released) {
+                if (complete) {
                     tc::fence_before_sync();
                     __syncwarp();
                     if (lane == 0) tc::mbar_arrive(&acc_empty[buf]);
@@ -1139,7 +1261,7 @@ static bool bs_plan(int M, int N, int K, bool resident, int grid_override, BsPla
         res_bytes = (size_t)pl.res_slots * (pl.nb * 128 + T::kApp * 128);
         if (64 + 2 * grp * T::kApp * 4 + pl.res_slots * T::kApp * 4 > 512) return false;   // accumulators + 2 scale sets + resident scale columns
     }
-    if (!resident) res_bytes = 128 * 128 * 2;          // output staging block of the streamed path's epilogue
+    if (!resident) res_bytes = bs_staging_bytes(pl.nb);
     const size_t avail = kBsSmemBudget - 1024;
     if (res_bytes + 3 * (size_t)stage > avail) return false;
     pl.stages = (int)((avail - res_bytes) / stage);
