@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kStThreads, 1) linear_stream_kernel(const Line
     int consumed = 0;
     bool timed_out = false;
     constexpr bool AMAX = VARIANT == ST_ARGMAX;
-    [[maybe_unused]] unsigned long long amax_mine = 0ull;      // AMAX: this thread's best key (its batch row is threadIdx.x % MT)
+    [[maybe_unused]] unsigned long long amax_mine = 0ull;      // AMAX: this thread's best key (its batch row is threadIdx.x / 4 % MT)
     [[maybe_unused]] bool amax_bad = false;
     for (int wave_q0 = quad_begin; wave_q0 < quad_end; wave_q0 += kStWaveQuads) {
         const int wave_quads = min(kStWaveQuads, quad_end - wave_q0);
@@ -153,28 +153,32 @@ __global__ void __launch_bounds__(kStThreads, 1) linear_stream_kernel(const Line
         __syncthreads();
         // ---- combine the warps' partial sums in warp order, apply the epilogue
         if (a.tp.size <= 1) {
-            for (int i = threadIdx.x; i < wave_quads * MT; i += kStThreads) {
-                const int ql = i / MT, m = i % MT;
+            // one thread per output, all of its partial sums in flight at once (one thread per quad, a read and a write at a time, kept the
+            // CTA for a microsecond per wave); the first lane of every four has the quad's values
+            const int outputs = wave_quads * MT * R;
+            for (int i0 = 0; i0 < outputs; i0 += kStThreads) {
+                const int i = i0 + threadIdx.x, r = i % R, m = i / R % MT, ql = i / (R * MT);
+                float s = 0.f;
+                if (i < outputs) {
+                    float* pp = &partial[ql * kStWarps * (R * MT) + r * MT + m];
+                    float q[kStWarps];
+#pragma unroll
+                    for (int w2 = 0; w2 < kStWarps; ++w2) q[w2] = pp[w2 * (R * MT)];
+#pragma unroll
+                    for (int w2 = 0; w2 < kStWarps; ++w2) { s += q[w2]; pp[w2 * (R * MT)] = 0.f; }
+                    s *= a.w_gscale * s_xscale_inv[m];
+                }
                 float v[R];
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    float s = 0.f;
-#pragma unroll
-                    for (int w2 = 0; w2 < kStWarps; ++w2) {
-                        float* pp = &partial[(ql * kStWarps + w2) * (R * MT) + r * MT + m];
-                        s += *pp;
-                        *pp = 0.f;
-                    }
-                    v[r] = s * (a.w_gscale * s_xscale_inv[m]);
-                }
-                if (m < a.M) {
+                for (int j = 0; j < R; ++j) v[j] = __shfl_sync(0xffffffffu, s, (lane & ~(R - 1)) + j);
+                if (i < outputs && r == 0 && m < a.M) {
                     if constexpr (AMAX) {
 #pragma unroll
-                        for (int r = 0; r < R; ++r) {
-                            const int n = (wave_q0 + ql) * R + r;
+                        for (int j = 0; j < R; ++j) {
+                            const int n = (wave_q0 + ql) * R + j;
                             if (n < a.N) {
-                                if (!(fabsf(v[r]) <= 3.0e38f)) amax_bad = true;
-                                const unsigned long long key = amax_key(v[r], n);
+                                if (!(fabsf(v[j]) <= 3.0e38f)) amax_bad = true;
+                                const unsigned long long key = amax_key(v[j], n);
                                 if (key > amax_mine) amax_mine = key;
                             }
                         }
@@ -253,7 +257,7 @@ __global__ void __launch_bounds__(kStThreads, 1) linear_stream_kernel(const Line
         __shared__ int s_amax_last;
         if (threadIdx.x < 8) s_amax[threadIdx.x] = 0ull;
         __syncthreads();
-        if (amax_mine != 0ull) atomicMax(&s_amax[threadIdx.x % MT], amax_mine);      // a thread only ever sees row threadIdx.x % MT
+        if (amax_mine != 0ull) atomicMax(&s_amax[threadIdx.x / R % MT], amax_mine);      // (a thread only ever sees this row)
         const int any_bad = __syncthreads_or(amax_bad ? 1 : 0);
         if ((int)threadIdx.x < a.M && s_amax[threadIdx.x] != 0ull) atomicMax(&a.amax_best[threadIdx.x], s_amax[threadIdx.x]);
         if (threadIdx.x == 0 && any_bad) atomicOr(&a.amax_ctl[1], 1u);
