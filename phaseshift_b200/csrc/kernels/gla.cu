@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(256) gla_rows_kernel(const GlaArgs a) {
 
 // ------------------------------------------------------------------------------------------------ chunked form (bf16)
 constexpr int kGC = 64;                 // rows of a block
-constexpr int kGPrepThreads = 512, kGOutThreads = 256;
+constexpr int kGPrepThreads = 1024, kGOutThreads = 512;
 constexpr int kGAPitch = kGC + 4;
 
 __device__ __forceinline__ uint32_t to_tf32(float x) { uint32_t r; asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x)); return r; }
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kGPrepThreads) gla_prepare_kernel(const GlaArg
         for (int i = t; i < dk * a.rank; i += kGPrepThreads) s2[(i / a.rank) * pw + i % a.rank] = bf16_to_f32(w[i]);
         __syncthreads();
         if constexpr (DKT > 0) {
-            // a thread owns one channel and every (512 / dk)-th row: eight weights at a time in registers, a1 as broadcast vectors
+            // a thread owns one channel and every (1024 / dk)-th row: eight weights at a time in registers, a1 as broadcast vectors
             constexpr int kStep = kGPrepThreads / DKT, kRows = kGC / kStep;
             const int d = t % DKT, r0 = t / DKT;
             float z[kRows];
@@ -327,28 +327,34 @@ __global__ void __launch_bounds__(kGPrepThreads) gla_prepare_kernel(const GlaArg
     __syncthreads();
     // ---- diagonal sub-blocks, pair by pair (sums local to the sub-block suffice: only differences enter)
 #pragma unroll 1
-    for (int blk = 0; blk < 4; ++blk) {
-        const int il = (blk & 1) ? 15 - warp : warp, i = blk * 16 + il;
+    for (int pass = 0; pass < 2; ++pass) {             // a warp takes rows w and 15 - w of two sub-blocks (equal work)
+        const int blk = 2 * pass + (warp >> 4), il = pass ? 15 - (warp & 15) : warp & 15, i = blk * 16 + il;
         if constexpr (DKT > 0) {
             constexpr int kU = DKT / 32;                // consecutive channels of a lane
             const int d = lane * kU;
             float qi[kU], bi[kU];
 #pragma unroll
             for (int u = 0; u < kU; ++u) { qi[u] = sQ[i * PQ + d + u]; bi[u] = sB[i * PQ + d + u]; }
-            for (int jl = 0; jl <= il; ++jl) {
-                const int j = blk * 16 + jl;
-                float kj[kU], bj[kU], s = 0.f;
-                if constexpr (kU == 4) {
-                    *reinterpret_cast<float4*>(kj) = *reinterpret_cast<const float4*>(sK + j * PK + d);
-                    *reinterpret_cast<float4*>(bj) = *reinterpret_cast<const float4*>(sB + j * PQ + d);
-                } else {
+            for (int jl = 0; jl <= il; jl += 2) {           // two keys at a time, so that their sums over the lanes overlap
+                float s[2];
 #pragma unroll
-                    for (int u = 0; u < kU; ++u) { kj[u] = sK[j * PK + d + u]; bj[u] = sB[j * PQ + d + u]; }
+                for (int e = 0; e < 2; ++e) {
+                    const int j = blk * 16 + min(jl + e, il);
+                    float kj[kU], bj[kU];
+                    if constexpr (kU == 4) {
+                        *reinterpret_cast<float4*>(kj) = *reinterpret_cast<const float4*>(sK + j * PK + d);
+                        *reinterpret_cast<float4*>(bj) = *reinterpret_cast<const float4*>(sB + j * PQ + d);
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < kU; ++u) { kj[u] = sK[j * PK + d + u]; bj[u] = sB[j * PQ + d + u]; }
+                    }
+                    s[e] = 0.f;
+#pragma unroll
+                    for (int u = 0; u < kU; ++u) s[e] = fmaf(qi[u] * kj[u], __expf(bi[u] - bj[u]), s[e]);
                 }
 #pragma unroll
-                for (int u = 0; u < kU; ++u) s = fmaf(qi[u] * kj[u], __expf(bi[u] - bj[u]), s);
-                s = warp_sum(s);
-                if (lane == 0) sA[i * kGAPitch + j] = s;
+                for (int o = 16; o > 0; o >>= 1) { s[0] += __shfl_xor_sync(0xffffffffu, s[0], o); s[1] += __shfl_xor_sync(0xffffffffu, s[1], o); }
+                if (lane < 2 && jl + lane <= il) sA[i * kGAPitch + blk * 16 + jl + lane] = lane ? s[1] : s[0];
             }
         } else {
         constexpr int kU = 8;
@@ -430,12 +436,12 @@ __global__ void __launch_bounds__(kGPrepThreads) gla_prepare_kernel(const GlaArg
         }
     }
     __syncthreads();
-    // ---- A v: a warp takes query blocks p and 3 - p (equal work) and every eighth column tile
+    // ---- A v: a warp takes query blocks p and 3 - p (equal work) and every sixteenth column tile
     {
         float* oi = a.oi + bh * kGC * dv;
         for (int half = 0; half < 2; ++half) {
             const int m = half == 0 ? (warp & 1) : 3 - (warp & 1);
-            for (int nt = warp >> 1; nt < dv / 8; nt += 8) {
+            for (int nt = warp >> 1; nt < dv / 8; nt += kGPrepThreads / 64) {
                 float acc[4] = {0.f, 0.f, 0.f, 0.f};
                 for (int k = 0; k < 16 * (m + 1); k += 8) {
                     uint32_t ah[4], al[4];
@@ -455,15 +461,15 @@ __global__ void __launch_bounds__(kGPrepThreads) gla_prepare_kernel(const GlaArg
             }
         }
     }
-    // ---- U = (k decayed to the block's end)^T v: 16 channels x 64 columns per task
+    // ---- U = (k decayed to the block's end)^T v: 16 channels x 32 columns per task
     {
         float* u = a.u + bh * dk * dv;
-        const int mt = dk / 16, ng = (dv + 63) / 64;
+        const int mt = dk / 16, ng = dv / 32;
         for (int task = warp; task < mt * ng; task += kGPrepThreads / 32) {
-            const int m = task % mt, nb = task / mt * 8, ne = min(8, dv / 8 - nb);
-            float acc[8][4];
+            const int m = task % mt, nb = task / mt * 4;
+            float acc[4][4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) { acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f; }
+            for (int j = 0; j < 4; ++j) { acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f; }
             const int c0 = m * 16 + g, c1 = c0 + 8;
             const float e0 = sE[3 * dk + c0], e1 = sE[3 * dk + c1];
 #pragma unroll 2
@@ -476,22 +482,18 @@ __global__ void __launch_bounds__(kGPrepThreads) gla_prepare_kernel(const GlaArg
                 split_tf32(sK[(k + tq + 4) * PK + c0] * f0, ah[2], al[2]);
                 split_tf32(sK[(k + tq + 4) * PK + c1] * f1, ah[3], al[3]);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    if (j < ne) {
-                        const uint32_t b0 = __float_as_uint(bf16_to_f32(sV[(k + tq) * PV + (nb + j) * 8 + g]));
-                        const uint32_t b1 = __float_as_uint(bf16_to_f32(sV[(k + tq + 4) * PV + (nb + j) * 8 + g]));
-                        mma_tf32_1688(acc[j], al, b0, b1);
-                        mma_tf32_1688(acc[j], ah, b0, b1);
-                    }
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t b0 = __float_as_uint(bf16_to_f32(sV[(k + tq) * PV + (nb + j) * 8 + g]));
+                    const uint32_t b1 = __float_as_uint(bf16_to_f32(sV[(k + tq + 4) * PV + (nb + j) * 8 + g]));
+                    mma_tf32_1688(acc[j], al, b0, b1);
+                    mma_tf32_1688(acc[j], ah, b0, b1);
                 }
             }
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (j < ne) {
-                    float* o = u + (size_t)c0 * dv + (nb + j) * 8 + 2 * tq;
-                    *reinterpret_cast<float2*>(o) = make_float2(acc[j][0], acc[j][1]);
-                    *reinterpret_cast<float2*>(o + 8 * dv) = make_float2(acc[j][2], acc[j][3]);
-                }
+            for (int j = 0; j < 4; ++j) {
+                float* o = u + (size_t)c0 * dv + (nb + j) * 8 + 2 * tq;
+                *reinterpret_cast<float2*>(o) = make_float2(acc[j][0], acc[j][1]);
+                *reinterpret_cast<float2*>(o + 8 * dv) = make_float2(acc[j][2], acc[j][3]);
             }
         }
     }
@@ -534,9 +536,9 @@ __device__ __forceinline__ void gla_cp_async16(void* dst, const void* src) {
 
 // grid = (blocks, H)
 template <int DKT, int DVT, bool FORGET>
-__global__ void __launch_bounds__(kGOutThreads) gla_output_kernel(const GlaArgs a) {
+__global__ void __launch_bounds__(kGOutThreads, 2) gla_output_kernel(const GlaArgs a) {
     extern __shared__ __align__(16) float gla_smem[];
-    __shared__ float s_ss[2][kGC];
+    __shared__ float s_ss[4][kGC];
     const int dk = DKT > 0 ? DKT : a.dk, dv = DVT > 0 ? DVT : a.dv;
     const int PQ = dk + 4, PS = dv + 8;
     float* sQ = gla_smem;                                  // [64][PQ]
@@ -555,10 +557,10 @@ __global__ void __launch_bounds__(kGOutThreads) gla_output_kernel(const GlaArgs 
         const int r = i / (dv / 4), c = (i % (dv / 4)) * 4;
         gla_cp_async16(sS + r * PS + c, S + (size_t)r * dv + c);
     }
-    constexpr int kNT = DVT > 0 ? DVT / 16 : 16;           // column tiles of eight per warp (half of the head)
-    const int m = warp & 3, half = warp >> 2, nt = dv / 16;
+    constexpr int kNT = DVT > 0 ? DVT / 32 : 8;            // column tiles of eight per warp (a quarter of the head)
+    const int m = warp & 3, part = warp >> 2, nt = dv / 32;
     float acc[kNT][4];
-    const float* oi = a.oi + bh * kGC * dv + (size_t)(m * 16 + g) * dv + half * (dv / 2) + 2 * tq;
+    const float* oi = a.oi + bh * kGC * dv + (size_t)(m * 16 + g) * dv + part * (dv / 4) + 2 * tq;
 #pragma unroll
     for (int j = 0; j < kNT; ++j) {
         if (j < nt) {
@@ -569,7 +571,7 @@ __global__ void __launch_bounds__(kGOutThreads) gla_output_kernel(const GlaArgs 
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     const float* q0 = sQ + (m * 16 + g) * PQ + tq;
-    const float* s0 = sS + tq * PS + half * (dv / 2) + g;
+    const float* s0 = sS + tq * PS + part * (dv / 4) + g;
     for (int k = 0; k < dk; k += 8) {
         uint32_t ah[4], al[4];
         split_tf32(q0[k], ah[0], al[0]);
@@ -588,7 +590,7 @@ __global__ void __launch_bounds__(kGOutThreads) gla_output_kernel(const GlaArgs 
             }
         }
     }
-    // ---- head norm over both column halves, gate, store
+    // ---- head norm over the column quarters, gate, store
     float ss[2] = {0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < kNT; ++j) {
@@ -599,21 +601,21 @@ __global__ void __launch_bounds__(kGOutThreads) gla_output_kernel(const GlaArgs 
     for (int r = 0; r < 2; ++r) {
         ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], 1);
         ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], 2);
-        if (tq == 0) s_ss[half][m * 16 + g + 8 * r] = ss[r];
+        if (tq == 0) s_ss[part][m * 16 + g + 8 * r] = ss[r];
     }
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         const int lr = m * 16 + g + 8 * r;
         if (lr >= n) continue;
-        const float inv = rsqrtf((s_ss[0][lr] + s_ss[1][lr]) / (float)a.dv_true + a.eps);
+        const float inv = rsqrtf(((s_ss[0][lr] + s_ss[1][lr]) + (s_ss[2][lr] + s_ss[3][lr])) / (float)a.dv_true + a.eps);
         const size_t row = (size_t)row0 + lr;
         const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(a.proj) + row * a.ld + a.g_off + h * dv;
         __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(a.out) + row * a.H * dv + h * dv;
 #pragma unroll
         for (int j = 0; j < kNT; ++j) {
             if (j < nt) {
-                const int d = half * (dv / 2) + j * 8 + 2 * tq;
+                const int d = part * (dv / 4) + j * 8 + 2 * tq;
                 const float2 wv = *reinterpret_cast<const float2*>(a.norm_w + d);
                 float gx = 1.f, gy = 1.f;
                 if (!FORGET || a.g_off >= 0) {
