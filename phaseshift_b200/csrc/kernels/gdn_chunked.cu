@@ -1,4 +1,4 @@
-// Gated DeltaNet, chunked (prefill) form: four launches per layer.
+// Gated DeltaNet, chunked (prefill) form: three launches per layer (four for other head sizes than 128).
 //
 // With G_t the running sum of the log decays g inside a 64-row chunk, D_t = exp(G_t) and S0 the state
 // entering the chunk, the exact recurrence
@@ -15,14 +15,13 @@
 //      g = -exp(A_log) softplus(a + dt_bias); then A and QKd from K K^T and Q K^T on the tensor cores, T by
 //      forward substitution in the four 16 x 16 diagonal blocks (one thread per column, out of registers) and
 //      -T_22 A_21 T_11 below them, for blocks of 16 and then of 32 rows, W and U as tensor-core products with T, and the decayed operands Qd = D q, Kd = (D_C/D_s) k, written to scratch.
-//   2. gdn_history : stores the raw inputs of each sequence's last rows in the conv ring (a separate
-//      launch so no CTA reads history that another CTA of the same step is overwriting).
-//   3. gdn_chunk_scan_umma : one CTA per (sequence, value head, 64-column slice of Dv) walks the chunks:
-//      Delta = U - W S0 ;  O = Qd S0 + QKd Delta ;  S = D_C S0 + Kd^T Delta.  Three small tensor-core
-//      products per chunk on tcgen05, no serial solve on the critical path; the state stays in tensor memory.
+//   2. gdn_chunk_scan_umma : one CTA per (sequence, value head) walks the chunks:
+//      Delta = U - W S0 ;  O = Qd S0 + QKd Delta ;  S = D_C S0 + Kd^T Delta.  Four small tensor-core
+//      products per chunk on tcgen05, no serial solve on the critical path; the state stays in tensor memory.  It also stores the
+//      raw inputs of each sequence's last rows in the conv ring (not the preparation, other CTAs of which still read the history).
 //      (gdn_chunk_scan_tc is the same walk on mma.sync for head sizes of 64, gdn_chunk_scan with fp32 CUDA-core
-//      products, selected by PS_GDN_SCAN=fp32.)
-//   4. gdn_post : RMSNorm over the head's Dv outputs (direct weight) * SiLU(z) -> bf16.
+//      products, selected by PS_GDN_SCAN=fp32; gdn_history stores the raw inputs for both.)
+//   3. gdn_post : RMSNorm over the head's Dv outputs (direct weight) * SiLU(z) -> bf16.
 //
 // All decay ratios have s <= t and g <= 0, so every exponential is <= 1.  The state and every accumulation
 // are fp32; the tensor-core products take TF32 operands (round-to-nearest copies; mma.sync in the preparation, tcgen05 in the scan).
@@ -66,7 +65,7 @@ template <int DK, int DV> struct GdnImage {
     __device__ static __forceinline__ int w(int r, int k) { return kWQ + at(2 * kChunk, r, k); }               // W over Qd, K = DK
     __device__ static __forceinline__ int qd(int r, int k) { return kWQ + at(2 * kChunk, kChunk + r, k); }
     __device__ static __forceinline__ int kdt(int d, int r) { return kKd + at(DK, d, r); }                     // Kd^T, K = rows of the chunk
-    __device__ static __forceinline__ int ut(int r, int n) { return kU + n * kChunk + r; }                     // U^T
+    __device__ static __forceinline__ int ut(int r, int n) { return kU + (((r >> 2) * DV + n) << 2) + (r & 3); }   // U^T, four rows of the chunk apiece
     __device__ static __forceinline__ int qk(int r, int c) { return kQK + at(kChunk, r, c); }
 };
 
@@ -102,12 +101,13 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const float (&a)[4], flo
 // (2048 rows, 32 heads) and 12 of 50 (37 rows) longer.
 __device__ __forceinline__ float gdn_silu(float x) { return __fdividef(x, 1.f + __expf(-x)); }
 
-// grid = (max chunks, Hv), block = 256 threads, two CTAs per SM (shared memory: Q and K tiles, the raw q|k input tile
+// grid = (max chunks, Hv), block = 512 threads, two CTAs per SM (shared memory: Q and K tiles, the raw q|k input tile
 // that A, T and the block-row temporaries later overwrite; V is convolved straight from global memory into Q's tile
-// once Q is dead).
+// once Q is dead).  2048 rows x 32 heads: 108 us, 111 with 256 threads; bound by issue.
+constexpr int kPrepThreads = 512;
 template <int DK, int DV>
-__global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArgs a) {
-    static_assert(DV <= DK && 256 % DK == 0 && 512 % DV == 0, "tile aliasing and the conv partition assume these");
+__global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prep_kernel(const GdnPrepArgs a) {
+    static_assert(DV <= DK && kPrepThreads % DK == 0 && 2 * kPrepThreads % DV == 0, "tile aliasing and the conv partition assume these");
     constexpr int CH = 2 * DK + DV, CQK = 2 * DK, PK = DK + 4, PV = DV + 4, RAWR = kChunk + 3;
     extern __shared__ __align__(16) float sm[];
     float* sQ = sm;                        // [64][DK+4]; after the decayed operands are written: V [64][DV+4]
@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
     float* sT = sA + kChunk * 65;          // 64 * 65 floats keep the T rows 16-byte aligned
     float* sM = sT + kChunk * kTP;
 
+    cudaTriggerProgrammaticLaunchCompletion();
     GdnSeqDesc2 sd; int chunk;
     if (!find_chunk(a.seqs, a.n_seqs, a.min_rows, blockIdx.x, sd, chunk)) return;
     const int h = blockIdx.y, t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -142,7 +143,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
         // all copies in flight at once
         constexpr int PPR = CQK / 8;
         const __nv_bfloat16* src0 = a.proj + (row0 - 3) * a.ld_proj;
-        for (int p = t; p < RAWR * PPR; p += 256) {
+        for (int p = t; p < RAWR * PPR; p += kPrepThreads) {
             const int rr = p / PPR, c = (p % PPR) * 8;
             const __nv_bfloat16* src = src0 + (size_t)rr * a.ld_proj + (c < DK ? q_off + c : k_off + (c - DK));
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(sRaw + rr * CQK + c)), "l"(src) : "memory");
@@ -151,7 +152,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
     } else {
         const bool vec = (a.ld_proj % 8) == 0;
         constexpr int PPR = CQK / 8;
-        for (int p = t; p < RAWR * PPR; p += 256) {
+        for (int p = t; p < RAWR * PPR; p += kPrepThreads) {
             const int rr = p / PPR - 3, c = (p % PPR) * 8;
             const int gc = c < DK ? q_off + c : k_off + (c - DK);
             uint4 v = make_uint4(0, 0, 0, 0);
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
         }
     }
     // ---- beta and the running log decay (last warp, two 32-wide halves)
-    if (warp == 7) {
+    if (warp == kPrepThreads / 32 - 1) {
         float g0 = 0.f, g1 = 0.f, b0 = 0.f, b1 = 0.f;
         const float Aexp = -__expf(a.A_log[h]), dtb = a.dt_bias[h];
         if (lane < C) {
@@ -197,7 +198,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
     __syncthreads();
     // ---- conv + SiLU of q and k: a thread owns a channel pair over a run of rows and slides its taps through registers
     {
-        constexpr int PARTS = 256 / DK, RUN = kChunk / PARTS;           // DK channel pairs x PARTS row runs = 256 threads
+        constexpr int PARTS = kPrepThreads / DK, RUN = kChunk / PARTS;       // DK channel pairs x PARTS row runs
         const int c = 2 * (t % DK), rb = (t / DK) * RUN;
         const int gc = c < DK ? q_off + c : k_off + (c - DK);
         const uint4 wraw = *reinterpret_cast<const uint4*>(a.conv_w + (size_t)gc * 4);     // two channels x four taps
@@ -217,10 +218,11 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
         }
     }
     __syncthreads();
-    // ---- L2 norms: warp w owns rows 8w .. 8w+7, four at a time so that their reductions overlap
+    // ---- L2 norms: warp w owns rows 4w .. 4w + 3, whose reductions overlap
     {
         constexpr int V = DK / 32;
-        for (int rb = warp * 8; rb < warp * 8 + 8; rb += 4) {
+        {
+            const int rb = warp * 4;
             float q[4][V], k[4][V], n[8];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -245,22 +247,22 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
     }
     __syncthreads();
     // ---- A (strictly lower) and QKd (lower incl. diagonal) on the tensor cores: warp -> rows 16 mt .., columns
-    //      32 ch .. 32 ch + 31; K K^T and Q K^T share the B fragments (B[k = d][n = s] = K[s][d])
+    //      16 ch .. 16 ch + 15; K K^T and Q K^T share the B fragments (B[k = d][n = s] = K[s][d])
     {
         const int g = lane >> 2, tq = lane & 3, mt = warp & 3, ch = warp >> 2;
-        float kk[4][4], qk[4][4];
+        float kk[2][4], qk[2][4];
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) { kk[nt][0] = kk[nt][1] = kk[nt][2] = kk[nt][3] = 0.f; qk[nt][0] = qk[nt][1] = qk[nt][2] = qk[nt][3] = 0.f; }
-        if (ch * 32 <= 16 * mt + 15) {                      // tiles entirely above the diagonal stay zero
+        for (int nt = 0; nt < 2; ++nt) { kk[nt][0] = kk[nt][1] = kk[nt][2] = kk[nt][3] = 0.f; qk[nt][0] = qk[nt][1] = qk[nt][2] = qk[nt][3] = 0.f; }
+        if (ch <= mt) {                                     // tiles entirely above the diagonal stay zero
             const float* kr = sK + (16 * mt + g) * PK + tq;
             const float* qr = sQ + (16 * mt + g) * PK + tq;
 #pragma unroll 4
             for (int ks = 0; ks < DK / 8; ++ks) {
                 const float ak[4] = {to_tf32(kr[8 * ks]), to_tf32(kr[8 * PK + 8 * ks]), to_tf32(kr[8 * ks + 4]), to_tf32(kr[8 * PK + 8 * ks + 4])};
                 const float aq[4] = {to_tf32(qr[8 * ks]), to_tf32(qr[8 * PK + 8 * ks]), to_tf32(qr[8 * ks + 4]), to_tf32(qr[8 * PK + 8 * ks + 4])};
-                const float* kb = sK + (32 * ch + g) * PK + 8 * ks + tq;
+                const float* kb = sK + (16 * ch + g) * PK + 8 * ks + tq;
 #pragma unroll
-                for (int nt = 0; nt < 4; ++nt) {
+                for (int nt = 0; nt < 2; ++nt) {
                     const float b0 = to_tf32(kb[8 * nt * PK]), b1 = to_tf32(kb[8 * nt * PK + 4]);
                     mma_tf32(kk[nt], ak, b0, b1);
                     mma_tf32(qk[nt], aq, b0, b1);
@@ -268,10 +270,10 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
             }
         }
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int tt = 16 * mt + g + (e >> 1) * 8, ss = 32 * ch + 8 * nt + 2 * tq + (e & 1);
+                const int tt = 16 * mt + g + (e >> 1) * 8, ss = 16 * ch + 8 * nt + 2 * tq + (e & 1);
                 const float dec = ss <= tt ? __expf(sG[tt] - sG[ss]) : 0.f;
                 sA[tt * 65 + ss] = ss < tt ? sBeta[tt] * dec * kk[nt][e] : 0.f;
                 (a.images ? scr[Image::qk(tt, ss)] : gQK[tt * kChunk + ss]) = a.round_tf32 ? to_tf32(dec * qk[nt][e]) : dec * qk[nt][e];
@@ -279,7 +281,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
     }
     __syncthreads();
     // ---- raw v inputs of this thread's conv run, requested now and used once Q's tile is free
-    constexpr int VPARTS = 512 / DV, VRUN = kChunk / VPARTS;             // DV / 2 channel pairs x VPARTS row runs = 256 threads
+    constexpr int VPARTS = 2 * kPrepThreads / DV, VRUN = kChunk / VPARTS;        // DV / 2 channel pairs x VPARTS row runs
     const int vc = 2 * (t % (DV / 2)), vrb = (t / (DV / 2)) * VRUN;
     uint32_t vraw[VRUN + 3];
     if (inner && (a.ld_proj & 1) == 0) {
@@ -322,14 +324,14 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
     } else {
         const float GC = sG[kChunk - 1];
         if (a.images) {
-            for (int i = t - kChunk; i < kChunk * DK / 4; i += 256 - kChunk) {
+            for (int i = t - kChunk; i < kChunk * DK / 4; i += kPrepThreads - kChunk) {
                 const int r = (i * 4) / DK, d = (i * 4) % DK;
                 const float eq = __expf(sG[r]);
                 const float4 q = *reinterpret_cast<const float4*>(sQ + r * PK + d);
                 *reinterpret_cast<float4*>(scr + Image::qd(r, d)) = make_float4(to_tf32(eq * q.x), to_tf32(eq * q.y), to_tf32(eq * q.z), to_tf32(eq * q.w));
             }
             // Kd^T: a thread takes eight rows of the chunk of one channel, whole 32-byte sectors of the tile
-            for (int i = t - kChunk; i < kChunk * DK / 8; i += 256 - kChunk) {
+            for (int i = t - kChunk; i < kChunk * DK / 8; i += kPrepThreads - kChunk) {
                 const int d = i % DK, r = i / DK * 8;
                 float k[8];
 #pragma unroll
@@ -337,7 +339,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
                 *reinterpret_cast<float4*>(scr + Image::kdt(d, r)) = make_float4(k[0], k[1], k[2], k[3]);
                 *reinterpret_cast<float4*>(scr + Image::kdt(d, r + 4)) = make_float4(k[4], k[5], k[6], k[7]);
             }
-        } else for (int i = t - kChunk; i < kChunk * DK / 4; i += 256 - kChunk) {
+        } else for (int i = t - kChunk; i < kChunk * DK / 4; i += kPrepThreads - kChunk) {
             const int r = (i * 4) / DK, d = (i * 4) % DK;
             const float eq = __expf(sG[r]), ek = __expf(GC - sG[r]);
             const float4 q = *reinterpret_cast<const float4*>(sQ + r * PK + d), k = *reinterpret_cast<const float4*>(sK + r * PK + d);
@@ -372,54 +374,46 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
     // ---- T below the diagonal blocks: -T_22 (A_21 T_11) for the two pairs of 16-row blocks, then for the two 32-row halves
     __syncthreads();
     {
-        const int pr = t >> 7, r = (t >> 3) & 15, c = 2 * (t & 7);                 // pair, row and columns of its 16 x 16 block
+        const int pr = t >> 8, r = (t >> 4) & 15, c = t & 15;                      // pair, row and column of its 16 x 16 block
         const int lo = 32 * pr, hi = lo + 16;
-        float x0 = 0.f, x1 = 0.f;
+        float x0 = 0.f;
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            const float av = sA[(hi + r) * 65 + lo + k];
-            const float2 tv = *reinterpret_cast<const float2*>(sT + (lo + k) * kTP + lo + c);
-            x0 = fmaf(av, tv.x, x0); x1 = fmaf(av, tv.y, x1);
-        }
-        sM[(16 * pr + r) * 36 + c] = x0; sM[(16 * pr + r) * 36 + c + 1] = x1;
-        sT[(lo + r) * kTP + hi + c] = 0.f; sT[(lo + r) * kTP + hi + c + 1] = 0.f;      // the halves are used whole below
+        for (int k = 0; k < 16; ++k) x0 = fmaf(sA[(hi + r) * 65 + lo + k], sT[(lo + k) * kTP + lo + c], x0);
+        sM[(16 * pr + r) * 36 + c] = x0;
+        sT[(lo + r) * kTP + hi + c] = 0.f;                                         // the halves are used whole below
         __syncthreads();
-        x0 = x1 = 0.f;
+        x0 = 0.f;
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            const float tv = sT[(hi + r) * kTP + hi + k];
-            const float2 mv = *reinterpret_cast<const float2*>(sM + (16 * pr + k) * 36 + c);
-            x0 = fmaf(tv, mv.x, x0); x1 = fmaf(tv, mv.y, x1);
-        }
-        sT[(hi + r) * kTP + lo + c] = -x0; sT[(hi + r) * kTP + lo + c + 1] = -x1;
+        for (int k = 0; k < 16; ++k) x0 = fmaf(sT[(hi + r) * kTP + hi + k], sM[(16 * pr + k) * 36 + c], x0);
+        sT[(hi + r) * kTP + lo + c] = -x0;
     }
     __syncthreads();
     {
-        const int r = t >> 3, c = 4 * (t & 7);
+        const int r = t >> 4, c = 2 * (t & 15);
         auto product = [&](const float* left, int lp, const float* right, int rp) {    // row r of left [32 x 32] times right's columns c ..
-            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            float2 x = make_float2(0.f, 0.f);
 #pragma unroll 8
             for (int k = 0; k < 32; ++k) {
                 const float l = left[r * lp + k];
-                const float4 v = *reinterpret_cast<const float4*>(right + k * rp + c);
-                x.x = fmaf(l, v.x, x.x); x.y = fmaf(l, v.y, x.y); x.z = fmaf(l, v.z, x.z); x.w = fmaf(l, v.w, x.w);
+                const float2 v = *reinterpret_cast<const float2*>(right + k * rp + c);
+                x.x = fmaf(l, v.x, x.x); x.y = fmaf(l, v.y, x.y);
             }
             return x;
         };
-        const float4 m = product(sA + 32 * 65, 65, sT, kTP);
-        *reinterpret_cast<float4*>(sM + r * 36 + c) = m;
+        const float2 m = product(sA + 32 * 65, 65, sT, kTP);
+        *reinterpret_cast<float2*>(sM + r * 36 + c) = m;
         __syncthreads();
-        const float4 x = product(sT + 32 * kTP + 32, kTP, sM, 36);
-        *reinterpret_cast<float4*>(sT + (32 + r) * kTP + c) = make_float4(-x.x, -x.y, -x.z, -x.w);
+        const float2 x = product(sT + 32 * kTP + 32, kTP, sM, 36);
+        *reinterpret_cast<float2*>(sT + (32 + r) * kTP + c) = make_float2(-x.x, -x.y);
     }
     __syncthreads();
-    // ---- W = T diag(beta D) K (warps 0-3) and U = T diag(beta) V (warps 4-7) on the tensor cores: warp -> rows
-    //      16 mt .., all columns of its matrix; T is lower triangular, so k-steps beyond the row tile are skipped
+    // ---- W = T diag(beta D) K (warps 0-7) and U = T diag(beta) V (warps 8-15) on the tensor cores: warp -> rows
+    //      16 mt .., half of the columns of its matrix; T is lower triangular, so k-steps beyond the row tile are skipped
     {
         const int g = lane >> 2, tq = lane & 3, mt = warp & 3;
-        const bool isW = warp < 4;
-        constexpr int NTW = (DK > DV ? DK : DV) / 8;
-        const int ntiles = (isW ? DK : DV) / 8;
+        const bool isW = warp < 8;
+        constexpr int NTW = (DK > DV ? DK : DV) / 16;
+        const int ntiles = (isW ? DK : DV) / 16, n0 = ((warp >> 2) & 1) * ntiles * 8;          // tiles of 8 columns from column n0 on
         const float* src = isW ? sK : sV;
         const int pitch = isW ? PK : PV;
         float acc[NTW][4];
@@ -430,8 +424,8 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
             const float at[4] = {to_tf32(tr[8 * ks]), to_tf32(tr[8 * kTP + 8 * ks]), to_tf32(tr[8 * ks + 4]), to_tf32(tr[8 * kTP + 8 * ks + 4])};
             const int s0 = 8 * ks + tq, s1 = s0 + 4;
             const float f0 = sBeta[s0] * (isW ? __expf(sG[s0]) : 1.f), f1 = sBeta[s1] * (isW ? __expf(sG[s1]) : 1.f);
-            const float* b0p = src + s0 * pitch + g;
-            const float* b1p = src + s1 * pitch + g;
+            const float* b0p = src + s0 * pitch + n0 + g;
+            const float* b1p = src + s1 * pitch + n0 + g;
 #pragma unroll
             for (int nt = 0; nt < NTW; ++nt)
                 if (nt < ntiles) mma_tf32(acc[nt], at, to_tf32(b0p[8 * nt] * f0), to_tf32(b1p[8 * nt] * f1));
@@ -445,7 +439,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
         if (a.images) {
 #pragma unroll
             for (int nt = 0; nt < NTW; ++nt) {
-                const int r = 16 * mt + g, c = 8 * nt + 2 * tq;
+                const int r = 16 * mt + g, c = n0 + 8 * nt + 2 * tq;
                 if (isW && nt < ntiles) {
                     *reinterpret_cast<float2*>(scr + Image::w(r, c)) = make_float2(acc[nt][0], acc[nt][1]);
                     *reinterpret_cast<float2*>(scr + Image::w(r + 8, c)) = make_float2(acc[nt][2], acc[nt][3]);
@@ -459,8 +453,8 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(const GdnPrepArg
 #pragma unroll
         for (int nt = 0; nt < NTW; ++nt)
             if (nt < ntiles) {
-                *reinterpret_cast<float2*>(dst + (size_t)(16 * mt + g) * dp + 8 * nt + 2 * tq) = make_float2(acc[nt][0], acc[nt][1]);
-                *reinterpret_cast<float2*>(dst + (size_t)(16 * mt + g + 8) * dp + 8 * nt + 2 * tq) = make_float2(acc[nt][2], acc[nt][3]);
+                *reinterpret_cast<float2*>(dst + (size_t)(16 * mt + g) * dp + n0 + 8 * nt + 2 * tq) = make_float2(acc[nt][0], acc[nt][1]);
+                *reinterpret_cast<float2*>(dst + (size_t)(16 * mt + g + 8) * dp + n0 + 8 * nt + 2 * tq) = make_float2(acc[nt][2], acc[nt][3]);
             }
     }
 }
@@ -810,45 +804,45 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_tc_kernel(const GdnScanArg
     }
 }
 
-// ---- the scan on tcgen05 (Dk = Dv = 128): the same products, with the state in tensor memory.  One CTA per (sequence, value head,
-// 64 columns of Dv); per chunk (TF32 operands from shared memory, fp32 accumulators):
-//     [P; R] = [W; Qd] S          128 x 64 x 128 into D1 (rows of P: lanes 0 .. 63)
-//     Delta = U - P               lanes 0 .. 63 to shared memory as Delta^T, rounded to TF32
-//     S     += Kd^T Delta         128 x 64 x 64 into D2, which the threads have scaled by D_C before
-//     [.; R] += [0; QKd] Delta    128 x 64 x 64 into D1 (the zero rows stay in shared memory)
-// then a TF32 copy of S goes to shared memory as the next chunk's operand and R to global memory.  The preparation kernel has laid the
-// operands out as shared-memory tiles (GdnImage), so one thread fetches a chunk with five bulk copies, each as soon as the products
-// that read the previous chunk's tile are done.
-// Warps 0-7: lane quadrant (warp & 3), columns 32 (warp >> 2) .. + 31; warp 8: copies; warp 9: products.
-// Rounding as in the mma.sync scan it replaces, which took 5.2 us per chunk (1500 of 9800 cycles to issue copies twice, 2700 and 2500
-// for the large products, bound by fragment loads from shared memory) and now takes 3.3 us.  2048 rows: 165 us before, 106 now with 32
-// heads, 169 and 115 with 48 (64 and 96 CTAs).  What bounds it: too few CTAs, and in each the chain of a chunk -- product, accumulator to
-// registers, operand to shared memory, barrier, next product -- at 6500 cycles with the tensor pipe 17 % and DRAM 29 % busy.  Fetching the
-// 128 KB of tiles is not the bound: with second buffers for them the scan took 105 us instead of 106.
+// ---- the scan on tcgen05 (Dk = Dv = 128): the same products transposed, with everything that a chunk hands to the next one in tensor
+// memory.  One CTA per (sequence, value head); lane n of tensor memory is column n of Dv.  Per chunk (TF32 operands, fp32 accumulators; A
+// from tensor memory, B from shared memory):
+//     P      = S^T W^T            128 x 64 x 128
+//     R      = S^T Qd^T           128 x 64 x 128, while the threads form
+//     Delta^T = U^T - P           rounded to TF32, back to tensor memory
+//     S^T   += Delta^T Kd         128 x 128 x 64, into S^T scaled by D_C
+//     R     += Delta^T QKd^T      128 x 64 x 64
+// then a TF32 copy of S^T becomes the next chunk's A operand, and R goes to global memory.
+// The preparation kernel has laid the B operands out as shared-memory tiles (GdnImage), so one thread fetches a chunk with three bulk
+// copies, a chunk ahead; U goes straight to the registers of the threads that subtract P from it.
+// Warps 0-7: lane quadrant (warp & 3), half (warp >> 2) of the columns of P and S; warps 8-11: outputs, one quadrant each; warp 12:
+// copies; warp 13: products.
+// With S and Delta as B operands in shared memory, two CTAs per head of 64 columns of Dv each took every accumulator through registers
+// into a swizzled tile and a proxy fence, 6500 cycles per chunk.  2048 rows: 32 heads 108 us with 64 CTAs, 113 with 32 here; 48 heads 150 and
+// 142; with the rows' history stored here and the launches overlapped a layer takes 28 us less.  What bounds it: the chain of a chunk, 5700
+// cycles -- S to tensor memory 1500, the product to P 2750, Delta 300, the product to S 1100.  Rounding on the integer pipe and P and R as
+// one product of 128 columns left it as it was; the copies are a chunk ahead.  Four warps that norm and gate the outputs here cannot keep up
+// (12 us a chunk).
+constexpr int kScanThreads = 448, kScanStageBytes = (2 * kChunk * 128 + 128 * kChunk + kChunk * kChunk) * 4;
+
 template <int DK, int DV>
-__global__ void __launch_bounds__(320, 1) gdn_chunk_scan_umma_kernel(const GdnScanArgs a) {
-    static_assert(DK == 128 && kChunk == 64 && kSlice == 64, "the tiles' row counts");
+__global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(const GdnScanArgs a, const GdnPrepArgs p) {
+    static_assert(DK == 128 && DV == 128 && kChunk == 64, "the tiles' row counts");
     using Image = GdnImage<DK, DV>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    constexpr int kBytesWQ = 128 * DK * 4, kBytesKd = DK * kChunk * 4, kBytesA3 = 128 * kChunk * 4, kBytesS = kSlice * DK * 4, kBytesD = kSlice * kChunk * 4;
-    unsigned char* sWQ = smem;                   // [4 panels][128 rows][128 B]
-    unsigned char* sKd = sWQ + kBytesWQ;         // [2][128][128 B]
-    unsigned char* sA3 = sKd + kBytesKd;         // [2][64 zero rows, 64 of QKd][128 B]
-    unsigned char* sS = sA3 + kBytesA3;          // S^T: [4 panels][64 columns][128 B]
-    unsigned char* sD = sS + kBytesS;            // Delta^T: [2 panels][64 columns][128 B]
-    float* sU = reinterpret_cast<float*>(sD + kBytesD);      // U^T: [64 columns][64 rows]
-    __shared__ __align__(8) uint64_t wq_full, u_full, kq_full, s_ready, d_ready, m1_done, m2_done, m3_done;
+    constexpr int kBytesWQ = 128 * DK * 4, kBytesKd = DK * kChunk * 4, kBytesQK = kChunk * kChunk * 4;
+    __shared__ __align__(8) uint64_t wq_full[2], kq_full[2], r_free[2], m3_done[2], s_ready, d_ready, m1_done, m2_done;
     __shared__ uint32_t tmem_slot;
-    __shared__ int s_abort, s_wq, s_u, s_kq;     // fills of each tile issued
+    __shared__ int s_abort, s_filled;            // chunks whose copies have been issued
 
-    const int c0 = blockIdx.x * kSlice, h = blockIdx.y, Hv = a.Hv;
+    const int h = blockIdx.x, Hv = a.Hv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const GdnSeqDesc2 sd = a.seqs[blockIdx.z];
+    const GdnSeqDesc2 sd = a.seqs[blockIdx.y];
     if (sd.n_rows <= a.min_rows || sd.slot < 0) return;
     PS_CHECK(PS_SLOT_OK(sd.slot) && PS_ROWS_OK(sd.row_start, sd.n_rows));
     int gc = 0;
-    for (int s = 0; s < (int)blockIdx.z; ++s) {
+    for (int s = 0; s < (int)blockIdx.y; ++s) {
         const GdnSeqDesc2 d = a.seqs[s];
         if (d.n_rows > a.min_rows && d.slot >= 0) gc += (d.n_rows + kChunk - 1) / kChunk;
     }
@@ -857,146 +851,171 @@ __global__ void __launch_bounds__(320, 1) gdn_chunk_scan_umma_kernel(const GdnSc
     const size_t scr_step = (size_t)Hv * chunk_scratch_floats(DK, DV);
 
     if (threadIdx.x == 0) {
-        tc::mbar_init(&wq_full, 1); tc::mbar_init(&u_full, 1); tc::mbar_init(&kq_full, 1);
-        tc::mbar_init(&s_ready, 8); tc::mbar_init(&d_ready, 4);
-        tc::mbar_init(&m1_done, 1); tc::mbar_init(&m2_done, 1); tc::mbar_init(&m3_done, 1);
+        for (int b = 0; b < 2; ++b) {
+            tc::mbar_init(&wq_full[b], 1); tc::mbar_init(&kq_full[b], 1); tc::mbar_init(&r_free[b], 4); tc::mbar_init(&m3_done[b], 1);
+        }
+        tc::mbar_init(&s_ready, 8); tc::mbar_init(&d_ready, 8); tc::mbar_init(&m1_done, 1); tc::mbar_init(&m2_done, 1);
         tc::fence_barrier_init();
-        s_abort = 0; s_wq = s_u = s_kq = 0;
+        s_abort = 0; s_filled = 0;
     }
-    if (warp == 9) {
-        tc::tmem_alloc(&tmem_slot, 128);
+    if (warp == 13) {
+        tc::tmem_alloc(&tmem_slot, 512);
         tc::tmem_relinquish();
     }
-    for (int i = threadIdx.x; i < 2 * 64 * 8; i += 320)       // the zero rows of both panels
-        *reinterpret_cast<uint4*>(sA3 + (i >> 9) * (128 * 128) + (i & 511) * 16) = make_uint4(0, 0, 0, 0);
-    tc::fence_proxy_async_smem();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t d1 = tmem_slot, d2 = d1 + 64;
+    cudaGridDependencySynchronize();
+    const uint32_t base = tmem_slot, tS = base, tA = base + 128, tD = base + 256, tP = base + 320, tR = base + 384;      // tR: two of 64
+    auto wait = [&](uint64_t* bar, uint32_t ph) {
+        const bool ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(bar, ph, a.budget, &s_abort));
+        if (ok) tc::fence_after_sync();
+        return ok;
+    };
+    auto arrive = [&](uint64_t* bar) {
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(bar);
+    };
 
-    if (warp == 8) {
+    if (warp == 12) {
         // ------------------------------------------------ copies
         if (tc::elect_one()) {
             for (int c = 0; c < nc; ++c) {
+                const int b = c & 1;
+                if (c >= 2 && !tc::mbar_wait_abortable(&m3_done[b], ((uint32_t)(c >> 1) & 1u) ^ 1u, a.budget, &s_abort)) break;
                 const float* scr = scr0 + c * scr_step;
-                const uint32_t before = (uint32_t)(c - 1) & 1u;
-                if (c > 0 && !tc::mbar_wait_abortable(&m1_done, before, a.budget, &s_abort)) break;      // [W; Qd] has been read
-                tc::mbar_expect_tx(&wq_full, kBytesWQ);
-                tc::bulk_load(sWQ, scr + Image::kWQ, kBytesWQ, &wq_full);
-                s_wq = c + 1;
-                // U is free with the Delta that was made of it, Kd and QKd with the products of that Delta
-                if (c > 0 && !tc::mbar_wait_abortable(&d_ready, before, a.budget, &s_abort)) break;
-                tc::mbar_expect_tx(&u_full, kBytesD);
-                tc::bulk_load(sU, scr + Image::kU + c0 * kChunk, kBytesD, &u_full);
-                s_u = c + 1;
-                if (c > 0 && !tc::mbar_wait_abortable(&m3_done, before, a.budget, &s_abort)) break;
-                tc::mbar_expect_tx(&kq_full, kBytesKd + kChunk * kChunk * 4);
-                tc::bulk_load(sKd, scr + Image::kKd, kBytesKd, &kq_full);
-#pragma unroll
-                for (int p = 0; p < 2; ++p) tc::bulk_load(sA3 + p * (128 * 128) + 64 * 128, scr + Image::kQK + p * (kChunk * 32), kChunk * 128, &kq_full);
-                s_kq = c + 1;
+                unsigned char* st = smem + b * kScanStageBytes;
+                tc::mbar_expect_tx(&wq_full[b], kBytesWQ);
+                tc::bulk_load(st, scr + Image::kWQ, kBytesWQ, &wq_full[b]);
+                tc::mbar_expect_tx(&kq_full[b], kBytesKd + kBytesQK);
+                tc::bulk_load(st + kBytesWQ, scr + Image::kKd, kBytesKd, &kq_full[b]);
+                tc::bulk_load(st + kBytesWQ + kBytesKd, scr + Image::kQK, kBytesQK, &kq_full[b]);
+                s_filled = c + 1;
             }
         }
-    } else if (warp == 9) {
+    } else if (warp == 13) {
         // ------------------------------------------------ products
         if (tc::elect_one()) {
-            constexpr uint32_t idesc = tc::idesc_tf32_f32(128, kSlice);
-            auto lo = [](const void* p) { return (tc::smem_u32(p) >> 4) | tc::kDescSw128LoFlags; };
-            const uint32_t wq = lo(sWQ), kd = lo(sKd), a3 = lo(sA3), st = lo(sS), dt = lo(sD);
-            // K-step j of 8: panel j / 4, 32 bytes inside its rows; panels of `ra` and `rb` rows
-            auto product = [&](uint32_t acc, uint32_t al, uint32_t bl, int steps, int ra, int rb, bool add) {
+            constexpr uint32_t id64 = tc::idesc_tf32_f32(128, 64), id128 = tc::idesc_tf32_f32(128, 128);
+            // K-step j of 8: panel j / 4 (of `rows` rows), 32 bytes inside its rows
+            auto product = [&](uint32_t acc, uint32_t at, uint32_t bl, int steps, int rows, uint32_t idesc, bool add) {
 #pragma unroll 4
                 for (int j = 0; j < steps; ++j)
-                    tc::mma_tf32_ss(acc, tc::desc_pack(al + (j >> 2) * (ra * 8) + (j & 3) * 2, tc::kDescSw128Hi),
-                                    tc::desc_pack(bl + (j >> 2) * (rb * 8) + (j & 3) * 2, tc::kDescSw128Hi), idesc, add || j > 0 ? 1u : 0u);
+                    tc::mma_tf32_ts(acc, at + 8 * j, tc::desc_pack(bl + (j >> 2) * (rows * 8) + (j & 3) * 2, tc::kDescSw128Hi), idesc, add || j > 0 ? 1u : 0u);
             };
             for (int c = 0; c < nc; ++c) {
-                const uint32_t ph = (uint32_t)c & 1u;
-                if (!tc::mbar_wait_abortable(&s_ready, ph, a.budget, &s_abort) || !tc::mbar_wait_abortable(&wq_full, ph, a.budget, &s_abort)) break;
+                const int b = c & 1;
+                const uint32_t ph = (uint32_t)c & 1u, ph2 = (uint32_t)(c >> 1) & 1u;
+                const uint32_t wq = (tc::smem_u32(smem + b * kScanStageBytes) >> 4) | tc::kDescSw128LoFlags, kd = wq + (kBytesWQ >> 4), qk = kd + (kBytesKd >> 4);
+                if (!tc::mbar_wait_abortable(&s_ready, ph, a.budget, &s_abort) || !tc::mbar_wait_abortable(&wq_full[b], ph2, a.budget, &s_abort)) break;
                 tc::fence_after_sync();
-                product(d1, wq, st, DK / 8, 128, kSlice, false);
+                product(tP, tA, wq, DK / 8, 128, id64, false);
                 tc::mma_commit(&m1_done);
-                if (!tc::mbar_wait_abortable(&d_ready, ph, a.budget, &s_abort) || !tc::mbar_wait_abortable(&kq_full, ph, a.budget, &s_abort)) break;
+                if (c >= 2 && !tc::mbar_wait_abortable(&r_free[b], ph2 ^ 1u, a.budget, &s_abort)) break;
                 tc::fence_after_sync();
-                product(d2, kd, dt, kChunk / 8, DK, kSlice, true);
+                product(tR + 64 * b, tA, wq + (64 * 128 >> 4), DK / 8, 128, id64, false);
+                if (!tc::mbar_wait_abortable(&d_ready, ph, a.budget, &s_abort) || !tc::mbar_wait_abortable(&kq_full[b], ph2, a.budget, &s_abort)) break;
+                tc::fence_after_sync();
+                product(tS, tD, kd, kChunk / 8, DK, id128, true);
                 tc::mma_commit(&m2_done);
-                product(d1, a3, dt, kChunk / 8, 128, kSlice, true);
-                tc::mma_commit(&m3_done);
+                product(tR + 64 * b, tD, qk, kChunk / 8, kChunk, id64, true);
+                tc::mma_commit(&m3_done[b]);
             }
+        }
+    } else if (warp < 8) {
+        // ------------------------------------------------ state and Delta: lane n = column of Dv
+        const int quad = warp & 3, half = warp >> 2, n = quad * 32 + lane;
+        const uint32_t at = (uint32_t)(quad * 32) << 16;
+        float* Sg = a.state + (((size_t)sd.slot * Hv + h) * DK + half * 64) * DV + n;         // rows of Dk: half * 64 ..
+        const float* dcs = a.dc + (size_t)gc * Hv + h;
+        uint32_t v[32], w[32];
+        float4 u[8];
+        auto load_u = [&](int c) {
+            const float4* src = reinterpret_cast<const float4*>(scr0 + c * scr_step + Image::kU) + half * 8 * DV + n;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) u[j] = __ldg(src + j * DV);
+        };
+        // 32 columns of S^T (from column `c0` of this half): TF32 copy for the products
+        auto copy_state = [&](const uint32_t (&x)[32], int c0) {
+            uint32_t t[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) t[j] = __float_as_uint(to_tf32(__uint_as_float(x[j])));
+            tc::tmem_st_32x32(tA + at + (uint32_t)(half * 64 + c0), t);
+        };
+        auto put_state = [&](uint32_t (&x)[32], int c0, float decay) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) x[j] = __float_as_uint(__uint_as_float(x[j]) * decay);
+            tc::tmem_st_32x32(tS + at + (uint32_t)(half * 64 + c0), x);
+        };
+#pragma unroll
+        for (int j = 0; j < 32; ++j) { v[j] = __float_as_uint(Sg[(size_t)j * DV]); w[j] = __float_as_uint(Sg[(size_t)(32 + j) * DV]); }
+        float decay = dcs[0];
+        for (int c = 0; c <= nc; ++c) {
+            if (c == nc) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) { Sg[(size_t)j * DV] = __uint_as_float(v[j]); Sg[(size_t)(32 + j) * DV] = __uint_as_float(w[j]); }
+                break;
+            }
+            const uint32_t ph = (uint32_t)c & 1u;
+            copy_state(v, 0);
+            copy_state(w, 32);
+            tc::tmem_st_wait();
+            arrive(&s_ready);
+            load_u(c);
+            put_state(v, 0, decay);              // (seen by the product that adds to it through d_ready)
+            put_state(w, 32, decay);
+            if (c + 1 < nc) decay = dcs[(size_t)(c + 1) * Hv];
+            if (!wait(&m1_done, ph)) break;
+            tc::tmem_ld_32x32(tP + at + (uint32_t)(half * 32), v);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                v[4 * j] = __float_as_uint(to_tf32(u[j].x - __uint_as_float(v[4 * j])));
+                v[4 * j + 1] = __float_as_uint(to_tf32(u[j].y - __uint_as_float(v[4 * j + 1])));
+                v[4 * j + 2] = __float_as_uint(to_tf32(u[j].z - __uint_as_float(v[4 * j + 2])));
+                v[4 * j + 3] = __float_as_uint(to_tf32(u[j].w - __uint_as_float(v[4 * j + 3])));
+            }
+            tc::tmem_st_32x32(tD + at + (uint32_t)(half * 32), v);
+            tc::tmem_st_wait();
+            arrive(&d_ready);
+            if (!wait(&m2_done, ph)) break;
+            tc::tmem_ld_32x32(tS + at + (uint32_t)(half * 64), v);
+            tc::tmem_ld_32x32(tS + at + (uint32_t)(half * 64 + 32), w);
+            tc::tmem_ld_wait();
         }
     } else {
-        // ------------------------------------------------ state, Delta and outputs
-        const int quad = warp & 3, n0 = (warp >> 2) * 32, row = quad * 32 + lane;         // row: TMEM lane
-        const uint32_t at = ((uint32_t)(quad * 32) << 16) + (uint32_t)n0;
-        float* Sg = a.state + (((size_t)sd.slot * Hv + h) * DK + row) * DV + c0 + n0;
-        const float* dcs = a.dc + (size_t)gc * Hv + h;
-        auto wait = [&](uint64_t* bar, uint32_t ph) {
-            const bool ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(bar, ph, a.budget, &s_abort));
-            if (ok) tc::fence_after_sync();
-            return ok;
-        };
-        // state row `row`, columns n0 .. + 31: TF32 copy as the operand S^T, and the accumulator scaled by the chunk's decay
-        auto put_state = [&](uint32_t (&v)[32], float decay) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const int n = n0 + j;
-                *reinterpret_cast<float*>(sS + quad * (kSlice * 128) + n * 128 + (((lane >> 2) ^ (n & 7)) << 4) + (lane & 3) * 4) = to_tf32(__uint_as_float(v[j]));
-                v[j] = __float_as_uint(__uint_as_float(v[j]) * decay);
+        // ------------------------------------------------ outputs: lane n = column of Dv
+        const int quad = warp & 3, n = quad * 32 + lane;
+        const uint32_t at = (uint32_t)(quad * 32) << 16;
+        // raw inputs of the sequence's last rows, for the convolution of later steps (the preparation has read what they replace)
+        {
+            constexpr int CH = 2 * DK + DV;
+            const int hk = h / (p.Hv / p.Hk), keep = min(p.ring, sd.n_rows);
+            __nv_bfloat16* hist = p.conv_state + ((size_t)sd.slot * Hv + h) * p.ring * CH;
+            for (int j = 0; j < keep; ++j) {
+                const int r = sd.n_rows - 1 - j;
+                const __nv_bfloat16* pr = p.proj + (size_t)(sd.row_start + r) * p.ld_proj;
+                __nv_bfloat16* dst = hist + (size_t)((sd.pos_start + r) % p.ring) * CH;
+                dst[n] = pr[hk * DK + n];
+                dst[DK + n] = pr[p.Hk * DK + hk * DK + n];
+                dst[2 * DK + n] = pr[2 * p.Hk * DK + h * DV + n];
             }
-            tc::tmem_st_32x32(d2 + at, v);
-            tc::tmem_st_wait();
-            tc::fence_proxy_async_smem();
-        };
-        auto arrive = [&](uint64_t* bar) {
-            tc::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(bar);
-        };
-        uint32_t v[32];
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-            const uint4 q = *reinterpret_cast<const uint4*>(Sg + j);
-            v[j] = q.x; v[j + 1] = q.y; v[j + 2] = q.z; v[j + 3] = q.w;
         }
-        put_state(v, dcs[0]);
-        arrive(&s_ready);
+        float* op = a.o + ((size_t)sd.row_start * Hv + h) * DV + n;
         for (int c = 0; c < nc; ++c) {
-            const uint32_t ph = (uint32_t)c & 1u;
-            const float next = c + 1 < nc ? dcs[(size_t)(c + 1) * Hv] : 1.f;
-            if (quad < 2) {
-                if (!wait(&m1_done, ph) || !wait(&u_full, ph)) break;
-                tc::tmem_ld_32x32(d1 + at, v);
-                tc::tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const int n = n0 + j;
-                    *reinterpret_cast<float*>(sD + quad * (kSlice * 128) + n * 128 + (((lane >> 2) ^ (n & 7)) << 4) + (lane & 3) * 4) =
-                        to_tf32(sU[n * kChunk + row] - __uint_as_float(v[j]));
-                }
-                tc::fence_proxy_async_smem();
-                arrive(&d_ready);
-            }
-            if (!wait(&m2_done, ph)) break;
-            tc::tmem_ld_32x32(d2 + at, v);
+            const int b = c & 1, rows = sd.n_rows - c * kChunk;
+            if (!wait(&m3_done[b], (uint32_t)(c >> 1) & 1u)) break;
+            uint32_t x[32], y[32];
+            tc::tmem_ld_32x32(tR + 64 * b + at, x);
+            tc::tmem_ld_32x32(tR + 64 * b + at + 32, y);
             tc::tmem_ld_wait();
-            if (c + 1 < nc) put_state(v, next);
-            else {
+            arrive(&r_free[b]);
+            float* o = op + (size_t)c * kChunk * (Hv * DV);
 #pragma unroll
-                for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(Sg + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-            }
-            if (quad >= 2) {
-                if (!wait(&m3_done, ph)) break;
-                tc::tmem_ld_32x32(d1 + at, v);
-                tc::tmem_ld_wait();
-            }
-            arrive(&s_ready);
-            const int r = c * kChunk + row - 64;
-            if (quad >= 2 && r < sd.n_rows) {
-                float* o = a.o + ((size_t)(sd.row_start + r) * Hv + h) * DV + c0 + n0;
+            for (int j = 0; j < 32; ++j) if (j < rows) o[(size_t)j * (Hv * DV)] = __uint_as_float(x[j]);
 #pragma unroll
-                for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(o + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-            }
+            for (int j = 0; j < 32; ++j) if (32 + j < rows) o[(size_t)(32 + j) * (Hv * DV)] = __uint_as_float(y[j]);
         }
     }
     tc::fence_before_sync();
@@ -1005,14 +1024,15 @@ __global__ void __launch_bounds__(320, 1) gdn_chunk_scan_umma_kernel(const GdnSc
         set_status(a.status, PS_DEV_WAIT_TIMEOUT);
         // copies still in flight get a bounded chance to land before the shared memory goes back to the next CTA
         const long long b = a.budget < 4000000ll ? a.budget : 4000000ll;
-        if (s_wq > 0) tc::mbar_wait(&wq_full, (uint32_t)(s_wq - 1) & 1u, b);
-        if (s_u > 0) tc::mbar_wait(&u_full, (uint32_t)(s_u - 1) & 1u, b);
-        if (s_kq > 0) tc::mbar_wait(&kq_full, (uint32_t)(s_kq - 1) & 1u, b);
+        for (int c = max(0, s_filled - 2); c < s_filled; ++c) {
+            tc::mbar_wait(&wq_full[c & 1], (uint32_t)(c >> 1) & 1u, b);
+            tc::mbar_wait(&kq_full[c & 1], (uint32_t)(c >> 1) & 1u, b);
+        }
     }
     __syncthreads();
-    if (warp == 9) {
+    if (warp == 13) {
         tc::fence_after_sync();
-        tc::tmem_dealloc(d1, 128);
+        tc::tmem_dealloc(base, 512);
     }
 }
 
@@ -1028,8 +1048,19 @@ __global__ void __launch_bounds__(256) gdn_post_kernel(const float* o, const __n
     const int row = item / Hv, h = item % Hv;
     if (row_slot[row] < 0 || !row_is_chunked(seqs, n_seqs, min_rows, row)) return;
     float v[E], z[E], w[E];
-    const float* op = o + ((size_t)row * Hv + h) * Dv + lane * E;
     const __nv_bfloat16* zp = proj + (size_t)row * ld_proj + z_off + h * Dv + lane * E;
+    // (the projection and the weights are older than the kernel that wrote `o`)
+    if (E == 4 && ld_proj % 4 == 0 && z_off % 4 == 0 && (uintptr_t)proj % 8 == 0 && (uintptr_t)norm_w % 8 == 0) {
+        const uint2 zb = *reinterpret_cast<const uint2*>(zp), wb = *reinterpret_cast<const uint2*>(norm_w + lane * E);
+        const float2 z0 = bf16x2_bits_to_f32x2(zb.x), z1 = bf16x2_bits_to_f32x2(zb.y), w0 = bf16x2_bits_to_f32x2(wb.x), w1 = bf16x2_bits_to_f32x2(wb.y);
+        z[0] = z0.x; z[1] = z0.y; z[E - 2] = z1.x; z[E - 1] = z1.y;
+        w[0] = w0.x; w[1] = w0.y; w[E - 2] = w1.x; w[E - 1] = w1.y;
+    } else {
+#pragma unroll
+        for (int e = 0; e < E; ++e) { z[e] = bf16_to_f32(zp[e]); w[e] = bf16_to_f32(norm_w[lane * E + e]); }
+    }
+    cudaGridDependencySynchronize();
+    const float* op = o + ((size_t)row * Hv + h) * Dv + lane * E;
     if constexpr (E == 4) {
         const float4 f = *reinterpret_cast<const float4*>(op);
         v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
@@ -1037,17 +1068,20 @@ __global__ void __launch_bounds__(256) gdn_post_kernel(const float* o, const __n
 #pragma unroll
         for (int e = 0; e < E; ++e) v[e] = op[e];
     }
-#pragma unroll
-    for (int e = 0; e < E; ++e) { z[e] = bf16_to_f32(zp[e]); w[e] = bf16_to_f32(norm_w[lane * E + e]); }
     float ss = 0.f;
 #pragma unroll
     for (int e = 0; e < E; ++e) ss = fmaf(v[e], v[e], ss);
     ss = warp_sum(ss);
     const float inv = rsqrtf(ss / (float)Dv + eps);
     __nv_bfloat16* dst = out + (size_t)row * (Hv * Dv) + h * Dv + lane * E;
+    uint32_t y[E / 2];
 #pragma unroll
-    for (int e = 0; e < E; e += 2)
-        *reinterpret_cast<__nv_bfloat162*>(dst + e) = __floats2bfloat162_rn(v[e] * inv * w[e] * silu_f(z[e]), v[e + 1] * inv * w[e + 1] * silu_f(z[e + 1]));
+    for (int e = 0; e < E; e += 2) y[e / 2] = f32x2_to_bf16x2_bits(v[e] * inv * w[e] * silu_f(z[e]), v[e + 1] * inv * w[e + 1] * silu_f(z[e + 1]));
+    if (E == 4 && (uintptr_t)out % 8 == 0) *reinterpret_cast<uint2*>(dst) = make_uint2(y[0], y[E / 2 - 1]);
+    else {
+#pragma unroll
+        for (int e = 0; e < E / 2; ++e) *reinterpret_cast<uint32_t*>(dst + 2 * e) = y[e];
+    }
 }
 
 }  // namespace ps
@@ -1062,14 +1096,14 @@ PS_API long long ps_gdn_chunked_scratch_floats(int rows, int n_seqs, int Hv, int
 
 namespace ps {
 template <int DK, int DV>
-static int launch_chunked(const GdnPrepArgs& p, const GdnScanArgs& s, int max_chunks, cudaStream_t stream) {
+static int launch_chunked(const GdnPrepArgs& p, const GdnScanArgs& s, const __nv_bfloat16* norm_w, float eps, __nv_bfloat16* out, int rows, int max_chunks,
+                          cudaStream_t stream) {
     const size_t raw_b = (size_t)(kChunk + 3) * (2 * DK) * 2, at_b = sizeof(float) * (kChunk * 65 + kChunk * kTP + 32 * 36);
     const size_t smem_a = sizeof(float) * (2 * kChunk * (DK + 4) + 2 * kChunk) + (raw_b > at_b ? raw_b : at_b);
     const size_t smem_b = sizeof(float) * (3 * kChunk * (DK + 4) + DK * (kSlice + 4) + kChunk * (kSlice + 4) + kChunk * 65);
     const size_t smem_t = sizeof(float) * (2 * kChunk * (DK + 4) + kChunk * (DK + 8) + DK * (kSlice + 8) + kChunk * (kSlice + 8) +
                                            kChunk * (kChunk + 4));
-    // a chunk's tiles, S^T, Delta^T and U^T of the tcgen05 scan, and slack for their alignment
-    const size_t smem_u = sizeof(float) * (2 * kChunk * DK + DK * kChunk + 2 * kChunk * kChunk + kSlice * DK + 2 * kSlice * kChunk) + 1024;
+    const size_t smem_u = 2 * kScanStageBytes + 1024;        // the tiles of two chunks of the tcgen05 scan, and slack for their alignment
     static bool set = false;
     static int use_tc = 1;
     constexpr bool kUmma = DK == 128 && DV == 128;
@@ -1085,14 +1119,22 @@ static int launch_chunked(const GdnPrepArgs& p, const GdnScanArgs& s, int max_ch
     GdnPrepArgs pp = p;
     pp.round_tf32 = use_tc;
     pp.images = use_tc && kUmma;
-    gdn_chunk_prep_kernel<DK, DV><<<dim3(max_chunks, p.Hv), 256, smem_a, stream>>>(pp);
+    gdn_chunk_prep_kernel<DK, DV><<<dim3(max_chunks, p.Hv), kPrepThreads, smem_a, stream>>>(pp);
     int err = PS_LAUNCH_CHECK();
     if (err) return err;
     const dim3 grid(DV / kSlice, p.Hv, p.n_seqs);
-    if (!use_tc) gdn_chunk_scan_kernel<DK, DV><<<grid, 256, smem_b, stream>>>(s);
-    else if constexpr (kUmma) gdn_chunk_scan_umma_kernel<DK, DV><<<grid, 320, smem_u, stream>>>(s);
-    else gdn_chunk_scan_tc_kernel<DK, DV><<<grid, 256, smem_t, stream>>>(s);
-    return PS_LAUNCH_CHECK();
+    if (use_tc && kUmma) {
+        if constexpr (kUmma) err = launch_pdl(gdn_chunk_scan_umma_kernel<DK, DV>, dim3(p.Hv, p.n_seqs), dim3(kScanThreads), smem_u, stream, s, p);
+    } else {
+        if (!use_tc) gdn_chunk_scan_kernel<DK, DV><<<grid, 256, smem_b, stream>>>(s);
+        else if constexpr (!kUmma) gdn_chunk_scan_tc_kernel<DK, DV><<<grid, 256, smem_t, stream>>>(s);
+        if ((err = PS_LAUNCH_CHECK())) return err;
+        gdn_history_kernel<<<dim3(p.Hv, p.ring, p.n_seqs), 128, 0, stream>>>(p);
+        err = PS_LAUNCH_CHECK();
+    }
+    if (err) return err;
+    return launch_pdl(gdn_post_kernel<DV / 32>, dim3((rows * p.Hv + 7) / 8), dim3(256), 0, stream, s.o, p.proj, p.ld_proj, 2 * p.Hk * DK + p.Hv * DV, norm_w, eps,
+                      p.Hv, rows, p.row_slot, out, p.seqs, p.n_seqs, p.min_rows);
 }
 }  // namespace ps
 
@@ -1115,19 +1157,7 @@ PS_API int ps_gdn_chunked(const void* proj, int ld_proj, int rows, int Hk, int H
     s.scratch = p.scratch; s.dc = p.dc; s.Hv = Hv; s.Dv = Dv; s.n_seqs = n_seqs; s.min_rows = min_rows; s.state = (float*)state; s.seqs = p.seqs;
     s.o = (float*)o; s.status = (uint32_t*)status; s.budget = g_ps_wait_budget_cycles;
     const int max_chunks = (rows + kChunk - 1) / kChunk + n_seqs;
-    int err;
-    if (Dk == 128 && Dv == 128) err = launch_chunked<128, 128>(p, s, max_chunks, stream);
-    else if (Dk == 64 && Dv == 64) err = launch_chunked<64, 64>(p, s, max_chunks, stream);
-    else return (int)cudaErrorInvalidValue;
-    if (err) return err;
-    gdn_history_kernel<<<dim3(Hv, ring, n_seqs), 128, 0, stream>>>(p);
-    if ((err = PS_LAUNCH_CHECK())) return err;
-    const int post_grid = (rows * Hv + 7) / 8, z_off = 2 * Hk * Dk + Hv * Dv;
-    if (Dv == 128)
-        gdn_post_kernel<4><<<post_grid, 256, 0, stream>>>((const float*)o, (const __nv_bfloat16*)proj, ld_proj, z_off, (const __nv_bfloat16*)norm_w,
-                                                         eps, Hv, rows, (const int*)row_slot, (__nv_bfloat16*)out, p.seqs, n_seqs, min_rows);
-    else
-        gdn_post_kernel<2><<<post_grid, 256, 0, stream>>>((const float*)o, (const __nv_bfloat16*)proj, ld_proj, z_off, (const __nv_bfloat16*)norm_w,
-                                                         eps, Hv, rows, (const int*)row_slot, (__nv_bfloat16*)out, p.seqs, n_seqs, min_rows);
-    return PS_LAUNCH_CHECK();
+    if (Dk == 128 && Dv == 128) return launch_chunked<128, 128>(p, s, (const __nv_bfloat16*)norm_w, eps, (__nv_bfloat16*)out, rows, max_chunks, stream);
+    if (Dk == 64 && Dv == 64) return launch_chunked<64, 64>(p, s, (const __nv_bfloat16*)norm_w, eps, (__nv_bfloat16*)out, rows, max_chunks, stream);
+    return (int)cudaErrorInvalidValue;
 }

@@ -624,7 +624,7 @@ class CudaOps(OpTrace):
                       c_int(Dv), ptr(gw.conv_w), ptr(gw.A_log), ptr(gw.dt_bias), ptr(gw.norm_w),
                       c_float(cfg.rms_norm_eps), ptr(gs.conv), c_int(st.sc.conv_ring), ptr(gs.rec), ptr(b.seq_desc),
                       c_int(n_seqs), ptr(b.row_slot), ptr(b.row_pos), c_int(T), ptr(scr), ptr(dc), ptr(o), ptr(out), ptr(self.status))
-            self.launches += 4
+            self.launches += 3 if (Dk, Dv) == (128, 128) else 4
             del long_rows
         if any_short:
             lk = ld = ldd = None
