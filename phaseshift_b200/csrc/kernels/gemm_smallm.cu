@@ -186,18 +186,19 @@ struct SmallMReduceArgs {
     const __nv_bfloat16* norm_w; float eps; __nv_bfloat16* normed; int ld_normed;      // gemm_smallm_norm_kernel
 };
 
-// Sum of the splits of four neighbouring columns (c a multiple of 4) of row m, in ascending order; four loads in flight.
+// Sum of the splits of four neighbouring columns (c a multiple of 4) of row m, in ascending order; eight loads in flight (their latency is
+// most of a reduction: with four, fourteen splits took four round trips to L2).
 __device__ __forceinline__ float4 smallm_sum4(const SmallMReduceArgs& a, int m, int c) {
     const float4* p = reinterpret_cast<const float4*>(a.partial + (size_t)m * a.N + c);
     const size_t step = (size_t)a.M * a.N / 4;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    int s = 0;
-    for (; s + 4 <= a.splits; s += 4) {
-        const float4 q[4] = {p[s * step], p[(s + 1) * step], p[(s + 2) * step], p[(s + 3) * step]};
+    for (int s = 0; s < a.splits; s += 8) {
+        float4 q[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) { v.x += q[i].x; v.y += q[i].y; v.z += q[i].z; v.w += q[i].w; }
+        for (int i = 0; i < 8; ++i) if (s + i < a.splits) q[i] = p[(s + i) * step];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) if (s + i < a.splits) { v.x += q[i].x; v.y += q[i].y; v.z += q[i].z; v.w += q[i].w; }
     }
-    for (; s < a.splits; ++s) { const float4 q = p[s * step]; v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w; }
     return v;
 }
 __device__ __forceinline__ float smallm_gated(const SmallMReduceArgs& a, float g, float u) {
