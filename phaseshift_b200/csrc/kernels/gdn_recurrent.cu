@@ -194,6 +194,182 @@ __global__ void __launch_bounds__(256) gdn_rows_kernel(const GdnArgs a) {
     }
 }
 
+// The same for sequences with several rows in the step (the rows of a drafted block, short prompts): what does not depend on the state --
+// convolution, norms, gates -- is prepared for eight rows at once, a warp per row, and the head norm and the gate follow for all eight;
+// between them a row costs the pass over the state and two barriers instead of six.  Every sum is formed in the order of the kernel
+// above, so rows have the same bits in both.  A single row takes longer here, hence two kernels.
+constexpr int kManyRows = 8;
+template <int DK, int DV>
+__global__ void __launch_bounds__(256) gdn_rows_many_kernel(const GdnArgs a) {
+    constexpr int CG = DV / 4, RG = 256 / CG, R = DK / RG, CH = 2 * DK + DV;
+    static_assert(DK % 32 == 0 && DV % 32 == 0, "a warp sums a row's channels in whole groups of 32");
+    __shared__ float s_qk[kManyRows][2 * DK], s_v[kManyRows][DV], s_o[kManyRows][DV];
+    __shared__ float s_row[kManyRows][5];                                // factors of q and k, k . q, beta, decay
+    __shared__ __align__(16) float s_part[RG][DV], s_partq[RG][DV];      // float4 accesses
+    __shared__ __align__(16) float s_vec[DV];
+
+    const int h = blockIdx.x;
+    const GdnSeqDesc sd = a.seqs[blockIdx.y];
+    if (sd.n_rows <= 0 || sd.n_rows > a.max_rows) return;
+    PS_CHECK(PS_SLOT_OK(sd.slot) && PS_ROWS_OK(sd.row_start, sd.n_rows) && sd.pos_start >= 0);
+    const int hk = h / (a.Hv / a.Hk);
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31, cg = t % CG, rg = t / CG;
+    const int q_off = hk * DK, k_off = a.Hk * DK + hk * DK, v_off = 2 * a.Hk * DK + h * DV;
+    const int z_off = 2 * a.Hk * DK + a.Hv * DV + h * DV;
+    const int b_off = 2 * a.Hk * DK + 2 * a.Hv * DV + h, a_off = b_off + a.Hv;
+
+    cudaTriggerProgrammaticLaunchCompletion();
+    float S[R][4];
+    {
+        // the recurrent state was last written by an earlier step, not by the stream predecessor
+        const float* sp = a.state_in + ((size_t)sd.slot * a.Hv + h) * DK * DV;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const float4 v = *reinterpret_cast<const float4*>(sp + (size_t)(rg + RG * r) * DV + cg * 4);
+            S[r][0] = v.x; S[r][1] = v.y; S[r][2] = v.z; S[r][3] = v.w;
+        }
+    }
+    cudaGridDependencySynchronize();
+    __nv_bfloat16* hist = a.conv_state + ((size_t)sd.slot * a.Hv + h) * a.ring * CH;
+    const float neg_expA = -__expf(a.A_log[h]);
+    const float dtb = a.dt_bias[h];
+
+    for (int first = 0; first < sd.n_rows; first += kManyRows) {
+        const int nb = min(kManyRows, sd.n_rows - first);
+        auto channel = [&](int c) { return c < DK ? q_off + c : (c < 2 * DK ? k_off + (c - DK) : v_off + (c - 2 * DK)); };
+        // ---- conv + SiLU for this head's channels
+        for (int i = t; i < nb * CH; i += 256) {
+            const int r = i / CH, c = i - r * CH, gc = channel(c), r_i = first + r, row = sd.row_start + r_i, pos = sd.pos_start + r_i;
+            const uint2 wraw = *reinterpret_cast<const uint2*>(a.conv_w + (size_t)gc * 4);
+            const float2 w01 = bf16x2_bits_to_f32x2(wraw.x), w23 = bf16x2_bits_to_f32x2(wraw.y);
+            float taps[3];
+#pragma unroll
+            for (int j = 1; j <= 3; ++j) {
+                float v = 0.f;
+                if (pos - j >= 0) {
+                    if (r_i - j >= 0) v = bf16_to_f32(a.proj[(size_t)(row - j) * a.ld_proj + gc]);
+                    else v = bf16_to_f32(hist[(size_t)((pos - j) % a.ring) * CH + c]);
+                }
+                taps[j - 1] = v;   // taps[0] = x_{t-1}, taps[2] = x_{t-3}
+            }
+            float y = w01.x * taps[2];
+            y = fmaf(w01.y, taps[1], y);
+            y = fmaf(w23.x, taps[0], y);
+            y = fmaf(w23.y, bf16_to_f32(a.proj[(size_t)row * a.ld_proj + gc]), y);
+            y = silu_f(y);
+            if (c < 2 * DK) s_qk[r][c] = y; else s_v[r][c - 2 * DK] = y;
+        }
+        __syncthreads();
+        // history of the sequence's last rows (what is still read of it lies before the first of these rows)
+        for (int i = t; i < nb * CH; i += 256) {
+            const int r = i / CH, c = i - r * CH, r_i = first + r;
+            if (r_i + a.ring >= sd.n_rows)
+                hist[(size_t)((sd.pos_start + r_i) % a.ring) * CH + c] = a.proj[(size_t)(sd.row_start + r_i) * a.ld_proj + channel(c)];
+        }
+        // ---- L2 norms, k.q, gates and (optionally) the beta / decay input projections of row `warp`
+        if (warp < nb) {
+            const int row = sd.row_start + first + warp;
+            const __nv_bfloat16* pr = a.proj + (size_t)row * a.ld_proj;
+            const float *q = s_qk[warp], *k = s_qk[warp] + DK;
+            float part[5] = {0.f, 0.f, 0.f, 0.f, 0.f};                  // lane w: the sum of warp w of the kernel above
+#pragma unroll
+            for (int w = 0; w < DK / 32; ++w) {
+                const float qv = q[32 * w + lane], kv = k[32 * w + lane];
+                const float qq = warp_sum(qv * qv), kk = warp_sum(kv * kv), qk = warp_sum(qv * kv);
+                if (lane == w) { part[0] = qq; part[1] = kk; part[4] = qk; }
+            }
+            if (a.ba_w != nullptr) {
+                const __nv_bfloat16* xr = a.xn + (size_t)row * a.ba_k;
+                const __nv_bfloat16* wb = a.ba_w + (size_t)h * a.ba_k;
+                const __nv_bfloat16* wa = a.ba_w + (size_t)(a.Hv + h) * a.ba_k;
+                for (int w = 0; w < 8; ++w) {
+                    float sb = 0.f, sa = 0.f;
+                    for (int i = (32 * w + lane) * 2; i < a.ba_k; i += 512) {
+                        const float2 xv = bf16x2_bits_to_f32x2(*reinterpret_cast<const uint32_t*>(xr + i));
+                        const float2 bv = bf16x2_bits_to_f32x2(__ldg(reinterpret_cast<const uint32_t*>(wb + i)));
+                        const float2 av = bf16x2_bits_to_f32x2(__ldg(reinterpret_cast<const uint32_t*>(wa + i)));
+                        sb = fmaf(xv.x, bv.x, sb); sb = fmaf(xv.y, bv.y, sb);
+                        sa = fmaf(xv.x, av.x, sa); sa = fmaf(xv.y, av.y, sa);
+                    }
+                    sb = warp_sum(sb); sa = warp_sum(sa);
+                    if (lane == w) { part[2] = sb; part[3] = sa; }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 5; ++i) part[i] = warp_sum(part[i]);
+            const float qn = rsqrtf(part[0] + 1e-6f) * rsqrtf((float)DK), kn = rsqrtf(part[1] + 1e-6f);
+            const float b_in = a.ba_w != nullptr ? bf16_to_f32(f32_to_bf16(part[2])) : bf16_to_f32(pr[b_off]);
+            const float a_in = a.ba_w != nullptr ? bf16_to_f32(f32_to_bf16(part[3])) : bf16_to_f32(pr[a_off]);
+            const float gate = neg_expA * softplus_f(a_in + dtb), d = __expf(gate);
+            if (lane == 0) { s_row[warp][0] = qn; s_row[warp][1] = kn; s_row[warp][2] = part[4] * qn * kn; s_row[warp][3] = sigmoid_f(b_in); s_row[warp][4] = d; }
+            if (a.log_k) {
+                for (int i = lane; i < DK; i += 32) a.log_k[((size_t)row * a.Hv + h) * DK + i] = k[i] * kn;
+                if (lane == 0) a.log_d[(size_t)row * a.Hv + h] = d;
+            }
+        }
+        __syncthreads();
+        // ---- row after row: one pass over the state each
+        for (int r = 0; r < nb; ++r) {
+            const float qn = s_row[r][0], kn = s_row[r][1], kq = s_row[r][2], beta = s_row[r][3], d = s_row[r][4];
+            float kreg[R], qreg[R];
+#pragma unroll
+            for (int j = 0; j < R; ++j) { kreg[j] = s_qk[r][DK + rg + RG * j] * kn; qreg[j] = s_qk[r][rg + RG * j] * qn; }
+            float p[4] = {0.f, 0.f, 0.f, 0.f}, pq[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) { S[j][c] *= d; p[c] = fmaf(S[j][c], kreg[j], p[c]); pq[c] = fmaf(S[j][c], qreg[j], pq[c]); }
+            }
+            *reinterpret_cast<float4*>(&s_part[rg][cg * 4]) = make_float4(p[0], p[1], p[2], p[3]);
+            *reinterpret_cast<float4*>(&s_partq[rg][cg * 4]) = make_float4(pq[0], pq[1], pq[2], pq[3]);
+            __syncthreads();
+            if (t < DV) {
+                float kv = 0.f, qv = 0.f;
+#pragma unroll
+                for (int g = 0; g < RG; ++g) { kv += s_part[g][t]; qv += s_partq[g][t]; }
+                const float delta = (s_v[r][t] - kv) * beta;
+                s_vec[t] = delta;
+                s_o[r][t] = fmaf(kq, delta, qv);
+                if (a.log_delta) a.log_delta[((size_t)(sd.row_start + first + r) * a.Hv + h) * DV + t] = delta;
+            }
+            __syncthreads();
+            const float4 dl = *reinterpret_cast<const float4*>(&s_vec[cg * 4]);
+            const float dlr[4] = {dl.x, dl.y, dl.z, dl.w};
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) S[j][c] = fmaf(kreg[j], dlr[c], S[j][c]);
+            }
+        }
+        // ---- head norm and gate of row `warp`
+        if (warp < nb) {
+            const int row = sd.row_start + first + warp;
+            float part = 0.f;
+#pragma unroll
+            for (int w = 0; w < DV / 32; ++w) {
+                const float o = s_o[warp][32 * w + lane], sq = warp_sum(o * o);
+                if (lane == w) part = sq;
+            }
+            const float inv = rsqrtf(warp_sum(part) / (float)DV + a.eps);
+#pragma unroll
+            for (int w = 0; w < DV / 32; ++w) {
+                const int i = 32 * w + lane;
+                const float y = s_o[warp][i] * inv * bf16_to_f32(a.norm_w[i]);
+                const float z = bf16_to_f32(a.proj[(size_t)row * a.ld_proj + z_off + i]);
+                a.out[(size_t)row * (a.Hv * DV) + h * DV + i] = f32_to_bf16(y * silu_f(z));
+            }
+        }
+        __syncthreads();      // the rows' vectors are rewritten by the next ones
+    }
+    {
+        float* sp = a.state_out + ((size_t)sd.slot * a.Hv + h) * DK * DV;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            *reinterpret_cast<float4*>(sp + (size_t)(rg + RG * r) * DV + cg * 4) =
+                make_float4(S[r][0], S[r][1], S[r][2], S[r][3]);
+    }
+}
+
 struct GdnReplayArgs {
     float* state; int Hv;            // [slots, Hv, Dk, Dv]: old state, updated in place
     const GdnSeqDesc* seqs;          // n_rows = number of accepted rows to re-apply
@@ -237,17 +413,12 @@ __global__ void __launch_bounds__(256) gdn_replay_kernel(const GdnReplayArgs a) 
 
 PS_DEFINE_LIMITS_SETTER(gdn_recurrent)
 
-// Contract: the kernel may load the recurrent state of its slots BEFORE its stream predecessor has finished
-// (programmatic dependent launch): the predecessor must therefore not write `state_in` of those slots.  Inside the
-// engine that holds -- a projection kernel always sits between two GDN launches of one layer.  A caller that runs two
-// ps_gdn_rows back to back on one slot and state buffer must put another kernel (or an event) between them, or set
-// PS_PDL=0.
-PS_API int ps_gdn_rows(const void* proj, int ld_proj, int Hk, int Hv, int Dk, int Dv, const void* conv_w,
+namespace ps {
+static int gdn_rows(bool many, const void* proj, int ld_proj, int Hk, int Hv, int Dk, int Dv, const void* conv_w,
                        const void* A_log, const void* dt_bias, const void* norm_w, float eps, void* conv_state,
                        int ring, const void* state_in, void* state_out, const void* seqs, int n_seqs, void* out,
                        void* log_k, void* log_delta, void* log_d, const void* ba_w, const void* xn, int ba_k, int max_rows,
                        cudaStream_t stream) {
-    using namespace ps;
     if (n_seqs <= 0 || Hk <= 0 || (Hv % Hk) || ring < 4) return (int)cudaErrorInvalidValue;
     GdnArgs a;
     a.proj = (const __nv_bfloat16*)proj; a.ld_proj = ld_proj; a.Hk = Hk; a.Hv = Hv;
@@ -259,9 +430,34 @@ PS_API int ps_gdn_rows(const void* proj, int ld_proj, int Hk, int Hv, int Dk, in
     a.max_rows = max_rows > 0 ? max_rows : 0x7fffffff;
     if (ba_w != nullptr && (ba_k & 1)) return (int)cudaErrorInvalidValue;
     dim3 grid(Hv, n_seqs);
-    if (Dk == 128 && Dv == 128) return launch_pdl(gdn_rows_kernel<128, 128>, grid, dim3(256), 0, stream, a);
-    if (Dk == 64 && Dv == 64) return launch_pdl(gdn_rows_kernel<64, 64>, grid, dim3(256), 0, stream, a);
+    if (Dk == 128 && Dv == 128) return launch_pdl(many ? gdn_rows_many_kernel<128, 128> : gdn_rows_kernel<128, 128>, grid, dim3(256), 0, stream, a);
+    if (Dk == 64 && Dv == 64) return launch_pdl(many ? gdn_rows_many_kernel<64, 64> : gdn_rows_kernel<64, 64>, grid, dim3(256), 0, stream, a);
     return (int)cudaErrorInvalidValue;
+}
+}  // namespace ps
+
+// Contract: the kernel may load the recurrent state of its slots BEFORE its stream predecessor has finished
+// (programmatic dependent launch): the predecessor must therefore not write `state_in` of those slots.  Inside the
+// engine that holds -- a projection kernel always sits between two GDN launches of one layer.  A caller that runs two
+// ps_gdn_rows back to back on one slot and state buffer must put another kernel (or an event) between them, or set
+// PS_PDL=0.
+PS_API int ps_gdn_rows(const void* proj, int ld_proj, int Hk, int Hv, int Dk, int Dv, const void* conv_w,
+                       const void* A_log, const void* dt_bias, const void* norm_w, float eps, void* conv_state,
+                       int ring, const void* state_in, void* state_out, const void* seqs, int n_seqs, void* out,
+                       void* log_k, void* log_delta, void* log_d, const void* ba_w, const void* xn, int ba_k, int max_rows,
+                       cudaStream_t stream) {
+    return ps::gdn_rows(false, proj, ld_proj, Hk, Hv, Dk, Dv, conv_w, A_log, dt_bias, norm_w, eps, conv_state, ring, state_in, state_out, seqs, n_seqs, out, log_k,
+                        log_delta, log_d, ba_w, xn, ba_k, max_rows, stream);
+}
+
+// The same results, sooner where sequences have several rows.
+PS_API int ps_gdn_rows_many(const void* proj, int ld_proj, int Hk, int Hv, int Dk, int Dv, const void* conv_w,
+                       const void* A_log, const void* dt_bias, const void* norm_w, float eps, void* conv_state,
+                       int ring, const void* state_in, void* state_out, const void* seqs, int n_seqs, void* out,
+                       void* log_k, void* log_delta, void* log_d, const void* ba_w, const void* xn, int ba_k, int max_rows,
+                       cudaStream_t stream) {
+    return ps::gdn_rows(true, proj, ld_proj, Hk, Hv, Dk, Dv, conv_w, A_log, dt_bias, norm_w, eps, conv_state, ring, state_in, state_out, seqs, n_seqs, out, log_k,
+                        log_delta, log_d, ba_w, xn, ba_k, max_rows, stream);
 }
 
 PS_API int ps_gdn_replay(void* state, int Hv, int Dk, int Dv, const void* seqs, int n_seqs, const void* log_k,

@@ -630,7 +630,9 @@ class CudaOps(OpTrace):
             lk = ld = ldd = None
             if log is not None:
                 lk, ld, ldd = log
-            _lib.call("ps_gdn_rows", ptr(proj), c_int(proj.stride(0)), c_int(hk), c_int(hv), c_int(Dk), c_int(Dv),
+            # several rows of a sequence share their preparation in a kernel of their own; it has the same bits
+            many = any(1 < n <= T for n in seq_rows) if any_long else b.multi_rows
+            _lib.call("ps_gdn_rows_many" if many else "ps_gdn_rows", ptr(proj), c_int(proj.stride(0)), c_int(hk), c_int(hv), c_int(Dk), c_int(Dv),
                       ptr(gw.conv_w), ptr(gw.A_log), ptr(gw.dt_bias), ptr(gw.norm_w), c_float(cfg.rms_norm_eps),
                       ptr(gs.conv), c_int(st.sc.conv_ring), ptr(gs.rec), ptr(state_out), ptr(b.seq_desc),
                       c_int(n_seqs), ptr(out), ptr(lk), ptr(ld), ptr(ldd),

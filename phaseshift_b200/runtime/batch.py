@@ -65,6 +65,7 @@ class StepBatch:
         # depend on this step's contents (attention covers max_context, GDN covers max_seqs descriptors)
         self.graph_static = False
         self.identity_out = False
+        self.multi_rows = False          # some sequence has more than one row in the step
         self.max_context = 1
         o = 0
         self.ids = self.d_int[o:o + max_rows]; o += max_rows
@@ -86,6 +87,7 @@ class StepBatch:
         # (identity_out: output row i is step row i for every i -- a pure decode batch -- so the output gather is the identity)
         self.n_seqs = len(seqs)
         self.seqs = list(seqs)
+        self.multi_rows = self.n_rows > self.n_seqs
 
     @property
     def max_visible_launch(self) -> int:

@@ -25,7 +25,7 @@ from ..models.registry import family_of
 from .batch import SeqRows, StepBatch, resolve_row_bucket
 from .state import ModelState, StateConfig
 
-GRAPH_MAX_ROWS = 8
+GRAPH_MAX_ROWS = 16             # plain steps of any kind; the kernels of a sequence with more rows are chosen by its length
 GRAPH_MAX_DECODE_ROWS = 64      # pure decode batches (one row per sequence) are also replayed from graphs
 GRAPH_MAX_VARIANT_ROWS = 16     # tapped / logged steps (speculative verification) replayed from graphs of their own
 
@@ -388,6 +388,7 @@ class Engine:
         return toks, out
 
     GREEDY_KEY_BIT = 1 << 48
+    MULTI_KEY_BIT = 1 << 49          # some sequence has several rows, and the family has kernels of its own for those
 
     @classmethod
     def graph_key(cls, bucket: int, n_out: int, identity_out: bool, greedy: bool = False) -> int:
@@ -412,6 +413,8 @@ class Engine:
         recurrent updates get graphs of their own (the tap and log tensors are fixed buffers, so the capture stays
         valid; Exact mode only changes which kernels the host picks, which the capture bakes in)."""
         key = self.graph_key(bucket, n_out, b.identity_out, greedy)
+        if b.multi_rows and getattr(self.runner, "many_row_kernels", False):
+            key |= self.MULTI_KEY_BIT
         kw = {}
         if variant is not None:
             taps, log, to_alt, exact = variant
