@@ -161,6 +161,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     __shared__ uint32_t tmem_base_slot;
     __shared__ int s_abort, s_bad, k_issued, k_consumed, v_issued, v_consumed, q_issued, q_consumed;
 
+    cudaGridDependencySynchronize();             // (the descriptors may be the predecessor's)
     const int* sd = a.seqs + 4 * blockIdx.z;
     const int row_start = sd[0], n_rows = sd[1], slot = sd[2], pos_start = sd[3];
     const int G = a.Hq / a.Hkv;
@@ -219,6 +220,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     tc::fence_after_sync();
     const uint32_t tmem = tmem_base_slot;
     const uint32_t tmem_o = tmem + 128;
+    cudaTriggerProgrammaticLaunchCompletion();   // with its tensor memory in hand
 
     int exp_row0 = 0;            // EXPANDED: row of the sequence's position 0, were it there
     if constexpr (EXPANDED) exp_row0 = expanded_row0(a.seqs, (int)blockIdx.z, a.min_rows, a.opt);
@@ -646,8 +648,7 @@ static int launch_attn_tc(dim3 grid, const CUtensorMap& mq, const CUtensorMap& m
         cudaFuncSetAttribute(attn_tc_kernel<DK, DV, DEC, SHARED, TRANSFORM, EXPANDED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         set = true;
     }
-    attn_tc_kernel<DK, DV, DEC, SHARED, TRANSFORM, EXPANDED><<<grid, kTcThreads, smem, stream>>>(mq, mk, mv, mr, a);
-    return PS_LAUNCH_CHECK();
+    return launch_pdl(attn_tc_kernel<DK, DV, DEC, SHARED, TRANSFORM, EXPANDED>, grid, dim3(kTcThreads), smem, stream, mq, mk, mv, mr, a);
 }
 
 }  // namespace ps

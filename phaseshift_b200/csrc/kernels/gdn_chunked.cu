@@ -122,6 +122,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prep_kernel(const G
     float* sM = sT + kChunk * kTP;
 
     cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     GdnSeqDesc2 sd; int chunk;
     if (!find_chunk(a.seqs, a.n_seqs, a.min_rows, blockIdx.x, sd, chunk)) return;
     const int h = blockIdx.y, t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -865,6 +866,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(co
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
     const uint32_t base = tmem_slot, tS = base, tA = base + 128, tD = base + 256, tP = base + 320, tR = base + 384;      // tR: two of 64
     auto wait = [&](uint64_t* bar, uint32_t ph) {
@@ -1043,13 +1045,14 @@ __global__ void __launch_bounds__(256) gdn_post_kernel(const float* o, const __n
                                                        const __nv_bfloat16* norm_w, float eps, int Hv, int rows, const int* row_slot,
                                                        __nv_bfloat16* out, const GdnSeqDesc2* seqs, int n_seqs, int min_rows) {
     constexpr int Dv = 32 * E;
+    cudaTriggerProgrammaticLaunchCompletion();
     const int item = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (item >= rows * Hv) return;
     const int row = item / Hv, h = item % Hv;
     if (row_slot[row] < 0 || !row_is_chunked(seqs, n_seqs, min_rows, row)) return;
     float v[E], z[E], w[E];
     const __nv_bfloat16* zp = proj + (size_t)row * ld_proj + z_off + h * Dv + lane * E;
-    // (the projection and the weights are older than the kernel that wrote `o`)
+    cudaGridDependencySynchronize();
     if (E == 4 && ld_proj % 4 == 0 && z_off % 4 == 0 && (uintptr_t)proj % 8 == 0 && (uintptr_t)norm_w % 8 == 0) {
         const uint2 zb = *reinterpret_cast<const uint2*>(zp), wb = *reinterpret_cast<const uint2*>(norm_w + lane * E);
         const float2 z0 = bf16x2_bits_to_f32x2(zb.x), z1 = bf16x2_bits_to_f32x2(zb.y), w0 = bf16x2_bits_to_f32x2(wb.x), w1 = bf16x2_bits_to_f32x2(wb.y);
@@ -1059,7 +1062,6 @@ __global__ void __launch_bounds__(256) gdn_post_kernel(const float* o, const __n
 #pragma unroll
         for (int e = 0; e < E; ++e) { z[e] = bf16_to_f32(zp[e]); w[e] = bf16_to_f32(norm_w[lane * E + e]); }
     }
-    cudaGridDependencySynchronize();
     const float* op = o + ((size_t)row * Hv + h) * Dv + lane * E;
     if constexpr (E == 4) {
         const float4 f = *reinterpret_cast<const float4*>(op);
@@ -1119,8 +1121,7 @@ static int launch_chunked(const GdnPrepArgs& p, const GdnScanArgs& s, const __nv
     GdnPrepArgs pp = p;
     pp.round_tf32 = use_tc;
     pp.images = use_tc && kUmma;
-    gdn_chunk_prep_kernel<DK, DV><<<dim3(max_chunks, p.Hv), kPrepThreads, smem_a, stream>>>(pp);
-    int err = PS_LAUNCH_CHECK();
+    int err = launch_pdl(gdn_chunk_prep_kernel<DK, DV>, dim3(max_chunks, p.Hv), dim3(kPrepThreads), smem_a, stream, pp);
     if (err) return err;
     const dim3 grid(DV / kSlice, p.Hv, p.n_seqs);
     if (use_tc && kUmma) {

@@ -17,8 +17,8 @@
 // kernels here are launched programmatically, the product asks for its first 128 KB of weights per SM before its rows exist, and the
 // reduction of a residual product norms the rows for the next one (gemm_smallm_norm_kernel).
 // May a product that starts early hold what its predecessors need?  It takes up to 128 columns of tensor memory and 97 KB; a predecessor
-// that wants more than what is left (512 columns or 200 KB: attention, CTA-pair and block-scaled GEMMs) either never triggers early
-// or fills the SM by its shared memory, so both are never resident together.
+// that wants more than what is left (512 columns or 200 KB: attention, CTA-pair and block-scaled GEMMs) has it before it lets its
+// successors start, or fills the SM by its shared memory, so that both are never resident together.
 //
 // The reference serves this regime with its RowBlock2/4/8 WMMA kernels (src/phaseshift/models/qwen35/
 // kernels/optimized/linear/psq4.hip:221-349); here it runs from a bf16 expansion that 180 GB of HBM can

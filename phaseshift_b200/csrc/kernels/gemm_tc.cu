@@ -14,6 +14,9 @@
 // Warp roles: warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner, warps 2..5 = epilogue.
 // Every mbarrier wait is bounded; a timeout sets PS_DEV_WAIT_TIMEOUT in the status word, the CTA
 // stops issuing, frees its tensor memory and returns.
+// The kernels are launched programmatically: a prompt is a chain of products, norms and mixers of 5 to 100 us whose set-up and, for CTA
+// pairs, first weights need not wait for the one before.  They take tensor memory only when their predecessors are done, and let their
+// successor start when they have it, so that nobody who waits holds what another needs.
 //
 // The reference's counterpart is its WMMA bf16 family (src/phaseshift/models/qwen35/kernels/optimized/
 // linear/bf16.hip:10-339) and the Prefill2D PSQ kernels (linear/psq4.hip:505-667); quantised weights
@@ -148,6 +151,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         tc::tma_prefetch_desc(&map_a);
         tc::tma_prefetch_desc(&map_w);
     }
+    cudaGridDependencySynchronize();
     if (warp == 1) {
         tc::tmem_alloc(&tmem_base_slot, BN);       // BN fp32 columns x 128 lanes
         tc::tmem_relinquish();
@@ -156,6 +160,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem_acc = tmem_base_slot;
+    cudaTriggerProgrammaticLaunchCompletion();
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
@@ -272,22 +277,37 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         tc::tma_prefetch_desc(&map_a);
         tc::tma_prefetch_desc(&map_w);
     }
+    __syncthreads();
+    tc::cluster_sync();              // both CTAs' barriers exist before either signals the other's
+    const uint32_t full0 = tc::cluster_addr(&full_bar[0], 0);
+    const uint32_t stage_bytes = 2 * kABytes + p.bn * kBK * 2;
+    const int early = min(k_iters, kPairStages);
+    if (warp == 0 && tc::elect_one()) {
+        // the first weights are on their way before the kernel that writes the rows is done
+        int tm, tn;
+        place(pair, tm, tn);         // (every pair has a tile)
+        for (int k = 0; k < early; ++k) {
+            if (rank == 0) tc::mbar_expect_tx(&full_bar[k], stage_bytes);
+            tc::tma_load_2d_pair(smem + k * kPairStageBytes + kABytes, &map_w, k * kBK, tn * p.bn + (int)rank * (p.bn >> 1), full0 + 8 * k);
+        }
+    }
+    __syncwarp();
+    cudaGridDependencySynchronize();
     if (warp == 1) {
         tc::tmem_alloc_pair(&tmem_base_slot, 512);
         tc::tmem_relinquish_pair();
     }
     tc::fence_before_sync();
     __syncthreads();
-    tc::cluster_sync();              // both CTAs' barriers exist before either signals the other's
+    tc::cluster_sync();
     tc::fence_after_sync();
     const uint32_t tmem_acc = tmem_base_slot;
+    cudaTriggerProgrammaticLaunchCompletion();
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer: this CTA's half of both operands
         if (tc::elect_one()) {
-            const uint32_t full0 = tc::cluster_addr(&full_bar[0], 0);
-            const uint32_t bytes = 2 * kABytes + p.bn * kBK * 2;
-            int s = 0;
+            int s = 0, ahead = early;
             uint32_t ph = 1;                 // the first round finds every stage free
             bool ok = true;
             for (int t = pair; t < p.tiles && ok; t += pairs) {
@@ -295,12 +315,17 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                 place(t, tm, tn);
                 const int ra = tm * kPairBM + (int)rank * kBM, rw = tn * p.bn + (int)rank * (p.bn >> 1);
                 for (int k = 0; k < k_iters; ++k) {
-                    ok = tc::mbar_wait_abortable(&empty_bar[s], ph, g.budget, &s_abort);
-                    if (!ok) break;
                     unsigned char* st = smem + s * kPairStageBytes;
-                    if (rank == 0) tc::mbar_expect_tx(&full_bar[s], bytes);
-                    tc::tma_load_2d_pair(st, &map_a, k * kBK, ra, full0 + 8 * s);
-                    tc::tma_load_2d_pair(st + kABytes, &map_w, k * kBK, rw, full0 + 8 * s);
+                    if (ahead > 0) {
+                        --ahead;
+                        tc::tma_load_2d_pair(st, &map_a, k * kBK, ra, full0 + 8 * s);
+                    } else {
+                        ok = tc::mbar_wait_abortable(&empty_bar[s], ph, g.budget, &s_abort);
+                        if (!ok) break;
+                        if (rank == 0) tc::mbar_expect_tx(&full_bar[s], stage_bytes);
+                        tc::tma_load_2d_pair(st, &map_a, k * kBK, ra, full0 + 8 * s);
+                        tc::tma_load_2d_pair(st + kABytes, &map_w, k * kBK, rw, full0 + 8 * s);
+                    }
                     if (++s == kPairStages) { s = 0; ph ^= 1u; }
                 }
             }
@@ -424,8 +449,7 @@ static int launch_gemm(const void* a, int lda, const void* w, int ldw, const Gem
         attr_set = true;
     }
     dim3 grid(((g.N + BN - 1) / BN) * ((g.M + kBM - 1) / kBM));
-    gemm_bf16_tc_kernel<BN, kGemmStages, kMinBlocks><<<grid, kGemmThreads, smem, stream>>>(map_a, map_w, g);
-    return PS_LAUNCH_CHECK();
+    return launch_pdl(gemm_bf16_tc_kernel<BN, kGemmStages, kMinBlocks>, grid, dim3(kGemmThreads), smem, stream, map_a, map_w, g);
 }
 
 // W rows of a pair's tile: the pairs work in waves of 74 tiles, so the width is chosen that loses least in the last wave.  A tile
@@ -461,8 +485,7 @@ static int launch_pair(const void* a, int lda, const void* w, int ldw, const Gem
         attr_set = true;
     }
     const int pairs = p.tiles < sms / 2 ? p.tiles : sms / 2;
-    gemm_bf16_pair_kernel<<<2 * pairs, kPairThreads, smem, stream>>>(map_a, map_w, p);
-    return PS_LAUNCH_CHECK();
+    return launch_pdl(gemm_bf16_pair_kernel, dim3(2 * pairs), dim3(kPairThreads), smem, stream, map_a, map_w, p);
 }
 
 }  // namespace ps

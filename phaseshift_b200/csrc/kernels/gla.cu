@@ -215,6 +215,8 @@ __global__ void __launch_bounds__(kGPrepThreads) gla_prepare_kernel(const GlaArg
     __nv_bfloat16* sV = reinterpret_cast<__nv_bfloat16*>(sB);       // [64][PV]
     float* sA = sB + kGC * max(PQ, PV / 2);             // [64][68]
     float* sE = sA + kGC * kGAPitch;                    // [4][dk]  B at the end of each 16-row sub-block
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     int seq, row0, n;
     if (!gla_find_block(a, blockIdx.x, seq, row0, n)) return;
     const int h = blockIdx.y, t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tq = lane & 3;
@@ -501,6 +503,8 @@ __global__ void __launch_bounds__(kGPrepThreads) gla_prepare_kernel(const GlaArg
 
 // grid = (ceil(H * dk * dv / 4 / 256), n_seqs): a thread carries four state elements through the sequence's blocks.
 __global__ void __launch_bounds__(256) gla_scan_kernel(const GlaArgs a) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     const GlaSeq sd = a.seqs[blockIdx.y];
     if (sd.slot < 0 || sd.n_rows <= a.rows_limit) return;
     const size_t per = (size_t)a.H * a.dk * a.dv;
@@ -543,6 +547,8 @@ __global__ void __launch_bounds__(kGOutThreads, 2) gla_output_kernel(const GlaAr
     const int PQ = dk + 4, PS = dv + 8;
     float* sQ = gla_smem;                                  // [64][PQ]
     float* sS = sQ + kGC * PQ;                             // [dk][PS]
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     int seq, row0, n;
     if (!gla_find_block(a, blockIdx.x, seq, row0, n)) return;
     const int h = blockIdx.y, t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tq = lane & 3;
@@ -637,14 +643,11 @@ static int launch_gla_chunked(const GlaArgs& a, int blocks, cudaStream_t stream)
         cudaFuncSetAttribute(gla_output_kernel<DKT, DVT, FORGET>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
         set = true;
     }
-    gla_prepare_kernel<DKT, DVT, FORGET><<<dim3(blocks, a.H), kGPrepThreads, s1, stream>>>(a);
-    int e = PS_LAUNCH_CHECK();
+    int e = launch_pdl(gla_prepare_kernel<DKT, DVT, FORGET>, dim3(blocks, a.H), dim3(kGPrepThreads), s1, stream, a);
     if (e) return e;
     const long long groups = (long long)a.H * a.dk * a.dv / 4;
-    gla_scan_kernel<<<dim3((unsigned)((groups + 255) / 256), a.n_seqs), 256, 0, stream>>>(a);
-    if ((e = PS_LAUNCH_CHECK())) return e;
-    gla_output_kernel<DKT, DVT, FORGET><<<dim3(blocks, a.H), kGOutThreads, s2, stream>>>(a);
-    return PS_LAUNCH_CHECK();
+    if ((e = launch_pdl(gla_scan_kernel, dim3((unsigned)((groups + 255) / 256), a.n_seqs), dim3(256), 0, stream, a))) return e;
+    return launch_pdl(gla_output_kernel<DKT, DVT, FORGET>, dim3(blocks, a.H), dim3(kGOutThreads), s2, stream, a);
 }
 
 template <bool FORGET>
