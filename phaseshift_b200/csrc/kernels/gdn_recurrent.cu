@@ -42,13 +42,24 @@ struct GdnArgs {
     int max_rows;                               // sequences with more rows in this step belong to the chunked kernels
 };
 
+// Sums over a CTA's warps: what warp_sum gives of the warps' sums in the first lanes (absent ones are 0).
+__device__ __forceinline__ float gdn_sum4(const float* p) { return (p[0] + p[2]) + (p[1] + p[3]); }
+__device__ __forceinline__ float gdn_sum8(const float* p) { return ((p[0] + p[4]) + (p[2] + p[6])) + ((p[1] + p[5]) + (p[3] + p[7])); }
+
+// A CTA is a chain of loads, sums and barriers, most of it latency; with many sequences the chip holds two CTAs per SM and a launch
+// takes as many such chains as there are rounds of them.  So what the predecessor has not written -- state, history, weights -- is
+// loaded before the wait for it, a thread keeps its channels' convolution in registers, and three barriers are left of eight: after the
+// channels and the warps' sums, after the pass over the state, after Delta.  One row through 32 heads of 128: 11.2 -> 7.7 us, 12
+// sequences 21.3 -> 14.7; 32 sequences through 48 heads 63 -> 42.7 (the state alone, read and written once, takes 31 of measured).
 template <int DK, int DV>
-__global__ void __launch_bounds__(256) gdn_rows_kernel(const GdnArgs a) {
+__global__ void __launch_bounds__(256, 2) gdn_rows_kernel(const GdnArgs a) {
     constexpr int CG = DV / 4;          // column groups of 4 consecutive columns
     constexpr int RG = 256 / CG;        // row groups
     constexpr int R = DK / RG;          // rows per thread
     constexpr int CH = 2 * DK + DV;     // conv channels owned by this head
-    __shared__ float s_q[DK], s_k[DK], s_v[DV], s_red[32], s_red4[192];
+    constexpr int NC = (CH + 255) / 256, G = DK / 32;
+    static_assert(2 * DK <= 256 && G <= 4 && DV <= 128, "a warp holds 32 channels of q or of k");
+    __shared__ float s_q[DK], s_k[DK], s_v[DV], s_sum[5][8], s_ss[4];     // sums of the warps: q.q, k.k, b, a, q.k; o.o
     __shared__ __align__(16) float s_part[RG][DV], s_partq[RG][DV];      // float4 accesses
     __shared__ __align__(16) float s_vec[DV];
 
@@ -57,15 +68,15 @@ __global__ void __launch_bounds__(256) gdn_rows_kernel(const GdnArgs a) {
     if (sd.n_rows <= 0 || sd.n_rows > a.max_rows) return;
     PS_CHECK(PS_SLOT_OK(sd.slot) && PS_ROWS_OK(sd.row_start, sd.n_rows) && sd.pos_start >= 0);
     const int hk = h / (a.Hv / a.Hk);
-    const int t = threadIdx.x, cg = t % CG, rg = t / CG;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31, cg = t % CG, rg = t / CG;
     const int q_off = hk * DK, k_off = a.Hk * DK + hk * DK, v_off = 2 * a.Hk * DK + h * DV;
     const int z_off = 2 * a.Hk * DK + a.Hv * DV + h * DV;
     const int b_off = 2 * a.Hk * DK + 2 * a.Hv * DV + h, a_off = b_off + a.Hv;
 
     cudaTriggerProgrammaticLaunchCompletion();
+    // ---- what was last written by an earlier step, not by the stream predecessor
     float S[R][4];
     {
-        // the recurrent state was last written by an earlier step, not by the stream predecessor
         const float* sp = a.state_in + ((size_t)sd.slot * a.Hv + h) * DK * DV;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -73,68 +84,87 @@ __global__ void __launch_bounds__(256) gdn_rows_kernel(const GdnArgs a) {
             S[r][0] = v.x; S[r][1] = v.y; S[r][2] = v.z; S[r][3] = v.w;
         }
     }
-    cudaGridDependencySynchronize();
     __nv_bfloat16* hist = a.conv_state + ((size_t)sd.slot * a.Hv + h) * a.ring * CH;
+    uint2 taps[NC];                      // the channel's four weights
+    __nv_bfloat16 past[NC][3];           // x_{t-1}, x_{t-2}, x_{t-3}
+#pragma unroll
+    for (int n = 0; n < NC; ++n) {
+        const int c = t + 256 * n;
+        taps[n] = make_uint2(0u, 0u);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) past[n][j] = __float2bfloat16(0.f);
+        if (c < CH) {
+            const int gc = c < DK ? q_off + c : (c < 2 * DK ? k_off + (c - DK) : v_off + (c - 2 * DK));
+            taps[n] = __ldg(reinterpret_cast<const uint2*>(a.conv_w + (size_t)gc * 4));
+#pragma unroll
+            for (int j = 1; j <= 3; ++j)
+                if (sd.pos_start - j >= 0) past[n][j - 1] = hist[(size_t)((sd.pos_start - j) % a.ring) * CH + c];
+        }
+    }
     const float neg_expA = -__expf(a.A_log[h]);
     const float dtb = a.dt_bias[h];
+    const float nw = t < DV ? bf16_to_f32(a.norm_w[t]) : 0.f;
+    if (t < 8) { s_sum[0][t] = s_sum[1][t] = s_sum[4][t] = 0.f; }
+    if (t < 4) s_ss[t] = 0.f;
+    __syncthreads();
+    cudaGridDependencySynchronize();
 
     for (int r_i = 0; r_i < sd.n_rows; ++r_i) {
         const int row = sd.row_start + r_i, pos = sd.pos_start + r_i;
         const __nv_bfloat16* pr = a.proj + (size_t)row * a.ld_proj;
-        // ---- conv + SiLU for this head's channels
-        for (int c = t; c < CH; c += 256) {
-            const int gc = c < DK ? q_off + c : (c < 2 * DK ? k_off + (c - DK) : v_off + (c - 2 * DK));
-            const uint2 wraw = *reinterpret_cast<const uint2*>(a.conv_w + (size_t)gc * 4);
-            const float2 w01 = bf16x2_bits_to_f32x2(wraw.x), w23 = bf16x2_bits_to_f32x2(wraw.y);
-            const __nv_bfloat16 xin = pr[gc];
-            float taps[3];
+        __nv_bfloat16 x[NC];
 #pragma unroll
-            for (int j = 1; j <= 3; ++j) {
-                float v = 0.f;
-                if (pos - j >= 0) {
-                    if (r_i - j >= 0) v = bf16_to_f32(a.proj[(size_t)(row - j) * a.ld_proj + gc]);
-                    else v = bf16_to_f32(hist[(size_t)((pos - j) % a.ring) * CH + c]);
-                }
-                taps[j - 1] = v;   // taps[0] = x_{t-1}, taps[2] = x_{t-3}
-            }
-            float y = w01.x * taps[2];
-            y = fmaf(w01.y, taps[1], y);
-            y = fmaf(w23.x, taps[0], y);
-            y = fmaf(w23.y, bf16_to_f32(xin), y);
-            y = silu_f(y);
-            if (c < DK) s_q[c] = y; else if (c < 2 * DK) s_k[c - DK] = y; else s_v[c - 2 * DK] = y;
+        for (int n = 0; n < NC; ++n) {
+            const int c = t + 256 * n, gc = c < DK ? q_off + c : (c < 2 * DK ? k_off + (c - DK) : v_off + (c - 2 * DK));
+            x[n] = c < CH ? pr[gc] : __float2bfloat16(0.f);
         }
-        __syncthreads();
-        // history write happens after every thread has read its taps for this row
-        for (int c = t; c < CH; c += 256) {
-            const int gc = c < DK ? q_off + c : (c < 2 * DK ? k_off + (c - DK) : v_off + (c - 2 * DK));
-            hist[(size_t)(pos % a.ring) * CH + c] = pr[gc];
-        }
-        // ---- L2 norms, k.q and (optionally) the beta / decay input projections: one fused block reduction
-        float red5[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int i = t; i < DK; i += 256) { red5[0] += s_q[i] * s_q[i]; red5[1] += s_k[i] * s_k[i]; red5[4] += s_q[i] * s_k[i]; }
-        if (a.ba_w != nullptr) {
+        const __nv_bfloat16 zb = t < DV ? pr[z_off + t] : __float2bfloat16(0.f);
+        float b_in = 0.f, a_in = 0.f;
+        if (a.ba_w == nullptr) { b_in = bf16_to_f32(pr[b_off]); a_in = bf16_to_f32(pr[a_off]); }
+        else {
+            // beta / decay input projections
             const __nv_bfloat16* xr = a.xn + (size_t)row * a.ba_k;
             const __nv_bfloat16* wb = a.ba_w + (size_t)h * a.ba_k;
             const __nv_bfloat16* wa = a.ba_w + (size_t)(a.Hv + h) * a.ba_k;
+            float sb = 0.f, sa = 0.f;
             for (int i = t * 2; i < a.ba_k; i += 512) {
                 const float2 xv = bf16x2_bits_to_f32x2(*reinterpret_cast<const uint32_t*>(xr + i));
                 const float2 bv = bf16x2_bits_to_f32x2(__ldg(reinterpret_cast<const uint32_t*>(wb + i)));
                 const float2 av = bf16x2_bits_to_f32x2(__ldg(reinterpret_cast<const uint32_t*>(wa + i)));
-                red5[2] = fmaf(xv.x, bv.x, red5[2]); red5[2] = fmaf(xv.y, bv.y, red5[2]);
-                red5[3] = fmaf(xv.x, av.x, red5[3]); red5[3] = fmaf(xv.y, av.y, red5[3]);
+                sb = fmaf(xv.x, bv.x, sb); sb = fmaf(xv.y, bv.y, sb);
+                sa = fmaf(xv.x, av.x, sa); sa = fmaf(xv.y, av.y, sa);
+            }
+            sb = warp_sum(sb); sa = warp_sum(sa);
+            if (lane == 0) { s_sum[2][warp] = sb; s_sum[3][warp] = sa; }
+        }
+        // ---- conv + SiLU for this thread's channels, whose history nobody else reads
+#pragma unroll
+        for (int n = 0; n < NC; ++n) {
+            const int c = t + 256 * n;
+            const float2 w01 = bf16x2_bits_to_f32x2(taps[n].x), w23 = bf16x2_bits_to_f32x2(taps[n].y);
+            float y = w01.x * bf16_to_f32(past[n][2]);
+            y = fmaf(w01.y, bf16_to_f32(past[n][1]), y);
+            y = fmaf(w23.x, bf16_to_f32(past[n][0]), y);
+            y = fmaf(w23.y, bf16_to_f32(x[n]), y);
+            y = silu_f(y);
+            past[n][2] = past[n][1]; past[n][1] = past[n][0]; past[n][0] = x[n];
+            if (c < CH) {
+                hist[(size_t)(pos % a.ring) * CH + c] = x[n];
+                if (c < DK) s_q[c] = y; else if (c < 2 * DK) s_k[c - DK] = y; else s_v[c - 2 * DK] = y;
+            }
+            if (n == 0 && warp < 2 * G) {
+                const float sq = warp_sum(y * y);
+                if (lane == 0) s_sum[warp < G ? 0 : 1][warp < G ? warp : warp - G] = sq;
             }
         }
-        block_sum_n<5>(red5, s_red4);
-        const float qn = rsqrtf(red5[0] + 1e-6f) * rsqrtf((float)DK);
-        const float kn = rsqrtf(red5[1] + 1e-6f);
-        const float kq = red5[4] * qn * kn;                       // k . q of the normalised vectors
-        float b_in, a_in;
-        if (a.ba_w != nullptr) {
-            b_in = bf16_to_f32(f32_to_bf16(red5[2])); a_in = bf16_to_f32(f32_to_bf16(red5[3]));
-        } else {
-            b_in = bf16_to_f32(pr[b_off]); a_in = bf16_to_f32(pr[a_off]);
+        __syncthreads();
+        if (t < DK) {
+            const float qk = warp_sum(s_q[t] * s_k[t]);               // (read after the next barrier)
+            if (lane == 0) s_sum[4][warp] = qk;
         }
+        const float qn = rsqrtf(gdn_sum4(s_sum[0]) + 1e-6f) * rsqrtf((float)DK);
+        const float kn = rsqrtf(gdn_sum4(s_sum[1]) + 1e-6f);
+        if (a.ba_w != nullptr) { b_in = bf16_to_f32(f32_to_bf16(gdn_sum8(s_sum[2]))); a_in = bf16_to_f32(f32_to_bf16(gdn_sum8(s_sum[3]))); }
         const float beta = sigmoid_f(b_in);
         const float gate = neg_expA * softplus_f(a_in + dtb);
         const float d = __expf(gate);
@@ -150,6 +180,10 @@ __global__ void __launch_bounds__(256) gdn_rows_kernel(const GdnArgs a) {
         }
         *reinterpret_cast<float4*>(&s_part[rg][cg * 4]) = make_float4(p[0], p[1], p[2], p[3]);
         *reinterpret_cast<float4*>(&s_partq[rg][cg * 4]) = make_float4(pq[0], pq[1], pq[2], pq[3]);
+        if (a.log_k) {
+            for (int i = t; i < DK; i += 256) a.log_k[((size_t)row * a.Hv + h) * DK + i] = s_k[i] * kn;
+            if (t == 0) a.log_d[(size_t)row * a.Hv + h] = d;
+        }
         __syncthreads();
         // delta = beta (v - S^T k);  o = S_new^T q = S^T q + (k.q) delta   with S_new = S + k delta^T
         float ov = 0.f;
@@ -157,21 +191,19 @@ __global__ void __launch_bounds__(256) gdn_rows_kernel(const GdnArgs a) {
             float kv = 0.f, qv = 0.f;
 #pragma unroll
             for (int g = 0; g < RG; ++g) { kv += s_part[g][t]; qv += s_partq[g][t]; }
+            const float kq = gdn_sum4(s_sum[4]) * qn * kn;            // k . q of the normalised vectors
             const float delta = (s_v[t] - kv) * beta;
             s_vec[t] = delta;
             ov = fmaf(kq, delta, qv);
             if (a.log_delta) a.log_delta[((size_t)row * a.Hv + h) * DV + t] = delta;
+            const float sq = warp_sum(ov * ov);
+            if (lane == 0) s_ss[warp] = sq;
         }
-        if (a.log_k) {
-            for (int i = t; i < DK; i += 256) a.log_k[((size_t)row * a.Hv + h) * DK + i] = s_k[i] * kn;
-            if (t == 0) a.log_d[(size_t)row * a.Hv + h] = d;
-        }
-        const float ss = block_sum(t < DV ? ov * ov : 0.f, s_red);      // its barriers also publish s_vec
+        __syncthreads();
         if (t < DV) {
-            const float inv = rsqrtf(ss / (float)DV + a.eps);
-            const float y = ov * inv * bf16_to_f32(a.norm_w[t]);
-            const float z = bf16_to_f32(pr[z_off + t]);
-            a.out[(size_t)row * (a.Hv * DV) + h * DV + t] = f32_to_bf16(y * silu_f(z));
+            const float inv = rsqrtf(gdn_sum4(s_ss) / (float)DV + a.eps);
+            const float y = ov * inv * nw;
+            a.out[(size_t)row * (a.Hv * DV) + h * DV + t] = f32_to_bf16(y * silu_f(bf16_to_f32(zb)));
         }
         // ---- S += k (x) delta (registers only)
         {
@@ -183,7 +215,7 @@ __global__ void __launch_bounds__(256) gdn_rows_kernel(const GdnArgs a) {
                 for (int c = 0; c < 4; ++c) S[r][c] = fmaf(kreg[r], dlr[c], S[r][c]);
             }
         }
-        __syncthreads();      // s_q / s_k / s_v / s_part / s_vec are rewritten by the next row
+        if (r_i + 1 < sd.n_rows) __syncthreads();      // the row's vectors and sums are rewritten by the next one
     }
     {
         float* sp = a.state_out + ((size_t)sd.slot * a.Hv + h) * DK * DV;
@@ -196,7 +228,7 @@ __global__ void __launch_bounds__(256) gdn_rows_kernel(const GdnArgs a) {
 
 // The same for sequences with several rows in the step (the rows of a drafted block, short prompts): what does not depend on the state --
 // convolution, norms, gates -- is prepared for eight rows at once, a warp per row, and the head norm and the gate follow for all eight;
-// between them a row costs the pass over the state and two barriers instead of six.  Every sum is formed in the order of the kernel
+// between them a row costs the pass over the state and two barriers instead of four.  Every sum is formed in the order of the kernel
 // above, so rows have the same bits in both.  A single row takes longer here, hence two kernels.
 constexpr int kManyRows = 8;
 template <int DK, int DV>
