@@ -235,10 +235,12 @@ __global__ void gemm_smallm_reduce4_kernel(const SmallMReduceArgs a) {
 // Residual epilogue and the next projection's RMSNorm (scale 1 + w) in one launch: the four CTAs of a cluster share a row, exchange
 // their sums of squares through distributed shared memory and write the new residual and its normed row.  Replaces a reduction
 // and a norm launch (2.9 + 6.5 us for 8 rows of 2560); with the early weights above, a step of 8 rows through 8 layers of 2560 x 9216
-// went from 1190 to 931 us, one of 32 rows through 4 layers of 5120 x 17408 from 2010 to 1780.  What bounds it: latency.
+// went from 1190 to 931 us, one of 32 rows through 4 layers of 5120 x 17408 from 2010 to 1780.  What bounds it: latency.  The sums are
+// written to the others instead of read from them: no CTA has to stay for a last cluster barrier (8 rows of 2560: 4.4 -> 4.3 us).
 constexpr int kSmNormCtas = 4, kSmNormThreads = 256, kSmNormItems = 4;       // rows of up to 4 * 4 * 4 * 256 columns
 __global__ void __cluster_dims__(kSmNormCtas, 1, 1) __launch_bounds__(kSmNormThreads) gemm_smallm_norm_kernel(const SmallMReduceArgs a) {
-    __shared__ float red[32], s_part;
+    __shared__ float red[32], s_part[kSmNormCtas];
+    tc::cluster_arrive();            // (the others have started when they are written to)
     const int m = blockIdx.x / kSmNormCtas, per = (a.N / 4 + kSmNormCtas - 1) / kSmNormCtas;
     const uint32_t rank = tc::cluster_ctarank();
     const int first = (int)rank * per, last = min(first + per, a.N / 4);         // this CTA's groups of four columns
@@ -268,11 +270,13 @@ __global__ void __cluster_dims__(kSmNormCtas, 1, 1) __launch_bounds__(kSmNormThr
         ss += x0.x * x0.x + x0.y * x0.y + x1.x * x1.x + x1.y * x1.y;
     }
     ss = block_sum(ss, red);
-    if (threadIdx.x == 0) s_part = ss;
+    // every CTA puts its sum into all of them, so that nobody reads from one that may have left
+    tc::cluster_wait();
+    if (threadIdx.x < kSmNormCtas) tc::cluster_store_f32(&s_part[rank], threadIdx.x, ss);
     tc::cluster_sync();
     ss = 0.f;
 #pragma unroll
-    for (int r = 0; r < kSmNormCtas; ++r) ss += tc::cluster_load_f32(&s_part, r);
+    for (int r = 0; r < kSmNormCtas; ++r) ss += s_part[r];
     const float inv = rsqrtf(ss / (float)a.N + a.eps);
 #pragma unroll
     for (int j = 0; j < kSmNormItems; ++j) {
@@ -283,7 +287,6 @@ __global__ void __cluster_dims__(kSmNormCtas, 1, 1) __launch_bounds__(kSmNormThr
             make_uint2(f32x2_to_bf16x2_bits(x[j].x * inv * (1.f + w0.x), x[j].y * inv * (1.f + w0.y)),
                        f32x2_to_bf16x2_bits(x[j].z * inv * (1.f + w1.x), x[j].w * inv * (1.f + w1.y)));
     }
-    tc::cluster_sync();              // nobody leaves while its sum may still be read
 }
 
 // Any even N and any alignment: one thread per output pair (two neighbouring columns); splits are added in ascending order.
