@@ -139,7 +139,7 @@ int launch_attn_prefill_tc(const void* q, int q_rows, const void* k_pool, const 
     a.Hq = Hq; a.Hkv = Hkv; a.scale_log2 = sm_scale * 1.4426950408889634f; a.min_rows = min_rows;
     a.gate = (const __nv_bfloat16*)gate; a.ld_gate = ld_gate; a.gate_head_stride = gate_head_stride; a.gate_offset = gate_offset;
     a.out = (__nv_bfloat16*)out; a.status = (uint32_t*)status; a.budget = g_ps_wait_budget_cycles; a.prof = g_attn_tc_prof;
-    a.split_tokens = 0; a.max_splits = 0; a.dec_max_rows = 0; a.part_acc = nullptr; a.part_ml = nullptr;
+    a.split_tokens = 0; a.max_splits = 0; a.dec_max_rows = 0; a.part_acc = nullptr; a.part_ml = nullptr; a.n_seqs = n_seqs; a.part_n = nullptr;
     a.opt = opt; a.k_groups = a.k_head = a.v_off = a.v_head = 0;
     const int tiles = (max_seq_rows + kTcRows - 1) / kTcRows;
     return launch_attn_tc_any<false>(D, k_pool == v_pool, dim3(tiles, Hq, n_seqs), mq, mk, mv, a, stream);
@@ -154,10 +154,12 @@ int launch_attn_prefill_tc(const void* q, int q_rows, const void* k_pool, const 
 // Reference: src/phaseshift/models/qwen35/kernels/optimized/attention/paged_decode.hip (split-KV decode); the grouped-query
 // packing onto one MMA tile has no counterpart there.
 // `options`: an AttnOptions (attn_options.cuh) or null; pass the same ones to the merge pass, which applies sink and gate.
-PS_API int ps_attn_decode_tc_ex(const void* q, int q_rows, const void* k_pool, const void* v_pool, const void* block_table,
-                             int max_blocks, int page_tokens, int num_pages, const void* seqs, int n_seqs, int dec_max_rows,
-                             int Hq, int Hkv, int D, float sm_scale, int split_tokens, int max_splits, int max_visible,
-                             void* part_acc, void* part_ml, void* status, const void* options, cudaStream_t stream) {
+// `part_n` ([rows, Hkv] int32): every SM takes an even share of all tiles and a row's partials are counted there
+// (`max_splits` must hold one for every 64 tokens); null: splits of `split_tokens`.
+static int attn_decode_tc(const void* q, int q_rows, const void* k_pool, const void* v_pool, const void* block_table,
+                          int max_blocks, int page_tokens, int num_pages, const void* seqs, int n_seqs, int dec_max_rows,
+                          int Hq, int Hkv, int D, float sm_scale, int split_tokens, int max_splits, int max_visible,
+                          void* part_acc, void* part_ml, void* part_n, void* status, const void* options, cudaStream_t stream) {
     using namespace ps;
     const AttnOptions opt = attn_options(options);
     if (!attn_options_ok(opt) || (k_pool == v_pool && attn_transforms_scores(opt)) || D % 64 || D < 64 || D > 256 || (page_tokens != 16 && page_tokens != 32 && page_tokens != 64) || Hkv <= 0 || (Hq % Hkv) || Hq / Hkv > 8 ||
@@ -180,7 +182,27 @@ PS_API int ps_attn_decode_tc_ex(const void* q, int q_rows, const void* k_pool, c
     a.status = (uint32_t*)status; a.budget = g_ps_wait_budget_cycles; a.prof = nullptr;
     a.split_tokens = split_tokens; a.max_splits = max_splits; a.dec_max_rows = dec_max_rows;
     a.part_acc = (float*)part_acc; a.part_ml = (float*)part_ml; a.opt = opt; a.k_groups = a.k_head = a.v_off = a.v_head = 0;
-    return launch_attn_tc_any<true>(D, k_pool == v_pool, dim3(n_splits, Hkv, n_seqs), mq, mk, mv, a, stream);
+    a.n_seqs = n_seqs; a.part_n = (int*)part_n;
+    const dim3 grid = part_n != nullptr ? dim3(sm_count()) : dim3(n_splits, Hkv, n_seqs);
+    return launch_attn_tc_any<true>(D, k_pool == v_pool, grid, mq, mk, mv, a, stream);
+}
+
+PS_API int ps_attn_decode_tc_ex(const void* q, int q_rows, const void* k_pool, const void* v_pool, const void* block_table,
+                             int max_blocks, int page_tokens, int num_pages, const void* seqs, int n_seqs, int dec_max_rows,
+                             int Hq, int Hkv, int D, float sm_scale, int split_tokens, int max_splits, int max_visible,
+                             void* part_acc, void* part_ml, void* status, const void* options, cudaStream_t stream) {
+    return attn_decode_tc(q, q_rows, k_pool, v_pool, block_table, max_blocks, page_tokens, num_pages, seqs, n_seqs, dec_max_rows, Hq, Hkv, D,
+                          sm_scale, split_tokens, max_splits, max_visible, part_acc, part_ml, nullptr, status, options, stream);
+}
+
+// Even shares; the caller merges with ps_paged_attention_merge_even.
+PS_API int ps_attn_decode_tc_even(const void* q, int q_rows, const void* k_pool, const void* v_pool, const void* block_table,
+                                  int max_blocks, int page_tokens, int num_pages, const void* seqs, int n_seqs, int dec_max_rows,
+                                  int Hq, int Hkv, int D, float sm_scale, int max_splits, int max_visible,
+                                  void* part_acc, void* part_ml, void* part_n, void* status, const void* options, cudaStream_t stream) {
+    if (part_n == nullptr) return (int)cudaErrorInvalidValue;
+    return attn_decode_tc(q, q_rows, k_pool, v_pool, block_table, max_blocks, page_tokens, num_pages, seqs, n_seqs, dec_max_rows, Hq, Hkv, D,
+                          sm_scale, ps::kTcTok, max_splits, max_visible, part_acc, part_ml, part_n, status, options, stream);
 }
 
 PS_API int ps_attn_decode_tc(const void* q, int q_rows, const void* k_pool, const void* v_pool, const void* block_table,

@@ -71,6 +71,7 @@ struct AttnTcArgs {
     // decode / verify variant (DEC): split-KV partials in the layout of the per-row kernel's merge pass
     int split_tokens; int max_splits; int dec_max_rows;
     float* part_acc; float* part_ml;
+    int n_seqs; int* part_n;     // with part_n [rows, Hkv]: even shares (below), and how many partials a row has
     AttnOptions opt;             // (sink and gate: the merge pass applies them for DEC)
     // expanded keys and values (EXPANDED): rows of consecutive tokens; columns of a head's keys, first column of its values
     int k_groups, k_head, v_off, v_head;
@@ -110,6 +111,14 @@ __device__ __forceinline__ float sigmoid_fast(float x) {
     return fmaf(0.5f, t, 0.5f);
 }
 
+// Barrier of the softmax warps: does `p` hold for all of them?
+__device__ __forceinline__ bool softmax_all(bool p) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, 256, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"((uint32_t)p) : "memory");
+    return r != 0;
+}
+
 // Expanded keys and values of a step (EXPANDED): the sequences with more than `min_rows` rows follow one another, each with the
 // tokens its rows see, from a multiple of the tile on.
 __device__ __forceinline__ int expanded_first(const int* sd, const AttnOptions& o) { return attn_first(o, sd[3]) / kTcTok * kTcTok; }
@@ -129,6 +138,12 @@ __device__ __forceinline__ int expanded_row0(const int* seqs, int s, int min_row
 // and one KV head: tile row 8 r + g is query head g of that KV head for the sequence's row r (grouped-query packing: the G <= 8
 // heads that share the KV head ride in one MMA tile, so K and V are read once for all of them), over the tokens of its
 // split; it leaves unnormalised partial outputs and (maximum, sum) pairs for the merge pass of paged_attention.cu.
+// With `part_n` the grid is one CTA per SM instead, and every CTA takes an even share of the tiles of all sequences and KV heads, in
+// their order: it works on the pieces of one or more (sequence, KV head) one after the other, its pipelines running on, and a
+// partial's number is that of its CTA among those that share the (sequence, KV head).  With 224 KB of shared memory a CTA has an SM to
+// itself, so splits of a fixed length run in rounds, each with its own set-up, and sequences of unequal length leave the last one
+// nearly empty.  Sequences of 5 to 100 % of a length, 4 KV heads of 256: 12 of up to 3001 tokens 29.7 -> 24.9 us, 24 of up to 3500 with keys
+// that are the values 47 -> 38.4.  What bounds it now: a tile's chain through the softmax warps, 1.5 us and more beside 0.7 or 1.4 of bytes.
 // TRANSFORM: query temperature and distance bias, applied to the scores before the maximum.
 // EXPANDED: keys and values were expanded per query head into rows of consecutive tokens (attn_latent.cu), the last 64-column
 // groups of the keys (`map_r`) are shared by all heads.
@@ -156,31 +171,101 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     unsigned char* sK = sQ + kTcQBytes;
     unsigned char* sV = sK + 2 * kTcKStage;
     unsigned char* sP = sV + 2 * kTcVStage;
-    __shared__ __align__(8) uint64_t q_full, k_full[4], v_full[2], s_full[2], p_full[2], pv_done[2], kv_free[4];
+    __shared__ __align__(8) uint64_t q_full, q_free, k_full[4], v_full[2], s_full[2], p_full[2], pv_done[2], kv_free[4];
     __shared__ float s_l[2][kTcRows];            // row sums of the two column halves, exchanged once at the end
     __shared__ uint32_t tmem_base_slot;
     __shared__ int s_abort, s_bad, k_issued, k_consumed, v_issued, v_consumed, q_issued, q_consumed;
 
     cudaGridDependencySynchronize();             // (the descriptors may be the predecessor's)
-    const int* sd = a.seqs + 4 * blockIdx.z;
-    const int row_start = sd[0], n_rows = sd[1], slot = sd[2], pos_start = sd[3];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = a.Hq / a.Hkv;
-    // tiles of the CTA: `n_keep` tiles of kept first positions from tile `keep0` on, then those from `t_first` on, T in all
-    int r_begin, nq, h, kvh, pos_q0, kv_end, t_first, T, keep0 = 0, n_keep = 0;
+    int row_start, n_rows, slot, pos_start;
+    auto read_seq = [&](int seq) {
+        const int* sd = a.seqs + 4 * seq;
+        row_start = sd[0]; n_rows = sd[1]; slot = sd[2]; pos_start = sd[3];
+    };
+    // tiles of the CTA's piece: of `n_keep` tiles of kept first positions from tile `keep0` on and then those from `t_first` on, T from
+    // the t_off-th on
+    int r_begin, nq, h, kvh, pos_q0, kv_end, t_first, T, keep0 = 0, n_keep = 0, t_off = 0;
     const int keep_tiles = EXPANDED ? 0 : (a.opt.keep_first + kTcTok - 1) / kTcTok;
-    if constexpr (DEC) {
-        if (slot < 0 || n_rows <= 0 || n_rows > a.dec_max_rows) return;
-        r_begin = 0; nq = 8 * n_rows; kvh = blockIdx.y; h = kvh * G;
+    // even shares: sequence, tiles of all its rows, first tile of (sequence, KV head) among all, tiles left, all tiles, CTAs with tiles
+    [[maybe_unused]] int seq = blockIdx.z, T_seq = 0, x0 = 0, left = 0, total = 0, n_ctas = 0;
+    [[maybe_unused]] auto tiles_of = [&](const int* sd) {
+        if (sd[2] < 0 || sd[1] <= 0 || sd[1] > a.dec_max_rows) return 0;
+        const int tf = attn_first(a.opt, sd[3]) / kTcTok;
+        return min(keep_tiles, tf) + (sd[3] + sd[1] + kTcTok - 1) / kTcTok - tf;
+    };
+    [[maybe_unused]] auto set_piece = [&]() {
+        read_seq(seq);
+        r_begin = 0; nq = 8 * n_rows; h = kvh * G;
         pos_q0 = pos_start; kv_end = pos_start + n_rows;
-        const int tps = a.split_tokens / kTcTok;                         // tiles per split
-        const int t_lo = attn_first(a.opt, pos_q0) / kTcTok;             // tile of the first token any row sees
-        const int t_end = min((kv_end + kTcTok - 1) / kTcTok, ((int)blockIdx.x + 1) * tps);
-        keep0 = (int)blockIdx.x * tps;
-        t_first = max(keep0, t_lo);
-        n_keep = max(0, min(min(keep_tiles, t_lo), keep0 + tps) - keep0);
-        T = n_keep + max(0, t_end - t_first);
-        if (T <= 0) return;
+        t_first = attn_first(a.opt, pos_q0) / kTcTok;
+        n_keep = min(keep_tiles, t_first);
+        T_seq = n_keep + (kv_end + kTcTok - 1) / kTcTok - t_first;
+        T = min(T_seq - t_off, left);
+        left -= T;
+    };
+    // the next piece of the CTA's share (every thread keeps its own place in it)
+    auto next_piece = [&]() -> bool {
+        if constexpr (!DEC) return false;
+        else {
+            if (left <= 0) return false;
+            x0 += T_seq; t_off = 0;
+            if (++kvh == a.Hkv) {
+                kvh = 0;
+                do if (++seq >= a.n_seqs) return false; while (tiles_of(a.seqs + 4 * seq) == 0);
+            }
+            set_piece();
+            return true;
+        }
+    };
+    const bool even = DEC && a.part_n != nullptr;
+    if constexpr (DEC) {
+        if (even) {
+            for (int s0 = 0; s0 < a.n_seqs; s0 += 32)
+                total += __reduce_add_sync(0xffffffffu, s0 + lane < a.n_seqs ? tiles_of(a.seqs + 4 * (s0 + lane)) : 0);
+            total *= a.Hkv;
+            n_ctas = min((int)gridDim.x, total);
+            const int cta = blockIdx.x;
+            if (cta >= n_ctas) return;
+            const int lo = (int)((long long)cta * total / n_ctas);
+            left = (int)((long long)(cta + 1) * total / n_ctas) - lo;
+            int before = 0;
+            for (int s0 = 0;; s0 += 32) {                                // the sequence of tile `lo`, which is below `total`
+                const int c = s0 + lane < a.n_seqs ? tiles_of(a.seqs + 4 * (s0 + lane)) : 0;
+                int sum = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
+                const uint32_t past = __ballot_sync(0xffffffffu, (before + sum) * a.Hkv > lo);
+                if (past != 0 || s0 + 32 >= a.n_seqs) {
+                    const int l = past != 0 ? __ffs(past) - 1 : 31;
+                    seq = s0 + l;
+                    T_seq = __shfl_sync(0xffffffffu, c, l);
+                    before += __shfl_sync(0xffffffffu, sum, l) - T_seq;
+                    break;
+                }
+                before += __shfl_sync(0xffffffffu, sum, 31);
+            }
+            const int at = lo - before * a.Hkv;
+            kvh = at / T_seq; t_off = at - kvh * T_seq;
+            x0 = lo - t_off;
+            set_piece();
+        } else {
+            read_seq(seq);
+            if (slot < 0 || n_rows <= 0 || n_rows > a.dec_max_rows) return;
+            r_begin = 0; nq = 8 * n_rows; kvh = blockIdx.y; h = kvh * G;
+            pos_q0 = pos_start; kv_end = pos_start + n_rows;
+            const int tps = a.split_tokens / kTcTok;                         // tiles per split
+            const int t_lo = attn_first(a.opt, pos_q0) / kTcTok;             // tile of the first token any row sees
+            const int t_end = min((kv_end + kTcTok - 1) / kTcTok, ((int)blockIdx.x + 1) * tps);
+            keep0 = (int)blockIdx.x * tps;
+            t_first = max(keep0, t_lo);
+            n_keep = max(0, min(min(keep_tiles, t_lo), keep0 + tps) - keep0);
+            T = n_keep + max(0, t_end - t_first);
+            if (T <= 0) return;
+        }
     } else {
+        read_seq(seq);
         const int tile = (int)gridDim.x - 1 - (int)blockIdx.x;
         r_begin = tile * kTcRows;
         if (r_begin >= n_rows || slot < 0 || n_rows <= a.min_rows) return;
@@ -192,13 +277,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         n_keep = min(keep_tiles, t_first);
         T = n_keep + (kv_end + kTcTok - 1) / kTcTok - t_first;
     }
-    auto tile_of = [&](int t) { return t < n_keep ? keep0 + t : t_first - n_keep + t; };
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto tile_of = [&](int t) { return t + t_off < n_keep ? keep0 + t + t_off : t_first - n_keep + t + t_off; };
     const bool cta_stamp = a.prof != nullptr && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
     if (cta_stamp) a.prof[15] = clock64();
 
     if (threadIdx.x == 0) {
-        tc::mbar_init(&q_full, 1);
+        tc::mbar_init(&q_full, 1); tc::mbar_init(&q_free, 2);
         for (int s = 0; s < 2; ++s) {
             tc::mbar_init(&k_full[s], 1); tc::mbar_init(&v_full[s], 1); tc::mbar_init(&s_full[s], 1);
             tc::mbar_init(&p_full[s], 8); tc::mbar_init(&pv_done[s], 1);
@@ -225,31 +309,35 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     int exp_row0 = 0;            // EXPANDED: row of the sequence's position 0, were it there
     if constexpr (EXPANDED) exp_row0 = expanded_row0(a.seqs, (int)blockIdx.z, a.min_rows, a.opt);
 
+    // In all roles `g` counts the tiles of earlier pieces: stages, buffers and phases go by a tile's number over all pieces.
+    // Q of the n-th piece: its buffer is free once both issuers' scores of the piece before are done.
+    auto load_q = [&](int n) -> bool {
+        if constexpr (DEC) {
+            if (n > 0 && !__all_sync(0xffffffffu, tc::mbar_wait_abortable(&q_free, (uint32_t)(n - 1) & 1u, a.budget, &s_abort))) return false;
+            // one 8-row box per (row of the sequence, 64-column group): the G heads of this KV head are consecutive rows
+            // of the [rows * Hq, D] view of q; tile rows 8 r + g with g >= G hold other heads' values and are never used
+            if (lane == 0) tc::mbar_expect_tx(&q_full, (uint32_t)n_rows * (uint32_t)kNB * 1024u);
+            __syncwarp();
+            for (int i = lane; i < kNB * n_rows; i += 32) {
+                const int r = i / kNB, c4 = i % kNB;
+                tc::tma_load_2d(sQ + c4 * (kTcRows * 128) + (8 * r) * 128, &map_q, c4 * 64, (row_start + r) * a.Hq + h, &q_full);
+            }
+        } else {
+            if (lane == 0) tc::mbar_expect_tx(&q_full, kTcQBytes);
+            __syncwarp();
+            if (lane < kNB) tc::tma_load_2d(sQ + lane * (kTcRows * 128), &map_q, h * DK + lane * 64, row_start + r_begin, &q_full);
+        }
+        if (lane == 0) q_issued = n + 1;
+        return true;
+    };
     if (SHARED && warp == 9) {
-        // the values arrive with the keys
+        // the values arrive with the keys; Q is this warp's
+        for (int piece = 0; load_q(piece) && next_piece(); ++piece) {}
     } else if (warp == 8 || warp == 9) {
         // ------------------------------------------------ TMA producers: warp 8 = Q and K, warp 9 = V.  One lane per box (a
         // tile is up to 16 boxes: pages x four 64-column groups): issuing them from one thread one after the other costs
         // more than a thousand cycles, and the stage's consumer is waiting for them.
         const bool isK = warp == 8;
-        if (isK) {
-            if constexpr (DEC) {
-                // one 8-row box per (row of the sequence, 64-column group): the G heads of this KV head are consecutive rows
-                // of the [rows * Hq, D] view of q; tile rows 8 r + g with g >= G hold other heads' values and are never used
-                if (lane == 0) tc::mbar_expect_tx(&q_full, (uint32_t)n_rows * (uint32_t)kNB * 1024u);
-                __syncwarp();
-                for (int i = lane; i < kNB * n_rows; i += 32) {
-                    const int r = i / kNB, c4 = i % kNB;
-                    tc::tma_load_2d(sQ + c4 * (kTcRows * 128) + (8 * r) * 128, &map_q, c4 * 64, (row_start + r) * a.Hq + h, &q_full);
-                }
-            } else {
-                if (lane == 0) tc::mbar_expect_tx(&q_full, kTcQBytes);
-                __syncwarp();
-                if (lane < kNB) tc::tma_load_2d(sQ + lane * (kTcRows * 128), &map_q, h * DK + lane * 64, row_start + r_begin, &q_full);
-            }
-            if (lane == 0) q_issued = 1;
-        }
-        const int* bt = a.block_table + (size_t)slot * a.max_blocks;
         const int pt = a.page_tokens, ppt = kTcTok / pt;            // a page is one box of pt token rows per 64-column group
         const int nb = isK ? kNB : kNBV, stage_bytes = isK ? kTcKStage : kTcVStage;
         const int pg = lane / nb, cb = lane % nb;
@@ -264,25 +352,34 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             else if (cb < a.k_groups) x += h * a.k_head;
             else { map = &map_r; x -= a.k_groups * 64; }
         }
-        for (int t = 0; t < T; ++t) {
-            const int b = t & kStageMask;
-            int page = 0;
-            const int blk = tile_of(t) * ppt + pg;
-            if (!EXPANDED && active && blk * pt < kv_end) {
-                page = bt[blk];
-                if (page < 0 || page >= a.num_pages) { s_bad = 1; page = 0; }
+        bool ok = true;
+        if (isK && !SHARED) ok = load_q(0);
+        for (int piece = 0, g = 0; ok; ++piece) {
+            const int* bt = a.block_table + (size_t)slot * a.max_blocks;
+            for (int t = 0; t < T && ok; ++t) {
+                const int n = g + t, b = n & kStageMask;
+                int page = 0;
+                const int blk = tile_of(t) * ppt + pg;
+                if (!EXPANDED && active && blk * pt < kv_end) {
+                    page = bt[blk];
+                    if (page < 0 || page >= a.num_pages) { s_bad = 1; page = 0; }
+                }
+                if constexpr (SHARED) {
+                    if (n >= 4) ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&kv_free[b], (uint32_t)((n - 4) >> 2) & 1u, a.budget, &s_abort));
+                } else {
+                    if (n >= 2) ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&freed[b], (uint32_t)((n - 2) >> 1) & 1u, a.budget, &s_abort));
+                }
+                if (!ok) break;
+                if (lane == 0) tc::mbar_expect_tx(&full[b], stage_bytes);
+                __syncwarp();
+                if (active)
+                    tc::tma_load_2d(stage0 + b * stage_bytes + cb * (kTcTok * 128) + pg * (pt * 128), map, x,
+                                    EXPANDED ? exp_row0 + (t_first + t) * kTcTok : (page * a.Hkv + kvh) * pt, &full[b]);
+                if (lane == 0) { if (isK) k_issued = n + 1; else v_issued = n + 1; }
+                if (isK && !SHARED && piece > 0 && t == 0) ok = load_q(piece);           // (the first tile need not wait for the buffer of Q)
             }
-            if constexpr (SHARED) {
-                if (t >= 4 && !__all_sync(0xffffffffu, tc::mbar_wait_abortable(&kv_free[b], (uint32_t)((t - 4) >> 2) & 1u, a.budget, &s_abort))) break;
-            } else {
-                if (t >= 2 && !__all_sync(0xffffffffu, tc::mbar_wait_abortable(&freed[b], (uint32_t)((t - 2) >> 1) & 1u, a.budget, &s_abort))) break;
-            }
-            if (lane == 0) tc::mbar_expect_tx(&full[b], stage_bytes);
-            __syncwarp();
-            if (active)
-                tc::tma_load_2d(stage0 + b * stage_bytes + cb * (kTcTok * 128) + pg * (pt * 128), map, x,
-                                EXPANDED ? exp_row0 + (t_first + t) * kTcTok : (page * a.Hkv + kvh) * pt, &full[b]);
-            if (lane == 0) { if (isK) k_issued = t + 1; else v_issued = t + 1; }
+            g += T;
+            if (!next_piece()) break;
         }
     } else if (warp == 10 || warp == 11) {
         // ------------------------------------------------ score issuers: warp 10 issues S(t) for even t, warp 11 for odd t.
@@ -292,28 +389,39 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             constexpr uint32_t idesc_s = tc::idesc_bf16_f32(kTcRows, kTcTok);
             const int b = warp - 10;
             const uint32_t q_addr = tc::smem_u32(sQ), k_addr0 = tc::smem_u32(sK);
-            bool ok = tc::mbar_wait_abortable(&q_full, 0, a.budget, &s_abort);
-            if (ok) q_consumed = 1;
-            for (int t = b; t < T && ok; t += 2) {
-                const uint32_t ph = (uint32_t)(t >> 1) & 1u;
-                const bool stamp = a.prof != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && t < 32;
-                if (stamp) a.prof[t * 16 + 8] = clock64();
-                // the score buffer is free once the softmax warps have read S(t - 2), which they signal with P(t - 2)
-                if (t >= 2 && !tc::mbar_wait_abortable(&p_full[b], ph ^ 1u, a.budget, &s_abort)) { ok = false; break; }
-                const int ks_ = t & kStageMask;                                          // the tile's stage
-                const uint32_t k_addr = k_addr0 + ks_ * kTcKStage;
-                if (!tc::mbar_wait_abortable(&k_full[ks_], (uint32_t)(t >> kStageLog) & 1u, a.budget, &s_abort)) { ok = false; break; }
-                if (stamp) a.prof[t * 16 + 9] = clock64();
-                atomicMax(&k_consumed, t + 1);
-                tc::fence_after_sync();
+            bool ok = true;
+            for (int piece = 0, g = 0; ok; ++piece) {
+                ok = tc::mbar_wait_abortable(&q_full, (uint32_t)piece & 1u, a.budget, &s_abort);
+                if (ok) atomicMax(&q_consumed, piece + 1);
+                const int first = (g & 1) == b ? 0 : 1;
+                for (int t = first; t < T && ok; t += 2) {
+                    const int n = g + t;
+                    const uint32_t ph = (uint32_t)(n >> 1) & 1u;
+                    const bool stamp = a.prof != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && t < 32;
+                    if (stamp) a.prof[t * 16 + 8] = clock64();
+                    // the score buffer is free once the softmax warps have read S(t - 2), which they signal with P(t - 2)
+                    if (n >= 2 && !tc::mbar_wait_abortable(&p_full[b], ph ^ 1u, a.budget, &s_abort)) { ok = false; break; }
+                    const int ks_ = n & kStageMask;                                          // the tile's stage
+                    const uint32_t k_addr = k_addr0 + ks_ * kTcKStage;
+                    if (!tc::mbar_wait_abortable(&k_full[ks_], (uint32_t)(n >> kStageLog) & 1u, a.budget, &s_abort)) { ok = false; break; }
+                    if (stamp) a.prof[t * 16 + 9] = clock64();
+                    atomicMax(&k_consumed, n + 1);
+                    tc::fence_after_sync();
 #pragma unroll
-                for (int ks = 0; ks < DK / 16; ++ks) {
-                    const uint64_t adesc = tc::smem_desc_sw128(q_addr + (ks >> 2) * (kTcRows * 128) + (ks & 3) * 32);
-                    const uint64_t bdesc = tc::smem_desc_sw128(k_addr + (ks >> 2) * (kTcTok * 128) + (ks & 3) * 32);
-                    tc::mma_bf16_ss(tmem + b * kTcTok, adesc, bdesc, idesc_s, ks > 0 ? 1u : 0u);
+                    for (int ks = 0; ks < DK / 16; ++ks) {
+                        const uint64_t adesc = tc::smem_desc_sw128(q_addr + (ks >> 2) * (kTcRows * 128) + (ks & 3) * 32);
+                        const uint64_t bdesc = tc::smem_desc_sw128(k_addr + (ks >> 2) * (kTcTok * 128) + (ks & 3) * 32);
+                        tc::mma_bf16_ss(tmem + b * kTcTok, adesc, bdesc, idesc_s, ks > 0 ? 1u : 0u);
+                    }
+                    tc::mma_commit(&s_full[b]);
+                    if (stamp) a.prof[t * 16 + 10] = clock64();
                 }
-                tc::mma_commit(&s_full[b]);
-                if (stamp) a.prof[t * 16 + 10] = clock64();
+                if constexpr (DEC) {                     // (one arrival of each issuer, also of one without a tile in a piece of one)
+                    if (ok && first < T) tc::mma_commit(&q_free);
+                    else if (ok) tc::mbar_arrive(&q_free);
+                }
+                g += T;
+                if (!next_piece()) break;
             }
         }
     } else if (warp == 12) {
@@ -321,25 +429,31 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         if (tc::elect_one()) {
             constexpr uint32_t idesc_o = tc::idesc_bf16_f32_bmn(kTcRows, DV);
             const uint32_t v_addr0 = tc::smem_u32(SHARED ? sK : sV), p_addr = tc::smem_u32(sP);
-            for (int t = 0; t < T; ++t) {
-                const int b = t & 1;
-                const uint32_t ph = (uint32_t)(t >> 1) & 1u;
-                const bool stamp = a.prof != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && t < 32;
-                if (!tc::mbar_wait_abortable(&p_full[b], ph, a.budget, &s_abort)) break;
-                if (stamp) a.prof[t * 16 + 11] = clock64();
-                const uint32_t v_addr = v_addr0 + (t & kStageMask) * kTcVStage;
-                if (!tc::mbar_wait_abortable(SHARED ? &k_full[t & 3] : &v_full[b], SHARED ? (uint32_t)(t >> 2) & 1u : ph, a.budget, &s_abort)) break;
-                v_consumed = t + 1;
-                tc::fence_after_sync();
+            bool ok = true;
+            for (int g = 0; ok;) {
+                for (int t = 0; t < T; ++t) {
+                    const int n = g + t, b = n & 1;
+                    const uint32_t ph = (uint32_t)(n >> 1) & 1u;
+                    const bool stamp = a.prof != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && t < 32;
+                    // (P of a piece's first tile comes from warps that have read the output of the piece before)
+                    if (!tc::mbar_wait_abortable(&p_full[b], ph, a.budget, &s_abort)) { ok = false; break; }
+                    if (stamp) a.prof[t * 16 + 11] = clock64();
+                    const uint32_t v_addr = v_addr0 + (n & kStageMask) * kTcVStage;
+                    if (!tc::mbar_wait_abortable(SHARED ? &k_full[n & 3] : &v_full[b], SHARED ? (uint32_t)(n >> 2) & 1u : ph, a.budget, &s_abort)) { ok = false; break; }
+                    v_consumed = n + 1;
+                    tc::fence_after_sync();
 #pragma unroll
-                for (int kk = 0; kk < kTcTok / 16; ++kk) {
-                    const uint64_t adesc = tc::smem_desc_sw128(p_addr + b * kTcPBuf + kk * 32);
-                    const uint64_t bdesc = tc::smem_desc_sw128_mn(v_addr + kk * (16 * 128), kTcTok * 128, 1024);
-                    tc::mma_bf16_ss(tmem_o, adesc, bdesc, idesc_o, (t > 0 || kk > 0) ? 1u : 0u);
+                    for (int kk = 0; kk < kTcTok / 16; ++kk) {
+                        const uint64_t adesc = tc::smem_desc_sw128(p_addr + b * kTcPBuf + kk * 32);
+                        const uint64_t bdesc = tc::smem_desc_sw128_mn(v_addr + kk * (16 * 128), kTcTok * 128, 1024);
+                        tc::mma_bf16_ss(tmem_o, adesc, bdesc, idesc_o, (t > 0 || kk > 0) ? 1u : 0u);
+                    }
+                    if constexpr (SHARED) tc::mma_commit(&kv_free[n & 3]);
+                    tc::mma_commit(&pv_done[b]);
+                    if (stamp) a.prof[t * 16 + 12] = clock64();
                 }
-                if constexpr (SHARED) tc::mma_commit(&kv_free[t & 3]);
-                tc::mma_commit(&pv_done[b]);
-                if (stamp) a.prof[t * 16 + 12] = clock64();
+                g += T;
+                if (!next_piece()) break;
             }
         }
     } else {
@@ -348,244 +462,255 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         const int quad = warp & 3, half = warp >> 2;
         const int row = quad * 32 + lane;
         const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
-        const int rp = DEC ? pos_q0 + (row >> 3) : pos_q0 + row;     // position of this thread's query row
-        const float sc = a.scale_log2;
-        const int lo = attn_first(a.opt, rp);                        // first token this row sees
-        const int lo_max = attn_first(a.opt, kv_end - 1);            // ... and the largest of any row
-        const int keep = EXPANDED ? 0 : a.opt.keep_first;
-        [[maybe_unused]] float row_scale = sc, bias_far = 0.f;
-        [[maybe_unused]] const float* bias = nullptr;                // this row's head, by distance
-        if constexpr (TRANSFORM) {
-            row_scale = sc * attn_temperature(a.opt, rp);
-            if (a.opt.bias != nullptr) {
-                bias = a.opt.bias + (size_t)(DEC ? min(h + (row & 7), a.Hq - 1) : h) * a.opt.bias_len;
-                bias_far = bias[a.opt.bias_len - 1] * 1.4426950408889634f;
-            }
-        }
-        float m_ref = 0.f, l_run = 0.f;
-        bool fresh = true;                                            // this row has not seen a token yet: m_ref is a placeholder
         bool ok = true;
-        // the epilogue reads this tile's gate values (one 512-byte run per row): ask for them now, so that they come from
-        // L2 then
-        if (!DEC && a.gate != nullptr && !a.opt.gate_per_head && half == 0 && row < nq)
-            tc::bulk_prefetch_l2(a.gate + (size_t)(row_start + r_begin + row) * a.ld_gate + (size_t)h * a.gate_head_stride + a.gate_offset, DV * 2);
-        for (int t = 0; t < T; ++t) {
-            const int b = t & 1;
-            const uint32_t ph = (uint32_t)(t >> 1) & 1u;
-            const int tt = tile_of(t);                                // tile index within the sequence
-            const int t0 = tt * kTcTok + half * 32;                   // first token of this thread's columns
-            const bool stamp = a.prof != nullptr && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && t < 32;
-            if (stamp) a.prof[t * 16 + 0] = clock64();
-            ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&s_full[b], ph, a.budget, &s_abort));
-            if (!ok) break;
-            tc::fence_after_sync();
-            if (stamp) a.prof[t * 16 + 1] = clock64();
-            // both threads of a row read all 64 scores and take the maximum themselves (cheaper than an exchange through
-            // shared memory); each then exponentiates its own 32 columns
-            uint32_t sr[32], so[32];
-            tc::tmem_ld_32x32(tmem + lane_base + b * kTcTok + half * 32, sr);
-            tc::tmem_ld_32x32(tmem + lane_base + b * kTcTok + (half ^ 1) * 32, so);
-            tc::tmem_ld_wait();
-            if (stamp) a.prof[t * 16 + 2] = clock64();
+        for (int g = 0;;) {
+            const int rp = DEC ? pos_q0 + (row >> 3) : pos_q0 + row;     // position of this thread's query row
+            const float sc = a.scale_log2;
+            const int lo = attn_first(a.opt, rp);                        // first token this row sees
+            const int lo_max = attn_first(a.opt, kv_end - 1);            // ... and the largest of any row
+            const int keep = EXPANDED ? 0 : a.opt.keep_first;
+            [[maybe_unused]] float row_scale = sc, bias_far = 0.f;
+            [[maybe_unused]] const float* bias = nullptr;                // this row's head, by distance
             if constexpr (TRANSFORM) {
-                const int to = tt * kTcTok + (half ^ 1) * 32;
-                if (bias == nullptr || rp - tt * kTcTok - (kTcTok - 1) >= a.opt.bias_len - 1) {      // the whole tile is far away
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        sr[j] = __float_as_uint(fmaf(__uint_as_float(sr[j]), row_scale, bias_far));
-                        so[j] = __float_as_uint(fmaf(__uint_as_float(so[j]), row_scale, bias_far));
-                    }
-                } else {
-                    const int far = a.opt.bias_len - 1;
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const float br = __ldg(bias + min(max(rp - t0 - j, 0), far)) * 1.4426950408889634f;
-                        const float bo = __ldg(bias + min(max(rp - to - j, 0), far)) * 1.4426950408889634f;
-                        sr[j] = __float_as_uint(fmaf(__uint_as_float(sr[j]), row_scale, br));
-                        so[j] = __float_as_uint(fmaf(__uint_as_float(so[j]), row_scale, bo));
-                    }
+                row_scale = sc * attn_temperature(a.opt, rp);
+                if (a.opt.bias != nullptr) {
+                    bias = a.opt.bias + (size_t)(DEC ? min(h + (row & 7), a.Hq - 1) : h) * a.opt.bias_len;
+                    bias_far = bias[a.opt.bias_len - 1] * 1.4426950408889634f;
                 }
             }
-            if (tt * kTcTok < lo_max) {                               // tokens before some row's block
-                const int to = tt * kTcTok + (half ^ 1) * 32;
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    if (t0 + j < lo && t0 + j >= keep) sr[j] = 0xff800000u;
-                    if (to + j < lo && to + j >= keep) so[j] = 0xff800000u;
-                }
-            }
-            if (tt * kTcTok + kTcTok - 1 > pos_q0) {                  // some row of the tile does not see every token
-                const int to = tt * kTcTok + (half ^ 1) * 32;
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    if (t0 + j > rp) sr[j] = 0xff800000u;             // -inf
-                    if (to + j > rp) so[j] = 0xff800000u;
-                }
-            }
-            float mq[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-            for (int j = 0; j < 32; ++j) mq[j & 3] = fmaxf(mq[j & 3], fmaxf(__uint_as_float(sr[j]), __uint_as_float(so[j])));
-            float mx = fmaxf(fmaxf(mq[0], mq[1]), fmaxf(mq[2], mq[3]));
-            if constexpr (!TRANSFORM) mx *= sc;                       // scale > 0, so the maximum commutes with it
-            if (stamp) a.prof[t * 16 + 3] = clock64();
-            float alpha = 1.f;
-            if (fresh) {                                              // (a row that sees nothing yet keeps a finite reference)
-                if (mx != -INFINITY) { m_ref = mx; fresh = false; }
-            }
-            else if (mx > m_ref + 8.f) { alpha = ex2_approx(m_ref - mx); m_ref = mx; }
-            const bool rescale = __any_sync(0xffffffffu, alpha != 1.f);
-            float sq[4] = {0.f, 0.f, 0.f, 0.f};
-            uint32_t pk[16];
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-                const float s0 = __uint_as_float(sr[j]), s1 = __uint_as_float(sr[j + 1]);
-                const float p0 = ex2_approx(TRANSFORM ? s0 - m_ref : fmaf(s0, sc, -m_ref));
-                const float p1 = ex2_approx(TRANSFORM ? s1 - m_ref : fmaf(s1, sc, -m_ref));
-                sq[(j >> 1) & 3] += p0 + p1;
-                pk[j >> 1] = f32x2_to_bf16x2_bits(p0, p1);
-            }
-            l_run = l_run * alpha + ((sq[0] + sq[1]) + (sq[2] + sq[3]));
-            if (t >= 2) {                                             // P buffer b was read by P V(t - 2)
-                ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&pv_done[b], (uint32_t)((t - 2) >> 1) & 1u, a.budget, &s_abort));
-                if (!ok) break;
-            }
-            if (stamp) a.prof[t * 16 + 4] = clock64();
-            unsigned char* prow = sP + b * kTcPBuf + row * 128;
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                *reinterpret_cast<uint4*>(prow + (((half * 4 + c) ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
-            if (t == T - 1 && kv_end < (tt + 1) * kTcTok) {
-                // token rows of the last V tile beyond the sequence's end: zero them (whole 128-byte rows, so the swizzle
-                // does not matter)
-                // (a shared tile has been read by S(t) already: the scores are here)
-                ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(SHARED ? &k_full[t & 3] : &v_full[b], SHARED ? (uint32_t)(t >> 2) & 1u : ph,
-                                                                     a.budget, &s_abort));
-                if (!ok) break;
-                const int jz = kv_end - tt * kTcTok;
-                unsigned char* vs = (SHARED ? sK : sV) + (t & kStageMask) * kTcVStage;
-                for (int i = (int)threadIdx.x; i < (kTcTok - jz) * kNBV * 8; i += 2 * kTcRows) {
-                    const int r = jz + i / (kNBV * 8), cb = i % (kNBV * 8) >> 3, c = i & 7;
-                    *reinterpret_cast<uint4*>(vs + cb * (kTcTok * 128) + r * 128 + c * 16) = make_uint4(0, 0, 0, 0);
-                }
-            }
-            if (stamp) a.prof[t * 16 + 5] = clock64();
-            tc::fence_proxy_async_smem();
-            if (stamp) a.prof[t * 16 + 6] = clock64();
-            if (rescale) {                                            // t >= 1: O must be complete up to P V(t - 1)
-                ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&pv_done[b ^ 1], (uint32_t)((t - 1) >> 1) & 1u, a.budget, &s_abort));
+            float m_ref = 0.f, l_run = 0.f;
+            bool fresh = true;                                            // this row has not seen a token yet: m_ref is a placeholder
+            // the epilogue reads this tile's gate values (one 512-byte run per row): ask for them now, so that they come from
+            // L2 then
+            if (!DEC && a.gate != nullptr && !a.opt.gate_per_head && half == 0 && row < nq)
+                tc::bulk_prefetch_l2(a.gate + (size_t)(row_start + r_begin + row) * a.ld_gate + (size_t)h * a.gate_head_stride + a.gate_offset, DV * 2);
+            for (int t = 0; t < T; ++t) {
+                const int n = g + t, b = n & 1;
+                const uint32_t ph = (uint32_t)(n >> 1) & 1u;
+                const int tt = tile_of(t);                                // tile index within the sequence
+                const int t0 = tt * kTcTok + half * 32;                   // first token of this thread's columns
+                const bool stamp = a.prof != nullptr && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && t < 32;
+                if (stamp) a.prof[t * 16 + 0] = clock64();
+                ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&s_full[b], ph, a.budget, &s_abort));
                 if (!ok) break;
                 tc::fence_after_sync();
+                if (stamp) a.prof[t * 16 + 1] = clock64();
+                // both threads of a row read all 64 scores and take the maximum themselves (cheaper than an exchange through
+                // shared memory); each then exponentiates its own 32 columns
+                uint32_t sr[32], so[32];
+                tc::tmem_ld_32x32(tmem + lane_base + b * kTcTok + half * 32, sr);
+                tc::tmem_ld_32x32(tmem + lane_base + b * kTcTok + (half ^ 1) * 32, so);
+                tc::tmem_ld_wait();
+                if (stamp) a.prof[t * 16 + 2] = clock64();
+                if constexpr (TRANSFORM) {
+                    const int to = tt * kTcTok + (half ^ 1) * 32;
+                    if (bias == nullptr || rp - tt * kTcTok - (kTcTok - 1) >= a.opt.bias_len - 1) {      // the whole tile is far away
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) {
+                            sr[j] = __float_as_uint(fmaf(__uint_as_float(sr[j]), row_scale, bias_far));
+                            so[j] = __float_as_uint(fmaf(__uint_as_float(so[j]), row_scale, bias_far));
+                        }
+                    } else {
+                        const int far = a.opt.bias_len - 1;
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) {
+                            const float br = __ldg(bias + min(max(rp - t0 - j, 0), far)) * 1.4426950408889634f;
+                            const float bo = __ldg(bias + min(max(rp - to - j, 0), far)) * 1.4426950408889634f;
+                            sr[j] = __float_as_uint(fmaf(__uint_as_float(sr[j]), row_scale, br));
+                            so[j] = __float_as_uint(fmaf(__uint_as_float(so[j]), row_scale, bo));
+                        }
+                    }
+                }
+                if (tt * kTcTok < lo_max) {                               // tokens before some row's block
+                    const int to = tt * kTcTok + (half ^ 1) * 32;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        if (t0 + j < lo && t0 + j >= keep) sr[j] = 0xff800000u;
+                        if (to + j < lo && to + j >= keep) so[j] = 0xff800000u;
+                    }
+                }
+                if (tt * kTcTok + kTcTok - 1 > pos_q0) {                  // some row of the tile does not see every token
+                    const int to = tt * kTcTok + (half ^ 1) * 32;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        if (t0 + j > rp) sr[j] = 0xff800000u;             // -inf
+                        if (to + j > rp) so[j] = 0xff800000u;
+                    }
+                }
+                float mq[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                for (int j = 0; j < 32; ++j) mq[j & 3] = fmaxf(mq[j & 3], fmaxf(__uint_as_float(sr[j]), __uint_as_float(so[j])));
+                float mx = fmaxf(fmaxf(mq[0], mq[1]), fmaxf(mq[2], mq[3]));
+                if constexpr (!TRANSFORM) mx *= sc;                       // scale > 0, so the maximum commutes with it
+                if (stamp) a.prof[t * 16 + 3] = clock64();
+                float alpha = 1.f;
+                if (fresh) {                                              // (a row that sees nothing yet keeps a finite reference)
+                    if (mx != -INFINITY) { m_ref = mx; fresh = false; }
+                }
+                else if (mx > m_ref + 8.f) { alpha = ex2_approx(m_ref - mx); m_ref = mx; }
+                const bool rescale = __any_sync(0xffffffffu, alpha != 1.f);
+                float sq[4] = {0.f, 0.f, 0.f, 0.f};
+                uint32_t pk[16];
+#pragma unroll
+                for (int j = 0; j < 32; j += 2) {
+                    const float s0 = __uint_as_float(sr[j]), s1 = __uint_as_float(sr[j + 1]);
+                    const float p0 = ex2_approx(TRANSFORM ? s0 - m_ref : fmaf(s0, sc, -m_ref));
+                    const float p1 = ex2_approx(TRANSFORM ? s1 - m_ref : fmaf(s1, sc, -m_ref));
+                    sq[(j >> 1) & 3] += p0 + p1;
+                    pk[j >> 1] = f32x2_to_bf16x2_bits(p0, p1);
+                }
+                l_run = l_run * alpha + ((sq[0] + sq[1]) + (sq[2] + sq[3]));
+                if (n >= 2) {                                             // P buffer b was read by P V(t - 2)
+                    ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&pv_done[b], (uint32_t)((n - 2) >> 1) & 1u, a.budget, &s_abort));
+                    if (!ok) break;
+                }
+                if (stamp) a.prof[t * 16 + 4] = clock64();
+                unsigned char* prow = sP + b * kTcPBuf + row * 128;
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    *reinterpret_cast<uint4*>(prow + (((half * 4 + c) ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+                if (t == T - 1 && kv_end < (tt + 1) * kTcTok) {
+                    // token rows of the last V tile beyond the sequence's end: zero them (whole 128-byte rows, so the swizzle
+                    // does not matter)
+                    // (a shared tile has been read by S(t) already: the scores are here)
+                    ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(SHARED ? &k_full[n & 3] : &v_full[b], SHARED ? (uint32_t)(n >> 2) & 1u : ph,
+                                                                         a.budget, &s_abort));
+                    if (!ok) break;
+                    const int jz = kv_end - tt * kTcTok;
+                    unsigned char* vs = (SHARED ? sK : sV) + (n & kStageMask) * kTcVStage;
+                    for (int i = (int)threadIdx.x; i < (kTcTok - jz) * kNBV * 8; i += 2 * kTcRows) {
+                        const int r = jz + i / (kNBV * 8), cb = i % (kNBV * 8) >> 3, c = i & 7;
+                        *reinterpret_cast<uint4*>(vs + cb * (kTcTok * 128) + r * 128 + c * 16) = make_uint4(0, 0, 0, 0);
+                    }
+                }
+                if (stamp) a.prof[t * 16 + 5] = clock64();
+                tc::fence_proxy_async_smem();
+                if (stamp) a.prof[t * 16 + 6] = clock64();
+                if (rescale) {                                            // t >= 1: O must be complete up to P V(t - 1)
+                    ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&pv_done[b ^ 1], (uint32_t)((n - 1) >> 1) & 1u, a.budget, &s_abort));
+                    if (!ok) break;
+                    tc::fence_after_sync();
+#pragma unroll 1
+                    for (int c0 = half * (DV / 2); c0 < (half + 1) * (DV / 2); c0 += 32) {
+                        uint32_t r[32];
+                        tc::tmem_ld_32x32(tmem_o + lane_base + c0, r);
+                        tc::tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * alpha);
+                        tc::tmem_st_32x32(tmem_o + lane_base + c0, r);
+                    }
+                    tc::tmem_st_wait();
+                }
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&p_full[b]);
+                if (stamp) a.prof[t * 16 + 7] = clock64();
+            }
+            // ---- epilogue: O / l -> bf16 rows staged in shared memory (Q and K stages are free once the last P V is done)
+            if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&pv_done[(g + T - 1) & 1], (uint32_t)((g + T - 1) >> 1) & 1u, a.budget, &s_abort));
+            if (cta_stamp) a.prof[2 * 16 + 15] = clock64();
+            s_l[half][row] = l_run;
+            asm volatile("bar.sync 1, 256;" ::: "memory");               // the eight softmax warps only; every one of them gets here
+            if (cta_stamp) a.prof[3 * 16 + 15] = clock64();
+            if constexpr (DEC) {
+                // partial result of this split for query row (r, g): unnormalised output, reference maximum (natural-log units, as
+                // the merge pass expects) and sum
+                const int r = row >> 3, gq = row & 7;
+                // the CTA that has tile x is the i-th with i total / n_ctas <= x < (i + 1) total / n_ctas
+                auto cta_of = [&](int x) { return (int)((((long long)x + 1) * n_ctas - 1) / total); };
+                const int part = even ? (int)blockIdx.x - cta_of(x0) : (int)blockIdx.x;
+                const bool mine = row < nq && gq < G && part < a.max_splits;
+                if (even && t_off == 0 && gq == 0 && half == 0 && row < nq)          // the (sequence, KV head) begins here
+                    a.part_n[(size_t)(row_start + r) * a.Hkv + kvh] = min(cta_of(x0 + T_seq - 1) - (int)blockIdx.x + 1, a.max_splits);
+                if (ok && quad * 32 < nq) {                              // warp-uniform: the tensor-memory loads are collective
+                    tc::fence_after_sync();
+                    const size_t idx = ((size_t)(row_start + (mine ? r : 0)) * a.Hq + h + (mine ? gq : 0)) * a.max_splits + part;
+                    float* dst = a.part_acc + idx * DV;
+#pragma unroll 1
+                    for (int c0 = half * (DV / 2); c0 < (half + 1) * (DV / 2); c0 += 32) {
+                        uint32_t rr[32];
+                        tc::tmem_ld_32x32(tmem_o + lane_base + c0, rr);
+                        tc::tmem_ld_wait();
+                        if (mine) {
+#pragma unroll
+                            for (int jj = 0; jj < 32; jj += 4)
+                                *reinterpret_cast<uint4*>(dst + c0 + jj) = make_uint4(rr[jj], rr[jj + 1], rr[jj + 2], rr[jj + 3]);
+                        }
+                    }
+                    if (mine && half == 0) {
+                        const float l = l_run + s_l[1][row];
+                        a.part_ml[idx * 2] = l > 0.f ? m_ref * 0.6931471805599453f : -3.0e38f;
+                        a.part_ml[idx * 2 + 1] = l;
+                    }
+                }
+            } else {
+            if (ok) {
+                tc::fence_after_sync();
+                float l = l_run + s_l[half ^ 1][row];
+                if (a.opt.sink != nullptr) l += ex2_approx(fmaf(a.opt.sink[h], 1.4426950408889634f, -m_ref));
+                float inv = l > 0.f ? 1.f / l : 0.f;
+                if (a.gate != nullptr && a.opt.gate_per_head && row < nq)
+                    inv *= sigmoid_f(bf16_to_f32(a.gate[(size_t)(row_start + r_begin + row) * a.ld_gate + (size_t)h * a.gate_head_stride + a.gate_offset]));
+                __nv_bfloat16* stg = reinterpret_cast<__nv_bfloat16*>(smem) + row * kTcOutPitch;
 #pragma unroll 1
                 for (int c0 = half * (DV / 2); c0 < (half + 1) * (DV / 2); c0 += 32) {
                     uint32_t r[32];
                     tc::tmem_ld_32x32(tmem_o + lane_base + c0, r);
                     tc::tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * alpha);
-                    tc::tmem_st_32x32(tmem_o + lane_base + c0, r);
-                }
-                tc::tmem_st_wait();
-            }
-            tc::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&p_full[b]);
-            if (stamp) a.prof[t * 16 + 7] = clock64();
-        }
-        // ---- epilogue: O / l -> bf16 rows staged in shared memory (Q and K stages are free once the last P V is done)
-        if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&pv_done[(T - 1) & 1], (uint32_t)((T - 1) >> 1) & 1u, a.budget, &s_abort));
-        if (cta_stamp) a.prof[2 * 16 + 15] = clock64();
-        s_l[half][row] = l_run;
-        asm volatile("bar.sync 1, 256;" ::: "memory");               // the eight softmax warps only; every one of them gets here
-        if (cta_stamp) a.prof[3 * 16 + 15] = clock64();
-        if constexpr (DEC) {
-            // partial result of this split for query row (r, g): unnormalised output, reference maximum (natural-log units, as
-            // the merge pass expects) and sum
-            const int r = row >> 3, g = row & 7;
-            const bool mine = row < nq && g < G;
-            if (ok && quad * 32 < nq) {                              // warp-uniform: the tensor-memory loads are collective
-                tc::fence_after_sync();
-                const size_t idx = ((size_t)(row_start + (mine ? r : 0)) * a.Hq + h + (mine ? g : 0)) * a.max_splits + blockIdx.x;
-                float* dst = a.part_acc + idx * DV;
-#pragma unroll 1
-                for (int c0 = half * (DV / 2); c0 < (half + 1) * (DV / 2); c0 += 32) {
-                    uint32_t rr[32];
-                    tc::tmem_ld_32x32(tmem_o + lane_base + c0, rr);
-                    tc::tmem_ld_wait();
-                    if (mine) {
+                    for (int j = 0; j < 32; j += 8) {
+                        uint32_t w[4];
 #pragma unroll
-                        for (int jj = 0; jj < 32; jj += 4)
-                            *reinterpret_cast<uint4*>(dst + c0 + jj) = make_uint4(rr[jj], rr[jj + 1], rr[jj + 2], rr[jj + 3]);
+                        for (int e = 0; e < 4; ++e)
+                            w[e] = f32x2_to_bf16x2_bits(__uint_as_float(r[j + 2 * e]) * inv, __uint_as_float(r[j + 2 * e + 1]) * inv);
+                        *reinterpret_cast<uint4*>(stg + c0 + j) = make_uint4(w[0], w[1], w[2], w[3]);
                     }
                 }
-                if (mine && half == 0) {
-                    const float l = l_run + s_l[1][row];
-                    a.part_ml[idx * 2] = l > 0.f ? m_ref * 0.6931471805599453f : -3.0e38f;
-                    a.part_ml[idx * 2 + 1] = l;
-                }
             }
-        } else {
-        if (ok) {
-            tc::fence_after_sync();
-            float l = l_run + s_l[half ^ 1][row];
-            if (a.opt.sink != nullptr) l += ex2_approx(fmaf(a.opt.sink[h], 1.4426950408889634f, -m_ref));
-            float inv = l > 0.f ? 1.f / l : 0.f;
-            if (a.gate != nullptr && a.opt.gate_per_head && row < nq)
-                inv *= sigmoid_f(bf16_to_f32(a.gate[(size_t)(row_start + r_begin + row) * a.ld_gate + (size_t)h * a.gate_head_stride + a.gate_offset]));
-            __nv_bfloat16* stg = reinterpret_cast<__nv_bfloat16*>(smem) + row * kTcOutPitch;
-#pragma unroll 1
-            for (int c0 = half * (DV / 2); c0 < (half + 1) * (DV / 2); c0 += 32) {
-                uint32_t r[32];
-                tc::tmem_ld_32x32(tmem_o + lane_base + c0, r);
-                tc::tmem_ld_wait();
+            if (cta_stamp) a.prof[4 * 16 + 15] = clock64();
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            if (cta_stamp) a.prof[5 * 16 + 15] = clock64();
+            if (ok) {
+                // 16-byte pieces, four per thread and pass so that the gate loads of a pass are in flight together
+                const __nv_bfloat16* stg0 = reinterpret_cast<const __nv_bfloat16*>(smem);
+                const int n_items = nq * (DV / 8);
+                const bool elementwise = a.gate != nullptr && !a.opt.gate_per_head;
+                for (int i0 = (int)threadIdx.x; i0 < n_items; i0 += 8 * kTcRows) {
+                    uint4 g[4];
 #pragma unroll
-                for (int j = 0; j < 32; j += 8) {
-                    uint32_t w[4];
+                    for (int u = 0; u < 4; ++u) {
+                        const int i = i0 + u * 2 * kTcRows;
+                        g[u] = make_uint4(0, 0, 0, 0);
+                        if (elementwise && i < n_items)
+                            g[u] = __ldg(reinterpret_cast<const uint4*>(a.gate + (size_t)(row_start + r_begin + i / (DV / 8)) * a.ld_gate +
+                                                                        (size_t)h * a.gate_head_stride + a.gate_offset + i % (DV / 8) * 8));
+                    }
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        w[e] = f32x2_to_bf16x2_bits(__uint_as_float(r[j + 2 * e]) * inv, __uint_as_float(r[j + 2 * e + 1]) * inv);
-                    *reinterpret_cast<uint4*>(stg + c0 + j) = make_uint4(w[0], w[1], w[2], w[3]);
-                }
-            }
-        }
-        if (cta_stamp) a.prof[4 * 16 + 15] = clock64();
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (cta_stamp) a.prof[5 * 16 + 15] = clock64();
-        if (ok) {
-            // 16-byte pieces, four per thread and pass so that the gate loads of a pass are in flight together
-            const __nv_bfloat16* stg0 = reinterpret_cast<const __nv_bfloat16*>(smem);
-            const int n_items = nq * (DV / 8);
-            const bool elementwise = a.gate != nullptr && !a.opt.gate_per_head;
-            for (int i0 = (int)threadIdx.x; i0 < n_items; i0 += 8 * kTcRows) {
-                uint4 g[4];
+                    for (int u = 0; u < 4; ++u) {
+                        const int i = i0 + u * 2 * kTcRows;
+                        if (i >= n_items) break;
+                        const int r = i / (DV / 8), c = i % (DV / 8);
+                        uint4 v = *reinterpret_cast<const uint4*>(stg0 + r * kTcOutPitch + c * 8);
+                        if (elementwise) {
+                            const uint32_t vw[4] = {v.x, v.y, v.z, v.w}, gw[4] = {g[u].x, g[u].y, g[u].z, g[u].w};
+                            uint32_t o[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int i = i0 + u * 2 * kTcRows;
-                    g[u] = make_uint4(0, 0, 0, 0);
-                    if (elementwise && i < n_items)
-                        g[u] = __ldg(reinterpret_cast<const uint4*>(a.gate + (size_t)(row_start + r_begin + i / (DV / 8)) * a.ld_gate +
-                                                                    (size_t)h * a.gate_head_stride + a.gate_offset + i % (DV / 8) * 8));
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int i = i0 + u * 2 * kTcRows;
-                    if (i >= n_items) break;
-                    const int r = i / (DV / 8), c = i % (DV / 8);
-                    uint4 v = *reinterpret_cast<const uint4*>(stg0 + r * kTcOutPitch + c * 8);
-                    if (elementwise) {
-                        const uint32_t vw[4] = {v.x, v.y, v.z, v.w}, gw[4] = {g[u].x, g[u].y, g[u].z, g[u].w};
-                        uint32_t o[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float2 vv = bf16x2_bits_to_f32x2(vw[e]), gg = bf16x2_bits_to_f32x2(gw[e]);
-                            o[e] = f32x2_to_bf16x2_bits(vv.x * sigmoid_fast(gg.x), vv.y * sigmoid_fast(gg.y));
+                            for (int e = 0; e < 4; ++e) {
+                                const float2 vv = bf16x2_bits_to_f32x2(vw[e]), gg = bf16x2_bits_to_f32x2(gw[e]);
+                                o[e] = f32x2_to_bf16x2_bits(vv.x * sigmoid_fast(gg.x), vv.y * sigmoid_fast(gg.y));
+                            }
+                            v = make_uint4(o[0], o[1], o[2], o[3]);
                         }
-                        v = make_uint4(o[0], o[1], o[2], o[3]);
+                        *reinterpret_cast<uint4*>(a.out + ((size_t)(row_start + r_begin + r) * a.Hq + h) * DV + c * 8) = v;
                     }
-                    *reinterpret_cast<uint4*>(a.out + ((size_t)(row_start + r_begin + r) * a.Hq + h) * DV + c * 8) = v;
                 }
             }
+            }   // prefill epilogue
+            if constexpr (!DEC) break;
+            g += T;
+            // the sums have been read, and all eight warps go on or none does: the barriers count all of them
+            if (!softmax_all(ok) || !next_piece()) break;
         }
-        }   // prefill epilogue
     }
     if (cta_stamp) a.prof[6 * 16 + 15] = clock64();
     tc::fence_before_sync();
@@ -596,7 +721,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             set_status(a.status, PS_DEV_WAIT_TIMEOUT);
             // copies still in flight get a bounded chance to land before the shared memory goes back to the next CTA
             const long long bd = a.budget < 4000000ll ? a.budget : 4000000ll;
-            if (q_issued > q_consumed) tc::mbar_wait(&q_full, 0, bd);
+            for (int c = q_consumed; c < q_issued; ++c) tc::mbar_wait(&q_full, (uint32_t)c & 1u, bd);
             for (int c = k_consumed; c < k_issued; ++c) tc::mbar_wait(&k_full[c & kStageMask], (uint32_t)(c >> kStageLog) & 1u, bd);
             for (int c = v_consumed; c < v_issued; ++c) tc::mbar_wait(&v_full[c & 1], (uint32_t)(c >> 1) & 1u, bd);
         }

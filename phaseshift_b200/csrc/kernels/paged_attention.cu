@@ -254,6 +254,7 @@ struct AttnMergeArgs {
     __nv_bfloat16* out;   // [rows, Hq*D]
     AttnOptions opt;
     int ring;             // > 0: split s of a row lies in slot s % ring of the partials
+    const int* part_n; int Hkv;   // or: a row's partials for the query heads of a KV head, [rows, Hkv], from slot 0 on
 };
 
 // grid = (Hq, rows), block = D threads.  The split weights exp(m_s - max m) are computed once, in
@@ -269,8 +270,10 @@ __global__ void paged_attn_merge_kernel(const AttnMergeArgs a) {
     const int h = blockIdx.x, row = blockIdx.y, d = threadIdx.x;
     const int visible = a.row_pos[row] + 1;
     if (visible < 0) return;                                            // position -2: a row another kernel of the step owns
-    const int n = (visible + a.split_tokens - 1) / a.split_tokens;      // 0 for a padding row
-    const int lo = visible > 0 ? attn_first(a.opt, visible - 1) : 0, s0 = lo / a.split_tokens;
+    const bool counted = !RING && a.part_n != nullptr;
+    const int n = visible <= 0 ? 0 : counted ? max(0, min(a.part_n[(size_t)row * a.Hkv + h / (a.Hq / a.Hkv)], a.max_splits)) :
+                                               (visible + a.split_tokens - 1) / a.split_tokens;      // 0 for a padding row
+    const int lo = visible > 0 && !counted ? attn_first(a.opt, visible - 1) : 0, s0 = counted ? 0 : lo / a.split_tokens;
     // splits of kept first positions before those of the run (no ring then)
     const int ks = RING ? 0 : min((min(a.opt.keep_first, lo) + a.split_tokens - 1) / a.split_tokens, s0);
     const int first = s0 - ks;                                          // the i-th split of the row, i from `first` on
@@ -348,7 +351,7 @@ PS_API int ps_paged_attention_ex(const void* q, const void* k_pool, const void* 
     m.part_acc = a.part_acc; m.part_ml = a.part_ml; m.row_pos = a.row_pos; m.rows = rows; m.Hq = Hq; m.D = D;
     m.split_tokens = split_tokens; m.max_splits = max_splits; m.gate = (const __nv_bfloat16*)gate;
     m.ld_gate = ld_gate; m.gate_head_stride = gate_head_stride; m.gate_offset = gate_offset;
-    m.out = (__nv_bfloat16*)out; m.opt = opt; m.ring = 0;
+    m.out = (__nv_bfloat16*)out; m.opt = opt; m.ring = 0; m.part_n = nullptr; m.Hkv = Hkv;
     return launch_pdl(paged_attn_merge_kernel<false>, dim3(Hq, rows), dim3(D), 0, stream, m);
 }
 
@@ -378,8 +381,25 @@ PS_API int ps_paged_attention_merge_ex(const void* part_acc, const void* part_ml
     m.part_acc = (const float*)part_acc; m.part_ml = (const float*)part_ml; m.row_pos = (const int*)row_pos; m.rows = rows; m.Hq = Hq; m.D = D;
     m.split_tokens = split_tokens; m.max_splits = max_splits; m.gate = (const __nv_bfloat16*)gate;
     m.ld_gate = ld_gate; m.gate_head_stride = gate_head_stride; m.gate_offset = gate_offset;
-    m.out = (__nv_bfloat16*)out; m.opt = opt; m.ring = ring;
+    m.out = (__nv_bfloat16*)out; m.opt = opt; m.ring = ring; m.part_n = nullptr; m.Hkv = Hq;
     return launch_pdl(ring > 0 ? paged_attn_merge_kernel<true> : paged_attn_merge_kernel<false>, dim3(Hq, rows), dim3(D), 0, stream, m);
+}
+
+// The merge pass for partials that were counted when they were made (ps_attn_decode_tc_even).
+PS_API int ps_paged_attention_merge_even(const void* part_acc, const void* part_ml, const void* part_n, const void* row_pos, int rows, int Hq,
+                                         int Hkv, int D, int max_splits, const void* gate, int ld_gate, int gate_head_stride,
+                                         int gate_offset, void* out, const void* options, cudaStream_t stream) {
+    using namespace ps;
+    const AttnOptions opt = attn_options(options);
+    if (part_n == nullptr || rows <= 0 || rows > 65535 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv) || D <= 0 || D > 1024 || max_splits > kAttnMaxSplits ||
+        !attn_options_ok(opt))
+        return (int)cudaErrorInvalidValue;
+    AttnMergeArgs m;
+    m.part_acc = (const float*)part_acc; m.part_ml = (const float*)part_ml; m.row_pos = (const int*)row_pos; m.rows = rows; m.Hq = Hq; m.D = D;
+    m.split_tokens = 1; m.max_splits = max_splits; m.gate = (const __nv_bfloat16*)gate;
+    m.ld_gate = ld_gate; m.gate_head_stride = gate_head_stride; m.gate_offset = gate_offset;
+    m.out = (__nv_bfloat16*)out; m.opt = opt; m.ring = 0; m.part_n = (const int*)part_n; m.Hkv = Hkv;
+    return launch_pdl(paged_attn_merge_kernel<false>, dim3(Hq, rows), dim3(D), 0, stream, m);
 }
 
 PS_API int ps_paged_attention_merge(const void* part_acc, const void* part_ml, const void* row_pos, int rows, int Hq, int D,

@@ -523,6 +523,8 @@ class CudaOps(OpTrace):
         if rows > SMALL_M_MAX and not self.exact_rows:
             want = max(1, (4 * 148) // (rows * hkv))
             split_tokens = max(split_tokens, -(-(-(-max_visible // want)) // 32) * 32)
+        # The kernel for bf16 pages below takes even shares of a batch's tokens instead, one per SM, however long its sequences are.
+        even = rows > SMALL_M_MAX and not self.exact_rows and self.max_splits * 64 >= max_visible
         pacc = self.buf("attn_part_acc" + geom, rows, hq * self.max_splits * D, torch.float32)
         pml = self.buf("attn_part_ml" + geom, rows, hq * self.max_splits * 2, torch.float32)
         # Decode / verify rows on the tensor cores: bf16 pages, head dims of whole 64s, every sequence handled here has at most 16 rows
@@ -536,6 +538,16 @@ class CudaOps(OpTrace):
                 and (b.graph_static or row_pos is b.row_pos_short or all(len(sq.token_ids) <= 16 for sq in b.seqs))):
             st_tok = -(-split_tokens // 64) * 64
             n_seqs = b.max_seqs if b.graph_static else b.n_seqs
+            if even:
+                part_n = self.buf(f"attn_part_n{hkv}", rows, hkv, torch.int32)
+                _lib.call("ps_attn_decode_tc_even", ptr(q), c_int(q.shape[0]), ptr(kv.k), ptr(kv.v), ptr(st.block_table),
+                          c_int(st.max_blocks), c_int(st.sc.page_tokens), c_int(st.num_pages), ptr(b.seq_desc), c_int(n_seqs),
+                          c_int(16), c_int(hq), c_int(hkv), c_int(D), sm, c_int(self.max_splits), c_int(max_visible), ptr(pacc),
+                          ptr(pml), ptr(part_n), ptr(st.status), opt)
+                _lib.call("ps_paged_attention_merge_even", ptr(pacc), ptr(pml), ptr(part_n), ptr(row_pos), c_int(rows), c_int(hq),
+                          c_int(hkv), c_int(D), c_int(self.max_splits), *gate, ptr(out), opt)
+                self.launches += 2
+                return out
             _lib.call("ps_attn_decode_tc_ex", ptr(q), c_int(q.shape[0]), ptr(kv.k), ptr(kv.v), ptr(st.block_table),
                       c_int(st.max_blocks), c_int(st.sc.page_tokens), c_int(st.num_pages), ptr(b.seq_desc), c_int(n_seqs),
                       c_int(16), c_int(hq), c_int(hkv), c_int(D), sm, c_int(st_tok), c_int(self.max_splits),
