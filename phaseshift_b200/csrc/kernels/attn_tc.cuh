@@ -143,7 +143,7 @@ __device__ __forceinline__ int expanded_row0(const int* seqs, int s, int min_row
 // partial's number is that of its CTA among those that share the (sequence, KV head).  With 224 KB of shared memory a CTA has an SM to
 // itself, so splits of a fixed length run in rounds, each with its own set-up, and sequences of unequal length leave the last one
 // nearly empty.  Sequences of 5 to 100 % of a length, 4 KV heads of 256: 12 of up to 3001 tokens 29.7 -> 24.9 us, 24 of up to 3500 with keys
-// that are the values 47 -> 38.4.  What bounds it now: a tile's chain through the softmax warps, 1.5 us and more beside 0.7 or 1.4 of bytes.
+// that are the values 47 -> 38.4 (35.8 since).  What bounds it now: a tile's chain through the softmax warps, 1.5 us and more beside 0.7 or 1.4 of bytes.
 // TRANSFORM: query temperature and distance bias, applied to the scores before the maximum.
 // EXPANDED: keys and values were expanded per query head into rows of consecutive tokens (attn_latent.cu), the last 64-column
 // groups of the keys (`map_r`) are shared by all heads.
@@ -316,11 +316,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             if (n > 0 && !__all_sync(0xffffffffu, tc::mbar_wait_abortable(&q_free, (uint32_t)(n - 1) & 1u, a.budget, &s_abort))) return false;
             // one 8-row box per (row of the sequence, 64-column group): the G heads of this KV head are consecutive rows
             // of the [rows * Hq, D] view of q; tile rows 8 r + g with g >= G hold other heads' values and are never used
-            if (lane == 0) tc::mbar_expect_tx(&q_full, (uint32_t)n_rows * (uint32_t)kNB * 1024u);
+            const int copies = nq <= 32 ? 4 : 1;                     // one for every quadrant of the accumulator's lanes
+            if (lane == 0) tc::mbar_expect_tx(&q_full, (uint32_t)(copies * n_rows) * (uint32_t)kNB * 1024u);
             __syncwarp();
-            for (int i = lane; i < kNB * n_rows; i += 32) {
-                const int r = i / kNB, c4 = i % kNB;
-                tc::tma_load_2d(sQ + c4 * (kTcRows * 128) + (8 * r) * 128, &map_q, c4 * 64, (row_start + r) * a.Hq + h, &q_full);
+            for (int i = lane; i < kNB * n_rows * copies; i += 32) {
+                const int c4 = i % kNB, r = i / kNB % n_rows, copy = i / kNB / n_rows;
+                tc::tma_load_2d(sQ + c4 * (kTcRows * 128) + (32 * copy + 8 * r) * 128, &map_q, c4 * 64, (row_start + r) * a.Hq + h, &q_full);
             }
         } else {
             if (lane == 0) tc::mbar_expect_tx(&q_full, kTcQBytes);
@@ -464,7 +465,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
         bool ok = true;
         for (int g = 0;;) {
-            const int rp = DEC ? pos_q0 + (row >> 3) : pos_q0 + row;     // position of this thread's query row
+            // decode with up to four rows: the query rows fill one quadrant, whose two warps share a scheduler and its exponential unit.  Q is
+            // there four times instead, so that every warp has the scores; the quadrants take every fourth pair of a half's columns
+            // each and write the probabilities of the first one's rows (24 sequences, keys that are the values: 38.8 -> 35.8 us; the pass
+            // from a tile's maximum to its probabilities had 900 of a tile's 2000 cycles)
+            const bool spread = DEC && nq <= 32;
+            const int qrow = spread ? lane : row;
+            const int rp = DEC ? pos_q0 + (qrow >> 3) : pos_q0 + row;    // position of this thread's query row
             const float sc = a.scale_log2;
             const int lo = attn_first(a.opt, rp);                        // first token this row sees
             const int lo_max = attn_first(a.opt, kv_end - 1);            // ... and the largest of any row
@@ -480,8 +487,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             }
             // decode: a warp without query rows only keeps the barriers' count, and rows that hold nothing (or another KV head's
             // queries) ask for no rescaling (8 rows of one sequence 721 -> 712 us per step of 8 layers, 24 sequences 833 -> 821 of 4)
-            const bool idle = DEC && quad * 32 >= nq, counts = !DEC || (row < nq && (row & 7) < G);
+            const bool idle = DEC && !spread && quad * 32 >= nq, counts = !DEC || (qrow < nq && (row & 7) < G);
             float m_ref = 0.f, l_run = 0.f;
+            [[maybe_unused]] float l4[4] = {0.f, 0.f, 0.f, 0.f};         // decode: sums of every fourth pair, so that both forms add alike
             bool fresh = true;                                            // this row has not seen a token yet: m_ref is a placeholder
             // the epilogue reads this tile's gate values (one 512-byte run per row): ask for them now, so that they come from
             // L2 then
@@ -554,26 +562,56 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     }
                     else if (mx > m_ref + 8.f && counts) { alpha = ex2_approx(m_ref - mx); m_ref = mx; }
                     rescale = __any_sync(0xffffffffu, alpha != 1.f);
-                    float sq[4] = {0.f, 0.f, 0.f, 0.f};
-                    uint32_t pk[16];
+                    if (spread) {
+                        float sum = 0.f;
+                        uint32_t pk[4];
 #pragma unroll
-                    for (int j = 0; j < 32; j += 2) {
-                        const float s0 = __uint_as_float(sr[j]), s1 = __uint_as_float(sr[j + 1]);
-                        const float p0 = ex2_approx(TRANSFORM ? s0 - m_ref : fmaf(s0, sc, -m_ref));
-                        const float p1 = ex2_approx(TRANSFORM ? s1 - m_ref : fmaf(s1, sc, -m_ref));
-                        sq[(j >> 1) & 3] += p0 + p1;
-                        pk[j >> 1] = f32x2_to_bf16x2_bits(p0, p1);
-                    }
-                    l_run = l_run * alpha + ((sq[0] + sq[1]) + (sq[2] + sq[3]));
-                    if (n >= 2) {                                             // P buffer b was read by P V(t - 2)
-                        ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&pv_done[b], (uint32_t)((n - 2) >> 1) & 1u, a.budget, &s_abort));
-                        if (!ok) break;
-                    }
-                    if (stamp) a.prof[t * 16 + 4] = clock64();
-                    unsigned char* prow = sP + b * kTcPBuf + row * 128;
+                        for (int i = 0; i < 4; ++i) {
+                            float p[2];
 #pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        *reinterpret_cast<uint4*>(prow + (((half * 4 + c) ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+                            for (int e = 0; e < 2; ++e) {
+                                const uint32_t x01 = quad & 1 ? sr[8 * i + 2 + e] : sr[8 * i + e], x23 = quad & 1 ? sr[8 * i + 6 + e] : sr[8 * i + 4 + e];
+                                const float sc_ = __uint_as_float(quad & 2 ? x23 : x01);
+                                p[e] = ex2_approx(TRANSFORM ? sc_ - m_ref : fmaf(sc_, sc, -m_ref));
+                            }
+                            sum += p[0] + p[1];
+                            pk[i] = f32x2_to_bf16x2_bits(p[0], p[1]);
+                        }
+                        l4[0] = fmaf(l4[0], alpha, sum);
+                        if (n >= 2) {                                     // P buffer b was read by P V(t - 2)
+                            ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&pv_done[b], (uint32_t)((n - 2) >> 1) & 1u, a.budget, &s_abort));
+                            if (!ok) break;
+                        }
+                        unsigned char* prow = sP + b * kTcPBuf + lane * 128 + 4 * quad;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint32_t*>(prow + (((half * 4 + i) ^ (lane & 7)) << 4)) = pk[i];
+                    } else {
+                        float sq[4] = {0.f, 0.f, 0.f, 0.f};
+                        uint32_t pk[16];
+#pragma unroll
+                        for (int j = 0; j < 32; j += 2) {
+                            const float s0 = __uint_as_float(sr[j]), s1 = __uint_as_float(sr[j + 1]);
+                            const float p0 = ex2_approx(TRANSFORM ? s0 - m_ref : fmaf(s0, sc, -m_ref));
+                            const float p1 = ex2_approx(TRANSFORM ? s1 - m_ref : fmaf(s1, sc, -m_ref));
+                            sq[(j >> 1) & 3] += p0 + p1;
+                            pk[j >> 1] = f32x2_to_bf16x2_bits(p0, p1);
+                        }
+                        if constexpr (DEC) {
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) l4[k] = fmaf(l4[k], alpha, sq[k]);
+                        } else {
+                            l_run = l_run * alpha + ((sq[0] + sq[1]) + (sq[2] + sq[3]));
+                        }
+                        if (n >= 2) {                                             // P buffer b was read by P V(t - 2)
+                            ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&pv_done[b], (uint32_t)((n - 2) >> 1) & 1u, a.budget, &s_abort));
+                            if (!ok) break;
+                        }
+                        if (stamp) a.prof[t * 16 + 4] = clock64();
+                        unsigned char* prow = sP + b * kTcPBuf + row * 128;
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            *reinterpret_cast<uint4*>(prow + (((half * 4 + c) ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+                    }
                 }
                 if (t == T - 1 && kv_end < (tt + 1) * kTcTok) {
                     // token rows of the last V tile beyond the sequence's end: zero them (whole 128-byte rows, so the swizzle
@@ -592,7 +630,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 if (stamp) a.prof[t * 16 + 5] = clock64();
                 tc::fence_proxy_async_smem();
                 if (stamp) a.prof[t * 16 + 6] = clock64();
-                if (rescale) {                                            // t >= 1: O must be complete up to P V(t - 1)
+                if (rescale && (!spread || quad == 0)) {                  // t >= 1: O must be complete up to P V(t - 1)
                     ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&pv_done[b ^ 1], (uint32_t)((n - 1) >> 1) & 1u, a.budget, &s_abort));
                     if (!ok) break;
                     tc::fence_after_sync();
@@ -615,7 +653,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             // ---- epilogue: O / l -> bf16 rows staged in shared memory (Q and K stages are free once the last P V is done)
             if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&pv_done[(g + T - 1) & 1], (uint32_t)((g + T - 1) >> 1) & 1u, a.budget, &s_abort));
             if (cta_stamp) a.prof[2 * 16 + 15] = clock64();
-            s_l[half][row] = l_run;
+            s_l[half][row] = DEC && !spread ? (l4[0] + l4[1]) + (l4[2] + l4[3]) : DEC ? l4[0] : l_run;
             asm volatile("bar.sync 1, 256;" ::: "memory");               // the eight softmax warps only; every one of them gets here
             if (cta_stamp) a.prof[3 * 16 + 15] = clock64();
             if constexpr (DEC) {
@@ -644,7 +682,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                         }
                     }
                     if (mine && half == 0) {
-                        const float l = l_run + s_l[1][row];
+                        float l = s_l[0][row] + s_l[1][row];
+                        if (spread)
+                            l = ((s_l[0][row] + s_l[0][row + 32]) + (s_l[0][row + 64] + s_l[0][row + 96])) +
+                                ((s_l[1][row] + s_l[1][row + 32]) + (s_l[1][row + 64] + s_l[1][row + 96]));
                         a.part_ml[idx * 2] = l > 0.f ? m_ref * 0.6931471805599453f : -3.0e38f;
                         a.part_ml[idx * 2 + 1] = l;
                     }
