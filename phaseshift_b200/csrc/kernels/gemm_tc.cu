@@ -15,7 +15,8 @@
 // Every mbarrier wait is bounded; a timeout sets PS_DEV_WAIT_TIMEOUT in the status word, the CTA
 // stops issuing, frees its tensor memory and returns.
 // The kernels are launched programmatically: a prompt is a chain of products, norms and mixers of 5 to 100 us whose set-up and, for CTA
-// pairs, first weights need not wait for the one before.  They take tensor memory only when their predecessors are done, and let their
+// pairs, first weights need not wait for the one before -- weights of the model, that is: a matrix that the predecessor has just expanded
+// (dequant_tiled.cu) is only sure to be there after the wait, so it is the caller who says that W is older.  They take tensor memory only when their predecessors are done, and let their
 // successor start when they have it, so that nobody who waits holds what another needs.
 //
 // The reference's counterpart is its WMMA bf16 family (src/phaseshift/models/qwen35/kernels/optimized/
@@ -245,6 +246,7 @@ struct PairArgs {
     GemmArgs g;
     int bn;              // W rows of a tile: a multiple of 32, at most 256
     int tiles_m, tiles;
+    int w_resident;      // no kernel that may still run writes W: it may be read before the wait for the stream predecessor
 };
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
@@ -281,8 +283,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     tc::cluster_sync();              // both CTAs' barriers exist before either signals the other's
     const uint32_t full0 = tc::cluster_addr(&full_bar[0], 0);
     const uint32_t stage_bytes = 2 * kABytes + p.bn * kBK * 2;
-    const int early = min(k_iters, kPairStages);
-    if (warp == 0 && tc::elect_one()) {
+    const int early = p.w_resident ? min(k_iters, kPairStages) : 0;
+    if (early > 0 && warp == 0 && tc::elect_one()) {
         // the first weights are on their way before the kernel that writes the rows is done
         int tm, tn;
         place(pair, tm, tn);         // (every pair has a tile)
@@ -466,10 +468,11 @@ static int pair_tile_cols(int tiles_m, int N, int pairs) {
     return best;
 }
 
-static int launch_pair(const void* a, int lda, const void* w, int ldw, const GemmArgs& g, cudaStream_t stream) {
+static int launch_pair(const void* a, int lda, const void* w, int ldw, const GemmArgs& g, bool w_resident, cudaStream_t stream) {
     const int sms = sm_count();
     PairArgs p;
     p.g = g;
+    p.w_resident = w_resident ? 1 : 0;
     p.tiles_m = (g.M + kPairBM - 1) / kPairBM;
     p.bn = pair_tile_cols(p.tiles_m, g.N, sms / 2);
     p.tiles = p.tiles_m * ((g.N + p.bn - 1) / p.bn);
@@ -492,9 +495,8 @@ static int launch_pair(const void* a, int lda, const void* w, int ldw, const Gem
 
 // out[M,N] = epilogue(A[M,K] . W[N,K]^T); A, W bf16 row-major (leading dimensions in elements, both
 // multiples of 8 and base pointers 16-byte aligned, as TMA requires).
-PS_API int ps_gemm_bf16_tc(const void* a, int lda, const void* w, int ldw, int M, int N, int K, int epilogue,
-                           const void* residual, int ld_res, void* out, int ldo, int out_f32, void* status,
-                           cudaStream_t stream) {
+static int gemm_bf16_tc(const void* a, int lda, const void* w, int ldw, int M, int N, int K, int epilogue, const void* residual, int ld_res,
+                        void* out, int ldo, int out_f32, void* status, bool w_resident, cudaStream_t stream) {
     using namespace ps;
     if (M <= 0 || N <= 0 || K <= 0 || (lda % 8) || (ldw % 8) || (K % 8) || ((uintptr_t)a % 16) || ((uintptr_t)w % 16))
         return (int)cudaErrorInvalidValue;
@@ -509,6 +511,20 @@ PS_API int ps_gemm_bf16_tc(const void* a, int lda, const void* w, int ldw, int M
     if (M <= kBM && N >= 512) return launch_gemm<32, 5, 2>(a, lda, w, ldw, g, stream);
     // short sums: the store of a tile takes longer than its products, so two CTAs per SM overlap them
     if (K <= 1024) return launch_gemm<128, 3, 2>(a, lda, w, ldw, g, stream);
-    if (M > kBM && N >= 256) return launch_pair(a, lda, w, ldw, g, stream);
+    if (M > kBM && N >= 256) return launch_pair(a, lda, w, ldw, g, w_resident, stream);
     return launch_gemm<128, 4, 1>(a, lda, w, ldw, g, stream);
+}
+
+PS_API int ps_gemm_bf16_tc(const void* a, int lda, const void* w, int ldw, int M, int N, int K, int epilogue,
+                           const void* residual, int ld_res, void* out, int ldo, int out_f32, void* status,
+                           cudaStream_t stream) {
+    return gemm_bf16_tc(a, lda, w, ldw, M, N, K, epilogue, residual, ld_res, out, ldo, out_f32, status, false, stream);
+}
+
+// The same for a W that no kernel of the stream writes while this one may already run (weights of the model): its first tiles are read before
+// the wait for the predecessor.
+PS_API int ps_gemm_bf16_tc_resident(const void* a, int lda, const void* w, int ldw, int M, int N, int K, int epilogue,
+                                    const void* residual, int ld_res, void* out, int ldo, int out_f32, void* status,
+                                    cudaStream_t stream) {
+    return gemm_bf16_tc(a, lda, w, ldw, M, N, K, epilogue, residual, ld_res, out, ldo, out_f32, status, true, stream);
 }

@@ -313,7 +313,9 @@ class CudaOps(OpTrace):
                       ptr(part), ptr(self.status))
             self.launches += 1 if direct else 2
             return out
-        _lib.call("ps_gemm_bf16_tc", ptr(a), c_int(a.stride(0)), ptr(wd), c_int(kp), c_int(M), c_int(W.N), c_int(kp),
+        # (the expansion above is this launch's predecessor: its result must not be read ahead of the wait for it)
+        _lib.call("ps_gemm_bf16_tc_resident" if W.rowmajor_bf16 is not None else "ps_gemm_bf16_tc", ptr(a), c_int(a.stride(0)), ptr(wd), c_int(kp),
+                  c_int(M), c_int(W.N), c_int(kp),
                   c_int(epi), ptr(residual), c_int(residual.stride(0) if residual is not None else 0), ptr(out),
                   c_int(out.stride(0)), c_int(1 if out_f32 else 0), ptr(self.status))
         self.launches += 1
@@ -1001,7 +1003,7 @@ class CudaOps(OpTrace):
                   c_int(st.sc.page_tokens), c_int(st.num_pages), ptr(b.seq_desc), c_int(b.n_seqs), c_int(T), ctypes.byref(opts), c_int(n),
                   ptr(lat), ptr(rot), ptr(st.status))
         N = s.ukv.shape[0]
-        _lib.call("ps_gemm_bf16_tc", ptr(lat), c_int(s.kv_rank), ptr(s.ukv), c_int(s.kv_rank), c_int(n), c_int(N), c_int(s.kv_rank),
+        _lib.call("ps_gemm_bf16_tc_resident", ptr(lat), c_int(s.kv_rank), ptr(s.ukv), c_int(s.kv_rank), c_int(n), c_int(N), c_int(s.kv_rank),
                   c_int(EPI_STORE), ptr(None), c_int(0), ptr(exp), c_int(N), c_int(0), ptr(self.status))
         self.launches += 2
         self._latent_turn(q, s.dim + s.rot, s.dim, q, s.dim + s.rot, s.dim, s, b)

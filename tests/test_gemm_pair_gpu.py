@@ -60,3 +60,29 @@ def test_pair_gemm_row_does_not_depend_on_the_others():
     _gemm(a, w, full)
     _gemm(a[:300], w, part)
     assert torch.equal(full[:300], part)
+
+
+@pytest.mark.parametrize("fmt", ["nvfp4", "mxfp8"])
+@pytest.mark.parametrize("M", [129, 600])
+def test_weights_expanded_into_one_scratch_in_turn(fmt, M):
+    """Block-quantised weights without tensor-core scales go through one scratch matrix, written by the launch before the product:
+    every product has its own weights, whatever the scratch held before."""
+    from phaseshift_b200.models.qwen35.config import tiny_config
+    from phaseshift_b200.models.qwen35.weights import LinearW
+    from phaseshift_b200.ops.cuda_ops import CudaOps
+    from phaseshift_b200.quant.formats import quantize
+    ops = CudaOps(tiny_config(), torch.device("cuda:0"))
+    N, K = 1536, 2048
+    g = torch.Generator(device="cuda").manual_seed(M)
+    ws = [LinearW(quantize(torch.randn(N, K, device="cuda", generator=g) * 0.03, fmt)) for _ in range(2)]
+    x = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    outs = [torch.empty(M, N, dtype=torch.bfloat16, device="cuda") for _ in range(8)]
+    for i, out in enumerate(outs):                     # nothing between the launches
+        ops.linear(x, ws[i % 2], name="y", out=out)
+    torch.cuda.synchronize()
+    assert int(ops.status[0]) == 0
+    for i, out in enumerate(outs):
+        # the expanded weights and the result are rounded to bf16 (2^-8 at most each); 32-bit sums of K products
+        want = x.double() @ ws[i % 2].dense().double().T
+        assert float((out.double() - want).norm() / want.norm()) < K * 2.0 ** -24 + 2 * 2.0 ** -8, i
+        assert torch.equal(out, outs[i % 2])
