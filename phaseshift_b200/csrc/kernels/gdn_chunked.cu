@@ -121,8 +121,8 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prep_kernel(const G
     float* sT = sA + kChunk * 65;          // 64 * 65 floats keep the T rows 16-byte aligned
     float* sM = sT + kChunk * kTP;
 
-    cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();   // (the scan takes a whole SM to wait on: not before the predecessor has left it)
     GdnSeqDesc2 sd; int chunk;
     if (!find_chunk(a.seqs, a.n_seqs, a.min_rows, blockIdx.x, sd, chunk)) return;
     const int h = blockIdx.y, t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -1045,7 +1045,6 @@ __global__ void __launch_bounds__(256) gdn_post_kernel(const float* o, const __n
                                                        const __nv_bfloat16* norm_w, float eps, int Hv, int rows, const int* row_slot,
                                                        __nv_bfloat16* out, const GdnSeqDesc2* seqs, int n_seqs, int min_rows) {
     constexpr int Dv = 32 * E;
-    cudaTriggerProgrammaticLaunchCompletion();
     const int item = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (item >= rows * Hv) return;
     const int row = item / Hv, h = item % Hv;
@@ -1053,6 +1052,7 @@ __global__ void __launch_bounds__(256) gdn_post_kernel(const float* o, const __n
     float v[E], z[E], w[E];
     const __nv_bfloat16* zp = proj + (size_t)row * ld_proj + z_off + h * Dv + lane * E;
     cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
     if (E == 4 && ld_proj % 4 == 0 && z_off % 4 == 0 && (uintptr_t)proj % 8 == 0 && (uintptr_t)norm_w % 8 == 0) {
         const uint2 zb = *reinterpret_cast<const uint2*>(zp), wb = *reinterpret_cast<const uint2*>(norm_w + lane * E);
         const float2 z0 = bf16x2_bits_to_f32x2(zb.x), z1 = bf16x2_bits_to_f32x2(zb.y), w0 = bf16x2_bits_to_f32x2(wb.x), w1 = bf16x2_bits_to_f32x2(wb.y);
@@ -1102,6 +1102,13 @@ static int launch_chunked(const GdnPrepArgs& p, const GdnScanArgs& s, const __nv
                           cudaStream_t stream) {
     const size_t raw_b = (size_t)(kChunk + 3) * (2 * DK) * 2, at_b = sizeof(float) * (kChunk * 65 + kChunk * kTP + 32 * 36);
     const size_t smem_a = sizeof(float) * (2 * kChunk * (DK + 4) + 2 * kChunk) + (raw_b > at_b ? raw_b : at_b);
+    // A preparation of few CTAs that starts while its predecessor drains is put on the first SMs that come free, two on each, where
+    // they take nearly twice as long.  Where every CTA can have an SM of its own it asks for more than half of the shared memory.
+    // In-projection, these kernels and out-projection of a layer, us, two on an SM / one: 32 heads, 64 rows 67.6 / 58.6, 100 rows 90.8 /
+    // 75.6; 48 heads, 37 rows 90.4 / 80.1, 100 rows 120.8 / 108.8; from 200 rows on alike.
+    constexpr size_t kAlone = 118 * 1024;
+    static_assert(2 * (kAlone + 1024) > 228 * 1024, "two of them do not fit an SM");
+    const size_t smem_p = (long long)max_chunks * p.Hv <= sm_count() && smem_a < kAlone ? kAlone : smem_a;
     const size_t smem_b = sizeof(float) * (3 * kChunk * (DK + 4) + DK * (kSlice + 4) + kChunk * (kSlice + 4) + kChunk * 65);
     const size_t smem_t = sizeof(float) * (2 * kChunk * (DK + 4) + kChunk * (DK + 8) + DK * (kSlice + 8) + kChunk * (kSlice + 8) +
                                            kChunk * (kChunk + 4));
@@ -1110,7 +1117,7 @@ static int launch_chunked(const GdnPrepArgs& p, const GdnScanArgs& s, const __nv
     static int use_tc = 1;
     constexpr bool kUmma = DK == 128 && DV == 128;
     if (!set) {
-        cudaFuncSetAttribute(gdn_chunk_prep_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a);
+        cudaFuncSetAttribute(gdn_chunk_prep_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem_a > kAlone ? smem_a : kAlone));
         cudaFuncSetAttribute(gdn_chunk_scan_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b);
         if constexpr (kUmma) cudaFuncSetAttribute(gdn_chunk_scan_umma_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_u);
         else cudaFuncSetAttribute(gdn_chunk_scan_tc_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t);
@@ -1121,7 +1128,7 @@ static int launch_chunked(const GdnPrepArgs& p, const GdnScanArgs& s, const __nv
     GdnPrepArgs pp = p;
     pp.round_tf32 = use_tc;
     pp.images = use_tc && kUmma;
-    int err = launch_pdl(gdn_chunk_prep_kernel<DK, DV>, dim3(max_chunks, p.Hv), dim3(kPrepThreads), smem_a, stream, pp);
+    int err = launch_pdl(gdn_chunk_prep_kernel<DK, DV>, dim3(max_chunks, p.Hv), dim3(kPrepThreads), smem_p, stream, pp);
     if (err) return err;
     const dim3 grid(DV / kSlice, p.Hv, p.n_seqs);
     if (use_tc && kUmma) {
