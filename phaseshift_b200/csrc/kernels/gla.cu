@@ -542,7 +542,7 @@ __device__ __forceinline__ void gla_cp_async16(void* dst, const void* src) {
 template <int DKT, int DVT, bool FORGET>
 __global__ void __launch_bounds__(kGOutThreads, 2) gla_output_kernel(const GlaArgs a) {
     extern __shared__ __align__(16) float gla_smem[];
-    __shared__ float s_ss[4][kGC];
+    __shared__ float s_ss[2][kGC], s_run[kGOutThreads / 2][2];
     const int dk = DKT > 0 ? DKT : a.dk, dv = DVT > 0 ? DVT : a.dv;
     const int PQ = dk + 4, PS = dv + 8;
     float* sQ = gla_smem;                                  // [64][PQ]
@@ -596,25 +596,38 @@ __global__ void __launch_bounds__(kGOutThreads, 2) gla_output_kernel(const GlaAr
             }
         }
     }
-    // ---- head norm over the column quarters, gate, store
+    // ---- head norm, gate, store.  The sum over a head has one order however many warps share its columns: a thread goes through a half of
+    // them, the second quarter's from where the first one's stopped.
     float ss[2] = {0.f, 0.f};
+    float* run = s_run[(part >> 1) * (kGOutThreads / 4) + m * 32 + lane];
+    auto add_columns = [&]() {
 #pragma unroll
-    for (int j = 0; j < kNT; ++j) {
-        ss[0] += acc[j][0] * acc[j][0] + acc[j][1] * acc[j][1];
-        ss[1] += acc[j][2] * acc[j][2] + acc[j][3] * acc[j][3];
+        for (int j = 0; j < kNT; ++j) {
+            ss[0] += acc[j][0] * acc[j][0] + acc[j][1] * acc[j][1];
+            ss[1] += acc[j][2] * acc[j][2] + acc[j][3] * acc[j][3];
+        }
+    };
+    if (!(part & 1)) {
+        add_columns();
+        run[0] = ss[0]; run[1] = ss[1];
     }
+    __syncthreads();
+    if (part & 1) {
+        ss[0] = run[0]; ss[1] = run[1];
+        add_columns();
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], 1);
-        ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], 2);
-        if (tq == 0) s_ss[part][m * 16 + g + 8 * r] = ss[r];
+        for (int r = 0; r < 2; ++r) {
+            ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], 1);
+            ss[r] += __shfl_xor_sync(0xffffffffu, ss[r], 2);
+            if (tq == 0) s_ss[part >> 1][m * 16 + g + 8 * r] = ss[r];
+        }
     }
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         const int lr = m * 16 + g + 8 * r;
         if (lr >= n) continue;
-        const float inv = rsqrtf(((s_ss[0][lr] + s_ss[1][lr]) + (s_ss[2][lr] + s_ss[3][lr])) / (float)a.dv_true + a.eps);
+        const float inv = rsqrtf((s_ss[0][lr] + s_ss[1][lr]) / (float)a.dv_true + a.eps);
         const size_t row = (size_t)row0 + lr;
         const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(a.proj) + row * a.ld + a.g_off + h * dv;
         __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(a.out) + row * a.H * dv + h * dv;
@@ -640,7 +653,7 @@ static int launch_gla_chunked(const GlaArgs& a, int blocks, cudaStream_t stream)
     static bool set = false;
     if (!set) {
         cudaFuncSetAttribute(gla_prepare_kernel<DKT, DVT, FORGET>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
-        cudaFuncSetAttribute(gla_output_kernel<DKT, DVT, FORGET>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+        cudaFuncSetAttribute(gla_output_kernel<DKT, DVT, FORGET>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);       // (+ 3 KB of its own)
         set = true;
     }
     int e = launch_pdl(gla_prepare_kernel<DKT, DVT, FORGET>, dim3(blocks, a.H), dim3(kGPrepThreads), s1, stream, a);
@@ -681,7 +694,7 @@ PS_DEFINE_LIMITS_SETTER(gla)
 PS_API int ps_gla_block_rows() { return ps::kGC; }
 PS_API int ps_gla_chunked_ok(int dk, int dv, int rank) {
     if (dk % 16 || dv % 32 || dk > 256 || dv > 256 || rank < 0) return 0;
-    if (ps::gla_prep_smem_floats(dk, dv) * 4 > 226 * 1024 || ((size_t)ps::kGC * (dk + 4) + (size_t)dk * (dv + 8)) * 4 > 226 * 1024) return 0;
+    if (ps::gla_prep_smem_floats(dk, dv) * 4 > 226 * 1024 || ((size_t)ps::kGC * (dk + 4) + (size_t)dk * (dv + 8)) * 4 > 224 * 1024) return 0;
     return (size_t)ps::kGC * rank + (size_t)dk * (rank + 1) <= (size_t)ps::kGC * (2 * dk + 12) ? 1 : 0;
 }
 

@@ -237,3 +237,12 @@ def test_gla_of_a_mixed_batch(H, dk, dv, dvt, rank, bias, tau, dtype):
 def test_gla_decoded_rows(graph):
     gla_case(2, 128, 128, 128, 16, [(5, 1), (0, 1), (9, 1)], BF, 1.0, 8.0, graph=graph)
     gla_case(2, 32, 96, 70, 3, [(5, 1), (0, 1), (9, 1)], BF, 1.0, 8.0, graph=graph)
+
+
+@pytest.mark.parametrize("dk,dv", [(192, 224), (240, 160), (160, 256)])
+def test_gla_of_the_largest_chunked_heads(dk, dv):
+    """Heads whose state and queries take the output kernel's shared memory to its end, beside what the kernel holds of its own."""
+    from phaseshift_b200.ops import _lib
+    import ctypes
+    assert _lib.lib().ps_gla_chunked_ok(ctypes.c_int(dk), ctypes.c_int(dv), ctypes.c_int(16))
+    gla_case(1, dk, dv, dv, 16, [(0, 70), (3, 130)], BF, 2.0, 16.0)
