@@ -25,7 +25,10 @@ from ..models.registry import family_of
 from .batch import SeqRows, StepBatch, resolve_row_bucket
 from .state import ModelState, StateConfig
 
-GRAPH_MAX_ROWS = 16             # plain steps of any kind; the kernels of a sequence with more rows are chosen by its length
+# Plain steps of up to 16 rows are captured at their first call, one graph per row bucket, number of output rows, and whether rows are single,
+# in order and greedy (at most 17 x 8 of the largest bucket; they share the workspaces and are kept).  12 rows through 8 layers of the 4B
+# shape: 1.05 ms as an ordinary step, 2.5 at the first call, 0.8 from then on.  Sequences with more rows: kernels are chosen by length.
+GRAPH_MAX_ROWS = 16
 GRAPH_MAX_DECODE_ROWS = 64      # pure decode batches (one row per sequence) are also replayed from graphs
 GRAPH_MAX_VARIANT_ROWS = 16     # tapped / logged steps (speculative verification) replayed from graphs of their own
 
