@@ -155,7 +155,7 @@ int launch_attn_prefill_tc(const void* q, int q_rows, const void* k_pool, const 
 // packing onto one MMA tile has no counterpart there.
 // `options`: an AttnOptions (attn_options.cuh) or null; pass the same ones to the merge pass, which applies sink and gate.
 // `part_n` ([rows, Hkv] int32): every SM takes an even share of all tiles and a row's partials are counted there
-// (`max_splits` must hold one for every 64 tokens); null: splits of `split_tokens`.
+// (`max_splits` must hold one for every 64 tokens, or one for every SM); null: splits of `split_tokens`.
 static int attn_decode_tc(const void* q, int q_rows, const void* k_pool, const void* v_pool, const void* block_table,
                           int max_blocks, int page_tokens, int num_pages, const void* seqs, int n_seqs, int dec_max_rows,
                           int Hq, int Hkv, int D, float sm_scale, int split_tokens, int max_splits, int max_visible,
@@ -168,7 +168,7 @@ static int attn_decode_tc(const void* q, int q_rows, const void* k_pool, const v
         return (int)cudaErrorInvalidValue;
     int n_splits = (max_visible + split_tokens - 1) / split_tokens;
     if (n_splits < 1) n_splits = 1;
-    if (n_splits > max_splits) return (int)cudaErrorInvalidValue;
+    if ((part_n != nullptr && n_splits > sm_count() ? sm_count() : n_splits) > max_splits) return (int)cudaErrorInvalidValue;
     CUtensorMap mq, mk, mv;
     int err = attn_map_2d(&mq, q, (uint64_t)q_rows * Hq, D, D, 8);                 // the [rows * Hq, D] view, 8-row boxes
     if (err) return err;

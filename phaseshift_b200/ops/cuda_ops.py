@@ -86,6 +86,7 @@ class CudaOps(OpTrace):
         self.force_tc = os.environ.get("PS_FORCE_TC", "0") == "1"   # single-row steps on the tensor-core kernel too
         self.bs_prefetch = os.environ.get("PS_BS_PREFETCH", "1") != "0"
         self._bs_plan_cache: Dict[tuple, bool] = {}
+        self.sms = torch.cuda.get_device_properties(device).multi_processor_count
         self._norm_cols = int(_lib.lib().ps_gemm_smallm_norm_cols())
         self._smallm_splits: Dict[Tuple[int, int], int] = {}                 # by (N, padded K)
         self.tickets = torch.zeros(ROW_BUCKETS[-1], dtype=torch.int32, device=device)      # one per sequence, zero between launches
@@ -521,12 +522,19 @@ class CudaOps(OpTrace):
         # Split length: 64 tokens give a single row enough CTAs to fill the GPU; a batch of many rows already does, and its
         # CTAs should rather amortise their set-up over a longer run of tokens (about four CTAs per SM in total).  Exact mode
         # and small batches keep the fixed length, so a row's summation order does not depend on its neighbours there.
+        # A captured step is launched for the engine's longest context; where it has few sequences of several rows (verification, short
+        # prompts) lengths made for that would leave each to a few CTAs (16 rows of one sequence with 16000 tokens, NVFP4 pages, engine of
+        # 131072 tokens, 8 layers of the 4B shape: 5255 us per step, and 1763 with a fixed length; 8-bit pages 1604 and 1057).
         split_tokens = self.split_tokens
         if rows > SMALL_M_MAX and not self.exact_rows:
-            want = max(1, (4 * 148) // (rows * hkv))
-            split_tokens = max(split_tokens, -(-(-(-max_visible // want)) // 32) * 32)
-        # The kernel for bf16 pages below takes even shares of a batch's tokens instead, one per SM, however long its sequences are.
-        even = rows > SMALL_M_MAX and not self.exact_rows and self.max_splits * 64 >= max_visible
+            if b.graph_static and b.multi_rows:
+                split_tokens = max(split_tokens, 256)
+            else:
+                want = max(1, (4 * 148) // (rows * hkv))
+                split_tokens = max(split_tokens, -(-(-(-max_visible // want)) // 32) * 32)
+        # The kernel for bf16 pages below takes even shares of a batch's tokens instead, one per SM, however long its sequences are: a
+        # sequence has at most a partial for each of its tiles and for each SM.
+        even = rows > SMALL_M_MAX and not self.exact_rows and self.max_splits >= min(-(-max_visible // 64), self.sms)
         pacc = self.buf("attn_part_acc" + geom, rows, hq * self.max_splits * D, torch.float32)
         pml = self.buf("attn_part_ml" + geom, rows, hq * self.max_splits * 2, torch.float32)
         # Decode / verify rows on the tensor cores: bf16 pages, head dims of whole 64s, every sequence handled here has at most 16 rows

@@ -391,7 +391,7 @@ class Engine:
         return toks, out
 
     GREEDY_KEY_BIT = 1 << 48
-    MULTI_KEY_BIT = 1 << 49          # some sequence has several rows, and the family has kernels of its own for those
+    MULTI_KEY_BIT = 1 << 49          # some sequence has several rows, and the family has kernels of its own for those or attention splits otherwise
 
     @classmethod
     def graph_key(cls, bucket: int, n_out: int, identity_out: bool, greedy: bool = False) -> int:
@@ -416,7 +416,7 @@ class Engine:
         recurrent updates get graphs of their own (the tap and log tensors are fixed buffers, so the capture stays
         valid; Exact mode only changes which kernels the host picks, which the capture bakes in)."""
         key = self.graph_key(bucket, n_out, b.identity_out, greedy)
-        if b.multi_rows and getattr(self.runner, "many_row_kernels", False):
+        if b.multi_rows and (bucket > 8 or getattr(self.runner, "many_row_kernels", False)):
             key |= self.MULTI_KEY_BIT
         kw = {}
         if variant is not None:
