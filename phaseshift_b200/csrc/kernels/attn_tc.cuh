@@ -729,8 +729,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                         const int i = i0 + u * 2 * kTcRows;
                         g[u] = make_uint4(0, 0, 0, 0);
                         if (elementwise && i < n_items)
-                            g[u] = __ldg(reinterpret_cast<const uint4*>(a.gate + (size_t)(row_start + r_begin + i / (DV / 8)) * a.ld_gate +
-                                                                        (size_t)h * a.gate_head_stride + a.gate_offset + i % (DV / 8) * 8));
+                            g[u] = __ldcg(reinterpret_cast<const uint4*>(a.gate + (size_t)(row_start + r_begin + i / (DV / 8)) * a.ld_gate +
+                                                                         (size_t)h * a.gate_head_stride + a.gate_offset + i % (DV / 8) * 8));
                     }
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {

@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prep_kernel(const G
             if (rr < C && pos0 + rr >= 0) {
                 if (r0 + rr >= 0) {
                     const __nv_bfloat16* src = a.proj + (size_t)((long long)row0 + rr) * a.ld_proj + gc;
-                    if (vec) v = __ldg(reinterpret_cast<const uint4*>(src));
+                    if (vec) v = *reinterpret_cast<const uint4*>(src);
                     else {
                         uint32_t w[4];
 #pragma unroll
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prep_kernel(const G
     if (inner && (a.ld_proj & 1) == 0) {
         const __nv_bfloat16* src = a.proj + (row0 + vrb - 3) * a.ld_proj + v_off + vc;
 #pragma unroll
-        for (int i = 0; i < VRUN + 3; ++i) vraw[i] = __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)i * a.ld_proj));
+        for (int i = 0; i < VRUN + 3; ++i) vraw[i] = *reinterpret_cast<const uint32_t*>(src + (size_t)i * a.ld_proj);
     } else {
         const bool even = (a.ld_proj & 1) == 0;
 #pragma unroll
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prep_kernel(const G
             if (rr < C && pos0 + rr >= 0) {
                 if (r0 + rr >= 0) {
                     const __nv_bfloat16* src = a.proj + (size_t)((long long)row0 + rr) * a.ld_proj + v_off + vc;
-                    v = even ? __ldg(reinterpret_cast<const uint32_t*>(src))
+                    v = even ? *reinterpret_cast<const uint32_t*>(src)
                              : ((uint32_t)__bfloat16_as_ushort(src[0]) | ((uint32_t)__bfloat16_as_ushort(src[1]) << 16));
                 } else {
                     v = *reinterpret_cast<const uint32_t*>(hist + (size_t)((pos0 + rr) % a.ring) * CH + CQK + vc);
@@ -936,7 +936,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_umma_kernel(co
         auto load_u = [&](int c) {
             const float4* src = reinterpret_cast<const float4*>(scr0 + c * scr_step + Image::kU) + half * 8 * DV + n;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) u[j] = __ldg(src + j * DV);
+            for (int j = 0; j < 8; ++j) u[j] = __ldcg(src + j * DV);      // (not __ldg: the preparation may still run when this kernel starts)
         };
         // 32 columns of S^T (from column `c0` of this half): TF32 copy for the products
         auto copy_state = [&](const uint32_t (&x)[32], int c0) {
