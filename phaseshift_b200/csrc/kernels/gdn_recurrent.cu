@@ -490,11 +490,12 @@ static int gdn_rows(bool many, const void* proj, int ld_proj, int Hk, int Hv, in
 }
 }  // namespace ps
 
-// Contract: the kernel may load the recurrent state of its slots BEFORE its stream predecessor has finished
-// (programmatic dependent launch): the predecessor must therefore not write `state_in` of those slots.  Inside the
-// engine that holds -- a projection kernel always sits between two GDN launches of one layer.  A caller that runs two
-// ps_gdn_rows back to back on one slot and state buffer must put another kernel (or an event) between them, or set
-// PS_PDL=0.
+// Contract of both entries: the kernel may load the recurrent state (`state_in`) and the convolution history (`conv_state`) of its slots,
+// and the layer's weights, BEFORE its stream predecessor has finished (programmatic dependent launch).  Nothing that may still run
+// then may write them.  A kernel between two launches on one slot is not enough to order them if it lets its successor start before it
+// has waited itself, as the few-row GEMM and the streaming projection do; a copy, an ordinary launch, a kernel that waits first or the
+// end of a graph is.  Inside the engine every step begins with the copy of its descriptors, or is a graph of its own, and has each
+// layer's mixer once per slot.  A caller that runs two launches back to back puts one of these between them, or sets PS_PDL=0.
 PS_API int ps_gdn_rows(const void* proj, int ld_proj, int Hk, int Hv, int Dk, int Dv, const void* conv_w,
                        const void* A_log, const void* dt_bias, const void* norm_w, float eps, void* conv_state,
                        int ring, const void* state_in, void* state_out, const void* seqs, int n_seqs, void* out,
@@ -504,7 +505,7 @@ PS_API int ps_gdn_rows(const void* proj, int ld_proj, int Hk, int Hv, int Dk, in
                         log_delta, log_d, ba_w, xn, ba_k, max_rows, stream);
 }
 
-// The same results, sooner where sequences have several rows.
+// The same results and the same contract, sooner where sequences have several rows.
 PS_API int ps_gdn_rows_many(const void* proj, int ld_proj, int Hk, int Hv, int Dk, int Dv, const void* conv_w,
                        const void* A_log, const void* dt_bias, const void* norm_w, float eps, void* conv_state,
                        int ring, const void* state_in, void* state_out, const void* seqs, int n_seqs, void* out,
