@@ -89,23 +89,23 @@ bool attn_prefill_tc_supported(int D, int page_tokens, int kv_fp8, const void* q
     return true;
 }
 
-template <int D, bool DEC>
+template <int D, bool DEC, bool EVEN>
 static int launch_attn_tc_size(bool shared, bool transform, dim3 grid, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                                const AttnTcArgs& a, cudaStream_t stream) {
     if (shared && transform) return (int)cudaErrorInvalidValue;          // no design has both; the callers take another kernel
-    if (shared) return launch_attn_tc<D, D, DEC, true, false, false>(grid, mq, mk, mv, mk, a, stream);
-    if (transform) return launch_attn_tc<D, D, DEC, false, true, false>(grid, mq, mk, mv, mk, a, stream);
-    return launch_attn_tc<D, D, DEC, false, false, false>(grid, mq, mk, mv, mk, a, stream);
+    if (shared) return launch_attn_tc<D, D, DEC, true, false, false, EVEN>(grid, mq, mk, mv, mk, a, stream);
+    if (transform) return launch_attn_tc<D, D, DEC, false, true, false, EVEN>(grid, mq, mk, mv, mk, a, stream);
+    return launch_attn_tc<D, D, DEC, false, false, false, EVEN>(grid, mq, mk, mv, mk, a, stream);
 }
-template <bool DEC>
+template <bool DEC, bool EVEN>
 static int launch_attn_tc_any(int D, bool shared, dim3 grid, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                               const AttnTcArgs& a, cudaStream_t stream) {
     const bool tr = attn_transforms_scores(a.opt);
     switch (D) {
-        case 64: return launch_attn_tc_size<64, DEC>(shared, tr, grid, mq, mk, mv, a, stream);
-        case 128: return launch_attn_tc_size<128, DEC>(shared, tr, grid, mq, mk, mv, a, stream);
-        case 192: return launch_attn_tc_size<192, DEC>(shared, tr, grid, mq, mk, mv, a, stream);
-        case 256: return launch_attn_tc_size<256, DEC>(shared, tr, grid, mq, mk, mv, a, stream);
+        case 64: return launch_attn_tc_size<64, DEC, EVEN>(shared, tr, grid, mq, mk, mv, a, stream);
+        case 128: return launch_attn_tc_size<128, DEC, EVEN>(shared, tr, grid, mq, mk, mv, a, stream);
+        case 192: return launch_attn_tc_size<192, DEC, EVEN>(shared, tr, grid, mq, mk, mv, a, stream);
+        case 256: return launch_attn_tc_size<256, DEC, EVEN>(shared, tr, grid, mq, mk, mv, a, stream);
         default: return (int)cudaErrorInvalidValue;
     }
 }
@@ -142,7 +142,7 @@ int launch_attn_prefill_tc(const void* q, int q_rows, const void* k_pool, const 
     a.split_tokens = 0; a.max_splits = 0; a.dec_max_rows = 0; a.part_acc = nullptr; a.part_ml = nullptr; a.n_seqs = n_seqs; a.part_n = nullptr;
     a.opt = opt; a.k_groups = a.k_head = a.v_off = a.v_head = 0;
     const int tiles = (max_seq_rows + kTcRows - 1) / kTcRows;
-    return launch_attn_tc_any<false>(D, k_pool == v_pool, dim3(tiles, Hq, n_seqs), mq, mk, mv, a, stream);
+    return launch_attn_tc_any<false, false>(D, k_pool == v_pool, dim3(tiles, Hq, n_seqs), mq, mk, mv, a, stream);
 }
 
 }  // namespace ps
@@ -183,8 +183,8 @@ static int attn_decode_tc(const void* q, int q_rows, const void* k_pool, const v
     a.split_tokens = split_tokens; a.max_splits = max_splits; a.dec_max_rows = dec_max_rows;
     a.part_acc = (float*)part_acc; a.part_ml = (float*)part_ml; a.opt = opt; a.k_groups = a.k_head = a.v_off = a.v_head = 0;
     a.n_seqs = n_seqs; a.part_n = (int*)part_n;
-    const dim3 grid = part_n != nullptr ? dim3(sm_count()) : dim3(n_splits, Hkv, n_seqs);
-    return launch_attn_tc_any<true>(D, k_pool == v_pool, grid, mq, mk, mv, a, stream);
+    return part_n != nullptr ? launch_attn_tc_any<true, true>(D, k_pool == v_pool, dim3(sm_count()), mq, mk, mv, a, stream)
+                             : launch_attn_tc_any<true, false>(D, k_pool == v_pool, dim3(n_splits, Hkv, n_seqs), mq, mk, mv, a, stream);
 }
 
 PS_API int ps_attn_decode_tc_ex(const void* q, int q_rows, const void* k_pool, const void* v_pool, const void* block_table,

@@ -138,7 +138,7 @@ __device__ __forceinline__ int expanded_row0(const int* seqs, int s, int min_row
 // and one KV head: tile row 8 r + g is query head g of that KV head for the sequence's row r (grouped-query packing: the G <= 8
 // heads that share the KV head ride in one MMA tile, so K and V are read once for all of them), over the tokens of its
 // split; it leaves unnormalised partial outputs and (maximum, sum) pairs for the merge pass of paged_attention.cu.
-// With `part_n` the grid is one CTA per SM instead, and every CTA takes an even share of the tiles of all sequences and KV heads, in
+// EVEN: with `part_n` the grid is one CTA per SM instead, and every CTA takes an even share of the tiles of all sequences and KV heads, in
 // their order: it works on the pieces of one or more (sequence, KV head) one after the other, its pipelines running on, and a
 // partial's number is that of its CTA among those that share the (sequence, KV head).  With 224 KB of shared memory a CTA has an SM to
 // itself, so splits of a fixed length run in rounds, each with its own set-up, and sequences of unequal length leave the last one
@@ -147,12 +147,13 @@ __device__ __forceinline__ int expanded_row0(const int* seqs, int s, int min_row
 // TRANSFORM: query temperature and distance bias, applied to the scores before the maximum.
 // EXPANDED: keys and values were expanded per query head into rows of consecutive tokens (attn_latent.cu), the last 64-column
 // groups of the keys (`map_r`) are shared by all heads.
-template <int DK, int DV, bool DEC, bool SHARED, bool TRANSFORM, bool EXPANDED>
+template <int DK, int DV, bool DEC, bool SHARED, bool TRANSFORM, bool EXPANDED, bool EVEN>
 __global__ void __launch_bounds__(kTcThreads, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_r, const AttnTcArgs a) {
     static_assert(!SHARED || DK == DV, "keys that are the values have their size");
     static_assert(!EXPANDED || (!DEC && !SHARED), "expanded keys and values are for prefill-sized steps");
+    static_assert(!EVEN || DEC, "shares of a batch's tiles are for decoding");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     using Shape = TcShape<DK, DV>;
     constexpr int kTcQBytes = Shape::kQBytes, kTcKStage = Shape::kKStage, kTcVStage = Shape::kVStage, kTcOutPitch = Shape::kOutPitch;
@@ -207,7 +208,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     };
     // the next piece of the CTA's share (every thread keeps its own place in it)
     auto next_piece = [&]() -> bool {
-        if constexpr (!DEC) return false;
+        if constexpr (!EVEN) return false;
         else {
             if (left <= 0) return false;
             x0 += T_seq; t_off = 0;
@@ -219,9 +220,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             return true;
         }
     };
-    const bool even = DEC && a.part_n != nullptr;
     if constexpr (DEC) {
-        if (even) {
+        if constexpr (EVEN) {
             for (int s0 = 0; s0 < a.n_seqs; s0 += 32)
                 total += __reduce_add_sync(0xffffffffu, s0 + lane < a.n_seqs ? tiles_of(a.seqs + 4 * (s0 + lane)) : 0);
             total *= a.Hkv;
@@ -316,7 +316,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             if (n > 0 && !__all_sync(0xffffffffu, tc::mbar_wait_abortable(&q_free, (uint32_t)(n - 1) & 1u, a.budget, &s_abort))) return false;
             // one 8-row box per (row of the sequence, 64-column group): the G heads of this KV head are consecutive rows
             // of the [rows * Hq, D] view of q; tile rows 8 r + g with g >= G hold other heads' values and are never used
-            const int copies = nq <= 32 ? 4 : 1;                     // one for every quadrant of the accumulator's lanes
+            const int copies = EVEN && nq <= 32 ? 4 : 1;             // one for every quadrant of the accumulator's lanes
             if (lane == 0) tc::mbar_expect_tx(&q_full, (uint32_t)(copies * n_rows) * (uint32_t)kNB * 1024u);
             __syncwarp();
             for (int i = lane; i < kNB * n_rows * copies; i += 32) {
@@ -417,7 +417,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     tc::mma_commit(&s_full[b]);
                     if (stamp) a.prof[t * 16 + 10] = clock64();
                 }
-                if constexpr (DEC) {                     // (one arrival of each issuer, also of one without a tile in a piece of one)
+                if constexpr (EVEN) {                     // (one arrival of each issuer, also of one without a tile in a piece of one)
                     if (ok && first < T) tc::mma_commit(&q_free);
                     else if (ok) tc::mbar_arrive(&q_free);
                 }
@@ -465,11 +465,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
         bool ok = true;
         for (int g = 0;;) {
-            // decode with up to four rows: the query rows fill one quadrant, whose two warps share a scheduler and its exponential unit.  Q is
-            // there four times instead, so that every warp has the scores; the quadrants take every fourth pair of a half's columns
-            // each and write the probabilities of the first one's rows (24 sequences, keys that are the values: 38.8 -> 35.8 us; the pass
-            // from a tile's maximum to its probabilities had 900 of a tile's 2000 cycles)
-            const bool spread = DEC && nq <= 32;
+            // shares with up to four rows per sequence: the query rows fill one quadrant, whose two warps share a scheduler and its exponential
+            // unit.  Q is there four times instead, so that every warp has the scores; the quadrants take every fourth pair of a half's
+            // columns each and write the probabilities of the first one's rows (24 sequences, keys that are the values: 38.8 -> 35.8 us; the
+            // pass from a tile's maximum to its probabilities had 900 of a tile's 2000 cycles).  A split of one or two tiles gains less by
+            // that than the copies of Q and the exchange of sums cost (one row at 4096 tokens 20.6 -> 22.4 us, 8 x 3000 77 -> 86).
+            const bool spread = EVEN && nq <= 32;
             const int qrow = spread ? lane : row;
             const int rp = DEC ? pos_q0 + (qrow >> 3) : pos_q0 + row;    // position of this thread's query row
             const float sc = a.scale_log2;
@@ -489,7 +490,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             // queries) ask for no rescaling (8 rows of one sequence 721 -> 712 us per step of 8 layers, 24 sequences 833 -> 821 of 4)
             const bool idle = DEC && !spread && quad * 32 >= nq, counts = !DEC || (qrow < nq && (row & 7) < G);
             float m_ref = 0.f, l_run = 0.f;
-            [[maybe_unused]] float l4[4] = {0.f, 0.f, 0.f, 0.f};         // decode: sums of every fourth pair, so that both forms add alike
+            [[maybe_unused]] float l4[4] = {0.f, 0.f, 0.f, 0.f};         // shares: sums of every fourth pair, so that spread or not adds alike
             bool fresh = true;                                            // this row has not seen a token yet: m_ref is a placeholder
             // the epilogue reads this tile's gate values (one 512-byte run per row): ask for them now, so that they come from
             // L2 then
@@ -596,7 +597,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                             sq[(j >> 1) & 3] += p0 + p1;
                             pk[j >> 1] = f32x2_to_bf16x2_bits(p0, p1);
                         }
-                        if constexpr (DEC) {
+                        if constexpr (EVEN) {
 #pragma unroll
                             for (int k = 0; k < 4; ++k) l4[k] = fmaf(l4[k], alpha, sq[k]);
                         } else {
@@ -653,7 +654,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             // ---- epilogue: O / l -> bf16 rows staged in shared memory (Q and K stages are free once the last P V is done)
             if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(&pv_done[(g + T - 1) & 1], (uint32_t)((g + T - 1) >> 1) & 1u, a.budget, &s_abort));
             if (cta_stamp) a.prof[2 * 16 + 15] = clock64();
-            s_l[half][row] = DEC && !spread ? (l4[0] + l4[1]) + (l4[2] + l4[3]) : DEC ? l4[0] : l_run;
+            s_l[half][row] = !EVEN ? l_run : spread ? l4[0] : (l4[0] + l4[1]) + (l4[2] + l4[3]);
             asm volatile("bar.sync 1, 256;" ::: "memory");               // the eight softmax warps only; every one of them gets here
             if (cta_stamp) a.prof[3 * 16 + 15] = clock64();
             if constexpr (DEC) {
@@ -662,9 +663,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 const int r = row >> 3, gq = row & 7;
                 // the CTA that has tile x is the i-th with i total / n_ctas <= x < (i + 1) total / n_ctas
                 auto cta_of = [&](int x) { return (int)((((long long)x + 1) * n_ctas - 1) / total); };
-                const int part = even ? (int)blockIdx.x - cta_of(x0) : (int)blockIdx.x;
+                const int part = EVEN ? (int)blockIdx.x - cta_of(x0) : (int)blockIdx.x;
                 const bool mine = row < nq && gq < G && part < a.max_splits;
-                if (even && t_off == 0 && gq == 0 && half == 0 && row < nq)          // the (sequence, KV head) begins here
+                if (EVEN && t_off == 0 && gq == 0 && half == 0 && row < nq)          // the (sequence, KV head) begins here
                     a.part_n[(size_t)(row_start + r) * a.Hkv + kvh] = min(cta_of(x0 + T_seq - 1) - (int)blockIdx.x + 1, a.max_splits);
                 if (ok && quad * 32 < nq) {                              // warp-uniform: the tensor-memory loads are collective
                     tc::fence_after_sync();
@@ -753,7 +754,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 }
             }
             }   // prefill epilogue
-            if constexpr (!DEC) break;
+            if constexpr (!EVEN) break;
             g += T;
             // the sums have been read, and all eight warps go on or none does: the barriers count all of them
             if (!softmax_all(ok) || !next_piece()) break;
@@ -811,16 +812,16 @@ static int attn_map_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64
     return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
-template <int DK, int DV, bool DEC, bool SHARED, bool TRANSFORM, bool EXPANDED>
+template <int DK, int DV, bool DEC, bool SHARED, bool TRANSFORM, bool EXPANDED, bool EVEN = false>
 static int launch_attn_tc(dim3 grid, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mr,
                           const AttnTcArgs& a, cudaStream_t stream) {
     constexpr size_t smem = TcShape<DK, DV>::kSmem;
     static bool set = false;
     if (!set) {
-        cudaFuncSetAttribute(attn_tc_kernel<DK, DV, DEC, SHARED, TRANSFORM, EXPANDED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(attn_tc_kernel<DK, DV, DEC, SHARED, TRANSFORM, EXPANDED, EVEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         set = true;
     }
-    return launch_pdl(attn_tc_kernel<DK, DV, DEC, SHARED, TRANSFORM, EXPANDED>, grid, dim3(kTcThreads), smem, stream, mq, mk, mv, mr, a);
+    return launch_pdl(attn_tc_kernel<DK, DV, DEC, SHARED, TRANSFORM, EXPANDED, EVEN>, grid, dim3(kTcThreads), smem, stream, mq, mk, mv, mr, a);
 }
 
 }  // namespace ps

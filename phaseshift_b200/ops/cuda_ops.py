@@ -533,8 +533,15 @@ class CudaOps(OpTrace):
                 want = max(1, (4 * 148) // (rows * hkv))
                 split_tokens = max(split_tokens, -(-(-(-max_visible // want)) // 32) * 32)
         # The kernel for bf16 pages below takes even shares of a batch's tokens instead, one per SM, however long its sequences are: a
-        # sequence has at most a partial for each of its tiles and for each SM.
+        # sequence has at most a partial for each of its tiles and for each SM.  Outside of a graph, where the step's lengths are known,
+        # splits that have an SM each and are no longer than a share and a few tiles are kept: they need no search for their place and
+        # no exchange between quadrants (16 query and 4 KV heads, shares / splits: 4 sequences of 4 rows and 2000 tokens 20.5 / 16.6 us,
+        # one of 9 rows and 4000 tokens 20.5 / 19.0; 12 single rows of 1000 tokens, 384 splits, 20.5 / 25.4).
+        st_tok = -(-split_tokens // 64) * 64
         even = rows > SMALL_M_MAX and not self.exact_rows and self.max_splits >= min(-(-max_visible // 64), self.sms)
+        if even and not b.graph_static:
+            lanes = hkv * b.n_seqs
+            even = -(-max_visible // st_tok) * lanes > self.sms or st_tok // 64 > -(-max_visible // 64) * lanes / self.sms + 5
         pacc = self.buf("attn_part_acc" + geom, rows, hq * self.max_splits * D, torch.float32)
         pml = self.buf("attn_part_ml" + geom, rows, hq * self.max_splits * 2, torch.float32)
         # Decode / verify rows on the tensor cores: bf16 pages, head dims of whole 64s, every sequence handled here has at most 16 rows
@@ -546,7 +553,6 @@ class CudaOps(OpTrace):
         if (self.attn_decode_tc and D % 64 == 0 and st.kv_fmt == 0 and st.sc.page_tokens in (16, 32, 64) and hq // hkv <= 8
                 and not (kv.k is kv.v and (spec.bias is not None or spec.temp_coef != 0.0))
                 and (b.graph_static or row_pos is b.row_pos_short or all(len(sq.token_ids) <= 16 for sq in b.seqs))):
-            st_tok = -(-split_tokens // 64) * 64
             n_seqs = b.max_seqs if b.graph_static else b.n_seqs
             if even:
                 part_n = self.buf(f"attn_part_n{hkv}", rows, hkv, torch.int32)

@@ -12,7 +12,7 @@ from phaseshift_b200.ops.specs import AttnSpec
 HQ, HKV, D = 8, 4, 64
 
 
-def launch(monkeypatch, kv_fmt, rows, multi, static, max_seq_len, visible):
+def launch(monkeypatch, kv_fmt, rows, multi, static, max_seq_len, visible, n_seqs=0):
     """(launcher, its split length or None) of a step's first attention launch."""
     calls = []
     monkeypatch.setattr(cuda_ops._lib, "call", lambda name, *args: calls.append((name, [getattr(x, "value", None) for x in args])))
@@ -25,7 +25,7 @@ def launch(monkeypatch, kv_fmt, rows, multi, static, max_seq_len, visible):
     t = torch.zeros(1)
     st = types.SimpleNamespace(kv_fmt=kv_fmt, kv_fp8=kv_fmt == 1, block_table=t, max_blocks=1, num_pages=1, status=t, sc=types.SimpleNamespace(page_tokens=16))
     b = types.SimpleNamespace(graph_static=static, multi_rows=multi, row_pos=t, row_pos_short=t, row_slot=t, seq_desc=t, max_seqs=16,
-                              n_seqs=1 if multi else rows, seqs=[types.SimpleNamespace(token_ids=[0] * (rows if multi else 1))])
+                              n_seqs=n_seqs or (1 if multi else rows), seqs=[types.SimpleNamespace(token_ids=[0] * (rows if multi else 1))])
     kv = types.SimpleNamespace(k=t, v=torch.zeros(1), k_scale=t, v_scale=t)
     buf = o.buf
     o.buf = lambda name, r, c, dtype=torch.bfloat16: buf(name, r, 1, dtype)          # (only addresses are used)
@@ -51,3 +51,12 @@ def test_captured_rows_of_one_sequence_have_a_fixed_length(monkeypatch, max_seq_
     assert launch(monkeypatch, 2, 16, False, True, max_seq_len, 0)[1] == max(o.split_tokens, -(-(-(-(max_seq_len + 1) // want)) // 32) * 32)
     assert launch(monkeypatch, 2, 16, True, False, max_seq_len, 1500)[1] == max(o.split_tokens, -(-(-(-1500 // want)) // 32) * 32)
     assert launch(monkeypatch, 2, 8, True, True, max_seq_len, 0)[1] == o.split_tokens
+
+
+def test_few_splits_are_kept_outside_of_a_graph(monkeypatch):
+    """One wave of splits that are no longer than a share and a few tiles needs no shares; anything else has them."""
+    assert launch(monkeypatch, 0, 16, True, False, 20000, 2000)[0] == "ps_attn_decode_tc_ex"           # 8 splits x 4 heads
+    assert launch(monkeypatch, 0, 16, False, False, 20000, 2000)[0] == "ps_attn_decode_tc_even"        # 8 x 4 x 16 sequences
+    # a few single rows beside a long prompt: rows and with them the splits' length are the prompt's
+    assert launch(monkeypatch, 0, 800, False, False, 20000, 2500, n_seqs=16)[0] == "ps_attn_decode_tc_even"
+    assert launch(monkeypatch, 0, 16, True, False, 20000, 18000)[0] == "ps_attn_decode_tc_even"        # 32 tiles a split, 8 a share
