@@ -230,10 +230,11 @@ __host__ __device__ __forceinline__ int sf_atom_off(int r, int j) { return (r & 
 
 // Threads per CTA: warp 0 producer, warp 1 MMA issuer, warps 2..5 epilogue, warp 6 scale-copy issuer; the resident variant
 // adds five more warps that only help in the activation prologue (one (slot, block) pair per thread instead of two in a row), the
-// streamed variant with HALVES = 2 four more epilogue warps.
+// streamed variant with HALVES = 2 four more epilogue warps.  HALVES: warps per TMEM lane quadrant of the epilogue that stages its outputs
+// (streamed activations, bf16 outputs of one rank's own sums); 0: the epilogue that stores directly, with four warps.
 // Warp 6 issues the scale-factor copies (tcgen05.cp) one stage ahead of the MMA warp: the two instruction streams of a
 // stage (copies: ~55 cycles each, MMAs: ~86 each at N = 16) run in parallel instead of back to back in one thread.
-template <bool RES, int HALVES> constexpr int bs_threads() { return RES ? 384 : kBsThreads + 32 + 128 * (HALVES - 1); }
+template <bool RES, int HALVES> constexpr int bs_threads() { return RES ? 384 : kBsThreads + 32 + (HALVES > 1 ? 128 : 0); }
 template <bool RES> constexpr int bs_group() { return RES ? 2 : 1; }      // K-panels per pipeline stage
 
 // Staging of the streamed epilogue: all of the tile's batch rows but the last 64 at once (32-bit words: a feature of two neighbouring rows),
@@ -364,8 +365,7 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* sBres = smem + (size_t)g.stages * kStage;                          // resident activation codes
-    // streamed path, bf16 outputs of one rank's own sums: outputs staged in shared memory, by all epilogue warps
-    const bool staged = !RES && !g.out_f32 && g.tp.size <= 1;
+    static_assert(!RES || HALVES == 0, "resident activations: outputs are stored directly");
     uint32_t* sSfRes = reinterpret_cast<uint32_t*>(sBres + (size_t)g.res_slots * kBTile);   // [slot][APP][32 rows] scale words
     __shared__ __align__(8) uint64_t full_bar[kBsMaxStages], empty_bar[kBsMaxStages], acc_full[2], acc_empty[2], drain_bar;
     __shared__ __align__(8) uint64_t sf_ready[4], sf_free[4];      // scale-factor columns of a stage parity: copied / consumed
@@ -408,7 +408,7 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         if (!RES) tc::tma_prefetch_desc(&map_x);
     } else if (threadIdx.x == 64) {
         for (int s = 0; s < stages; ++s) tc::mbar_init(&empty_bar[s], 1);
-        for (int b = 0; b < 2; ++b) { tc::mbar_init(&acc_full[b], 1); tc::mbar_init(&acc_empty[b], staged ? 4 * HALVES : 4); }
+        for (int b = 0; b < 2; ++b) { tc::mbar_init(&acc_full[b], 1); tc::mbar_init(&acc_empty[b], HALVES > 0 ? 4 * HALVES : 4); }
         tc::mbar_init(&drain_bar, 1);
         for (int b = 0; b < 4; ++b) { tc::mbar_init(&sf_ready[b], 1); tc::mbar_init(&sf_free[b], 1); }
         tc::fence_barrier_init();
@@ -769,7 +769,9 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 }
             }
         }
-    } else if (staged) {
+    } else if (HALVES == 0 && warp >= 6) {
+        // (only help in the prologue)
+    } else if constexpr (HALVES > 0) {
         // ------------------------------------------------ epilogue of the streamed path: HALVES warps per TMEM lane quadrant (warp % 4), which
         // take turns at the blocks of 32 batch rows.  The accumulator (one: the scale factors take the rest of the tensor memory) is only held
         // until its values are in registers, as bf16 pairs of rows; everything else -- staging, activation, stores -- runs under the next
@@ -909,7 +911,7 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             if (prof) prof_ework += clock64() - te1;
         }
         if (prof && et == 0) { g.prof[9] = clock64(); g.prof[11] = prof_ewait; g.prof[12] = prof_ework; g.prof[13] = seg; }
-    } else if (warp < 6) {
+    } else {
         // ------------------------------------------------ epilogue: warps 2..5 own TMEM lane quadrant (warp % 4)
         // Control flow below depends only on values that are uniform over the 128 epilogue threads, so every
         // named barrier is reached by all of them even after a wait has run out (`ok` only gates memory work;
@@ -1291,7 +1293,7 @@ static bool bs_plan(int M, int N, int K, bool resident, int grid_override, BsPla
     return true;
 }
 
-template <int FMT, int NB, bool RES, int HALVES = 2>
+template <int FMT, int NB, bool RES, int HALVES>
 static int bs_launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mn, const BsArgs& a, const BsPlan& pl,
                      cudaStream_t stream) {
     static bool attr_set = false;
@@ -1320,12 +1322,15 @@ static int bs_dispatch(const void* w_codes, long long w_row_bytes, long long w_p
     }
     const CUtensorMap& mn = map_next != nullptr ? *map_next : mw;
     if (map_next == nullptr) a.next_total = 0;
-    if (resident) return pl.nb == 16 ? bs_launch<FMT, 16, true>(mw, mx, mn, a, pl, stream) : bs_launch<FMT, 32, true>(mw, mx, mn, a, pl, stream);
+    if (resident) return pl.nb == 16 ? bs_launch<FMT, 16, true, 0>(mw, mx, mn, a, pl, stream) : bs_launch<FMT, 32, true, 0>(mw, mx, mn, a, pl, stream);
+    // 32-bit outputs and the ranks' partial sums: four warps that store directly
+    if (a.out_f32 || a.tp.size > 1)
+        return pl.nb == 128 ? bs_launch<FMT, 128, false, 0>(mw, mx, mn, a, pl, stream) : bs_launch<FMT, 256, false, 0>(mw, mx, mn, a, pl, stream);
     // One block of rows: four epilogue warps do, and leave registers for the next kernel of the step, the quantiser of the next product's
     // rows, to start beside this one (both feed-forward products of the 27B shape, NVFP4 and MXFP8: 9 rows 78.5 us with eight warps, 75.0
     // with four; with two blocks, 64 rows, 76.8 and 79.2).
     if (a.M <= 32) return bs_launch<FMT, 128, false, 1>(mw, mx, mn, a, pl, stream);
-    return pl.nb == 128 ? bs_launch<FMT, 128, false>(mw, mx, mn, a, pl, stream) : bs_launch<FMT, 256, false>(mw, mx, mn, a, pl, stream);
+    return pl.nb == 128 ? bs_launch<FMT, 128, false, 2>(mw, mx, mn, a, pl, stream) : bs_launch<FMT, 256, false, 2>(mw, mx, mn, a, pl, stream);
 }
 
 }  // namespace ps
