@@ -779,7 +779,7 @@ gemm_bs_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         // 15000 of products (34816 x 5120, 2048 rows).
         // With few rows a tile's products are over in a moment and the end of the last tile shows: blocks without rows are neither
         // summed, staged nor looked at, and the partials of two contributors are in flight.  Both feed-forward products of the 27B shape,
-        // us, with every block of a tile done / now: 9 rows 81.0 / 74.4, 32 rows 81.3 / 75.8, 64 rows 81.7 / 76.8, 128 rows 89.0 / 89.8.
+        // us, with every block of a tile done / now: 9 rows 81.6 / 73.5, 32 rows 81.3 / 74.8, 64 rows 81.6 / 73.5, 128 rows 89.0 / 86.2.
         // Control flow depends only on values that are uniform over the epilogue's threads, so every barrier is reached by all of them
         // even after a wait has run out (`ok` only gates memory work).
         constexpr int STEP = 32 * HALVES, EPI = 128 * HALVES;
@@ -1327,8 +1327,8 @@ static int bs_dispatch(const void* w_codes, long long w_row_bytes, long long w_p
     if (a.out_f32 || a.tp.size > 1)
         return pl.nb == 128 ? bs_launch<FMT, 128, false, 0>(mw, mx, mn, a, pl, stream) : bs_launch<FMT, 256, false, 0>(mw, mx, mn, a, pl, stream);
     // One block of rows: four epilogue warps do, and leave registers for the next kernel of the step, the quantiser of the next product's
-    // rows, to start beside this one (both feed-forward products of the 27B shape, NVFP4 and MXFP8: 9 rows 78.5 us with eight warps, 75.0
-    // with four; with two blocks, 64 rows, 76.8 and 79.2).
+    // rows, to start beside this one (both feed-forward products of the 27B shape, NVFP4 and MXFP8: 9 rows 77.4 us with eight warps, 74.3
+    // with four; with two blocks, 64 rows, 73.0 and 78.9).
     if (a.M <= 32) return bs_launch<FMT, 128, false, 1>(mw, mx, mn, a, pl, stream);
     return pl.nb == 128 ? bs_launch<FMT, 128, false, 2>(mw, mx, mn, a, pl, stream) : bs_launch<FMT, 256, false, 2>(mw, mx, mn, a, pl, stream);
 }

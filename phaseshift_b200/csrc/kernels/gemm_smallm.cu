@@ -186,18 +186,19 @@ struct SmallMReduceArgs {
     const __nv_bfloat16* norm_w; float eps; __nv_bfloat16* normed; int ld_normed;      // gemm_smallm_norm_kernel
 };
 
-// Sum of the splits of four neighbouring columns (c a multiple of 4) of row m, in ascending order; eight loads in flight (their latency is
+// Sum of the splits of four neighbouring columns (c a multiple of 4) of row m, in ascending order; F loads in flight (their latency is
 // most of a reduction: with four, fourteen splits took four round trips to L2).
+template <int F>
 __device__ __forceinline__ float4 smallm_sum4(const SmallMReduceArgs& a, int m, int c) {
     const float4* p = reinterpret_cast<const float4*>(a.partial + (size_t)m * a.N + c);
     const size_t step = (size_t)a.M * a.N / 4;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s < a.splits; s += 8) {
-        float4 q[8];
+    for (int s = 0; s < a.splits; s += F) {
+        float4 q[F];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) if (s + i < a.splits) q[i] = p[(s + i) * step];
+        for (int i = 0; i < F; ++i) if (s + i < a.splits) q[i] = p[(s + i) * step];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) if (s + i < a.splits) { v.x += q[i].x; v.y += q[i].y; v.z += q[i].z; v.w += q[i].w; }
+        for (int i = 0; i < F; ++i) if (s + i < a.splits) { v.x += q[i].x; v.y += q[i].y; v.z += q[i].z; v.w += q[i].w; }
     }
     return v;
 }
@@ -207,6 +208,7 @@ __device__ __forceinline__ float smallm_gated(const SmallMReduceArgs& a, float g
 }
 
 // One thread per four output columns (N a multiple of 4, rows of `out` and the residual 16- / 8-byte aligned).
+template <int F>
 __global__ void gemm_smallm_reduce4_kernel(const SmallMReduceArgs a) {
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
@@ -214,7 +216,7 @@ __global__ void gemm_smallm_reduce4_kernel(const SmallMReduceArgs a) {
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= a.M * quads) return;
     const int m = id / quads, c = (id - m * quads) * 4;
-    float4 v = smallm_sum4(a, m, c);
+    float4 v = smallm_sum4<F>(a, m, c);
     if (a.epilogue == 2 || a.epilogue == 3 || a.epilogue == 5) {
         *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(a.out) + (size_t)m * a.ldo + (c >> 1)) =
             f32x2_to_bf16x2_bits(smallm_gated(a, v.x, v.y), smallm_gated(a, v.z, v.w));
@@ -238,6 +240,7 @@ __global__ void gemm_smallm_reduce4_kernel(const SmallMReduceArgs a) {
 // went from 1190 to 931 us, one of 32 rows through 4 layers of 5120 x 17408 from 2010 to 1780.  What bounds it: latency.  The sums are
 // written to the others instead of read from them: no CTA has to stay for a last cluster barrier (8 rows of 2560: 4.4 -> 4.3 us).
 constexpr int kSmNormCtas = 4, kSmNormThreads = 256, kSmNormItems = 4;       // rows of up to 4 * 4 * 4 * 256 columns
+template <int F>
 __global__ void __cluster_dims__(kSmNormCtas, 1, 1) __launch_bounds__(kSmNormThreads) gemm_smallm_norm_kernel(const SmallMReduceArgs a) {
     __shared__ float red[32], s_part[kSmNormCtas];
     tc::cluster_arrive();            // (the others have started when they are written to)
@@ -259,7 +262,7 @@ __global__ void __cluster_dims__(kSmNormCtas, 1, 1) __launch_bounds__(kSmNormThr
         const int i = first + threadIdx.x + j * kSmNormThreads, c = 4 * i;
         x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i >= last) continue;
-        const float4 v = smallm_sum4(a, m, c);
+        const float4 v = smallm_sum4<F>(a, m, c);
         const uint2 rb = *reinterpret_cast<const uint2*>(a.residual + (size_t)m * a.ld_res + c);
         const float2 r0 = bf16x2_bits_to_f32x2(rb.x), r1 = bf16x2_bits_to_f32x2(rb.y);
         const uint2 o = make_uint2(f32x2_to_bf16x2_bits(bf16_to_f32(f32_to_bf16(v.x)) + r0.x, bf16_to_f32(f32_to_bf16(v.y)) + r0.y),
@@ -411,10 +414,16 @@ PS_API int ps_gemm_smallm_normed(const void* a, int lda, const void* w, int ldw,
     r.partial = g.partial; r.splits = g.splits; r.M = M; r.N = N; r.epilogue = epilogue;
     r.residual = (const __nv_bfloat16*)residual; r.ld_res = ld_res; r.out = out; r.ldo = ldo; r.out_f32 = out_f32;
     r.norm_w = (const __nv_bfloat16*)norm_w; r.eps = eps; r.normed = (__nv_bfloat16*)normed; r.ld_normed = ld_normed;
-    if (norm_w != nullptr) return launch_pdl(gemm_smallm_norm_kernel, dim3(M * kSmNormCtas), dim3(kSmNormThreads), 0, stream, r);
+    // loads in flight: as many as there are splits, up to eight; registers for more cost wide outputs, which have few splits, their occupancy
+    // (34816 x 5120, two splits, 24 / 64 rows: eight 120.3 / 133.5 us, two 116.8 / 129.4)
+    const int f = g.splits <= 2 ? 2 : g.splits <= 4 ? 4 : 8;
+    if (norm_w != nullptr)
+        return launch_pdl(f == 2 ? gemm_smallm_norm_kernel<2> : f == 4 ? gemm_smallm_norm_kernel<4> : gemm_smallm_norm_kernel<8>, dim3(M * kSmNormCtas),
+                          dim3(kSmNormThreads), 0, stream, r);
     if (N % 4 == 0 && (uintptr_t)partial % 16 == 0 && (epilogue != 1 || rows8(residual, ld_res)) &&
         (gated ? (uintptr_t)out % 4 == 0 && ldo % 2 == 0 : out_f32 ? (uintptr_t)out % 16 == 0 && ldo % 4 == 0 : rows8(out, ldo)))
-        return launch_pdl(gemm_smallm_reduce4_kernel, dim3((unsigned)((M * (N >> 2) + 255) / 256)), dim3(256), 0, stream, r);
+        return launch_pdl(f == 2 ? gemm_smallm_reduce4_kernel<2> : f == 4 ? gemm_smallm_reduce4_kernel<4> : gemm_smallm_reduce4_kernel<8>,
+                          dim3((unsigned)((M * (N >> 2) + 255) / 256)), dim3(256), 0, stream, r);
     const long long n = (long long)M * (N >> 1);
     return launch_pdl(gemm_smallm_reduce_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, r);
 }
