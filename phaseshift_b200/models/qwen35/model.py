@@ -24,7 +24,7 @@ FUSED_BA_MAX_ROWS = 8
 
 
 class Qwen35Runner:
-    many_row_kernels = True  # steps in which a sequence has several rows launch other kernels than single rows, hence other graphs
+    many_row_kernels = True  # steps in which sequences have many rows launch other kernels than single rows, hence other graphs
     any_rows = True          # a step computes the rows it has, not its bucket's (runtime/engine.py: _eager_rows)
 
     def __init__(self, weights: EngineWeights, state: ModelState, ops, tp=None):

@@ -527,7 +527,7 @@ class CudaOps(OpTrace):
         # 131072 tokens, 8 layers of the 4B shape: 5255 us per step, and 1763 with a fixed length; 8-bit pages 1604 and 1057).
         split_tokens = self.split_tokens
         if rows > SMALL_M_MAX and not self.exact_rows:
-            if b.graph_static and b.multi_rows:
+            if b.graph_static and b.several_rows:
                 split_tokens = max(split_tokens, 256)
             else:
                 want = max(1, (4 * 148) // (rows * hkv))
@@ -659,7 +659,7 @@ class CudaOps(OpTrace):
             if log is not None:
                 lk, ld, ldd = log
             # several rows of a sequence share their preparation in a kernel of their own; it has the same bits
-            many = any(1 < n <= T for n in seq_rows) if any_long else b.multi_rows
+            many = any(3 < n <= T for n in seq_rows) if any_long else b.multi_rows
             _lib.call("ps_gdn_rows_many" if many else "ps_gdn_rows", ptr(proj), c_int(proj.stride(0)), c_int(hk), c_int(hv), c_int(Dk), c_int(Dv),
                       ptr(gw.conv_w), ptr(gw.A_log), ptr(gw.dt_bias), ptr(gw.norm_w), c_float(cfg.rms_norm_eps),
                       ptr(gs.conv), c_int(st.sc.conv_ring), ptr(gs.rec), ptr(state_out), ptr(b.seq_desc),

@@ -65,7 +65,10 @@ class StepBatch:
         # depend on this step's contents (attention covers max_context, GDN covers max_seqs descriptors)
         self.graph_static = False
         self.identity_out = False
-        self.multi_rows = False          # some sequence has more than one row in the step
+        self.several_rows = False        # some sequence has more than one row in the step
+        # More than three rows a sequence: the delta rule's kernel that prepares rows together is sooner from there on (us with 48 heads, row after
+        # row / together: two rows 6.1 / 7.0, three 7.9 / 8.0, four 9.7 / 8.9, eight 17.1 / 12.0; three sequences of two rows 7.6 / 8.9)
+        self.multi_rows = False
         self.max_context = 1
         o = 0
         self.ids = self.d_int[o:o + max_rows]; o += max_rows
@@ -87,7 +90,7 @@ class StepBatch:
         # (identity_out: output row i is step row i for every i -- a pure decode batch -- so the output gather is the identity)
         self.n_seqs = len(seqs)
         self.seqs = list(seqs)
-        self.multi_rows = self.n_rows > self.n_seqs
+        self.several_rows, self.multi_rows = self.n_rows > self.n_seqs, self.n_rows > 3 * self.n_seqs
 
     @property
     def max_visible_launch(self) -> int:

@@ -391,7 +391,8 @@ class Engine:
         return toks, out
 
     GREEDY_KEY_BIT = 1 << 48
-    MULTI_KEY_BIT = 1 << 49          # some sequence has several rows, and the family has kernels of its own for those or attention splits otherwise
+    MULTI_KEY_BIT = 1 << 49          # sequences have many rows, and the family has kernels of its own for those
+    SEVERAL_KEY_BIT = 1 << 50        # some sequence has several rows: attention splits otherwise
 
     @classmethod
     def graph_key(cls, bucket: int, n_out: int, identity_out: bool, greedy: bool = False) -> int:
@@ -416,8 +417,10 @@ class Engine:
         recurrent updates get graphs of their own (the tap and log tensors are fixed buffers, so the capture stays
         valid; Exact mode only changes which kernels the host picks, which the capture bakes in)."""
         key = self.graph_key(bucket, n_out, b.identity_out, greedy)
-        if b.multi_rows and (bucket > 8 or getattr(self.runner, "many_row_kernels", False)):
+        if b.multi_rows and getattr(self.runner, "many_row_kernels", False):
             key |= self.MULTI_KEY_BIT
+        if b.several_rows and bucket > 8:
+            key |= self.SEVERAL_KEY_BIT
         kw = {}
         if variant is not None:
             taps, log, to_alt, exact = variant

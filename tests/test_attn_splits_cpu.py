@@ -24,7 +24,7 @@ def launch(monkeypatch, kv_fmt, rows, multi, static, max_seq_len, visible, n_seq
     o.max_splits = -(-(max_seq_len + 1) // o.split_tokens)
     t = torch.zeros(1)
     st = types.SimpleNamespace(kv_fmt=kv_fmt, kv_fp8=kv_fmt == 1, block_table=t, max_blocks=1, num_pages=1, status=t, sc=types.SimpleNamespace(page_tokens=16))
-    b = types.SimpleNamespace(graph_static=static, multi_rows=multi, row_pos=t, row_pos_short=t, row_slot=t, seq_desc=t, max_seqs=16,
+    b = types.SimpleNamespace(graph_static=static, several_rows=multi, row_pos=t, row_pos_short=t, row_slot=t, seq_desc=t, max_seqs=16,
                               n_seqs=n_seqs or (1 if multi else rows), seqs=[types.SimpleNamespace(token_ids=[0] * (rows if multi else 1))])
     kv = types.SimpleNamespace(k=t, v=torch.zeros(1), k_scale=t, v_scale=t)
     buf = o.buf
@@ -60,3 +60,11 @@ def test_few_splits_are_kept_outside_of_a_graph(monkeypatch):
     # a few single rows beside a long prompt: rows and with them the splits' length are the prompt's
     assert launch(monkeypatch, 0, 800, False, False, 20000, 2500, n_seqs=16)[0] == "ps_attn_decode_tc_even"
     assert launch(monkeypatch, 0, 16, True, False, 20000, 18000)[0] == "ps_attn_decode_tc_even"        # 32 tiles a split, 8 a share
+
+
+def test_rows_of_a_step_that_share_their_preparation():
+    from phaseshift_b200.runtime.batch import SeqRows, StepBatch
+    b = StepBatch(16, 4, torch.device("cpu"), pinned=False)
+    for rows, several, many in (([1], False, False), ([1, 1, 1], False, False), ([2], True, False), ([3, 3], True, False), ([4], True, True), ([5, 3], True, True)):
+        b.fill([SeqRows(i, 0, [0] * n, ()) for i, n in enumerate(rows)])
+        assert (b.several_rows, b.multi_rows) == (several, many), rows
