@@ -240,7 +240,6 @@ __global__ void gemm_smallm_reduce4_kernel(const SmallMReduceArgs a) {
 // went from 1190 to 931 us, one of 32 rows through 4 layers of 5120 x 17408 from 2010 to 1780.  What bounds it: latency.  The sums are
 // written to the others instead of read from them: no CTA has to stay for a last cluster barrier (8 rows of 2560: 4.4 -> 4.3 us).
 constexpr int kSmNormCtas = 4, kSmNormThreads = 256, kSmNormItems = 4;       // rows of up to 4 * 4 * 4 * 256 columns
-template <int F>
 __global__ void __cluster_dims__(kSmNormCtas, 1, 1) __launch_bounds__(kSmNormThreads) gemm_smallm_norm_kernel(const SmallMReduceArgs a) {
     __shared__ float red[32], s_part[kSmNormCtas];
     tc::cluster_arrive();            // (the others have started when they are written to)
@@ -262,7 +261,7 @@ __global__ void __cluster_dims__(kSmNormCtas, 1, 1) __launch_bounds__(kSmNormThr
         const int i = first + threadIdx.x + j * kSmNormThreads, c = 4 * i;
         x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i >= last) continue;
-        const float4 v = smallm_sum4<F>(a, m, c);
+        const float4 v = smallm_sum4<8>(a, m, c);
         const uint2 rb = *reinterpret_cast<const uint2*>(a.residual + (size_t)m * a.ld_res + c);
         const float2 r0 = bf16x2_bits_to_f32x2(rb.x), r1 = bf16x2_bits_to_f32x2(rb.y);
         const uint2 o = make_uint2(f32x2_to_bf16x2_bits(bf16_to_f32(f32_to_bf16(v.x)) + r0.x, bf16_to_f32(f32_to_bf16(v.y)) + r0.y),
@@ -414,16 +413,14 @@ PS_API int ps_gemm_smallm_normed(const void* a, int lda, const void* w, int ldw,
     r.partial = g.partial; r.splits = g.splits; r.M = M; r.N = N; r.epilogue = epilogue;
     r.residual = (const __nv_bfloat16*)residual; r.ld_res = ld_res; r.out = out; r.ldo = ldo; r.out_f32 = out_f32;
     r.norm_w = (const __nv_bfloat16*)norm_w; r.eps = eps; r.normed = (__nv_bfloat16*)normed; r.ld_normed = ld_normed;
-    // loads in flight: as many as there are splits, up to eight; registers for more cost wide outputs, which have few splits, their occupancy
-    // (34816 x 5120, two splits, 24 / 64 rows: eight 120.3 / 133.5 us, two 116.8 / 129.4)
-    const int f = g.splits <= 2 ? 2 : g.splits <= 4 ? 4 : 8;
-    if (norm_w != nullptr)
-        return launch_pdl(f == 2 ? gemm_smallm_norm_kernel<2> : f == 4 ? gemm_smallm_norm_kernel<4> : gemm_smallm_norm_kernel<8>, dim3(M * kSmNormCtas),
-                          dim3(kSmNormThreads), 0, stream, r);
+    if (norm_w != nullptr) return launch_pdl(gemm_smallm_norm_kernel, dim3(M * kSmNormCtas), dim3(kSmNormThreads), 0, stream, r);
+    // With more than two CTAs for an SM, registers for loads that no split has cost occupancy (two splits, 34816 x 5120, 24 / 64 rows: room for eight
+    // 120.3 / 133.5 us, for two 116.8 / 129.4; three splits, 12352 x 2560, 32 rows: 13.85 and, for four, 13.58; 16 rows: 12.97 and 13.18).
+    const int ctas = (M * (N >> 2) + 255) / 256, f = ctas <= 2 * sm_count() || g.splits > 4 ? 8 : g.splits > 2 ? 4 : 2;
     if (N % 4 == 0 && (uintptr_t)partial % 16 == 0 && (epilogue != 1 || rows8(residual, ld_res)) &&
         (gated ? (uintptr_t)out % 4 == 0 && ldo % 2 == 0 : out_f32 ? (uintptr_t)out % 16 == 0 && ldo % 4 == 0 : rows8(out, ldo)))
         return launch_pdl(f == 2 ? gemm_smallm_reduce4_kernel<2> : f == 4 ? gemm_smallm_reduce4_kernel<4> : gemm_smallm_reduce4_kernel<8>,
-                          dim3((unsigned)((M * (N >> 2) + 255) / 256)), dim3(256), 0, stream, r);
+                          dim3((unsigned)ctas), dim3(256), 0, stream, r);
     const long long n = (long long)M * (N >> 1);
     return launch_pdl(gemm_smallm_reduce_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, r);
 }
