@@ -103,7 +103,8 @@ __device__ __forceinline__ float gdn_silu(float x) { return __fdividef(x, 1.f + 
 
 // grid = (max chunks, Hv), block = 512 threads, two CTAs per SM (shared memory: Q and K tiles, the raw q|k input tile
 // that A, T and the block-row temporaries later overwrite; V is convolved straight from global memory into Q's tile
-// once Q is dead).  2048 rows x 32 heads: 108 us, 111 with 256 threads; bound by issue.
+// once Q is dead).  2048 rows x 32 heads: 105.5 us, 106 with 256 threads; x 48 heads 162 and 159; 100 rows x
+// 32 heads 23 and 31; bound by issue.
 constexpr int kPrepThreads = 512;
 template <int DK, int DV>
 __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prep_kernel(const GdnPrepArgs a) {
@@ -819,8 +820,8 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_tc_kernel(const GdnScanArg
 // Warps 0-7: lane quadrant (warp & 3), half (warp >> 2) of the columns of P and S; warps 8-11: outputs, one quadrant each; warp 12:
 // copies; warp 13: products.
 // With S and Delta as B operands in shared memory, two CTAs per head of 64 columns of Dv each took every accumulator through registers
-// into a swizzled tile and a proxy fence, 6500 cycles per chunk.  2048 rows: 32 heads 108 us with 64 CTAs, 113 with 32 here; 48 heads 150 and
-// 142; with the rows' history stored here and the launches overlapped a layer takes 28 us less.  What bounds it: the chain of a chunk, 5700
+// into a swizzled tile and a proxy fence, 6500 cycles per chunk.  2048 rows, the launch alone: 32 heads 102 us with 64 CTAs, 94 with 32 here; 48 heads
+// 110 and 100, and the rows' history was a launch of 4.5 us; all launches of a layer back to back 226 -> 217 and 298 -> 289 us.  What bounds it: the chain of a chunk, 5700
 // cycles -- S to tensor memory 1500, the product to P 2750, Delta 300, the product to S 1100.  Rounding on the integer pipe and P and R as
 // one product of 128 columns left it as it was; the copies are a chunk ahead.  Four warps that norm and gate the outputs here cannot keep up
 // (12 us a chunk).
@@ -1146,7 +1147,7 @@ static int launch_chunked(const GdnPrepArgs& p, const GdnScanArgs& s, const __nv
 }
 }  // namespace ps
 
-// (All launches, 2048 rows: 343 us before the tcgen05 scan and the shorter preparation, 239 now with 32 heads; 421 and 309 with 48.)
+// (All launches back to back, 2048 rows: 217 us with 32 heads, 289 with 48; 100 rows 30.5 and 31.)
 // Chunked GDN mixer for prefill-sized steps.  `scratch` holds ps_gdn_chunked_scratch_floats() floats,
 // `dc` one float per (chunk, head), `o` [rows, Hv, Dv] floats.
 PS_API int ps_gdn_chunked(const void* proj, int ld_proj, int rows, int Hk, int Hv, int Dk, int Dv, const void* conv_w,
